@@ -533,6 +533,7 @@ int vx_cc_apply(vx_cc* c, const uint32_t* src, const uint32_t* dst, const uint8_
   if (!c || (n && (!src || !dst || !add))) return fail(VX_ERR_INVALID, "null argument");
   if (n == 0) {
     c->c->last_repaired = 0;
+    c->c->repaired_pending = false;
     return VX_OK;
   }
   size_t v_after = 0;
@@ -547,8 +548,7 @@ int vx_cc_labels(vx_cc* c, uint32_t* out, size_t cap, size_t* n) {
 
 int vx_cc_last_repaired_vertices(vx_cc* c, uint64_t* out) {
   if (!c || !out) return fail(VX_ERR_INVALID, "null argument");
-  *out = c->c->last_repaired;
-  return VX_OK;
+  return vxh::cc_last_repaired(c->c, out);
 }
 
 int vx_mrbfs_create(vx_graph* g, const uint32_t* roots, size_t k, vx_mrbfs** out) {

@@ -11,10 +11,12 @@
 //   2. the components of the endpoints of every effective deletion are marked
 //      affected, and their vertices counted (last_repaired_vertices);
 //   3. the batch is committed to the graph;
-//   4. affected vertices restart as singletons and are united along their
-//      arcs to other affected vertices in the post-batch graph;
+//   4. affected vertices are united anew along their arcs to other affected
+//      vertices in the post-batch graph (unite_rows below);
 //   5. the final additions are united;
 //   6. every label is compressed to its root.
+// Nothing of this waits on the host: without an effective deletion the kernels
+// of steps 2 and 4 return at once, and the affected count is read when asked.
 // The partition equals the reference's after every batch.  The labels are the
 // components' smallest ids, where the reference's are whichever union-find
 // roots its union order left (the reference's tests compare labels only for
@@ -66,35 +68,158 @@ __global__ void cc_identity_kernel(uint32_t* label, uint32_t lo, uint32_t hi) {
   for (uint32_t v = lo + blockIdx.x * blockDim.x + threadIdx.x; v < hi; v += gridDim.x * blockDim.x) label[v] = v;
 }
 
-// Unites u with every live neighbour v of u (v > u: each undirected edge once)
-// that passes the filter: all of them (only_affected == 0), or those where
-// both ends are affected.  One warp per row.
-__global__ void cc_rows_kernel(vxb::DevAdj a, uint32_t V, uint32_t* label, const uint32_t* aff, int only_affected) {
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < V; u += nw) {
-    if (only_affected && !((aff[u >> 5] >> (u & 31)) & 1u)) continue;
-    auto visit = [&](bool valid, uint32_t v, uint32_t) {
-      if (!valid || v <= u || v >= V) return;
-      if (only_affected && !((aff[v >> 5] >> (v & 31)) & 1u)) return;
-      cc_union(label, u, v);
-    };
-    frontier::warp_row(a, u, visit);
+// ---- uniting a vertex set along its arcs ------------------------------------
+// All vertices (aff == null), or those of a bitmap, united along every live arc
+// with both ends in the set.  Uniting arc by arc makes every arc of a skewed
+// graph race for one root: R-MAT 2^20 (32M arcs) took 3.41 ms however little
+// the batch cut.  Almost all of those arcs lie inside one giant component that
+// two arcs per vertex already reveal, so (the sampling order of Sutton,
+// Ben-Nun and Barak, "Optimizing parallel graph connectivity computation via
+// subgraph sampling", IPDPS 2018):
+//   hook    label[v] = the smaller of v and its first neighbour (rows are
+//           sorted, so that is the smallest): one plain store each, no cycle;
+//           the trees are then compressed;
+//   link    v is united with its second neighbour (almost always equal by
+//           now: two label loads);
+//   sample  the commonest root of 256 vertices is taken for the giant one;
+//   rows    only vertices of other sets unite along their whole rows.
+// An arc between two sets is seen from an end outside the giant, as both
+// directions are stored, so the partition is the same whichever root is taken
+// (none when no sample hit the set).  Each pass is a coalesced sweep of the
+// vertices with a few dependent loads each, bound by their latency; at R-MAT
+// 2^20 they take 84 us together (hook 13, compress 29, link 24, sample 6, rows 12).
+
+constexpr uint32_t kNoRoot = 0xFFFFFFFFu;
+constexpr uint32_t kProbe = 4;     // arcs of each row part looked at for a live neighbour in the set
+constexpr uint32_t kSamples = 256;
+
+__device__ __forceinline__ bool in_set(const uint32_t* aff, uint32_t v) {
+  return !aff || ((aff[v >> 5] >> (v & 31)) & 1u);
+}
+
+// The smallest neighbour of v above `after` in the set among the first kProbe
+// arcs of its base row and of its delta row; kNoRoot if there is none.
+__device__ __forceinline__ uint32_t probe_row(const vxb::DevAdj& a, uint32_t v, uint32_t V, const uint32_t* aff,
+                                              uint32_t after, bool any_after) {
+  uint64_t b, e;
+  vxb::base_range(a, v, b, e);
+  const uint2 dr = a.drow[v];
+  uint32_t best = kNoRoot;
+  for (uint32_t k = 0; k < kProbe && b + k < e; ++k) {
+    const uint32_t x = a.col[b + k];
+    if ((x & vxb::kTomb) || x >= V || (any_after && x <= after) || !in_set(aff, x)) continue;
+    best = x;
+    break;
+  }
+  for (uint32_t k = 0; k < kProbe && k < dr.y; ++k) {
+    const uint32_t x = a.darena[dr.x + k];
+    if (x >= V || (any_after && x <= after) || !in_set(aff, x)) continue;
+    best = min(best, x);
+    break;
+  }
+  return best;
+}
+
+__global__ void cc_hook_kernel(vxb::DevAdj a, uint32_t V, uint32_t n, uint32_t* label, const uint32_t* aff,
+                               const uint32_t* any) {
+  if (any && !*any) return;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    if (!in_set(aff, v)) continue;
+    const uint32_t x = probe_row(a, v, V, aff, 0u, false);
+    label[v] = min(v, x);
   }
 }
 
-// Every label becomes its root.  The walk only reads: with path halving, a
-// thread that read a vertex's old parent could store it back after the
-// vertex's own thread had stored the root, leaving a label that is not a
-// root.  Here each thread stores only its own label, and a concurrent reader
-// sees either the old parent or the root, both ancestors.
-__global__ void cc_compress_kernel(uint32_t* label, uint32_t V) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    uint32_t x = v, p = __ldcg(&label[v]);
-    while (p != x) {
-      x = p;
-      p = __ldcg(&label[x]);
+__global__ void cc_link_kernel(vxb::DevAdj a, uint32_t V, uint32_t n, uint32_t* label, const uint32_t* aff,
+                               const uint32_t* any) {
+  if (any && !*any) return;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    if (!in_set(aff, v)) continue;
+    const uint32_t x = probe_row(a, v, V, aff, 0u, false);
+    if (x == kNoRoot) continue;
+    const uint32_t y = probe_row(a, v, V, aff, x, true);
+    if (x > v) cc_union(label, v, x);  // a vertex hooked to itself: its first arc is still to be united
+    if (y != kNoRoot && __ldcg(&label[v]) != __ldcg(&label[y])) cc_union(label, v, y);
+  }
+}
+
+// The root of v, read only (no halving: nothing is stored behind a union's back).
+__device__ __forceinline__ uint32_t cc_root(const uint32_t* label, uint32_t v) {
+  uint32_t p = __ldcg(&label[v]);
+  while (p != v) {
+    v = p;
+    p = __ldcg(&label[v]);
+  }
+  return v;
+}
+
+// One block: the commonest root of kSamples vertices spread over [0, n), those
+// outside the set not counted.
+__global__ void __launch_bounds__(kSamples) cc_sample_kernel(const uint32_t* label, uint32_t n, const uint32_t* aff,
+                                                             const uint32_t* any, uint32_t* giant) {
+  __shared__ uint32_t root[kSamples];
+  __shared__ unsigned long long best;
+  if (any && !*any) return;
+  const uint32_t t = threadIdx.x;
+  // one vertex at a hashed place in each of kSamples equal parts
+  const uint64_t lo = (uint64_t)n * t / kSamples, hi = (uint64_t)n * (t + 1) / kSamples;
+  uint32_t r = kNoRoot;
+  if (hi > lo) {
+    const uint32_t v = (uint32_t)(lo + vxb::mix64(t) % (hi - lo));
+    if (in_set(aff, v)) r = cc_root(label, v);
+  }
+  root[t] = r;
+  if (t == 0) best = kNoRoot;  // no count, no root
+  __syncthreads();
+  if (r != kNoRoot) {
+    uint32_t c = 0;
+    for (uint32_t k = 0; k < kSamples; ++k) c += root[k] == r;
+    atomicMax(&best, (unsigned long long)c << 32 | r);
+  }
+  __syncthreads();
+  if (t == 0) *giant = (uint32_t)best;
+}
+
+// The rows of the set's vertices outside the giant: a lane each finds them, the
+// warp walks them.
+__global__ void cc_rows_kernel(vxb::DevAdj a, uint32_t V, uint32_t n, uint32_t* label, const uint32_t* aff,
+                               const uint32_t* any, const uint32_t* giant) {
+  if (any && !*any) return;
+  const uint32_t big = *giant, lane = threadIdx.x & 31;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t v0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; v0 < n; v0 += nw * 32) {
+    const uint32_t v = v0 + lane;
+    const bool mine = v < n && in_set(aff, v) && frontier::degree_of(a, v) != 0u && cc_root(label, v) != big;
+    uint32_t rows = __ballot_sync(0xFFFFFFFFu, mine);
+    while (rows) {
+      const uint32_t u = v0 + (uint32_t)__ffs(rows) - 1;
+      rows &= rows - 1;
+      auto visit = [&](bool valid, uint32_t x, uint32_t) {
+        if (valid && x < V && in_set(aff, x)) cc_union(label, u, x);
+      };
+      frontier::warp_row(a, u, visit);
     }
-    __stcg(&label[v], x);
+  }
+}
+
+// Every label becomes its root.  The walk halves the paths it takes, so the long
+// chains that hooking leaves on a lattice shorten for everybody (2048 x 2048,
+// two batches and the label read: 3.8 ms against 15.4 ms without, and 5.5 ms
+// arc by arc).  It lowers by atomicMin: ancestors are always
+// smaller ids, so a thread that read an old parent cannot store it back over
+// the root another thread stored meanwhile.
+__global__ void cc_compress_kernel(uint32_t* label, uint32_t V, const uint32_t* any) {
+  if (any && !*any) return;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const uint32_t first = __ldcg(&label[v]);
+    uint32_t x = v, p = first;
+    while (p != x) {
+      const uint32_t gp = __ldcg(&label[p]);
+      if (gp != p && x != v) atomicMin(&label[x], gp);
+      x = p;
+      p = gp;
+    }
+    if (x != first) atomicMin(&label[v], x);
   }
 }
 
@@ -117,26 +242,32 @@ __global__ void cc_mark_roots_kernel(const uint32_t* fu, const uint32_t* fv, con
 
 // Affected vertices (their root is marked) as a bitmap, counted.
 __global__ void cc_mark_vertices_kernel(const uint32_t* label, uint32_t n_old, const uint32_t* aroot, uint32_t* aff,
-                                        unsigned long long* count) {
-  unsigned long long c = 0;
-  for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < (n_old + 31) / 32; w += gridDim.x * blockDim.x) {
-    uint32_t bits = 0;
-    for (uint32_t k = 0; k < 32; ++k) {
-      const uint32_t v = w * 32 + k;
-      if (v >= n_old) break;
+                                        const uint32_t* any, unsigned long long* count) {
+  if (!*any) return;
+  // a lane per vertex, so the labels are read whole lines at a time, a ballot
+  // per bitmap word, and one counter update per block (one per warp serialised
+  // on the counter: 28 us at 2^20 vertices)
+  __shared__ uint32_t total;
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  uint32_t c = 0;
+  const uint32_t lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (n_old + 31) / 32; w += nw) {
+    const uint32_t v = w * 32 + lane;
+    bool hit = false;
+    if (v < n_old) {
       const uint32_t r = label[v];
-      if ((aroot[r >> 5] >> (r & 31)) & 1u) bits |= 1u << k;
+      hit = (aroot[r >> 5] >> (r & 31)) & 1u;
     }
-    aff[w] = bits;
-    c += __popc(bits);
+    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, hit);
+    if (lane == 0) {
+      aff[w] = bits;
+      c += __popc(bits);
+    }
   }
-  c = vxb::warp_sum(c);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
-}
-
-__global__ void cc_reset_affected_kernel(uint32_t* label, uint32_t n_old, const uint32_t* aff) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n_old; v += gridDim.x * blockDim.x)
-    if ((aff[v >> 5] >> (v & 31)) & 1u) label[v] = v;
+  if (lane == 0 && c) atomicAdd(&total, c);
+  __syncthreads();
+  if (threadIdx.x == 0 && total) atomicAdd(count, (unsigned long long)total);
 }
 
 // Step 5: the final additions of the batch (their edges exist now).
@@ -175,6 +306,25 @@ int ensure_labels(Components* c, size_t V) {
   return 0;
 }
 
+// Unites the vertices [0, n) of the set (all, or the affected ones, whose
+// kernels run only when *any is set) in the graph of V vertices.  Labels of the
+// set need not hold anything before; afterwards they lead to the sets' roots.
+void unite_rows(Components* c, uint32_t V, uint32_t n, const uint32_t* aff, const uint32_t* any) {
+  cudaStream_t s = c->g->stream;
+  const vxb::DevAdj a = c->g->view().out;
+  uint32_t* giant = c->ctr + 1;
+  count_launch();
+  cc_hook_kernel<<<cc_grid(n), kCcThreads, 0, s>>>(a, V, n, c->label, aff, any);
+  count_launch();
+  cc_compress_kernel<<<cc_grid(n), kCcThreads, 0, s>>>(c->label, n, any);
+  count_launch();
+  cc_link_kernel<<<cc_grid(n), kCcThreads, 0, s>>>(a, V, n, c->label, aff, any);
+  count_launch();
+  cc_sample_kernel<<<1, kSamples, 0, s>>>(c->label, n, aff, any, giant);
+  count_launch();
+  cc_rows_kernel<<<cc_grid(n), kCcThreads, 0, s>>>(a, V, n, c->label, aff, any, giant);
+}
+
 }  // namespace
 
 int cc_rebuild(Components* c) {
@@ -183,16 +333,14 @@ int cc_rebuild(Components* c) {
   if (int rc = ensure_labels(c, std::max<size_t>(V, 1))) return rc;
   cudaStream_t s = g->stream;
   if (V) {
+    unite_rows(c, (uint32_t)V, (uint32_t)V, nullptr, nullptr);
     count_launch();
-    cc_identity_kernel<<<cc_grid(V), kCcThreads, 0, s>>>(c->label, 0, (uint32_t)V);
-    count_launch();
-    cc_rows_kernel<<<cc_grid(32ull * V), kCcThreads, 0, s>>>(g->view().out, (uint32_t)V, c->label, nullptr, 0);
-    count_launch();
-    cc_compress_kernel<<<cc_grid(V), kCcThreads, 0, s>>>(c->label, (uint32_t)V);
+    cc_compress_kernel<<<cc_grid(V), kCcThreads, 0, s>>>(c->label, (uint32_t)V, nullptr);
     VX_CUDA_TRY(cudaGetLastError());
   }
   c->n = V;
   c->last_repaired = V;
+  c->repaired_pending = false;
   return 0;
 }
 
@@ -206,7 +354,7 @@ int cc_create(Components** out, Graph* g) {
   c->g = g;
   if (cudaMalloc(&c->ctr, 16) != cudaSuccess) {
     set_error("components: counter allocation failed");
-    delete c;
+    cc_destroy(c);
     return -4;
   }
   if (int rc = cc_rebuild(c)) {
@@ -231,9 +379,13 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
   Graph* g = c->g;
   cudaStream_t s = g->stream;
   c->last_repaired = 0;
+  c->repaired_pending = false;
   if (n == 0) return 0;  // an empty batch changes nothing (connected_components.hpp:32-35)
   const uint32_t n_old = (uint32_t)c->n;
-  if (int rc = graph_stage_batch(g, n, vertex_bound)) return rc;
+  if (int rc = graph_stage_batch(g, n, vertex_bound)) return rc;  // also grows the graph
+  const size_t V = g->V;
+  // before the marks: a growth replaces their bitmaps
+  if (int rc = ensure_labels(c, std::max<size_t>(V, 1))) return rc;
   BatchBuffers& B = g->batch;
   const uint32_t* F = &g->ctr->final_arcs;
   const uint32_t words_old = (n_old + 31) / 32;
@@ -245,36 +397,36 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
     count_launch();
     cc_mark_roots_kernel<<<cc_grid(m), kCcThreads, 0, s>>>(B.fu, B.fv, B.ff, F, c->label, n_old, c->aroot, any);
     count_launch();
-    cc_mark_vertices_kernel<<<cc_grid(words_old), kCcThreads, 0, s>>>(c->label, n_old, c->aroot, c->aff, count);
+    cc_mark_vertices_kernel<<<std::min(cc_grid(n_old), 148u * 8u), kCcThreads, 0, s>>>(c->label, n_old, c->aroot, c->aff, any, count);
   }
-  uint32_t hc[4] = {0, 0, 0, 0};
-  VX_CUDA_TRY(cudaMemcpyAsync(hc, c->ctr, 16, cudaMemcpyDeviceToHost, s));
-  VX_CUDA_TRY(cudaStreamSynchronize(s));
-  c->last_repaired = (size_t)hc[2] | ((size_t)hc[3] << 32);
-  const bool affected = hc[0] != 0;
+  c->repaired_pending = true;  // the count is read by cc_last_repaired
   if (int rc = graph_commit_batch(g)) return rc;
-  const size_t V = g->V;
-  if (int rc = ensure_labels(c, std::max<size_t>(V, 1))) return rc;
   if (V > n_old) {
     count_launch();
     cc_identity_kernel<<<cc_grid(V - n_old), kCcThreads, 0, s>>>(c->label, n_old, (uint32_t)V);
     VX_CUDA_TRY(cudaMemsetAsync(c->aff + words_old, 0, ((V + 31) / 32 + 1 - words_old) * 4, s));
   }
-  if (affected) {
-    count_launch();
-    cc_reset_affected_kernel<<<cc_grid(n_old), kCcThreads, 0, s>>>(c->label, n_old, c->aff);
-    count_launch();
-    cc_rows_kernel<<<cc_grid(32ull * V), kCcThreads, 0, s>>>(g->view().out, (uint32_t)V, c->label, c->aff, 1);
-  }
+  if (n_old) unite_rows(c, (uint32_t)V, n_old, c->aff, any);
   count_launch();
   cc_union_adds_kernel<<<cc_grid(m), kCcThreads, 0, s>>>(B.fu, B.fv, B.ff, F, c->label);
   count_launch();
-  cc_compress_kernel<<<cc_grid(V), kCcThreads, 0, s>>>(c->label, (uint32_t)V);
+  cc_compress_kernel<<<cc_grid(V), kCcThreads, 0, s>>>(c->label, (uint32_t)V, nullptr);
   // the marks start clear for the next batch
   VX_CUDA_TRY(cudaMemsetAsync(c->aroot, 0, ((c->cap / 32) + 1) * 4, s));
   VX_CUDA_TRY(cudaMemsetAsync(c->aff, 0, ((c->cap / 32) + 1) * 4, s));
   VX_CUDA_TRY(cudaGetLastError());
   c->n = V;
+  return 0;
+}
+
+int cc_last_repaired(Components* c, uint64_t* out) {
+  if (c->repaired_pending) {
+    VX_CUDA_TRY(cudaMemcpyAsync(c->g->pinned_scalar, c->ctr + 2, 8, cudaMemcpyDeviceToHost, c->g->stream));
+    VX_CUDA_TRY(cudaStreamSynchronize(c->g->stream));
+    c->last_repaired = (size_t)c->g->pinned_scalar[0];
+    c->repaired_pending = false;
+  }
+  *out = c->last_repaired;
   return 0;
 }
 
