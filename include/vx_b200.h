@@ -340,7 +340,7 @@ int vx_multiroot_bfs(vx_graph* g, const uint32_t* roots, size_t k, uint32_t* out
  * (the kernel indexes d_dist and the scratch bitmaps by column id and does not
  * check it) and rows must be free of duplicates; a source at or beyond
  * `vertices` gives all-unreachable and *reachable = 0, as in the reference.  All other working
- * memory is one file-scope device array (~8.5 MB per GPU that loads the
+ * memory is one file-scope device array (~6.5 MB per GPU that loads the
  * library, held until exit), so at most 262,144 vertices (larger counts
  * return VX_ERR_RANGE).  Calls share that array: calls that overlap on the
  * GPU race, so issue them one at a time per device.  The first call on a

@@ -42,9 +42,10 @@ using namespace frontier;
 
 constexpr int kThreads = 512;
 enum { kModeFull = 0, kModePre = 1, kModePost = 2 };
-// slots past the vertex count in each candidate list: the per-block segments
-// of ceil(V / blocks) slots cover at most V + blocks - 1 (blocks <= 148 * 4)
-constexpr uint32_t kListSlack = 1024;
+// Slots of each bottom-up candidate list for V vertices: the blocks' segments
+// of whole tiles (BuTiles) hold at most V / 16 + 32 vertices per block more
+// than V (at most 1,024 blocks).
+constexpr size_t list_slots(size_t V) { return V + V / 16 + 32 * 1024; }
 
 struct Params {
   vxb::DevGraph g;
@@ -60,7 +61,7 @@ struct Params {
   uint32_t* lst_t;
   uint32_t* tent;
   uint32_t* bul;      // bottom-up candidate lists A (bul[0, bul_half)) and B (bul[bul_half, 2 * bul_half)),
-  uint32_t bul_half;  // each cut into one segment per block (bul_half >= V + blocks)
+  uint32_t bul_half;  // each cut into one segment per block (bul_half >= list_slots(V))
   unsigned long long* sw;  // support words of the pre-batch cascade (zero between batches)
   unsigned long long* ring;  // work ring of the repair phases (kSent between phases)
   uint32_t ring_mask;
@@ -83,6 +84,7 @@ struct Params {
   float alpha, beta;
   uint32_t large_row;
   uint32_t nblocks;
+  uint32_t deltas;  // the graph may hold delta rows (zero: their table need not be read)
   unsigned long long* trace;  // optional per-level {time, n_f | bottom-up << 63}
   // optional accounting of the update launch's algorithmic bytes (null: off):
   // [0] row arcs scanned by the repair, [1] vertices it visited, [2] delta-row
@@ -96,8 +98,8 @@ constexpr uint32_t kTraceLevels = 256;
 // Time budgets of the repair phases.  On a deep graph one batch can move the
 // distances of millions of vertices, and the cascade or the relaxation then
 // walks them level by level, for far longer than a full BFS takes.  A phase
-// that has run longer than handover x the last full BFS's time drops the rest
-// of its queue and a BFS finishes its work, so a batch costs at most about
+// that has run longer than handover x the last full BFS's time (as it would
+// be inside the launch) drops the rest of its queue and a BFS finishes its work, so a batch costs at most about
 // twice the cheaper of the two; either way the result is the same.  The
 // deadline is set by thread 0 before the barrier that precedes the phase's
 // drain, which reads it once and compares it with the clock every round.  The cascade's BFS compares distances over every vertex of the
@@ -119,84 +121,160 @@ __device__ __forceinline__ void acct_add(const Params& p, int k, unsigned long l
 // Grid barrier; returns false once any block recorded a device error (a
 // barrier that gave up waiting, a loop bound), so every persistent loop ends.
 __device__ __forceinline__ bool sync_grid(const Params& p) {
-  vxb::grid_barrier(p.bar, p.nblocks, &p.c->err);
-  return __ldcg(&p.c->err) == 0u;
+  __shared__ uint32_t failed;
+  vxb::grid_barrier_then(p.bar, p.nblocks, &p.c->err, [&] { failed = __ldcg(&p.c->err); });
+  return failed == 0u;
 }
 
 
-// ------------------------------------------------------------ top-down --
+// The row bounds of u; the delta row is read only where the graph may hold
+// one (a loaded or compacted graph has none, and the load is one more random
+// 32-byte sector per vertex).
+__device__ __forceinline__ void row_of(const Params& p, const DevAdj& a, uint32_t u, uint64_t& b, uint32_t& nb,
+                                       uint2& dr) {
+  uint64_t e;
+  vxb::base_range(a, u, b, e);
+  nb = (uint32_t)(e - b);
+  dr = p.deltas ? a.drow[u] : make_uint2(0u, 0u);
+}
 
+__device__ __forceinline__ uint32_t row_len(const Params& p, const DevAdj& a, uint32_t u) {
+  uint64_t b;
+  uint32_t nb;
+  uint2 dr;
+  row_of(p, a, u, b, nb, dr);
+  return nb + dr.y;
+}
+
+// ------------------------------------------------------------ top-down --
+//
+// A level is a chain of dependent round trips per arc (column, visited word,
+// claim), so its time is the number of steps a warp takes times that chain.
+// Every path below hands TdVisit::visit four arcs per lane at once, whose
+// loads and atomics are all in flight together.  A 4096 x 4096 lattice (160
+// levels of up to 644,000 vertices with 4 arcs each): 4.15 -> 2.33 ms, with the
+// one-block levels and the direction rule below; its widest levels (57 us) move
+// some 200 MB of scattered sectors through L2.
+
+constexpr int kVisit = 4;  // arcs a lane has in flight per step
+
+template <class Queue>
 struct TdVisit {
   const Params* p;
   uint32_t* dist;
   uint32_t level;
   uint32_t* qout;
-  uint32_t* fbn;
+  uint32_t* fbn;  // bitmap of the next frontier, or null when no bottom-up level reads it as it is made
   uint32_t* cnt_n;
-  bool want_deg;
-  unsigned long long mloc;
-  BlockQueue* bq;
-  // Claim x for the next level (warp-uniform).
-  __device__ __forceinline__ void operator()(bool valid, uint32_t x, uint32_t) {
-    bool claim = false;
-    const uint32_t bit = 1u << (x & 31);
-    if (valid) {
-      const uint32_t w = p->vis[x >> 5];
-      if (!(w & bit)) {
-        // the row length is loaded before the claim, so both are in flight together
-        const uint64_t deg = want_deg ? degree_of(p->g.out, x) : 0ull;
-        claim = !(atomicOr(&p->vis[x >> 5], bit) & bit);
-        if (claim) mloc += deg;
+  Queue* bq;
+  unsigned long long mloc;  // arcs of the vertices this lane claimed
+  // Claims the heads of one step's arcs for the next level (warp-uniform);
+  // bit 31 of an entry marks a dead arc or none.
+  __device__ __forceinline__ void visit(const uint32_t (&x)[kVisit]) {
+    uint32_t w[kVisit];
+#pragma unroll
+    for (int j = 0; j < kVisit; ++j) w[j] = (x[j] & kTomb) ? FULL : p->vis[x[j] >> 5];
+    // the row lengths are loaded before the claims, so both are in flight together
+    uint32_t deg[kVisit];
+#pragma unroll
+    for (int j = 0; j < kVisit; ++j) deg[j] = (w[j] >> (x[j] & 31)) & 1u ? 0u : row_len(*p, p->g.out, x[j]);
+#pragma unroll
+    for (int j = 0; j < kVisit; ++j) {
+      const uint32_t bit = 1u << (x[j] & 31);
+      if (!(w[j] & bit)) w[j] = atomicOr(&p->vis[x[j] >> 5], bit);
+    }
+    uint32_t m[kVisit];
+#pragma unroll
+    for (int j = 0; j < kVisit; ++j) {
+      const uint32_t bit = 1u << (x[j] & 31);
+      const bool claim = !(w[j] & bit);
+      m[j] = __ballot_sync(FULL, claim);
+      if (claim) {
+        mloc += deg[j];
+        dist[x[j]] = level + 1;
+        if (fbn) atomicOr(&fbn[x[j] >> 5], bit);
       }
     }
-    if (claim) {
-      dist[x] = level + 1;
-      atomicOr(&fbn[x >> 5], bit);
-    }
-    bq_push(*bq, claim, x, cnt_n, qout);
-  }
-  __device__ __forceinline__ void flush(unsigned long long* dst) {
-    if (!want_deg) return;
-    const unsigned long long sum = vxb::warp_sum(mloc);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(dst, sum);
-    mloc = 0;
+    bq_push_n(*bq, m, x, cnt_n, qout);
   }
 };
 
-__device__ void td_level(const Params& p, TdVisit& t, const uint32_t* qin, uint32_t n_f, uint32_t* cnt_big) {
-  const DevAdj& a = p.g.out;
+// Rows arr[start, start + len) of the lanes (len 0: none): rows of >= 32 arcs
+// walked by the whole warp, shorter ones as one flattened list (a warp scan of
+// the lengths, then each arc's owner by a 5-step shuffle search), 128 arcs
+// per step either way.
+template <class Visit>
+__device__ __forceinline__ void td_rows(Visit& t, const uint32_t* arr, uint64_t start, uint32_t len) {
   const int lane = threadIdx.x & 31;
-  if (n_f <= nwarps()) {
-    // small frontier: one warp per vertex, so no warp walks several rows
-    for (uint32_t i = gwarp(); i < n_f; i += nwarps()) {
-      const uint32_t u = qin[i];
-      const bool big = degree_of(a, u) >= p.large_row;
-      if (big) {
-        if (lane == 0) p.big[atomicAdd(cnt_big, 1u)] = u;
-        continue;
+  uint32_t med = __ballot_sync(FULL, len >= 32);
+  while (med) {
+    const int l = __ffs(med) - 1;
+    med &= med - 1;
+    const uint64_t s = __shfl_sync(FULL, start, l);
+    const uint32_t n = __shfl_sync(FULL, len, l);
+    for (uint32_t k0 = 0; k0 < n; k0 += 32 * kVisit) {
+      uint32_t x[kVisit];
+#pragma unroll
+      for (int j = 0; j < kVisit; ++j) {
+        const uint32_t k = k0 + 32 * j + lane;
+        x[j] = k < n ? arr[s + k] : kTomb;
       }
-      warp_row(a, u, t);
+      t.visit(x);
     }
-    return;
   }
-  for (uint32_t base = gwarp() * 32; base < n_f; base += nwarps() * 32) {
-    const uint32_t i = base + lane;
-    const bool act = i < n_f;
-    const uint32_t u = act ? qin[i] : 0u;
-    uint64_t b = 0, e = 0;
-    uint2 dr = make_uint2(0, 0);
-    if (act) {
-      vxb::base_range(a, u, b, e);
-      dr = a.drow[u];
+  if (len >= 32) len = 0;
+  uint32_t incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const uint32_t excl = incl - len;
+  const uint32_t total = __shfl_sync(FULL, incl, 31);
+  start -= excl;  // arc k of the list is arr[start + k] in its owner's lane
+  for (uint32_t k0 = 0; k0 < total; k0 += 32 * kVisit) {
+    uint32_t x[kVisit];
+#pragma unroll
+    for (int j = 0; j < kVisit; ++j) {
+      const uint32_t k = k0 + 32 * j + lane;
+      int owner = 0;
+#pragma unroll
+      for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t ex = __shfl_sync(FULL, excl, owner + step);
+        if (ex <= k) owner += step;
+      }
+      const uint64_t s = __shfl_sync(FULL, start, owner);
+      x[j] = k < total ? arr[s + k] : kTomb;
     }
-    const bool big = act && (e - b) + dr.y >= p.large_row;
+    t.visit(x);
+  }
+}
+
+// A frontier of more than kLbMax vertices: up to 32 of them per warp, fewer
+// when that leaves warps without any.  Rows of at least large_row arcs are
+// listed (p.big, their lengths in p.bul, free outside the bottom-up levels)
+// for grid_rows.
+template <class Visit>
+__device__ void td_level(const Params& p, Visit& t, const uint32_t* qin, uint32_t n_f, uint32_t* cnt_big) {
+  const DevAdj& a = p.g.out;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t per = min(32u, (n_f + nwarps() - 1) / nwarps());
+  for (uint32_t base = gwarp() * per; base < n_f; base += nwarps() * per) {
+    const bool act = lane < per && base + lane < n_f;
+    const uint32_t u = act ? qin[base + lane] : 0u;
+    uint64_t b = 0;
+    uint32_t nb = 0;
+    uint2 dr = make_uint2(0u, 0u);
+    if (act) row_of(p, a, u, b, nb, dr);
+    const bool big = act && nb + dr.y >= p.large_row;
     const uint32_t slot = vxb::warp_append(big, cnt_big);
     if (big) {
       p.big[slot] = u;
-      b = e = 0;
-      dr = make_uint2(0, 0);
+      p.bul[slot] = nb + dr.y;
+      nb = dr.y = 0;
     }
-    expand_lanes(a, u, b, e, dr, t);
+    td_rows(t, a.col, b, nb);
+    if (p.deltas) td_rows(t, a.darena, dr.x, dr.y);
   }
 }
 
@@ -213,24 +291,25 @@ struct LbStage {
   uint32_t dx[kLbMax];
 };
 
-__device__ void td_level_lb(const Params& p, TdVisit& t, const uint32_t* qin, uint32_t n_f, LbStage& st) {
+template <int kT>
+__device__ void lb_stage(const Params& p, const uint32_t* qin, uint32_t n_f, LbStage& st) {
   const DevAdj& a = p.g.out;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // stage: two frontier entries per thread (blockDim 512 covers kLbMax)
-  uint32_t len[2], sum = 0;
+  constexpr int kPer = kLbMax / kT;  // frontier entries per thread
+  uint32_t len[kPer], sum = 0;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint32_t i = threadIdx.x * 2 + h;
+  for (int h = 0; h < kPer; ++h) {
+    const uint32_t i = threadIdx.x * kPer + h;
     len[h] = 0;
     if (i < n_f) {
-      const uint32_t u = qin[i];
-      uint64_t b, e;
-      vxb::base_range(a, u, b, e);
-      const uint2 dr = a.drow[u];
+      uint64_t b;
+      uint32_t nb;
+      uint2 dr;
+      row_of(p, a, qin[i], b, nb, dr);
       st.base[i] = b;
-      st.blen[i] = (uint32_t)(e - b);
+      st.blen[i] = nb;
       st.dx[i] = dr.x;
-      len[h] = (uint32_t)(e - b) + dr.y;
+      len[h] = nb + dr.y;
     }
     sum += len[h];
   }
@@ -240,81 +319,193 @@ __device__ void td_level_lb(const Params& p, TdVisit& t, const uint32_t* qin, ui
     const uint32_t y = __shfl_up_sync(FULL, incl, o);
     if (lane >= o) incl += y;
   }
-  __shared__ uint32_t wsum[kThreads / 32];
+  __shared__ uint32_t wsum[kT / 32];
   if (lane == 31) wsum[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    const uint32_t w = lane < kThreads / 32 ? wsum[lane] : 0u;
+    const uint32_t w = lane < kT / 32 ? wsum[lane] : 0u;
     uint32_t wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(FULL, wi, o);
       if (lane >= o) wi += y;
     }
-    if (lane < kThreads / 32) wsum[lane] = wi - w;
+    if (lane < kT / 32) wsum[lane] = wi - w;
   }
   __syncthreads();
   uint32_t ex = wsum[warp] + incl - sum;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint32_t i = threadIdx.x * 2 + h;
+  for (int h = 0; h < kPer; ++h) {
+    const uint32_t i = threadIdx.x * kPer + h;
     if (i < n_f) st.pref[i] = ex;
     ex += len[h];
+    if (i + 1 == n_f) st.pref[n_f] = ex;
   }
-  if (threadIdx.x * 2 + 1 == n_f - 1 || (threadIdx.x * 2 == n_f - 1)) st.pref[n_f] = ex;
   __syncthreads();
-  const uint32_t M = st.pref[n_f];
-  for (uint32_t e0 = gwarp() * 32; e0 < M; e0 += nwarps() * 32) {
-    const uint32_t e = e0 + lane;
-    bool valid = false;
-    uint32_t x = 0;
-    if (e < M) {
-      uint32_t lo = 0, hi = n_f;  // last i with pref[i] <= e
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (st.pref[mid] <= e) lo = mid;
-        else hi = mid;
-      }
-      const uint32_t j = e - st.pref[lo];
-      if (j < st.blen[lo]) {
-        x = a.col[st.base[lo] + j];
-        valid = !(x & kTomb);
-        x &= kIdMask;
-      } else {
-        x = a.darena[st.dx[lo] + (j - st.blen[lo])];
-        valid = true;
-      }
-    }
-    t(valid, x, 0u);
-  }
-  __syncthreads();  // st is reused by the next level
 }
 
-// Rows of at least large_row arcs: every warp of the grid takes a slice.
-template <class F>
-__device__ void grid_rows(const DevAdj& a, const uint32_t* rows, uint32_t n, F& f) {
-  const int lane = threadIdx.x & 31;
-  for (uint32_t r = 0; r < n; ++r) {
-    const uint32_t u = rows[r];
-    uint64_t b, e;
-    vxb::base_range(a, u, b, e);
-    for (uint64_t j0 = b + (uint64_t)gwarp() * 32; j0 < e; j0 += (uint64_t)nwarps() * 32) {
-      const uint64_t j = j0 + lane;
-      const uint32_t x = j < e ? a.col[j] : kTomb;
-      f(!(x & kTomb), x & kIdMask, u);
+// The staged rows' arcs, 32 per warp and round over `warps` warps, four rounds
+// at a time (a frontier of fewer arcs still spreads over every warp).
+template <class Visit>
+__device__ void lb_visit(const Params& p, Visit& t, uint32_t n_f, const LbStage& st, uint32_t warp, uint32_t warps) {
+  const DevAdj& a = p.g.out;
+  const uint32_t M = st.pref[n_f];
+  for (uint32_t e0 = warp * 32; e0 < M; e0 += warps * 32 * kVisit) {
+    uint32_t x[kVisit];
+#pragma unroll
+    for (int j = 0; j < kVisit; ++j) {
+      const uint32_t e = e0 + j * warps * 32 + (threadIdx.x & 31);
+      x[j] = kTomb;
+      if (e < M) {
+        uint32_t lo = 0, hi = n_f;  // last i with pref[i] <= e
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (st.pref[mid] <= e) lo = mid;
+          else hi = mid;
+        }
+        const uint32_t k = e - st.pref[lo];
+        x[j] = k < st.blen[lo] ? a.col[st.base[lo] + k] : a.darena[st.dx[lo] + (k - st.blen[lo])];
+      }
     }
-    const uint2 dr = a.drow[u];
-    for (uint32_t j0 = dr.x + gwarp() * 32; j0 < dr.x + dr.y; j0 += nwarps() * 32) {
-      const uint32_t j = j0 + lane;
-      const bool ok = j < dr.x + dr.y;
-      f(ok, ok ? a.darena[j] : 0u, u);
-    }
+    t.visit(x);
   }
+}
+
+// The listed rows of at least large_row arcs, in slices of 128 arcs dealt to
+// the warps of the grid.
+template <class Visit>
+__device__ void grid_rows(const Params& p, Visit& t, uint32_t n) {
+  const DevAdj& a = p.g.out;
+  const uint32_t lane = threadIdx.x & 31;
+  constexpr uint32_t kSlice = 32 * kVisit;
+  for_my_rows(p.bul, n, kSlice, [&](uint32_t r, uint32_t len, uint32_t s0) {
+    uint64_t b;
+    uint32_t nb;
+    uint2 dr;
+    row_of(p, a, p.big[r], b, nb, dr);
+    for (uint64_t k0 = (uint64_t)s0 * kSlice; k0 < len; k0 += (uint64_t)nwarps() * kSlice) {
+      uint32_t x[kVisit];
+#pragma unroll
+      for (int j = 0; j < kVisit; ++j) {
+        const uint64_t k = k0 + 32 * j + lane;
+        x[j] = k >= len ? kTomb : (k < nb ? a.col[b + k] : a.darena[dr.x + (uint32_t)(k - nb)]);
+      }
+      t.visit(x);
+    }
+  });
+}
+
+// What a block adds up over a level and reads back after it (shared memory).
+struct LevelWords {
+  unsigned long long m;   // arcs of the vertices the block claimed
+  uint32_t n;             // vertices it claimed without queueing them
+  uint32_t failed, n_f, nbig;
+  unsigned long long m_f;
+};
+
+// The end of a level's pass: the block's sums and queued vertices go out (one
+// update of each counter per block), the grid meets, and the block reads the
+// level's figures.  Block-uniform; false once any block recorded an error.
+template <class Queue>
+__device__ __forceinline__ bool level_end(const Params& p, LevelWords& lw, Queue& bq, uint32_t nloc,
+                                          unsigned long long mloc, uint32_t slot, uint32_t* nbig) {
+  BfsCounters* c = p.c;
+  constexpr uint32_t kCap = sizeof(bq.items) / sizeof(bq.items[0]);
+  mloc = vxb::warp_sum(mloc);
+  nloc = vxb::warp_sum(nloc);
+  if ((threadIdx.x & 31) == 0) {
+    if (mloc) atomicAdd(&lw.m, mloc);
+    if (nloc) atomicAdd(&lw.n, nloc);
+  }
+  __syncthreads();
+  const uint32_t q = min(bq.cnt, kCap);
+  if (threadIdx.x == 0) {
+    const uint32_t n = lw.n;
+    if (lw.m) atomicAdd(&c->lvl_m[slot], lw.m);
+    if (q + n) bq.gbase = atomicAdd(&c->lvl_n[slot], q + n);  // queued or counted, not both
+    lw.m = 0;
+    lw.n = 0;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < q; i += blockDim.x) p.q[slot][bq.gbase + i] = bq.items[i];
+  if (threadIdx.x == 0) bq.cnt = 0;  // read by every thread before the block barrier above
+  vxb::grid_barrier_then(p.bar, p.nblocks, &c->err, [&] {
+    lw.failed = __ldcg(&c->err);
+    lw.n_f = ld_cg(&c->lvl_n[slot]);
+    lw.m_f = __ldcg(&c->lvl_m[slot]);
+    lw.nbig = nbig ? ld_cg(nbig) : 0u;
+  });
+  return lw.failed == 0u;
+}
+
+// The block's sum of v (every thread gets it; red is per-block scratch).
+template <int kT>
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v, unsigned long long* red) {
+  v = vxb::warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  unsigned long long s = 0;
+#pragma unroll
+  for (int k = 0; k < kT / 32; ++k) s += red[k];
+  return s;
+}
+
+// ---- levels of one block ----
+// A frontier of a few hundred vertices keeps one block busy for about as long
+// as the grid takes to meet at a barrier: block 0 runs such levels by itself,
+// frontier in shared memory and block barriers only, until the frontier
+// outgrows it, while the others wait at the grid barrier that ends the
+// stretch.  A level takes 3 us instead of 8 to 10.  The limits are where a
+// level of one block (four arcs per thread and step) costs what a level of
+// the grid does.  A stretch is bounded so that the waiting blocks' barrier is.
+constexpr uint32_t kSoloArcs = 4096;
+constexpr uint32_t kSoloLevels = 4096;
+
+// Words of the barrier array past the barrier word (zero between searches):
+// what a stretch hands back (two sets of 8), and the length of a queue made
+// from a bitmap.
+constexpr uint32_t kSoloWord = 8, kQueueWord = 28;
+static_assert(kQueueWord < vxb::kBarrierWords, "the barrier array holds these words");
+
+struct SoloState {
+  uint32_t level, n_f, reached;
+  unsigned long long m_f, m_visited;
+};
+
+__device__ __forceinline__ bool solo_fits(uint32_t n_f, unsigned long long m_f) {
+  return n_f <= kLbMax && m_f <= kSoloArcs;
+}
+
+// Block 0, block-uniform: levels from s.level on, the frontier in qin; the
+// frontier after the last one is left in qout (its size added to *cnt_n).
+template <int kT, class Queue>
+__device__ void solo_levels(const Params& p, uint32_t* dist, const uint32_t* qin, uint32_t* qout, uint32_t* cnt_n,
+                            Queue& bq, LbStage& st, unsigned long long* red, unsigned long long* trace,
+                            SoloState& s) {
+  const uint32_t* in = qin;
+  for (uint32_t k = 0; s.n_f && solo_fits(s.n_f, s.m_f) && k < kSoloLevels; ++k, ++s.level) {
+    s.reached += s.n_f;
+    s.m_visited += s.m_f;
+    if (trace && threadIdx.x == 0 && s.level < kTraceLevels) {
+      trace[2 * s.level] = globaltimer();
+      trace[2 * s.level + 1] = s.n_f;
+    }
+    lb_stage<kT>(p, in, s.n_f, st);  // ends with a block barrier: the entries are read
+    in = bq.items;
+    if (threadIdx.x == 0) bq.cnt = 0;
+    __syncthreads();
+    // an overflow of bq's slots goes to qout: more than kLbMax entries, so it is the last level here
+    TdVisit<Queue> t{&p, dist, s.level, qout, nullptr, cnt_n, &bq, 0ull};
+    lb_visit(p, t, s.n_f, st, threadIdx.x >> 5, kT / 32);
+    s.m_f = block_sum<kT>(t.mloc, red);  // its barriers also cover the pushes
+    s.n_f = bq.cnt;
+    __threadfence_block();
+  }
+  bq_flush(bq, cnt_n, qout);
 }
 
 // ----------------------------------------------------------- bottom-up --
-
-constexpr uint32_t kBuHead = 8;  // arcs a lane scans itself before the warp helps
 
 // Appends v where pred holds to a block-private list segment (seg, counter
 // n in shared memory), in lane order within the warp.  Warp-uniform.
@@ -328,157 +519,296 @@ __device__ __forceinline__ void seg_append(bool pred, uint32_t v, uint32_t* seg,
   if (pred) seg[base + __popc(m & vxb::lanemask_lt())] = v;
 }
 
-// Bottom-up over this block's segment of a candidate list: lin[0, nin) holds
-// vertices that may still be reached (unvisited when the list was made,
-// in-degree > 0; the first list is every such vertex of the block's range,
-// built by the full BFS's initialisation, later ones the previous level's
-// misses).  One warp per 32 entries: each lane scans the first kBuHead
-// in-arcs of its row, the rest of longer rows is scanned by the whole warp 32
-// arcs at a time, every scan stops at the first parent in the frontier
-// bitmap.  Entries visited since the list was made are skipped; entries that
-// find no parent go to the block's segment of the other list (lout, counter
-// nout in shared memory), so isolated vertices cost nothing and a later level
-// scans only the vertices still unreached.  Entries are loaded two groups
-// ahead and their visited words and row bounds one group ahead, so those
-// loads are in flight while a group is scanned.  Block-uniform.
-__device__ void bu_list_level(const Params& p, uint32_t* dist, uint32_t level, const uint32_t* fbc, uint32_t* fbn,
-                              uint32_t* qout, uint32_t* cnt_n, BlockQueue& bq, const uint32_t* lin, uint32_t nin,
-                              uint32_t* lout, uint32_t* nout) {
-  const DevAdj& a = p.g.in;
-  const int lane = threadIdx.x & 31;
-  const uint32_t step = kThreads;  // the block's warps take consecutive 32-entry groups
-  uint32_t base = (threadIdx.x >> 5) * 32;
-  uint32_t v1 = base + step + lane < nin ? lin[base + step + lane] : kUnreachable;
-  uint32_t v0 = base + lane < nin ? lin[base + lane] : kUnreachable;
-  uint32_t vis0 = 0;
-  uint64_t b0 = 0, e0 = 0;
-  uint2 dr0 = make_uint2(0, 0);
-  if (v0 != kUnreachable) {
-    vis0 = p.vis[v0 >> 5];
-    vxb::base_range(a, v0, b0, e0);
-    dr0 = a.drow[v0];
+// A bottom-up level scans the in-rows of the unvisited vertices for a parent
+// in the frontier bitmap.  Each scan is a chain of round trips (columns, bitmap
+// words), a warp has some 500 vertices, and most of them find their parent
+// among the first arcs (rows are sorted, and in skewed graphs the hubs that
+// fill the frontier sit at small ids): the level's time is the number of steps
+// a warp takes times one step's chain.  So a warp gathers its vertices in a
+// ring in shared memory until every lane of a step has kR of them (R-MAT graphs
+// have two isolated vertices in five), reads the first 8 arcs of each (kR x 4
+// loads in flight), and scans the longer rows still looking four at a time,
+// eight lanes each (one after another by the whole warp, each paid its own
+// chain).  R-MAT 22, the level that reaches 1.8M of 2.4M vertices: 103 us with
+// one vertex per lane and step, 87 us with two (of about 40 us for its 250 MB
+// of mostly single 32-byte sectors); one is enough, and 10% faster in all, on
+// graphs of a few thousand arcs per block, which kT = 512 serves.  Putting the
+// long rows back into the ring instead (24 or 56 arcs left): no gain on large
+// graphs, 41 -> 44 us in all at 30,000 vertices.
+constexpr uint32_t kBuStep = 8;  // arcs of a vertex a lane scans by itself
+
+constexpr uint64_t kBuDelta = 1ull << 63;
+struct BuEntry {
+  uint64_t at;    // next arc: base position, or arena position with kBuDelta set
+  uint32_t v;
+  uint32_t left;  // arcs left of that part of the row
+};
+
+// The vertices waiting for a step, per warp: fewer than 32 * kR before a
+// refill of 32 or a step's returns (for their delta rows).
+template <int kT, int kR>
+struct BuStage {
+  BuEntry e[kT / 32][32 * kR * 2];
+};
+
+// The vertices of a block in bottom-up levels: tiles of 2^shift bitmap words
+// dealt to the blocks in turn, at least 16 a block where the graph has them
+// (so that no block has all the small ids, an R-MAT graph's hubs; one range per
+// block measured the same within 2% at R-MAT 20 to 22).
+struct BuTiles {
+  uint32_t shift, per_block;  // words per tile (log2), tiles of each block
+  __device__ BuTiles(uint32_t words, uint32_t blocks) {
+    shift = 0;
+    while (shift < 6 && (words >> (shift + 1)) >= blocks * 16u) ++shift;
+    const uint32_t tiles = (words + (1u << shift) - 1) >> shift;
+    per_block = (tiles + blocks - 1) / blocks;
   }
-  for (; base < nin; base += step) {
-    const uint32_t v = v0, visw = vis0;
-    uint64_t b = b0, e = e0;
-    uint2 dr = dr0;
-    // advance the pipeline: row bounds of the next group, entries of the one after
-    v0 = v1;
-    vis0 = 0;
-    b0 = e0 = 0;
-    dr0 = make_uint2(0, 0);
+  // the block's words are 0 .. words() - 1 in its own count
+  __device__ uint32_t words() const { return per_block << shift; }
+  __device__ uint32_t word_of(uint32_t local) const {
+    return (((local >> shift) * gridDim.x + blockIdx.x) << shift) + (local & ((1u << shift) - 1u));
+  }
+  __device__ uint32_t local_of(uint32_t word) const {
+    return (((word >> shift) / gridDim.x) << shift) + (word & ((1u << shift) - 1u));
+  }
+};
+
+// Where a level's finds and misses go.  Vertices found may be counted and set
+// in the bitmaps only (bq null): the queue is then made from the bitmap if a
+// top-down level follows (queueing 1.8M vertices past the blocks' buffers took
+// tens of thousands of updates of one counter).  A block's bitmap words are its
+// own, so their bits are gathered in shared memory where it holds them.
+template <class Queue>
+struct BuOut {
+  uint32_t* dist;
+  uint32_t level;
+  const uint32_t* fbc;
+  uint32_t* fbn;
+  uint32_t* bits;   // the block's words in shared memory, or null
+  BuTiles tiles;
+  uint32_t* lout;   // this block's segment of the next list, and its length (shared memory)
+  uint32_t* nout;
+  Queue* bq;        // the next frontier's queue, or null
+  uint32_t* qout;
+  uint32_t* cnt_n;
+  uint32_t nloc;    // vertices this lane found and did not queue
+};
+
+// Every scan stops at the first parent.  refill(ring, cnt) appends up to 32
+// vertices, false when there are no more.  Whole warp.
+template <int kR, class Queue, class Refill>
+__device__ __forceinline__ void bu_scan(const Params& p, BuOut<Queue>& o, BuEntry* ring, Refill&& refill) {
+  const DevAdj& a = p.g.in;
+  const uint32_t lane = threadIdx.x & 31, lt = vxb::lanemask_lt();
+  uint32_t cnt = 0;
+  bool more = true;
+  for (;;) {
+    while (more && cnt < 32 * kR) more = refill(ring, cnt);
+    if (!cnt) break;
+    __syncwarp();
+    const uint32_t n = min(cnt, 32u * kR);
+    cnt -= n;
+    BuEntry e[kR];
+    bool found[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const uint32_t k = 32 * r + lane;
+      e[r] = k < n ? ring[cnt + k] : BuEntry{0ull, kUnreachable, 0u};
+      found[r] = false;
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k0 = 0; k0 < kBuStep; k0 += 4) {
+      uint32_t x[kR][4];
+#pragma unroll
+      for (int r = 0; r < kR; ++r) {
+        const uint32_t* arr = (e[r].at & kBuDelta ? a.darena : a.col) + (e[r].at & ~kBuDelta) + k0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) x[r][j] = !found[r] && k0 + j < e[r].left ? arr[j] : kTomb;
+      }
+#pragma unroll
+      for (int r = 0; r < kR; ++r)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) found[r] = found[r] || (!(x[r][j] & kTomb) && test_bit(o.fbc, x[r][j]));
+    }
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      // long rows: four at a time, eight lanes each, 32 arcs per step
+      uint32_t coop = __ballot_sync(FULL, !found[r] && e[r].left > kBuStep);
+      while (coop) {
+        const uint32_t sub = lane >> 3, g = lane & 7;
+        int l = -1;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          if (k == sub) l = __ffs(coop) - 1;
+          coop &= coop - 1;
+        }
+        const uint64_t at = __shfl_sync(FULL, e[r].at, l < 0 ? 0 : l) + kBuStep;
+        const uint32_t tot = __shfl_sync(FULL, e[r].left, l < 0 ? 0 : l) - kBuStep;
+        const uint32_t* arr = (at & kBuDelta ? a.darena : a.col) + (at & ~kBuDelta);
+        bool on = l >= 0, hit_l = false;
+        for (uint32_t k0 = 0; __any_sync(FULL, on); k0 += 32) {
+          uint32_t x[4];
+          bool hit = false;
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j) x[j] = on && k0 + 8 * j + g < tot ? arr[k0 + 8 * j + g] : kTomb;
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j) hit = hit || (!(x[j] & kTomb) && test_bit(o.fbc, x[j]));
+          if ((__ballot_sync(FULL, hit) >> (8 * sub)) & 0xFFu) {
+            hit_l = true;
+            on = false;
+          }
+          on = on && k0 + 32 < tot;
+        }
+        const uint32_t got = __reduce_or_sync(FULL, hit_l && g == 0 ? 1u << l : 0u);
+        found[r] = found[r] || ((got >> lane) & 1u);
+      }
+      const uint32_t v = e[r].v;
+      const bool real = v != kUnreachable;
+      bool look = false;
+      if (p.deltas && real && !found[r] && !(e[r].at & kBuDelta)) {  // back for the delta row
+        const uint2 dr = a.drow[v];
+        e[r].at = dr.x | kBuDelta;
+        e[r].left = dr.y;
+        look = dr.y != 0u;
+      }
+      if (found[r]) {
+        o.dist[v] = o.level + 1;
+        const uint32_t bit = 1u << (v & 31);
+        if (o.bits) {
+          atomicOr(&o.bits[o.tiles.local_of(v >> 5)], bit);
+        } else {
+          atomicOr(&p.vis[v >> 5], bit);
+          atomicOr(&o.fbn[v >> 5], bit);
+        }
+        o.nloc += o.bq == nullptr;
+      }
+      if (o.bq) bq_push(*o.bq, found[r], v, o.cnt_n, o.qout);
+      seg_append(real && !found[r] && !look, v, o.lout, o.nout);
+      const uint32_t back = __ballot_sync(FULL, look);
+      if (look) ring[cnt + __popc(back & lt)] = e[r];
+      cnt += __popc(back);
+    }
+  }
+}
+
+// The first arcs of v's in-row for the ring.
+__device__ __forceinline__ BuEntry bu_entry(uint32_t v, uint64_t b, uint32_t nb, uint2 dr) {
+  return nb ? BuEntry{b, v, nb} : BuEntry{dr.x | kBuDelta, v, dr.y};
+}
+
+// The first bottom-up level: every unvisited vertex of the block's tiles with a
+// nonempty in-row; a warp reads the visited words and row bounds of 32 vertices
+// at a time, one refill ahead.  (Listing the candidates in the initialisation
+// pass instead cost a chain of loads per 512 vertices of a block there, also in
+// searches that never go bottom-up.)
+template <int kT, int kR, class Queue>
+__device__ void bu_first_level(const Params& p, BuOut<Queue>& o, BuStage<kT, kR>& st) {
+  const DevAdj& a = p.g.in;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t nw = o.tiles.words();
+  uint32_t w = warp, v = 0, vis0 = FULL, n0 = 0;  // v: this lane's vertex of the word loaded
+  uint64_t b0 = 0;
+  uint2 d0 = make_uint2(0u, 0u);
+  auto load = [&] {
+    vis0 = FULL;
+    if (w >= nw) return;
+    const uint64_t x = (uint64_t)o.tiles.word_of(w) * 32 + lane;
+    if (x >= p.V) return;
+    v = (uint32_t)x;
+    vis0 = p.vis[v >> 5];
+    row_of(p, a, v, b0, n0, d0);
+  };
+  load();
+  bu_scan<kR>(p, o, st.e[warp], [&](BuEntry* ring, uint32_t& cnt) {
+    if (w >= nw) return false;
+    const bool cand = !((vis0 >> lane) & 1u) && n0 + d0.y != 0u;
+    const uint32_t m = __ballot_sync(FULL, cand);
+    if (cand) ring[cnt + __popc(m & vxb::lanemask_lt())] = bu_entry(v, b0, n0, d0);
+    cnt += __popc(m);
+    w += kT / 32;
+    load();
+    return w < nw;
+  });
+}
+
+// Later bottom-up levels: the block's segment lin[0, nin) of the list the
+// level before left (entries visited since are skipped).  Entries are loaded
+// two refills ahead, their visited words and row bounds one.
+template <int kT, int kR, class Queue>
+__device__ void bu_list_level(const Params& p, BuOut<Queue>& o, BuStage<kT, kR>& st, const uint32_t* lin,
+                              uint32_t nin) {
+  const DevAdj& a = p.g.in;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t base = warp * 32;
+  uint32_t v0 = base + lane < nin ? lin[base + lane] : kUnreachable;
+  uint32_t v1 = base + kT + lane < nin ? lin[base + kT + lane] : kUnreachable;
+  uint32_t vis0 = FULL, n0 = 0;
+  uint64_t b0 = 0;
+  uint2 d0 = make_uint2(0u, 0u);
+  auto load = [&] {
+    vis0 = FULL;
     if (v0 != kUnreachable) {
       vis0 = p.vis[v0 >> 5];
-      vxb::base_range(a, v0, b0, e0);
-      dr0 = a.drow[v0];
+      row_of(p, a, v0, b0, n0, d0);
     }
-    const uint32_t i2 = base + 2 * step + lane;
-    v1 = i2 < nin ? lin[i2] : kUnreachable;
-    const bool todo = v != kUnreachable && !((visw >> (v & 31)) & 1u);
-    if (!todo) {
-      b = e = 0;
-      dr = make_uint2(0, 0);
-    }
-    const uint32_t nb = (uint32_t)(e - b), total = nb + dr.y;
-    bool found = false;
-    // every lane first scans the head of its own row (rows are sorted, and in
-    // skewed graphs the hubs that fill the frontier sit at small ids), four
-    // independent loads in flight per step
-    const uint32_t head = todo ? min(total, kBuHead) : 0u;
-    for (uint32_t k = 0; k < head && !found; k += 4) {
-      uint32_t x[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t kk = k + j;
-        x[j] = kk >= head ? kTomb : (kk < nb ? a.col[b + kk] : a.darena[dr.x + (kk - nb)]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) found = found || (!(x[j] & kTomb) && test_bit(fbc, x[j]));
-    }
-    // the rest of the longer rows: whole warp, 32 arcs per step, early exit
-    uint32_t longm = __ballot_sync(FULL, todo && !found && total > head);
-    while (longm) {
-      const int l = __ffs(longm) - 1;
-      longm &= longm - 1;
-      const uint64_t bb = __shfl_sync(FULL, b, l);
-      const uint32_t nbl = __shfl_sync(FULL, nb, l), tot = __shfl_sync(FULL, total, l);
-      const uint32_t dx = __shfl_sync(FULL, dr.x, l);
-      bool hit_l = false;
-      for (uint32_t k0 = kBuHead; k0 < tot; k0 += 32) {
-        const uint32_t k = k0 + lane;
-        bool hit = false;
-        if (k < tot) {
-          const uint32_t x = k < nbl ? a.col[bb + k] : a.darena[dx + (k - nbl)];
-          hit = !(x & kTomb) && test_bit(fbc, x);
-        }
-        if (__any_sync(FULL, hit)) {
-          hit_l = true;
-          break;
-        }
-      }
-      if (lane == l) found = hit_l;
-    }
-    if (found) dist[v] = level + 1;
-    // visited and next-frontier bits: OR-combined over runs of lanes on the
-    // same bitmap word (list entries come in ascending runs), one atomic per
-    // run; a word that recurs outside its run is ORed again, which is harmless
-    const uint32_t word = v >> 5;
-    uint32_t bits = found ? 1u << (v & 31) : 0u;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, bits, o);
-      const uint32_t wy = __shfl_up_sync(FULL, word, o);
-      if (lane >= o && wy == word) bits |= y;
-    }
-    const uint32_t wnext = __shfl_down_sync(FULL, word, 1);
-    if (bits && (lane == 31 || wnext != word)) {
-      atomicOr(&p.vis[word], bits);
-      atomicOr(&fbn[word], bits);
-    }
-    bq_push(bq, found, v, cnt_n, qout);
-    seg_append(todo && !found, v, lout, nout);
-  }
-  bq_flush(bq, cnt_n, qout);
+  };
+  load();
+  bu_scan<kR>(p, o, st.e[warp], [&](BuEntry* ring, uint32_t& cnt) {
+    if (base >= nin) return false;
+    const uint32_t v = v0;
+    const bool cand = !((vis0 >> (v & 31)) & 1u);
+    const uint32_t m = __ballot_sync(FULL, cand);
+    if (cand) ring[cnt + __popc(m & vxb::lanemask_lt())] = bu_entry(v, b0, n0, d0);
+    cnt += __popc(m);
+    base += kT;
+    v0 = v1;
+    const uint32_t i = base + kT + lane;
+    v1 = i < nin ? lin[i] : kUnreachable;
+    load();
+    return base < nin;
+  });
 }
 
 // ------------------------------------------------------------ full BFS --
 
-__device__ void full_bfs(const Params& p, BlockQueue& bq, LbStage& lbst, uint32_t* dist,
-                         unsigned long long* trace) {
+// kT threads per block; lbst and bu may share memory.  wbits[0, wbits_n): shared
+// words for the block's part of a bitmap.
+template <bool kInRepair, int kT, int kR, class Queue>
+__device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, kR>& bu, uint32_t* wbits,
+                         uint32_t wbits_n, uint32_t* dist, unsigned long long* trace) {
   BfsCounters* c = p.c;
   const unsigned long long t_start = gtid() == 0 ? globaltimer() : 0ull;  // the repair phases' time budget
   __shared__ uint32_t seg_n[2];  // entries of this block's segment of each candidate list
-  if (threadIdx.x == 0) bq.cnt = 0;
+  __shared__ unsigned long long red[kT / 32];
+  __shared__ LevelWords lw;
+  if (threadIdx.x == 0) {
+    bq.cnt = 0;
+    lw.m = 0;
+    lw.n = 0;
+  }
   const uint32_t V = p.V;
   const uint32_t words = (V + 31) >> 5;
   // one pass sets every vertex unreached and the source at level 0 (bits
-  // past V count as visited, so bottom-up never scans them), and lists the
-  // bottom-up candidates: every vertex but the source with a nonempty in-row
-  // (isolated vertices never enter a bottom-up level).  Each block takes a
-  // contiguous range of vertices and lists its candidates in its own segment
-  // of list A (shared-memory counter, no global atomics); a bottom-up level
-  // scans the block's own segment.
+  // past V count as visited, so bottom-up never scans them)
   const uint32_t s = p.source;
   const bool has_source = s < V;
-  const uint32_t seg = (V + gridDim.x - 1) / gridDim.x;  // vertices (and list slots) per block
-  const uint32_t seg_lo = blockIdx.x * seg, seg_hi = min(V, seg_lo + seg);
-  if (threadIdx.x == 0) seg_n[0] = seg_n[1] = 0;
-  __syncthreads();
-  for (uint32_t i0 = seg_lo; i0 < seg_hi; i0 += kThreads) {
-    const uint32_t i = i0 + threadIdx.x;
-    bool cand = false;
-    if (i < seg_hi) {
-      dist[i] = i == s ? 0u : kUnreachable;
-      cand = has_source && i != s && degree_of(p.g.in, i) != 0u;
+  if ((reinterpret_cast<uintptr_t>(dist) & 15) == 0) {  // a caller's own buffer may start anywhere
+    const uint4 none = make_uint4(kUnreachable, kUnreachable, kUnreachable, kUnreachable);
+    for (uint32_t i = gtid(); i < V / 4; i += nthreads()) {
+      uint4 d = none;
+      if (i == s / 4) d = make_uint4(s % 4 == 0 ? 0u : d.x, s % 4 == 1 ? 0u : d.y, s % 4 == 2 ? 0u : d.z, s % 4 == 3 ? 0u : d.w);
+      reinterpret_cast<uint4*>(dist)[i] = d;
     }
-    seg_append(cand, i, p.bul + seg_lo, &seg_n[0]);
+    for (uint32_t i = V / 4 * 4 + gtid(); i < V; i += nthreads()) dist[i] = i == s ? 0u : kUnreachable;
+  } else {
+    for (uint32_t i = gtid(); i < V; i += nthreads()) dist[i] = i == s ? 0u : kUnreachable;
   }
   for (uint32_t i = gtid(); i < words; i += nthreads()) {
     const uint32_t lo = i * 32;
     const uint32_t sbit = has_source && i == (s >> 5) ? 1u << (s & 31) : 0u;
     p.vis[i] = ((lo + 32 <= V) ? 0u : (FULL << (V - lo))) | sbit;
-    p.fb[0][i] = sbit;
-    p.fb[1][i] = p.fb[2][i] = 0u;
+    p.fb[0][i] = p.fb[1][i] = p.fb[2][i] = 0u;
   }
   if (gtid() == 0) {
     for (int k = 0; k < 3; ++k) {
@@ -489,7 +819,7 @@ __device__ void full_bfs(const Params& p, BlockQueue& bq, LbStage& lbst, uint32_
     if (has_source) {
       p.q[0][0] = s;
       c->lvl_n[0] = 1;
-      c->lvl_m[0] = degree_of(p.g.out, s);
+      c->lvl_m[0] = row_len(p, p.g.out, s);
     } else {
       c->reachable = 0;
       c->levels = 0;
@@ -499,85 +829,186 @@ __device__ void full_bfs(const Params& p, BlockQueue& bq, LbStage& lbst, uint32_
   if (!sync_grid(p) || !has_source) return;
   unsigned long long m_visited = 0;
   uint32_t reached = 0;
-  bool bottom_up = false, left_bu = false;
+  bool bottom_up = false, left_bu = false, bu_listed = false;
+  bool queued = true;  // the current frontier is in its queue
   uint32_t prev_n = 0;
   uint32_t level = 0;
   // the frontier size and arc count of the current level, read once after the
-  // barrier that ends the level before it
+  // barrier that ends the level before it; a bottom-up level does not count arcs
   uint32_t n_f = ld_cg(&c->lvl_n[0]);
   unsigned long long m_f = __ldcg(&c->lvl_m[0]);
-  // bottom-up candidate lists: the first bottom-up level reads list 0
-  uint32_t lin = 0;
-  for (;; ++level) {
+  bool m_known = true;
+  // bottom-up candidate lists, cut into one segment per block: the first
+  // bottom-up level leaves list 0
+  const BuTiles tiles(words, gridDim.x);
+  const uint32_t seg = tiles.words() * 32;  // vertices (and list slots) per block
+  uint32_t lin = 1;
+  uint32_t bits = 0;  // bit k: fb[k] holds the bits of its level's frontier
+  // queues, bitmaps and counters rotate over three slots; a stretch of one
+  // block's levels takes one turn
+  for (uint32_t turn = 0;; ++turn) {
     if (level > V + 1) {
       if (gtid() == 0) atomicOr(&c->err, vxb::kErrLoopBound);
       break;
     }
-    const int cur = level % 3, nxt = (level + 1) % 3, clr = (level + 2) % 3;
+    const uint32_t cur = turn % 3, nxt = (turn + 1) % 3, clr = (turn + 2) % 3;
     if (n_f == 0) break;
-    reached += n_f;
-    m_visited += m_f;
-    if (!bottom_up && !left_bu) {
-      const unsigned long long m_u = p.total_arcs > m_visited ? p.total_arcs - m_visited : 0ull;
-      if ((double)m_f * p.alpha > (double)m_u && level > 0) bottom_up = true;
-    } else if (bottom_up && (double)n_f * p.beta < (double)V && n_f < prev_n) {
-      bottom_up = false;
-      left_bu = true;
-    }
     if (gtid() == 0) {
       c->lvl_n[clr] = 0;
       c->lvl_m[clr] = 0;
       c->lvl_big[clr] = 0;
-      if (trace && level < kTraceLevels) {
-        trace[2 * level] = globaltimer();
-        trace[2 * level + 1] = (unsigned long long)n_f | ((unsigned long long)bottom_up << 63);
+    }
+    if (bottom_up && (double)n_f * p.beta < (double)V && n_f < prev_n) {
+      bottom_up = false;
+      left_bu = true;
+      if (!queued) {  // the frontier's queue, from its bitmap (at most once per search)
+        for (uint32_t i0 = gtid() & ~31u; i0 < words; i0 += nthreads()) {
+          const uint32_t i = i0 + (threadIdx.x & 31);
+          uint32_t w = i < words ? p.fb[cur][i] : 0u;
+          while (__any_sync(FULL, w != 0u)) {
+            bq_push(bq, w != 0u, i * 32 + (uint32_t)__ffs(w) - 1, p.bar + kQueueWord, p.q[cur]);
+            w &= w - 1;
+          }
+        }
+        bq_flush(bq, p.bar + kQueueWord, p.q[cur]);
+        if (!sync_grid(p)) return;
+        if (gtid() == 0) p.bar[kQueueWord] = 0u;
+        queued = true;
       }
     }
-    // clear the frontier bitmap of level-1: through its queue when it was
-    // small, else word by word (plain stores, no dependent queue loads)
-    if ((unsigned long long)prev_n * 8 < words) {
-      for (uint32_t i = gtid(); i < prev_n; i += nthreads()) p.fb[clr][p.q[clr][i] >> 5] = 0u;
-    } else {
-      for (uint32_t i = gtid(); i < words; i += nthreads()) p.fb[clr][i] = 0u;
+    if (!bottom_up && m_known && solo_fits(n_f, m_f)) {
+      for (uint32_t k = 0; k < 3; ++k)
+        if ((bits >> k) & 1u)
+          for (uint32_t i = gtid(); i < words; i += nthreads()) p.fb[k][i] = 0u;
+      bits = 0;
+      // the state after the stretch, one set per parity of the turn (a block
+      // may still read the last stretch's set while block 0 runs the next)
+      uint32_t* out = p.bar + kSoloWord + 8 * (turn & 1);
+      if (blockIdx.x == 0) {
+        SoloState st{level, n_f, reached, m_f, m_visited};
+        solo_levels<kT>(p, dist, p.q[cur], p.q[nxt], &c->lvl_n[nxt], bq, lbst, red, trace, st);
+        if (threadIdx.x == 0) {
+          out[0] = st.level;
+          out[1] = st.reached;
+          *reinterpret_cast<unsigned long long*>(out + 2) = st.m_visited;
+          c->lvl_m[nxt] = st.m_f;
+        }
+      }
+      __shared__ SoloState after;
+      vxb::grid_barrier_then(p.bar, p.nblocks, &c->err, [&] {
+        lw.failed = __ldcg(&c->err);
+        after = SoloState{ld_cg(&out[0]), ld_cg(&c->lvl_n[nxt]), ld_cg(&out[1]), __ldcg(&c->lvl_m[nxt]),
+                          __ldcg(reinterpret_cast<unsigned long long*>(out + 2))};
+      });
+      if (lw.failed) return;
+      prev_n = n_f;
+      level = after.level;
+      n_f = after.n_f;
+      reached = after.reached;
+      m_f = after.m_f;
+      m_visited = after.m_visited;
+      continue;
     }
+    reached += n_f;
+    m_visited += m_f;
+    if (!bottom_up && !left_bu && level > 0) {
+      // bottom-up when the frontier's rows hold more than 1 / alpha of the
+      // arcs of unvisited vertices, and (at the default alpha) more arcs than
+      // there are vertices: the first bottom-up level sweeps every vertex, so
+      // a thin frontier of a low-degree graph is cheaper pushed (4096 x 4096
+      // lattice, 620,000 vertices of frontier: three bottom-up levels took 480 us,
+      // top-down ones take 170)
+      const unsigned long long m_u = p.total_arcs > m_visited ? p.total_arcs - m_visited : 0ull;
+      const double am = (double)m_f * p.alpha;
+      bottom_up = am > (double)m_u && am > 14.0 * (double)V;
+    }
+    if (gtid() == 0 && trace && level < kTraceLevels) {
+      trace[2 * level] = globaltimer();
+      trace[2 * level + 1] = (unsigned long long)n_f | ((unsigned long long)bottom_up << 63);
+    }
+    if ((bits >> clr) & 1u)
+      for (uint32_t i = gtid(); i < words; i += nthreads()) p.fb[clr][i] = 0u;
+    bits &= ~(1u << clr);
+    unsigned long long mloc = 0;
+    uint32_t nloc = 0;
+    const bool td = !bottom_up;
     if (bottom_up) {
+      if (!((bits >> cur) & 1u)) {  // the level before kept no bitmap
+        for (uint32_t i = gtid(); i < n_f; i += nthreads()) {
+          const uint32_t v = p.q[cur][i];
+          atomicOr(&p.fb[cur][v >> 5], 1u << (v & 31));
+        }
+        if (!sync_grid(p)) return;
+        bits |= 1u << cur;
+      }
       const uint32_t lout = lin ^ 1u;
       if (threadIdx.x == 0) seg_n[lout] = 0;
+      // the queue is kept where the block's shared buffer takes it whole or the
+      // level is not the first (which reaches most of a graph's vertices)
+      const bool push = seg <= sizeof(bq.items) / sizeof(bq.items[0]) || bu_listed;
+      const uint32_t nwords = tiles.words();
+      const bool local = nwords <= wbits_n;
+      if (local)
+        for (uint32_t i = threadIdx.x; i < nwords; i += kT) wbits[i] = 0u;
       __syncthreads();
-      bu_list_level(p, dist, level, p.fb[cur], p.fb[nxt], p.q[nxt], &c->lvl_n[nxt], bq, p.bul + lin * p.bul_half + seg_lo,
-                    seg_n[lin], p.bul + lout * p.bul_half + seg_lo, &seg_n[lout]);
-      lin = lout;
-      if (!sync_grid(p)) return;
-      prev_n = n_f;
-      n_f = ld_cg(&c->lvl_n[nxt]);
-      m_f = __ldcg(&c->lvl_m[nxt]);
-    } else {
-      TdVisit t{&p, dist, level, p.q[nxt], p.fb[nxt], &c->lvl_n[nxt], !left_bu, 0ull, &bq};
-      if (n_f <= kLbMax) td_level_lb(p, t, p.q[cur], n_f, lbst);
-      else td_level(p, t, p.q[cur], n_f, &c->lvl_big[cur]);
-      t.flush(&c->lvl_m[nxt]);
-      bq_flush(bq, &c->lvl_n[nxt], p.q[nxt]);
-      if (!sync_grid(p)) return;
-      // three independent loads: the next level's figures stand unless hub rows remain
-      prev_n = n_f;
-      const uint32_t nbig = ld_cg(&c->lvl_big[cur]);
-      n_f = ld_cg(&c->lvl_n[nxt]);
-      m_f = __ldcg(&c->lvl_m[nxt]);
-      if (nbig) {
-        grid_rows(p.g.out, p.big, nbig, t);
-        t.flush(&c->lvl_m[nxt]);
-        bq_flush(bq, &c->lvl_n[nxt], p.q[nxt]);
-        if (!sync_grid(p)) return;
-        n_f = ld_cg(&c->lvl_n[nxt]);
-        m_f = __ldcg(&c->lvl_m[nxt]);
+      uint32_t* lists = p.bul + (size_t)blockIdx.x * seg;
+      BuOut<Queue> o{dist,  level, p.fb[cur], p.fb[nxt], local ? wbits : nullptr, tiles, lists + (size_t)lout * p.bul_half,
+                     &seg_n[lout], push ? &bq : nullptr, p.q[nxt], &c->lvl_n[nxt], 0u};
+      if (!bu_listed) bu_first_level(p, o, bu);
+      else bu_list_level(p, o, bu, lists + (size_t)lin * p.bul_half, seg_n[lin]);
+      if (local) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < nwords; i += kT) {
+          const uint32_t w = wbits[i];
+          if (!w) continue;
+          const uint32_t g = tiles.word_of(i);  // no other block writes it
+          p.vis[g] |= w;
+          p.fb[nxt][g] = w;
+        }
       }
+      bu_listed = true;
+      lin = lout;
+      bits |= 1u << nxt;
+      m_known = false;
+      nloc = o.nloc;
+      queued = push;
+    } else {
+      // a small frontier's level keeps the bitmap (few claims); after a
+      // larger one a bottom-up level makes it from the queue
+      const bool keep = n_f <= kLbMax && !left_bu;
+      TdVisit<Queue> t{&p, dist, level, p.q[nxt], keep ? p.fb[nxt] : nullptr, &c->lvl_n[nxt], &bq, 0ull};
+      if (n_f <= kLbMax) {
+        lb_stage<kT>(p, p.q[cur], n_f, lbst);
+        lb_visit(p, t, n_f, lbst, gwarp(), nwarps());
+      } else {
+        td_level(p, t, p.q[cur], n_f, &c->lvl_big[cur]);
+      }
+      if (keep) bits |= 1u << nxt;
+      m_known = true;
+      queued = true;
+      mloc = t.mloc;
     }
+    if (!level_end(p, lw, bq, nloc, mloc, nxt, td ? &c->lvl_big[cur] : nullptr)) return;
+    prev_n = n_f;
+    if (lw.nbig) {  // hub rows remain
+      TdVisit<Queue> t{&p, dist, level, p.q[nxt], nullptr, &c->lvl_n[nxt], &bq, 0ull};
+      grid_rows(p, t, lw.nbig);
+      if (!level_end(p, lw, bq, 0u, t.mloc, nxt, nullptr)) return;
+    }
+    n_f = lw.n_f;
+    m_f = lw.m_f;
+    ++level;
   }
   if (gtid() == 0) {
     c->reachable = reached;
     c->levels = level;
     c->arcs = m_visited;
-    c->full_ns = globaltimer() - t_start;
+    // for the repair phases' time budget: what a full BFS takes inside an update
+    // launch, by the measure of the kernel's own time (its 512 threads per SM take
+    // 1.2 to 1.45 times as long at R-MAT 20 to 22 and on the lattice, and the
+    // handover adds a few passes)
+    const unsigned long long t = globaltimer() - t_start;
+    c->full_ns = kInRepair ? t : t + t / 2 + 20000ull;
     if (trace && level < kTraceLevels) {
       trace[2 * level] = globaltimer();
       trace[2 * level + 1] = 0;
@@ -741,6 +1172,16 @@ struct RepairSmem {
   uint32_t late;     // the round started past the phase's deadline (its items are dropped)
   uint32_t flagged;  // this block has raised the phase's handover flag
 };
+
+// The full BFS inside a repair kernel, in the shared memory its phases do not
+// hold at that point.
+__device__ void bfs_in_repair(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t* dist,
+                              unsigned long long* trace) {
+  using Stage = BuStage<kThreads, 1>;
+  static_assert(sizeof(Stage) <= sizeof(LbStage) && alignof(LbStage) >= alignof(Stage), "the two share memory");
+  full_bfs<true>(p, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm), (uint32_t)(sizeof(sm) / 4), dist,
+           trace);
+}
 
 // Drains the ring; W::process(sm, n) handles sm.items[0, n) block-uniformly,
 // with sm.late set for a round that starts at or past the deadline (a
@@ -1210,7 +1651,7 @@ __device__ void clear_workspace(const Params& p);
 // affected list stays empty, so the post-batch repair only relaxes the
 // insertions.  The BFS distances go to tent (zero between phases), which the
 // comparison pass zeroes again.
-__device__ bool cascade_by_bfs(const Params& p, BlockQueue& bq, LbStage& lb) {
+__device__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
   BfsCounters* c = p.c;
   clear_workspace(p);
   reset_ring(p);
@@ -1224,7 +1665,7 @@ __device__ bool cascade_by_bfs(const Params& p, BlockQueue& bq, LbStage& lb) {
     c->a_n = 0;
     c->a_bfs = 0;
   }
-  full_bfs(p, bq, lb, p.tent, nullptr);  // also sets the reachable count of the graph without the deletions
+  bfs_in_repair(p, sm, lb, bq, p.tent, nullptr);  // also sets the reachable count of the graph without the deletions
   if (!sync_grid(p)) return false;
   uint32_t raised = 0;
   for (uint32_t v = gtid(); v < p.dist_len; v += nthreads()) {
@@ -1267,7 +1708,7 @@ __device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue
     p.c->rtrace[7] = ld_cg(p.rq_tail);
     for (int k = 0; k < 6; ++k) p.c->rtrace[9 + k] = __ldcg(&p.rq_stat[k]);
   }
-  if (ld_cg(&p.c->cbig)) return cascade_by_bfs(p, bq, lb);
+  if (ld_cg(&p.c->cbig)) return cascade_by_bfs(p, sm, bq, lb);
   if (gtid() == 0) p.c->affected = ld_cg(&p.c->a_n);
   return true;
 }
@@ -1571,7 +2012,7 @@ __device__ void repair_post(const Params& p, RepairSmem& sm, LbStage& lb, BlockQ
   if (fallback) clear_workspace(p);
   else if (!repair_relax(p, sm, lb)) return;
   if (!sync_grid(p)) return;
-  full_bfs(p, bq, lb, p.dist, p.trace);
+  bfs_in_repair(p, sm, lb, bq, p.dist, p.trace);
   if (gtid() == 0) {
     if (fallback) {
       c->full = 1;
@@ -1950,16 +2391,30 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
   if (gtid() == 0) c->rmb[0] = c->rmb[1] = 0u;
 }
 
-// The full BFS has a kernel of its own, so that its registers are allocated
-// apart from the repair phases' (the repair kernel runs it too, for the
-// fallback and the budget handovers).
-__global__ void __launch_bounds__(kThreads, 3) bfs_full_kernel(Params p) {
-  __shared__ BlockQueue bq;
-  __shared__ LbStage lb;
-  full_bfs(p, bq, lb, p.dist, p.trace);
+// The full BFS has a kernel of its own (the repair kernels run it too, for the
+// fallback and the budget handovers), one block of 1,024 threads per SM: the
+// grid barrier's cost grows with the blocks that meet at it, and 32 warps with
+// four arcs per lane in flight keep the memory as busy as 48 with one did.
+// R-MAT of 30,000 vertices: 75 us with 444 blocks of 512 threads, 56 with 296,
+// 45 with 148.  Graphs of fewer than kWideArcs arcs take 512 threads, whose
+// block barriers are cheaper (40 us; R-MAT 2^20, 31M arcs: 89 us with 512, 77 with
+// 1,024; R-MAT 2^22: 244 and 168).
+template <int kT>
+struct FullSmem {
+  BlockQueueOf<8192> bq;
+  LbStage lb;
+  BuStage<kT, kT / 512> bu;
+  uint32_t bits[8192];
+};
+
+template <int kT>
+__global__ void __launch_bounds__(kT, 1024 / kT) bfs_full_kernel(Params p) {
+  extern __shared__ __align__(16) unsigned char full_smem[];
+  FullSmem<kT>& sm = *reinterpret_cast<FullSmem<kT>*>(full_smem);
+  full_bfs<false>(p, sm.bq, sm.lb, sm.bu, sm.bits, 8192u, p.dist, p.trace);
 }
 
-__global__ void __launch_bounds__(kThreads, 3) bfs_kernel(Params p, int mode) {
+__global__ void __launch_bounds__(kThreads, 2) bfs_kernel(Params p, int mode) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
@@ -1967,6 +2422,10 @@ __global__ void __launch_bounds__(kThreads, 3) bfs_kernel(Params p, int mode) {
   else repair_post(p, sm, lb, bq);
 }
 
+// Registers for two blocks per SM: the launches of two graphs (on their own
+// streams) then run side by side, which a block with 128 registers a thread
+// (no spills, 2% faster alone) does not allow: 10,000-op batches on three R-MAT
+// 22 graphs in turn 86 us a batch, 111 us with 128 registers.
 __global__ void __launch_bounds__(kThreads, 2) bfs_stream_kernel(Params p, StreamArgs s) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
@@ -2109,7 +2568,7 @@ static int ensure_capacity(Bfs* b, size_t V) {
   rc |= realloc_copy(&b->lst_a, c, 0, 0);
   rc |= realloc_copy(&b->lst_t, c, 0, 0);
   rc |= realloc_copy(&b->tent, c, 0, 0);
-  rc |= realloc_copy(&b->bul, 2 * (c + kListSlack), 0, 0);
+  rc |= realloc_copy(&b->bul, 2 * list_slots(c), 0, 0);
   const cudaError_t e = cudaStreamSynchronize(s);
   for (uint32_t* p : old) cudaFree(p);
   if (rc) return -4;
@@ -2171,7 +2630,7 @@ static Params make_params(Bfs* b, uint32_t V, uint32_t dist_len) {
   p.lst_t = b->lst_t;
   p.tent = b->tent;
   p.bul = b->bul;
-  p.bul_half = (uint32_t)(b->cap + kListSlack);
+  p.bul_half = (uint32_t)list_slots(b->cap);
   p.sw = reinterpret_cast<unsigned long long*>(b->sw);
   p.ring = b->ring;
   p.ring_mask = b->ring_slots ? (uint32_t)(b->ring_slots - 1) : 0u;
@@ -2195,6 +2654,7 @@ static Params make_params(Bfs* b, uint32_t V, uint32_t dist_len) {
   p.trace = b->trace;
   p.acct = b->acct_on ? b->acct : nullptr;
   p.bar = b->barrier;
+  p.deltas = (g->adj[0].arena_bound | g->in().arena_bound) != 0;
   return p;
 }
 
@@ -2211,15 +2671,43 @@ static int grid_of(const void* kernel, int* grid) {
   return 0;
 }
 
-static int launch(Bfs* b, Params& p, int mode) {
-  const bool full = mode == kModeFull;
-  const void* kernel = full ? (const void*)bfs_full_kernel : (const void*)bfs_kernel;
-  int* grid = full ? &b->full_grid : &b->grid;
-  if (int rc = grid_of(kernel, grid)) return rc;
-  p.nblocks = (uint32_t)*grid;
-  void* args[] = {&p, &mode};  // the full-BFS kernel takes p alone
+// One block per SM, fewer for a graph whose arcs one step of fewer blocks covers
+// (kT threads of kVisit arcs): 2,000 vertices 38 us with 148 blocks, 32 with 20.
+template <int kT>
+static int launch_full_t(Params& p, cudaStream_t s) {
+  static std::atomic<int> sms_dev[64];  // SMs of a device whose kernel has its shared memory limit set
+  int dev = 0;
+  VX_CUDA_TRY(cudaGetDevice(&dev));
+  int sms = dev < 64 ? sms_dev[dev].load(std::memory_order_acquire) : 0;
+  if (!sms) {
+    VX_CUDA_TRY(cudaFuncSetAttribute(bfs_full_kernel<kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(FullSmem<kT>)));
+    VX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (dev < 64) sms_dev[dev].store(sms, std::memory_order_release);
+  }
+  const uint64_t want = std::max<uint64_t>(p.V, p.total_arcs) / (kT * kVisit) + 8;
+  p.nblocks = (uint32_t)std::min<uint64_t>(want, (uint64_t)sms);
+  void* args[] = {&p};
   vxh::count_launch();
-  VX_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(*grid), dim3(kThreads), args, 0, b->g->stream));
+  VX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bfs_full_kernel<kT>, dim3(p.nblocks), dim3(kT), args,
+                                          sizeof(FullSmem<kT>), s));
+  return 0;
+}
+
+// Launches the full BFS (p.V, p.total_arcs set); p.nblocks is set here.
+constexpr uint64_t kWideArcs = 1ull << 24;
+static int launch_full(Params& p, cudaStream_t s) {
+  return std::max<uint64_t>(p.V, p.total_arcs) >= kWideArcs ? launch_full_t<1024>(p, s) : launch_full_t<512>(p, s);
+}
+
+static int launch(Bfs* b, Params& p, int mode) {
+  if (mode == kModeFull) return launch_full(p, b->g->stream);
+  if (int rc = grid_of((const void*)bfs_kernel, &b->grid)) return rc;
+  p.nblocks = (uint32_t)b->grid;
+  void* args[] = {&p, &mode};
+  vxh::count_launch();
+  VX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bfs_kernel, dim3(b->grid), dim3(kThreads), args, 0,
+                                          b->g->stream));
   return 0;
 }
 
@@ -2409,6 +2897,7 @@ static int launch_stream(Bfs* b, Params& p, StreamArgs& sa) {
   // update step measured 13% faster at R-MAT 22 and R-MAT 20
   const uint32_t want = b->tune.update_blocks ? b->tune.update_blocks : (uint32_t)sm_count();
   p.nblocks = want < (uint32_t)b->stream_grid ? want : (uint32_t)b->stream_grid;
+  p.deltas = 1;  // the launch inserts delta rows itself
   void* args[] = {&p, &sa};
   count_launch();
   VX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bfs_stream_kernel, dim3(p.nblocks), dim3(kThreads), args,
@@ -2761,11 +3250,11 @@ int bfs_digest(Bfs* b, uint64_t* out) {
 // direction-optimising BFS kernel as recompute() on a CSR the caller already
 // holds in device memory, writing distances into the caller's buffer, and
 // keeps every other buffer (visited and frontier bitmaps, frontier queues,
-// counters, barrier words, the empty delta-row table) in one file-scope
+// counters, barrier words) in one file-scope
 // device array.  It allocates nothing.
 //
 // Limits and sharing: at most kStaticMaxVertices vertices; every GPU that
-// loads this library holds the array (about 8.5 MB) until the process exits;
+// loads this library holds the array (about 6.5 MB) until the process exits;
 // all calls share it and it keeps the last call's contents, so calls that
 // overlap on the GPU (different streams, different threads) race -- issue
 // them one at a time per device.  The first call on a device looks up the
@@ -2782,8 +3271,7 @@ struct StaticBfsScratch {
   uint32_t fb[3][kStaticWords];
   uint32_t q[3][kStaticMaxVertices];
   uint32_t big[kStaticMaxVertices];
-  uint32_t bul[2 * (kStaticMaxVertices + kListSlack)];  // the bottom-up candidate lists
-  uint2 drow[kStaticMaxVertices];  // kept all-zero: a plain CSR has no delta rows
+  uint32_t bul[2 * list_slots(kStaticMaxVertices)];  // the bottom-up candidate lists
   BfsCounters ctr;
   uint32_t bar[vxb::kBarrierWords];
 };
@@ -2832,10 +3320,9 @@ extern "C" int vx_bfs_csr_static(const uint64_t* d_out_offsets, const uint32_t* 
   }
   StaticBfsScratch* sc = static_cast<StaticBfsScratch*>(addr);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // what must start at zero: counters, barrier words, the delta-row table
+  // what must start at zero: counters, barrier words (a plain CSR has no delta rows to read)
   VX_CUDA_TRY(cudaMemsetAsync(&sc->ctr, 0, sizeof(vxh::BfsCounters), s));
   VX_CUDA_TRY(cudaMemsetAsync(sc->bar, 0, sizeof(sc->bar), s));
-  VX_CUDA_TRY(cudaMemsetAsync(sc->drow, 0, (size_t)vertices * sizeof(uint2), s));
   vxh::Params p;
   memset(&p, 0, sizeof(p));
   auto adj = [&](const uint64_t* off, const uint32_t* col) {
@@ -2844,7 +3331,6 @@ extern "C" int vx_bfs_csr_static(const uint64_t* d_out_offsets, const uint32_t* 
     a.off = off;
     a.col = const_cast<uint32_t*>(col);
     a.Vb = vertices;
-    a.drow = sc->drow;
     return a;
   };
   p.g.out = adj(d_out_offsets, d_out_cols);
@@ -2862,25 +3348,14 @@ extern "C" int vx_bfs_csr_static(const uint64_t* d_out_offsets, const uint32_t* 
   }
   p.big = sc->big;
   p.bul = sc->bul;
-  p.bul_half = vxh::kStaticMaxVertices + vxh::kListSlack;
+  p.bul_half = (uint32_t)vxh::list_slots(vxh::kStaticMaxVertices);
   p.c = &sc->ctr;
   p.total_arcs = arcs;
   p.alpha = 14.0f;
   p.beta = 24.0f;
   p.large_row = 1024;
   p.bar = sc->bar;
-  int per_sm = 0, sms = 0;
-  VX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vxh::bfs_full_kernel, vxh::kThreads, 0));
-  VX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (per_sm < 1) {
-    vxh::set_error("vx_bfs_csr_static: BFS kernel cannot be resident on an SM");
-    return -3;
-  }
-  p.nblocks = (uint32_t)(per_sm * sms);
-  void* args[] = {&p};
-  vxh::count_launch();
-  VX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)vxh::bfs_full_kernel, dim3(p.nblocks), dim3(vxh::kThreads),
-                                          args, 0, s));
+  if (int rc = vxh::launch_full(p, s)) return rc;
   uint32_t err = 0;
   unsigned long long reach = 0;
   VX_CUDA_TRY(cudaMemcpyAsync(&err, &sc->ctr.err, sizeof(err), cudaMemcpyDeviceToHost, s));

@@ -51,7 +51,7 @@ struct BfsCounters {
   // the number of vertices whose distance that BFS raised
   uint32_t cbig;
   uint32_t a_bfs;
-  // globaltimer ns the last full BFS took, and the time at which the running
+  // ns the last full BFS took (or would have inside an update launch), and the time at which the running
   // repair phase hands over to a BFS (~0: never)
   unsigned long long full_ns;
   unsigned long long deadline;
@@ -128,7 +128,6 @@ struct Bfs {
   bool staged_classified = true;
   BfsTuning tune;
   int grid = 0;       // blocks of the repair kernel
-  int full_grid = 0;  // blocks of the full-BFS kernel
   int stream_grid = 0;
   unsigned long long* acct = nullptr;  // algorithmic-byte accounting (5 counters), when on
   bool acct_on = false;

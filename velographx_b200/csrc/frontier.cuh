@@ -77,77 +77,6 @@ __device__ __forceinline__ void for_my_rows(const uint32_t* len, uint32_t n, uin
 
 constexpr uint32_t FULL = 0xFFFFFFFFu;
 
-// Flattened expansion of per-lane segments arr[start, start+len) across the
-// warp (Merrill-style gather: warp scan of the lengths, then each lane finds
-// the owner of element k by a 5-step shuffle search).  f(valid, x, owner) is
-// called warp-uniformly.
-template <class F>
-__device__ __forceinline__ void gather_segments(const uint32_t* arr, uint64_t start, uint32_t len, uint32_t u,
-                                                bool tombs, F& f) {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const uint32_t excl = incl - len;
-  const uint32_t total = __shfl_sync(FULL, incl, 31);
-  for (uint32_t k0 = 0; k0 < total; k0 += 32) {
-    const uint32_t k = k0 + lane;
-    const bool ok = k < total;
-    int owner = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-      const int cand = owner + step;
-      const uint32_t ex = __shfl_sync(FULL, excl, cand & 31);
-      if (cand < 32 && ex <= k) owner = cand;
-    }
-    const uint64_t st = __shfl_sync(FULL, start, owner);
-    const uint32_t ex = __shfl_sync(FULL, excl, owner);
-    const uint32_t ou = __shfl_sync(FULL, u, owner);
-    const uint32_t x = ok ? arr[st + (k - ex)] : kTomb;
-    f(ok && !(tombs && (x & kTomb)), x & kIdMask, ou);
-  }
-}
-
-// Expands the rows of the (up to) 32 lane vertices: rows of >= 32 arcs are
-// walked by the whole warp, shorter ones flattened across lanes.  Lanes pass
-// an empty range (b == e, dr.y == 0) when they have no row.
-template <class F>
-__device__ __forceinline__ void expand_lanes(const DevAdj& a, uint32_t u, uint64_t b, uint64_t e, uint2 dr, F& f) {
-  const int lane = threadIdx.x & 31;
-  uint32_t blen = (uint32_t)(e - b), dlen = dr.y;
-  uint32_t med = __ballot_sync(FULL, blen >= 32);
-  while (med) {
-    const int l = __ffs(med) - 1;
-    med &= med - 1;
-    const uint64_t bb = __shfl_sync(FULL, b, l), ee = __shfl_sync(FULL, e, l);
-    const uint32_t uu = __shfl_sync(FULL, u, l);
-    for (uint64_t j0 = bb; j0 < ee; j0 += 32) {
-      const uint64_t j = j0 + lane;
-      const uint32_t x = j < ee ? a.col[j] : kTomb;
-      f(!(x & kTomb), x & kIdMask, uu);
-    }
-  }
-  if (blen >= 32) blen = 0;
-  gather_segments(a.col, b, blen, u, true, f);
-  med = __ballot_sync(FULL, dlen >= 32);
-  while (med) {
-    const int l = __ffs(med) - 1;
-    med &= med - 1;
-    const uint32_t bb = __shfl_sync(FULL, dr.x, l), ee = bb + __shfl_sync(FULL, dr.y, l);
-    const uint32_t uu = __shfl_sync(FULL, u, l);
-    for (uint32_t j0 = bb; j0 < ee; j0 += 32) {
-      const uint32_t j = j0 + lane;
-      const bool ok = j < ee;
-      f(ok, ok ? a.darena[j] : 0u, uu);
-    }
-  }
-  if (dlen >= 32) dlen = 0;
-  gather_segments(a.darena, (uint64_t)dr.x, dlen, u, false, f);
-}
-
 // The whole warp walks one row (all lanes pass the same u); f as above.
 template <class F>
 __device__ __forceinline__ void warp_row(const DevAdj& a, uint32_t u, F& f) {
@@ -177,15 +106,18 @@ __device__ __forceinline__ uint64_t globaltimer() {
 // (shared atomics); the block flushes with one global atomic per phase.  Warps
 // that find the buffer full append straight to the global queue.
 constexpr uint32_t kBlockQueueCap = 2048;
-struct BlockQueue {
+template <uint32_t kCap>
+struct BlockQueueOf {
   uint32_t cnt;
   uint32_t gbase;
-  uint32_t items[kBlockQueueCap];
+  uint32_t items[kCap];
 };
+using BlockQueue = BlockQueueOf<kBlockQueueCap>;
 
 // gbase0: the global counter's value that corresponds to gq[0] (a counter
 // that is not reset between uses, as the bottom-up candidate lists use).
-__device__ __forceinline__ void bq_push(BlockQueue& bq, bool pred, uint32_t v, uint32_t* gcnt, uint32_t* gq,
+template <uint32_t kCap>
+__device__ __forceinline__ void bq_push(BlockQueueOf<kCap>& bq, bool pred, uint32_t v, uint32_t* gcnt, uint32_t* gq,
                                         uint32_t gbase0 = 0u) {
   const uint32_t mask = __ballot_sync(FULL, pred);
   if (!mask) return;
@@ -196,21 +128,52 @@ __device__ __forceinline__ void bq_push(BlockQueue& bq, bool pred, uint32_t v, u
   if (lane == leader) base = atomicAdd(&bq.cnt, n);
   base = __shfl_sync(FULL, base, leader);
   const uint32_t r = __popc(mask & vxb::lanemask_lt());
-  const uint32_t spill = base + n > kBlockQueueCap ? base + n - max(base, kBlockQueueCap) : 0u;
+  const uint32_t spill = base + n > kCap ? base + n - max(base, kCap) : 0u;
   uint32_t gb = 0;
   if (spill && lane == leader) gb = atomicAdd(gcnt, spill);
   gb = __shfl_sync(FULL, gb, leader);
   if (pred) {
     const uint32_t slot = base + r;
-    if (slot < kBlockQueueCap) bq.items[slot] = v;
-    else gq[(gb - gbase0) + (slot - max(base, kBlockQueueCap))] = v;
+    if (slot < kCap) bq.items[slot] = v;
+    else gq[(gb - gbase0) + (slot - max(base, kCap))] = v;
+  }
+}
+
+// The lanes' entries v[j] where bit `lane` of mask[j] is set (masks are
+// warp-uniform), one reservation for all of them.
+template <int N, uint32_t kCap>
+__device__ __forceinline__ void bq_push_n(BlockQueueOf<kCap>& bq, const uint32_t (&mask)[N], const uint32_t (&v)[N],
+                                          uint32_t* gcnt, uint32_t* gq) {
+  uint32_t n = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) n += __popc(mask[j]);
+  if (!n) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(&bq.cnt, n);
+  base = __shfl_sync(FULL, base, 0);
+  const uint32_t first = max(base, kCap);  // slots from here on overflow to the global queue
+  uint32_t gb = 0;
+  if (base + n > first) {
+    if (lane == 0) gb = atomicAdd(gcnt, base + n - first);
+    gb = __shfl_sync(FULL, gb, 0);
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if ((mask[j] >> lane) & 1u) {
+      const uint32_t slot = base + __popc(mask[j] & vxb::lanemask_lt());
+      if (slot < kCap) bq.items[slot] = v[j];
+      else gq[gb + (slot - first)] = v[j];
+    }
+    base += __popc(mask[j]);
   }
 }
 
 // Block-uniform: moves the buffered entries to the global queue.
-__device__ __forceinline__ void bq_flush(BlockQueue& bq, uint32_t* gcnt, uint32_t* gq, uint32_t gbase0 = 0u) {
+template <uint32_t kCap>
+__device__ __forceinline__ void bq_flush(BlockQueueOf<kCap>& bq, uint32_t* gcnt, uint32_t* gq, uint32_t gbase0 = 0u) {
   __syncthreads();
-  const uint32_t n = min(bq.cnt, kBlockQueueCap);
+  const uint32_t n = min(bq.cnt, kCap);
   if (threadIdx.x == 0) bq.gbase = n ? atomicAdd(gcnt, n) : 0u;
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) gq[(bq.gbase - gbase0) + i] = bq.items[i];

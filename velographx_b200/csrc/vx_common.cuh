@@ -158,7 +158,12 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* a, uint32_t 
 constexpr uint32_t kBarrierWords = 32;
 constexpr uint32_t kBarrierSpinLimit = 1u << 22;
 
-__device__ __forceinline__ void grid_barrier(uint32_t* bar, uint32_t nblocks, uint32_t* err) {
+// Thread 0 of each block runs after() between the wait and the block's release:
+// words the whole block needs next are loaded there once and handed on in
+// shared memory (every warp loading them by itself is thousands of requests
+// for one line, which its L2 slice serves one after another).
+template <class F>
+__device__ __forceinline__ void grid_barrier_then(uint32_t* bar, uint32_t nblocks, uint32_t* err, F&& after) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const uint32_t inc = blockIdx.x == 0 ? 0x80000000u - (nblocks - 1u) : 1u;
@@ -174,8 +179,13 @@ __device__ __forceinline__ void grid_barrier(uint32_t* bar, uint32_t nblocks, ui
       if (spins > 64) __nanosleep(spins < 1024 ? 32 : 256);
     }
     __threadfence();
+    after();
   }
   __syncthreads();
+}
+
+__device__ __forceinline__ void grid_barrier(uint32_t* bar, uint32_t nblocks, uint32_t* err) {
+  grid_barrier_then(bar, nblocks, err, [] {});
 }
 
 }  // namespace vxb
