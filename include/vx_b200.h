@@ -266,7 +266,7 @@ int vx_bfs_window_trace(vx_bfs* b, uint64_t* out, size_t cap, size_t* n);
  * value.  No reference counterpart. */
 int vx_bfs_set_window_pull_fraction(vx_bfs* b, float frac);
 /* Time budget of the repair phases, in multiples of the last full BFS's time
- * (default 1): a deletion cascade that runs longer hands over to a BFS of the
+ * plus 0.1 ms (default 1): a deletion cascade that runs longer hands over to a BFS of the
  * graph without the batch's deletions (the affected set is the vertices
  * whose distance it raises), a relaxation that runs longer to a full BFS of
  * the post-batch graph; 0 hands over at a phase's first work-ring round, a

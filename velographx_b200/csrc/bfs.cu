@@ -21,6 +21,7 @@
 //              relaxation from them and from the heads of inserted arcs.
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -98,20 +99,24 @@ constexpr uint32_t kTraceLevels = 256;
 // Time budgets of the repair phases.  On a deep graph one batch can move the
 // distances of millions of vertices, and the cascade or the relaxation then
 // walks them level by level, for far longer than a full BFS takes.  A phase
-// that has run longer than handover x the last full BFS's time (as it would
-// be inside the launch) drops the rest of its queue and a BFS finishes its work, so a batch costs at most about
+// that has run longer than handover x (the last full BFS's time + 0.1 ms) drops the rest of its queue and a BFS finishes its work, so a batch costs at most about
 // twice the cheaper of the two; either way the result is the same.  The
 // deadline is set by thread 0 before the barrier that precedes the phase's
 // drain, which reads it once and compares it with the clock every round.  The cascade's BFS compares distances over every vertex of the
 // phase graph, so it may hand over only when the distance vector spans it.
 constexpr unsigned long long kNever = ~0ull;
+// What handing over costs beside the BFS (clearing, the comparison pass,
+// barriers, the launch's smaller blocks): without it 100,000-op batches at
+// R-MAT 20, whose cascades take 110 us against a BFS of 70, hand over and take
+// 280.
+constexpr double kHandoverNs = 100e3;
 
 __device__ __forceinline__ void set_deadline(const Params& p) {
   const float h = p.handover;
   const unsigned long long f = p.c->full_ns;
   p.c->deadline = h < 0.0f || (h > 0.0f && f == 0ull)
                       ? kNever
-                      : globaltimer() + (unsigned long long)((double)h * (double)f);
+                      : globaltimer() + (unsigned long long)((double)h * ((double)f + kHandoverNs));
 }
 
 __device__ __forceinline__ void acct_add(const Params& p, int k, unsigned long long v) {
@@ -128,14 +133,16 @@ __device__ __forceinline__ bool sync_grid(const Params& p) {
 
 
 // The row bounds of u; the delta row is read only where the graph may hold
-// one (a loaded or compacted graph has none, and the load is one more random
-// 32-byte sector per vertex).
+// one (a loaded or compacted graph has none) and the row's dirty bit is set
+// (every delta row's is): the table is one more random 32-byte sector per
+// vertex, the bits stay in L2.  The bits are read past L1, which may hold them
+// as they were before the launch's own insertions.
 __device__ __forceinline__ void row_of(const Params& p, const DevAdj& a, uint32_t u, uint64_t& b, uint32_t& nb,
                                        uint2& dr) {
   uint64_t e;
   vxb::base_range(a, u, b, e);
   nb = (uint32_t)(e - b);
-  dr = p.deltas ? a.drow[u] : make_uint2(0u, 0u);
+  dr = p.deltas && (ld_cg(&a.dirty[u >> 5]) >> (u & 31)) & 1u ? a.drow[u] : make_uint2(0u, 0u);
 }
 
 __device__ __forceinline__ uint32_t row_len(const Params& p, const DevAdj& a, uint32_t u) {
@@ -1003,12 +1010,11 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     c->reachable = reached;
     c->levels = level;
     c->arcs = m_visited;
-    // for the repair phases' time budget: what a full BFS takes inside an update
-    // launch, by the measure of the kernel's own time (its 512 threads per SM take
-    // 1.2 to 1.45 times as long at R-MAT 20 to 22 and on the lattice, and the
-    // handover adds a few passes)
+    // for the repair phases' time budget: the kernel's time (inside an update
+    // launch, 512 threads per SM take 1.2 to 1.45 times as long at R-MAT 20 to 22
+    // and on the lattice)
     const unsigned long long t = globaltimer() - t_start;
-    c->full_ns = kInRepair ? t : t + t / 2 + 20000ull;
+    c->full_ns = kInRepair ? t - t / 4 : t;
     if (trace && level < kTraceLevels) {
       trace[2 * level] = globaltimer();
       trace[2 * level + 1] = 0;
@@ -1161,6 +1167,40 @@ __device__ void block_rows(const DevAdj& a, const T* items, uint32_t n, LbStage&
   __syncthreads();  // st is reused by the next call
 }
 
+// The words a repair phase decides by, as of the last grid barrier.
+struct RepairWords {
+  unsigned long long deadline;
+  uint32_t failed, touched, affected, fallback, cbig, rbig, tail, big_b, multi_rm;
+};
+
+// Grid barrier of the repair phases: thread 0 of each block loads the words
+// above once, all in flight together (each phase loading what it needs in
+// every thread cost a dependent round trip per word and thousands of requests
+// for one line).  False once any block recorded a device error.
+__device__ __forceinline__ bool sync_words(const Params& p, RepairWords& w) {
+  BfsCounters* c = p.c;
+  vxb::grid_barrier_then(p.bar, p.nblocks, &c->err, [&] {
+    RepairWords r;
+    r.failed = __ldcg(&c->err);
+    r.touched = ld_cg(&c->touched_n);
+    r.affected = ld_cg(&c->a_n);
+    r.fallback = ld_cg(&c->fallback);
+    r.cbig = ld_cg(&c->cbig);
+    r.rbig = ld_cg(&c->rbig);
+    r.tail = ld_cg(p.rq_tail);
+    r.big_b = ld_cg(&c->big_b);
+    r.multi_rm = ld_cg(&c->multi_rm);
+    r.deadline = __ldcg(&c->deadline);
+    w = r;
+  });
+  return w.failed == 0u;
+}
+
+// Warps (threads) numbered across the blocks first, so that a few items spread
+// over every SM.
+__device__ __forceinline__ uint32_t dealt_warp() { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
+__device__ __forceinline__ uint32_t dealt_thread() { return threadIdx.x * gridDim.x + blockIdx.x; }
+
 // Shared memory of one block for the repair phases.
 struct RepairSmem {
   unsigned long long items[kThreads];  // claimed ring items
@@ -1171,16 +1211,17 @@ struct RepairSmem {
   uint32_t g0, n, stop, nsv, nex, fallback;
   uint32_t late;     // the round started past the phase's deadline (its items are dropped)
   uint32_t flagged;  // this block has raised the phase's handover flag
+  RepairWords w;     // kept across a BFS in the memory before it
 };
 
 // The full BFS inside a repair kernel, in the shared memory its phases do not
 // hold at that point.
-__device__ void bfs_in_repair(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t* dist,
+__device__ __noinline__ void bfs_in_repair(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t* dist,
                               unsigned long long* trace) {
   using Stage = BuStage<kThreads, 1>;
   static_assert(sizeof(Stage) <= sizeof(LbStage) && alignof(LbStage) >= alignof(Stage), "the two share memory");
-  full_bfs<true>(p, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm), (uint32_t)(sizeof(sm) / 4), dist,
-           trace);
+  full_bfs<true>(p, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm),
+                 (uint32_t)(offsetof(RepairSmem, w) / 4), dist, trace);
 }
 
 // Drains the ring; W::process(sm, n) handles sm.items[0, n) block-uniformly,
@@ -1406,7 +1447,11 @@ __device__ __forceinline__ bool find_parent(const Params& p, const DevAdj& a, ui
 // arc that failed once fails again.  In-rows longer than kChunk arcs are
 // scanned in place over their first chunk only; when it holds no witness the
 // rest goes to a chunked pass (chunk_check), and the saved position kChunk
-// tells later checks to go straight to a new pass.
+// tells later checks to go straight to a new pass.  A candidate's first check
+// (kFirst) answers no request and starts at position 0: nothing relies on it
+// clearing the request bit, and neither that nor the saved state is a round
+// trip of its chain.
+template <bool kFirst>
 __device__ void check_vertex(const Params& p, uint32_t x) {
   const DevAdj& a = p.g.in;
   const int lane = threadIdx.x & 31;
@@ -1416,12 +1461,14 @@ __device__ void check_vertex(const Params& p, uint32_t x) {
   uint64_t b, e;
   vxb::base_range(a, x, b, e);
   const uint2 dr = a.drow[x];
-  if (lane == 0) atomicAnd(&p.inq[1][x >> 5], ~(1u << (x & 31)));
-  __syncwarp();
-  __threadfence();  // the request bit is clear before the state (witness, affected bits) is read
+  if (!kFirst) {
+    if (lane == 0) atomicAnd(&p.inq[1][x >> 5], ~(1u << (x & 31)));
+    __syncwarp();
+    __threadfence();  // the request bit is clear before the state (witness, affected bits) is read
+  }
   const uint32_t nb = (uint32_t)(e - b), total = nb + dr.y;
   const uint32_t lim = min(total, kChunk);
-  uint32_t k0 = (uint32_t)__ldcg(&p.sw[x]);
+  uint32_t k0 = kFirst ? 0u : (uint32_t)__ldcg(&p.sw[x]);
   bool resolved = false;
   uint32_t kw = 0, yw = 0;
   while (k0 < lim && !resolved) {
@@ -1579,7 +1626,7 @@ struct Cascade {
     const uint32_t nsv = sm.nsv, nex = sm.nex;
     for (uint32_t i = t >> 5; i < nsv; i += kThreads / 32) {
       if (sm.cnt[i]) chunk_check(P, sm.sv[i], sm.cnt[i] - 1);
-      else check_vertex(P, sm.sv[i]);
+      else check_vertex<false>(P, sm.sv[i]);
     }
     if (nex) {
       if (t < nex) sm.d[t] = P.dist[item_vertex(sm.ex[t])];
@@ -1636,7 +1683,7 @@ __device__ void register_candidates(const Params& p) {
   }
 }
 
-__device__ void clear_workspace(const Params& p);
+__device__ void clear_workspace(const Params& p, uint32_t touched, uint32_t affected);
 
 // The cascade past its time budget (a cut near the root of a deep graph
 // leaves millions of vertices affected, and the cascade walks them level by
@@ -1651,9 +1698,9 @@ __device__ void clear_workspace(const Params& p);
 // affected list stays empty, so the post-batch repair only relaxes the
 // insertions.  The BFS distances go to tent (zero between phases), which the
 // comparison pass zeroes again.
-__device__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
+__device__ __noinline__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
   BfsCounters* c = p.c;
-  clear_workspace(p);
+  clear_workspace(p, sm.w.touched, sm.w.affected);
   reset_ring(p);
   if (!sync_grid(p)) return false;
   unsigned long long arcs = 0;
@@ -1697,19 +1744,19 @@ __device__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, BlockQueue& bq, 
 // batch's affected count.
 __device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t ncand) {
   if (gtid() == 0) set_deadline(p);
-  for (uint32_t i = gwarp(); i < ncand; i += nwarps()) check_vertex(p, p.lst_t[i]);
-  if (!sync_grid(p)) return false;
-  if (ld_cg(p.rq_tail)) {
+  for (uint32_t i = dealt_warp(); i < ncand; i += nwarps()) check_vertex<true>(p, p.lst_t[i]);
+  if (!sync_words(p, sm.w)) return false;
+  if (sm.w.tail) {
     Cascade w{&p, &lb};
-    drain(p, sm, w, p.cascade_bfs ? __ldcg(&p.c->deadline) : kNever);
-    if (!sync_grid(p)) return false;
+    drain(p, sm, w, p.cascade_bfs ? sm.w.deadline : kNever);
+    if (!sync_words(p, sm.w)) return false;
   }
   if (gtid() == 0) {  // the drain statistics of the phase trace
-    p.c->rtrace[7] = ld_cg(p.rq_tail);
+    p.c->rtrace[7] = sm.w.tail;
     for (int k = 0; k < 6; ++k) p.c->rtrace[9 + k] = __ldcg(&p.rq_stat[k]);
   }
-  if (ld_cg(&p.c->cbig)) return cascade_by_bfs(p, sm, bq, lb);
-  if (gtid() == 0) p.c->affected = ld_cg(&p.c->a_n);
+  if (sm.w.cbig) return cascade_by_bfs(p, sm, bq, lb);
+  if (gtid() == 0) p.c->affected = sm.w.affected;
   return true;
 }
 
@@ -1731,8 +1778,7 @@ __device__ void repair_pre(const Params& p, RepairSmem& sm, LbStage& lb, BlockQu
 
 // -------------------------------------------------- post-batch repair --
 
-__device__ void clear_workspace(const Params& p) {
-  const uint32_t nt = ld_cg(&p.c->touched_n), na = ld_cg(&p.c->a_n);
+__device__ void clear_workspace(const Params& p, uint32_t nt, uint32_t na) {
   for (uint32_t i = gtid(); i < nt; i += nthreads()) {
     p.sw[p.lst_t[i]] = 0ull;
     p.tent[p.lst_t[i]] = 0u;  // chunk counts left by a pass the fallback dropped
@@ -1785,17 +1831,18 @@ __device__ void seed_relax(const Params& p, bool lowered, uint32_t v, long long&
       queue = true;
     } else {
       acct_add(p, 0, deg);
+      // the row's columns, then their labels, are in flight together
       const uint32_t dv = ld_cg(&p.dist[v]);
-      for (uint32_t k = 0; k < deg; ++k) {
-        uint32_t x;
-        if (k < e - b) {
-          x = a.col[b + k];
-          if (x & kTomb) continue;
-        } else {
-          x = a.darena[dr.x + (k - (uint32_t)(e - b))];
-        }
-        if (x < p.dist_len && lower(p, x, dv + 1, reach)) push_one(p, x);
-      }
+      uint32_t x[kInlineRelax], dx[kInlineRelax];
+#pragma unroll
+      for (uint32_t k = 0; k < kInlineRelax; ++k)
+        x[k] = k < e - b ? a.col[b + k] : k < deg ? a.darena[dr.x + (k - (uint32_t)(e - b))] : kTomb;
+#pragma unroll
+      for (uint32_t k = 0; k < kInlineRelax; ++k)
+        dx[k] = !(x[k] & kTomb) && x[k] < p.dist_len ? ld_cg(&p.dist[x[k]]) : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < kInlineRelax; ++k)
+        if (dx[k] > dv + 1 && lower(p, x[k], dv + 1, reach)) push_one(p, x[k]);
     }
   }
   lower_and_push(p, queue, v);
@@ -1880,6 +1927,51 @@ __device__ void boundary_seeds(const Params& p, RepairSmem& sm, LbStage& lb, uin
   }
 }
 
+// A few affected vertices (no more than the grid has warps): a warp each, no
+// block barriers; the blocks' last warps take them first, so that the inserted
+// arcs' seeds, which the first ones take, run beside them.
+__device__ void boundary_seeds_few(const Params& p, uint32_t na, long long& reach) {
+  const DevAdj& a = p.g.in;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t i = (blockDim.x / 32 - 1 - (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
+  if (i >= na) return;
+  const uint32_t v = p.lst_a[i];
+  uint64_t b, e;
+  vxb::base_range(a, v, b, e);
+  const uint2 dr = a.drow[v];
+  const uint32_t nb = (uint32_t)(e - b), total = nb + dr.y;
+  if (total > kBigBoundary) {
+    if (lane == 0) {
+      p.tent[i] = kUnreachable;
+      p.big[atomicAdd(&p.c->big_b, 1u)] = i;
+    }
+    return;
+  }
+  if (lane == 0) acct_add(p, 0, total);
+  uint32_t best = kUnreachable;
+  for (uint32_t k0 = 0; k0 < total; k0 += 128) {
+    uint32_t x[4], dx[4], aw[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t k = k0 + 32 * j + lane;
+      x[j] = k < nb ? a.col[b + k] : k < total ? a.darena[dr.x + (k - nb)] : kTomb;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool live = !(x[j] & kTomb) && x[j] < p.dist_len;
+      dx[j] = live ? p.dist[x[j]] : kUnreachable;
+      aw[j] = live ? p.aff[x[j] >> 5] : FULL;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (dx[j] != kUnreachable && !((aw[j] >> (x[j] & 31)) & 1u)) best = min(best, dx[j] + 1);
+  }
+  best = __reduce_min_sync(FULL, best);
+  bool seed = false;
+  if (lane == 0 && best != kUnreachable) seed = lower(p, v, best, reach);
+  seed_relax(p, seed, v, reach);
+}
+
 // Boundary distances of the hub entries p.big[0, nb) (indices into lst_a):
 // each hub gets its own group of nwarps / nb warps (at least one), which fold
 // 32-arc slices of its row into p.tent[i] by atomicMin, so many hubs are
@@ -1920,6 +2012,17 @@ __device__ void grid_boundary_min(const Params& p, uint32_t nb) {
 // The post-batch repair proper (everything but the fallback); true when the
 // batch's distances are to come from a full BFS of the post-batch graph
 // instead (the relaxation passed its budget), with the workspace cleared.
+// kInvalidated: the caller invalidated the affected vertices (invalidate) and
+// sm.w holds the words of the barrier after that.
+__device__ __forceinline__ void invalidate(const Params& p, uint32_t na) {
+  for (uint32_t i = dealt_thread(); i < na; i += nthreads()) p.dist[p.lst_a[i]] = kUnreachable;
+  if (gtid() == 0 && na) {
+    reach_add(p, -(long long)na);
+    p.c->big_b = 0;
+  }
+}
+
+template <bool kInvalidated>
 __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
   BfsCounters* c = p.c;
   const int lane = threadIdx.x & 31;
@@ -1928,24 +2031,22 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
   // kernel or a kernel boundary
   stamp(p, 3);
   if (gtid() == 0) set_deadline(p);
-  const uint32_t na = ld_cg(&c->a_n);
+  const uint32_t na = kInvalidated ? sm.w.affected : ld_cg(&c->a_n);
   if (gtid() == 0) acct_add(p, 1, na);  // invalidated and re-seeded
   long long reach = 0;
   if (na > 0) {
-    // invalidate the affected vertices (repair_affected, bfs.hpp:272-283)
-    for (uint32_t i = gtid(); i < na; i += nthreads()) p.dist[p.lst_a[i]] = kUnreachable;
-    if (gtid() == 0) {
-      reach_add(p, -(long long)na);
-      c->big_b = 0;
+    if (!kInvalidated) {  // the affected vertices (repair_affected, bfs.hpp:272-283)
+      invalidate(p, na);
+      if (!sync_words(p, sm.w)) return false;
     }
-    if (!sync_grid(p)) return false;
     stamp(p, 4);
-    boundary_seeds(p, sm, lb, na, reach);
+    if (na <= nwarps()) boundary_seeds_few(p, na, reach);
+    else boundary_seeds(p, sm, lb, na, reach);
   }
   // inserted arcs relax their heads (bfs.hpp:91-96)
   const uint32_t F = *p.F;
-  for (uint32_t base = gwarp() * 32; base < F; base += nwarps() * 32) {
-    const uint32_t i = base + lane;
+  for (uint32_t base = (dealt_thread() - lane * gridDim.x); base < F; base += nthreads()) {
+    const uint32_t i = base + lane * gridDim.x;
     bool lowered = false;
     uint32_t v = 0;
     if (i < F && (p.ff[i] & kFAdd)) {
@@ -1958,11 +2059,11 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
     }
     seed_relax(p, lowered, v, reach);
   }
-  if (!sync_grid(p)) return false;
-  const uint32_t nbig = na ? ld_cg(&c->big_b) : 0u;
+  if (!sync_words(p, sm.w)) return false;
+  const uint32_t nbig = na ? sm.w.big_b : 0u;
   if (nbig) {
     grid_boundary_min(p, nbig);
-    if (!sync_grid(p)) return false;
+    if (!sync_words(p, sm.w)) return false;
     for (uint32_t base = gwarp() * 32; base < nbig; base += nwarps() * 32) {
       const uint32_t r = base + lane;
       bool seed = false;
@@ -1976,41 +2077,46 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
       }
       seed_relax(p, seed, v, reach);
     }
-    if (!sync_grid(p)) return false;
+    if (!sync_words(p, sm.w)) return false;
   }
   stamp(p, 5);
-  if (ld_cg(p.rq_tail)) {  // the relaxation runs only when a seed left work queued
+  if (sm.w.tail) {  // the relaxation runs only when a seed left work queued
     Relax w{&p, &lb, &reach};
-    drain(p, sm, w, __ldcg(&p.c->deadline));
-    if (!sync_grid(p)) return false;
-    if (ld_cg(&c->rbig)) {
+    drain(p, sm, w, sm.w.deadline);
+    if (!sync_words(p, sm.w)) return false;
+    if (sm.w.rbig) {
       // the relaxation passed its budget: a full BFS of the post-batch graph
       // gives the distances and the reachable count (the repair's counters
       // -- candidates, affected, no full recompute -- stand)
-      clear_workspace(p);
+      clear_workspace(p, sm.w.touched, sm.w.affected);
       reset_ring(p);
       return true;
     }
   }
   stamp(p, 6);
   if (gtid() == 0) {
-    c->rtrace[8] = ld_cg(p.rq_tail);
+    c->rtrace[8] = sm.w.tail;
     for (int k = 0; k < 6; ++k) c->rtrace[15 + k] = __ldcg(&p.rq_stat[k]);
   }
   reach = vxb::warp_sum(reach);
   if (lane == 0) reach_add(p, reach);
-  clear_workspace(p);
+  clear_workspace(p, sm.w.touched, sm.w.affected);
   reset_ring(p);
   return false;
 }
 
 // Post-batch repair (bfs.hpp:72-97): the fallback's full BFS or the repair,
 // which may itself hand over to a full BFS; one call site serves both.
+template <bool kInvalidated>
 __device__ void repair_post(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
-  const bool fallback = ld_cg(&c->fallback) != 0u;
-  if (fallback) clear_workspace(p);
-  else if (!repair_relax(p, sm, lb)) return;
+  const bool fallback = kInvalidated ? sm.w.fallback != 0u : ld_cg(&c->fallback) != 0u;
+  if (fallback) {
+    if (kInvalidated) clear_workspace(p, sm.w.touched, sm.w.affected);
+    else clear_workspace(p, ld_cg(&c->touched_n), ld_cg(&c->a_n));
+  } else if (!repair_relax<kInvalidated>(p, sm, lb)) {
+    return;
+  }
   if (!sync_grid(p)) return;
   bfs_in_repair(p, sm, lb, bq, p.dist, p.trace);
   if (gtid() == 0) {
@@ -2035,18 +2141,20 @@ __device__ void repair_post(const Params& p, RepairSmem& sm, LbStage& lb, BlockQ
 // per-batch counters make every batch checkable.
 
 struct StreamArgs {
-  const uint32_t* fu;        // canonical arcs of the stream, batch-major
-  const uint32_t* fv;
-  uint8_t* ff;               // in: desired state (bit 0); out: classification flags
-  uint64_t* fpos;
-  const uint32_t* boff;      // nb + 1 offsets of the batches' arcs
-  const uint32_t* bcnt;      // nb arc counts
+  // canonical arcs of the stream, batch-major: [0] of the out-adjacency, sorted
+  // by (u, v); [1] of a directed graph's in-adjacency, the same arcs as (v, u)
+  const uint32_t* fu[2];
+  const uint32_t* fv[2];
+  uint8_t* ff[2];            // in: desired state (bit 0); out: classification flags
+  uint64_t* fpos[2];
+  const uint32_t* cnt[2];    // arc counts: nb of them for [0], one for [1]
+  uint32_t* scratch[2];      // one batch's arcs: the insertions of each row run
+  const uint32_t* boff;      // nb + 1 offsets of the batches' arcs (null: one batch)
   const uint32_t* vpost;     // vertex count after each batch
-  uint32_t* scratch;         // one batch's arcs: the insertions of each row run
   unsigned long long* digest;  // nb digests of the distances (optional)
   uint32_t* bstats;          // nb x 4: candidates, affected, full recompute, reachable (optional)
   GraphCounters* gc;
-  unsigned long long arena_cap;
+  unsigned long long arena_cap[2];
   double frac;
   uint32_t nb, V0, len0;
   uint32_t v_single;    // vertex count after the batch when vpost is null (one staged batch)
@@ -2081,8 +2189,8 @@ __device__ __forceinline__ bool delta_op(uint8_t f, bool insertion) {
 // Delta removals of one row run (whole warp): the row's sorted delta list
 // keeps every entry that is not a removal of the run (delta_remove_kernel of
 // the per-batch path, on the canonical arcs directly).
-__device__ void run_remove(const vxb::DevAdj& a, const uint32_t* fv, const uint8_t* ff, uint32_t s, uint32_t e, uint32_t u,
-                           GraphCounters* gc, unsigned long long* acct) {
+__device__ void run_remove(const vxb::DevAdj& a, int dir, const uint32_t* fv, const uint8_t* ff, uint32_t s, uint32_t e,
+                           uint32_t u, GraphCounters* gc, unsigned long long* acct) {
   const int lane = threadIdx.x & 31;
   bool any = false;
   for (uint32_t k = s + lane; k < e; k += 32) any |= delta_op(ff[k], false);
@@ -2109,8 +2217,8 @@ __device__ void run_remove(const vxb::DevAdj& a, const uint32_t* fv, const uint8
   if (lane == 0) {
     a.drow[u].y = written;
     if (acct) atomicAdd(acct, (unsigned long long)(row.y + written));
-    atomicAdd(&gc->delta_live[0], (unsigned long long)(-(long long)(row.y - written)));
-    gdev::mark_dirty(a.dirty, u, &gc->dirty_rows[0]);
+    atomicAdd(&gc->delta_live[dir], (unsigned long long)(-(long long)(row.y - written)));
+    gdev::mark_dirty(a.dirty, u, &gc->dirty_rows[dir]);
   }
 }
 
@@ -2118,8 +2226,8 @@ __device__ void run_remove(const vxb::DevAdj& a, const uint32_t* fv, const uint8
 // compacted into scratch[s, s + nB) and merged into the row's delta list, in
 // place when its block has room, else into a new power-of-two arena block
 // (delta_insert_kernel of the per-batch path).
-__device__ void run_insert(const vxb::DevAdj& a, const uint32_t* fv, const uint8_t* ff, uint32_t* scratch, uint32_t s,
-                           uint32_t e, uint32_t u, GraphCounters* gc, unsigned long long arena_cap,
+__device__ void run_insert(const vxb::DevAdj& a, int dir, const uint32_t* fv, const uint8_t* ff, uint32_t* scratch,
+                           uint32_t s, uint32_t e, uint32_t u, GraphCounters* gc, unsigned long long arena_cap,
                            unsigned long long* acct) {
   const int lane = threadIdx.x & 31;
   uint32_t nB = 0;
@@ -2142,7 +2250,7 @@ __device__ void run_insert(const vxb::DevAdj& a, const uint32_t* fv, const uint8
     uint32_t ncap = 8;
     while (ncap < cnew) ncap <<= 1;
     unsigned long long off = 0;
-    if (lane == 0) off = atomicAdd(&gc->arena_top[0], (unsigned long long)ncap);
+    if (lane == 0) off = atomicAdd(&gc->arena_top[dir], (unsigned long long)ncap);
     off = __shfl_sync(FULL, off, 0);
     if (off + ncap > arena_cap) {
       if (lane == 0) atomicOr(&gc->err, vxb::kErrArenaOverflow);
@@ -2155,47 +2263,294 @@ __device__ void run_insert(const vxb::DevAdj& a, const uint32_t* fv, const uint8
     }
   }
   if (lane == 0) {
-    atomicAdd(&gc->delta_live[0], (unsigned long long)nB);
+    atomicAdd(&gc->delta_live[dir], (unsigned long long)nB);
     if (acct) atomicAdd(acct, (unsigned long long)(row.y + cnew));
-    gdev::mark_dirty(a.dirty, u, &gc->dirty_rows[0]);
+    gdev::mark_dirty(a.dirty, u, &gc->dirty_rows[dir]);
   }
 }
 
-// The row runs of the batch's canonical arcs [0, F): delta removals
-// (kInsert false) or insertions (true).  A run of one arc whose delta row
-// holds at most 7 arcs (8 for a removal) -- most runs of a batch -- is done by
-// one lane: the row's block (capacity >= 8, 8-aligned in the arena) is loaded
-// as two 16-byte words, edited in registers and stored back; a row without a
-// block gets 8 slots from one warp-aggregated arena allocation.  The other
-// runs are queued in shared memory and done by the block's warps (run_insert,
-// run_remove).  Arcs are dealt round-robin (arc i to block i mod gridDim), so
-// a small batch still spreads over every block.  Block-uniform.
-template <bool kInsert>
-__device__ void commit_runs(const Params& p, const StreamArgs& s, uint32_t off, uint32_t F, RepairSmem& sm) {
-  const vxb::DevAdj& a = p.g.out;
-  const uint32_t* fu = s.fu + off;
-  const uint32_t* fv = s.fv + off;
-  const uint8_t* ff = s.ff + off;
-  const int lane = threadIdx.x & 31;
-  const uint32_t per_round = gridDim.x * kThreads;
-  for (uint32_t r0 = 0; r0 < F; r0 += per_round) {
+// ---- the commit's two passes over the canonical arcs ----
+//
+// Removals first (before the cascade reads the rows), insertions after it.
+// Arcs of one row are consecutive (a run) and only they touch that row, so
+// whoever takes an arc that is a run by itself -- most of a batch -- classifies
+// it, tombstones it or edits its delta row and registers it as a deletion
+// candidate in one go.  Delta removals of longer runs need the whole run's
+// classification: they are left to a second pass behind a grid barrier, which
+// a batch without any skips.  On a delta row of at most 7 arcs (8 for a removal)
+// one lane does a single arc: the row's block (capacity >= 8, 8-aligned in the
+// arena) is loaded as two 16-byte words, edited in registers and stored back; a
+// row without a block gets 8 slots from one warp-aggregated arena allocation.
+// The rest is queued in shared memory and done by the block's warps (run_insert,
+// run_remove).  Arcs are dealt round-robin (arc i to block i mod gridDim), so a
+// small batch still spreads over every block.
+
+// Position of x in the sorted a[lo, hi), compared by the low 31 bits, or hi
+// where it is missing; whole warp: 32 pivots per round trip.
+__device__ __forceinline__ uint64_t warp_find(const uint32_t* a, uint64_t lo, uint64_t hi, uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t end = hi;
+  while (hi - lo > 32) {
+    const uint64_t step = (hi - lo + 31) / 32;
+    const uint64_t k = lo + step * (lane + 1) - 1;  // last entry of this lane's part
+    const bool below = k < hi && (a[k] & kIdMask) < x;
+    const uint32_t n = __popc(__ballot_sync(FULL, below));  // parts before the one that may hold x
+    lo += step * n;
+    if (lo >= hi) return end;
+    hi = hi < lo + step ? hi : lo + step;
+  }
+  const bool hit = lo + lane < hi && (a[lo + lane] & kIdMask) == x;
+  const uint32_t m = __ballot_sync(FULL, hit);
+  return m ? lo + (uint32_t)(__ffs(m) - 1) : end;
+}
+
+struct ArcWork {
+  const Params* p;
+  const StreamArgs* s;
+  const vxb::DevAdj* a;
+  int dir;
+  const uint32_t* fu;  // the batch's arcs
+  const uint32_t* fv;
+  uint8_t* ff;
+  uint64_t* fpos;
+  uint32_t F;
+  long long tombs;     // this lane's change of the tombstone count, and rows it dirtied
+  uint32_t dirtied;
+
+  // A deletion candidate (bfs.hpp:52-63) is the head of a deleted
+  // shortest-parent arc; its first touch records it in the touched list, whose
+  // length after the pass is their number.  Warp-uniform.
+  __device__ __forceinline__ void candidate(bool arc, uint32_t u, uint32_t v, uint8_t f) {
+    if (dir) return;
+    bool first = false;
+    if (arc && !(f & kFAdd) && (f & kFCur) && is_sp(*p, u, v))
+      first = !(atomicOr(&p->sw[v], kSwTouched) & kSwTouched);
+    const uint32_t slot = vxb::warp_append(first, &p->c->touched_n);
+    if (first) p->lst_t[slot] = v;
+  }
+
+  // Whether arc i's row has other arcs in the batch.
+  __device__ __forceinline__ bool in_run(uint32_t i, uint32_t u) const {
+    return (i > 0 && fu[i - 1] == u) || (i + 1 < F && fu[i + 1] == u);
+  }
+
+  // The delta removals of run [st, ...), classified before; whole warp.
+  __device__ void remove_run(uint32_t st) {
+    run_remove(*a, dir, fv, ff, st, run_end(fu, st, F), fu[st], s->gc, p->acct ? p->acct + 2 : nullptr);
+  }
+
+  // The sums of the pass into the graph's counters.
+  __device__ __forceinline__ void flush() {
+    tombs = vxb::warp_sum(tombs);
+    dirtied = vxb::warp_sum(dirtied);
+    if ((threadIdx.x & 31) == 0 && tombs) atomicAdd(&s->gc->tombs[dir], (unsigned long long)tombs);
+    if ((threadIdx.x & 31) == 0 && dirtied) atomicAdd(&s->gc->dirty_rows[dir], (unsigned long long)dirtied);
+    tombs = 0;
+    dirtied = 0;
+  }
+};
+
+// A delta row of at most 8 arcs in registers: its block's 8 slots.
+struct SmallRow {
+  uint32_t x[8];
+  __device__ __forceinline__ void load(const uint32_t* block) {
+    const uint4* q = reinterpret_cast<const uint4*>(block);
+    const uint4 q0 = q[0], q1 = q[1];
+    x[0] = q0.x, x[1] = q0.y, x[2] = q0.z, x[3] = q0.w;
+    x[4] = q1.x, x[5] = q1.y, x[6] = q1.z, x[7] = q1.w;
+  }
+  __device__ __forceinline__ uint32_t below(uint32_t n, uint32_t v) const {  // entries < v among the first n
+    uint32_t k = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) k += (j < n && x[j] < v) ? 1u : 0u;
+    return k;
+  }
+  __device__ __forceinline__ bool holds(uint32_t n, uint32_t v) const {
+    bool h = false;
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) h = h || (j < n && x[j] == v);
+    return h;
+  }
+};
+
+// The removal pass.  A batch of few arcs takes a warp per arc: its row searches
+// read 32 pivots per round trip instead of 7, and the chain of such a batch is
+// its longest row's.  With the classification, the removals and the candidates
+// in three passes and two barriers 950 arcs at R-MAT 20 took 20 us, now 7 to 8;
+// 20,000 arcs at R-MAT 22 22 us, now 15.  Block-uniform.
+__device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
+  const Params& p = *w.p;
+  const vxb::DevAdj& a = *w.a;
+  const uint32_t lane = threadIdx.x & 31;
+  bool multi = false;  // a delta removal left to removal_runs
+  if (w.F <= 2 * nwarps()) {
+    for (uint32_t i = dealt_warp(); i < w.F; i += nwarps()) {
+      const uint32_t u = w.fu[i], v = w.fv[i];
+      uint8_t f = w.ff[i];
+      uint64_t b, e;
+      vxb::base_range(a, u, b, e);
+      const uint2 row = a.drow[u];
+      const bool small = row.y <= 32u, run = w.in_run(i, u);
+      const uint32_t x = small && lane < row.y ? a.darena[row.x + lane] : 0u;  // in flight with the base search
+      uint64_t q = ~0ull;
+      const uint32_t held = __ballot_sync(FULL, small && lane < row.y && x == v);
+      if (!w.s->classified) {
+        const uint64_t at = warp_find(a.col, b, e, v);
+        bool cur;
+        f &= kFAdd;
+        if (at < e) {
+          f |= kFInBase;
+          cur = !(a.col[at] & kTomb);
+          q = at;
+        } else {
+          cur = small ? held != 0u : warp_find(a.darena, row.x, row.x + row.y, v) < row.x + row.y;
+        }
+        if (cur) f |= kFCur;
+        if (cur != ((f & kFAdd) != 0)) f |= kFChanged;
+        if (lane == 0) {
+          w.ff[i] = f;
+          w.fpos[i] = q;
+        }
+      } else {
+        q = w.fpos[i];
+      }
+      // lane 0 does what is not a search
+      if (lane == 0) w.tombs += gdev::tomb_arc(a, u, f, q, 0, w.dirtied);
+      w.candidate(lane == 0, u, v, f);
+      if (!delta_op(f, false)) continue;
+      if (run) {
+        multi = true;
+      } else if (small) {  // the entries above the arc move down
+        const uint32_t k = (uint32_t)__ffs(held) - 1;
+        if (lane > k && lane < row.y) a.darena[row.x + lane - 1] = x;
+        if (lane == 0) {
+          a.drow[u].y = row.y - 1;
+          atomicAdd(&w.s->gc->delta_live[w.dir], ~0ull);
+          acct_add(p, 2, 2ull * row.y - 1);
+          w.dirtied += gdev::mark_dirty_count(a.dirty, u);
+        }
+      } else {
+        __syncwarp();
+        w.remove_run(i);
+      }
+    }
+  } else {
+    for (uint32_t r0 = 0; r0 < w.F; r0 += nthreads()) {
+      if (threadIdx.x == 0) sm.nsv = 0;
+      __syncthreads();
+      const uint32_t i = r0 + dealt_thread();
+      const bool act = i < w.F;
+      bool queue = false;
+      uint32_t u = 0, v = 0;
+      uint8_t f = 0;
+      long long dlive = 0;
+      if (act) {
+        u = w.fu[i];
+        v = w.fv[i];
+        f = w.ff[i];
+        uint64_t b, e;
+        vxb::base_range(a, u, b, e);
+        const uint2 row = a.drow[u];
+        SmallRow r = {};
+        if (row.y && row.y <= 8u) r.load(a.darena + row.x);  // in flight with the base search
+        uint64_t q = ~0ull;
+        if (!w.s->classified) {
+          const uint64_t at = vxb::lower_bound_masked(a.col, b, e, v);
+          const uint32_t c = at < e ? a.col[at] : kTomb;
+          bool cur;
+          f &= kFAdd;
+          if (at < e && (c & kIdMask) == v) {
+            f |= kFInBase;
+            cur = !(c & kTomb);
+            q = at;
+          } else {
+            cur = row.y <= 8u ? r.holds(row.y, v) : gdev::bsearch_u32(a.darena, row.x, row.x + row.y, v);
+          }
+          if (cur) f |= kFCur;
+          if (cur != ((f & kFAdd) != 0)) f |= kFChanged;
+          w.ff[i] = f;
+          w.fpos[i] = q;
+        } else {
+          q = w.fpos[i];
+        }
+        w.tombs += gdev::tomb_arc(a, u, f, q, 0, w.dirtied);
+        if (delta_op(f, false)) {
+          if (w.in_run(i, u)) {
+            multi = true;
+          } else if (row.y > 8u) {
+            queue = true;
+          } else {
+            const uint32_t pos = r.below(row.y, v);
+            auto out = [&](uint32_t k) { return k < pos ? r.x[k] : r.x[k < 7 ? k + 1 : 7]; };
+            uint4* dst = reinterpret_cast<uint4*>(a.darena + row.x);
+            dst[0] = make_uint4(out(0), out(1), out(2), out(3));
+            dst[1] = make_uint4(out(4), out(5), out(6), out(7));
+            a.drow[u].y = row.y - 1;
+            dlive = -1;
+            acct_add(p, 2, 2ull * row.y - 1);
+            w.dirtied += gdev::mark_dirty_count(a.dirty, u);
+          }
+        }
+      }
+      w.candidate(act, u, v, f);
+      dlive = vxb::warp_sum(dlive);
+      if (lane == 0 && dlive) atomicAdd(&w.s->gc->delta_live[w.dir], (unsigned long long)dlive);
+      if (queue) sm.sv[atomicAdd(&sm.nsv, 1u)] = i;
+      __syncthreads();
+      const uint32_t nq = sm.nsv;
+      for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k]);
+      __syncthreads();  // the list is rebuilt by the next round
+    }
+  }
+  if (__any_sync(FULL, multi) && lane == 0) p.c->multi_rm = 1u;
+  w.flush();
+}
+
+// The second removal pass: delta removals of runs of several arcs, a warp per
+// run.  Block-uniform.
+__device__ void removal_runs(ArcWork& w, RepairSmem& sm) {
+  for (uint32_t r0 = 0; r0 < w.F; r0 += nthreads()) {
     if (threadIdx.x == 0) sm.nsv = 0;
     __syncthreads();
-    const uint32_t i = r0 + threadIdx.x * gridDim.x + blockIdx.x;
+    const uint32_t i = r0 + dealt_thread();
+    if (i + 1 < w.F) {
+      const uint32_t u = w.fu[i];
+      if (w.fu[i + 1] == u && (i == 0 || w.fu[i - 1] != u)) sm.sv[atomicAdd(&sm.nsv, 1u)] = i;
+    }
+    __syncthreads();
+    const uint32_t nq = sm.nsv;
+    for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k]);
+    __syncthreads();  // the list is rebuilt by the next round
+  }
+}
+
+// The insertion pass: tombstoned base arcs the batch re-adds revived, delta
+// insertions made.  Block-uniform.
+__device__ void insertion_pass(ArcWork& w, RepairSmem& sm) {
+  const Params& p = *w.p;
+  const vxb::DevAdj& a = *w.a;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t r0 = 0; r0 < w.F; r0 += nthreads()) {
+    if (threadIdx.x == 0) sm.nsv = 0;
+    __syncthreads();
+    const uint32_t i = r0 + dealt_thread();
     bool job = false, queue = false, need_block = false;
     uint32_t u = 0, v = 0;
     uint2 row = make_uint2(0, 0);
-    if (i < F) {
-      u = fu[i];
-      if (i == 0 || fu[i - 1] != u) {
-        if (i + 1 < F && fu[i + 1] == u) {
+    if (i < w.F) {
+      u = w.fu[i];
+      const uint8_t f = w.ff[i];
+      if ((f & kFInBase) && (f & kFChanged) && (f & kFAdd))
+        w.tombs += gdev::tomb_arc(a, u, f, w.fpos[i], 1, w.dirtied);
+      if (i == 0 || w.fu[i - 1] != u) {
+        if (i + 1 < w.F && w.fu[i + 1] == u) {
           queue = true;  // a run of several arcs
-        } else if (delta_op(ff[i], kInsert)) {
-          v = fv[i];
+        } else if (delta_op(f, true)) {
+          v = w.fv[i];
           row = a.drow[u];
-          if (kInsert ? row.y < 8u : row.y <= 8u) {
+          if (row.y < 8u) {
             job = true;
-            need_block = kInsert && a.dcap[u] == 0u;  // no block yet (then the row is empty)
+            need_block = a.dcap[u] == 0u;  // no block yet (then the row is empty)
           } else {
             queue = true;
           }
@@ -2207,12 +2562,12 @@ __device__ void commit_runs(const Params& p, const StreamArgs& s, uint32_t off, 
     if (nm) {
       const int leader = __ffs(nm) - 1;
       unsigned long long b0 = 0;
-      if (lane == leader) b0 = atomicAdd(&s.gc->arena_top[0], 8ull * (unsigned long long)__popc(nm));
+      if ((int)lane == leader) b0 = atomicAdd(&w.s->gc->arena_top[w.dir], 8ull * (unsigned long long)__popc(nm));
       b0 = __shfl_sync(FULL, b0, leader);
       const unsigned long long o = b0 + 8ull * __popc(nm & vxb::lanemask_lt());
       if (need_block) {
-        if (o + 8 > s.arena_cap) {
-          atomicOr(&s.gc->err, vxb::kErrArenaOverflow);
+        if (o + 8 > w.s->arena_cap[w.dir]) {
+          atomicOr(&w.s->gc->err, vxb::kErrArenaOverflow);
           job = false;
         } else {
           base_off = (uint32_t)o;
@@ -2220,54 +2575,38 @@ __device__ void commit_runs(const Params& p, const StreamArgs& s, uint32_t off, 
       }
     }
     long long dlive = 0;
-    unsigned long long dirtied = 0;
     if (job) {
-      uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (row.y) {
-        const uint4* src = reinterpret_cast<const uint4*>(a.darena + row.x);
-        const uint4 q0 = src[0], q1 = src[1];
-        x[0] = q0.x, x[1] = q0.y, x[2] = q0.z, x[3] = q0.w;
-        x[4] = q1.x, x[5] = q1.y, x[6] = q1.z, x[7] = q1.w;
-      }
-      // output k: an insertion takes x[k] below the new arc's position, the arc
-      // at it and x[k - 1] above; a removal takes x[k] below the arc, x[k + 1] from it on
-      uint32_t pos = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) pos += ((uint32_t)k < row.y && x[k] < v) ? 1u : 0u;
-      auto out = [&](int k) -> uint32_t {
-        if (kInsert) return (uint32_t)k < pos ? x[k] : ((uint32_t)k == pos ? v : x[k > 0 ? k - 1 : 0]);
-        return (uint32_t)k < pos ? x[k] : x[k < 7 ? k + 1 : 7];
-      };
+      SmallRow r = {};
+      if (row.y) r.load(a.darena + row.x);
+      // output k: x[k] below the new arc's position, the arc at it, x[k - 1] above
+      const uint32_t pos = r.below(row.y, v);
+      auto out = [&](uint32_t k) { return k < pos ? r.x[k] : (k == pos ? v : r.x[k > 0 ? k - 1 : 0]); };
       uint4* dst = reinterpret_cast<uint4*>(a.darena + base_off);
       dst[0] = make_uint4(out(0), out(1), out(2), out(3));
       dst[1] = make_uint4(out(4), out(5), out(6), out(7));
-      dlive = kInsert ? 1 : -1;
-      acct_add(p, 2, kInsert ? 2ull * row.y + 1 : 2ull * row.y - 1);
-      a.drow[u] = make_uint2(base_off, kInsert ? row.y + 1 : row.y - 1);
+      dlive = 1;
+      acct_add(p, 2, 2ull * row.y + 1);
+      a.drow[u] = make_uint2(base_off, row.y + 1);
       if (need_block) a.dcap[u] = 8u;
-      const uint32_t bit = 1u << (u & 31);
-      dirtied = (atomicOr(&a.dirty[u >> 5], bit) & bit) ? 0ull : 1ull;
+      w.dirtied += gdev::mark_dirty_count(a.dirty, u);
     }
     dlive = vxb::warp_sum(dlive);
-    dirtied = vxb::warp_sum(dirtied);
-    if (lane == 0 && dlive) atomicAdd(&s.gc->delta_live[0], (unsigned long long)dlive);
-    if (lane == 0 && dirtied) atomicAdd(&s.gc->dirty_rows[0], dirtied);
+    if (lane == 0 && dlive) atomicAdd(&w.s->gc->delta_live[w.dir], (unsigned long long)dlive);
     if (queue) sm.sv[atomicAdd(&sm.nsv, 1u)] = i;
     __syncthreads();
     const uint32_t nq = sm.nsv;
     for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) {
-      const uint32_t st = sm.sv[k], en = run_end(fu, st, F);
-      unsigned long long* ac = p.acct ? p.acct + 2 : nullptr;
-      if (kInsert) run_insert(a, fv, ff, s.scratch, st, en, fu[st], s.gc, s.arena_cap, ac);
-      else run_remove(a, fv, ff, st, en, fu[st], s.gc, ac);
+      const uint32_t st = sm.sv[k], en = run_end(w.fu, st, w.F);
+      run_insert(a, w.dir, w.fv, w.ff, w.s->scratch[w.dir], st, en, w.fu[st], w.s->gc, w.s->arena_cap[w.dir],
+                 p.acct ? p.acct + 2 : nullptr);
     }
     __syncthreads();  // the list is rebuilt by the next round
   }
+  w.flush();
 }
 
 __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
-  const int lane = threadIdx.x & 31;
   unsigned long long tmark = globaltimer();
   auto phase = [&](int k) {  // gtid 0 accumulates the time since the previous mark
     if (gtid() == 0) {
@@ -2281,67 +2620,50 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     for (int k = 0; k < (int)(sizeof(c->rtrace) / sizeof(c->rtrace[0])); ++k) c->rtrace[k] = 0;
     c->handovers[0] = c->handovers[1] = 0;
   }
+  const int ndir = p.g.directed ? 2 : 1;
   for (uint32_t bi = 0; bi < s.nb; ++bi) {
-    const uint32_t off = s.boff ? s.boff[bi] : 0u, F = s.bcnt[bi];
+    const uint32_t off = s.boff ? s.boff[bi] : 0u, F = s.cnt[0][bi];
     const uint32_t Vpre = bi ? s.vpost[bi - 1] : s.V0, lpre = bi ? s.vpost[bi - 1] : s.len0;
     const uint32_t Vpost = s.vpost ? s.vpost[bi] : s.v_single;
     Params q = p;
-    q.fu = s.fu + off;
-    q.fv = s.fv + off;
-    q.ff = s.ff + off;
-    q.F = &s.bcnt[bi];
+    q.fu = s.fu[0] + off;
+    q.fv = s.fv[0] + off;
+    q.ff = s.ff[0] + off;
+    q.F = &s.cnt[0][bi];
     q.V = Vpre;
     q.dist_len = lpre;
     const unsigned long long lim = (unsigned long long)((double)Vpre * s.frac);
     q.fallback_limit = lim < 1 ? 1 : lim;
-    if (gtid() == 0) {  // last_* counters and the repair lists start empty (bfs.hpp:30-33)
-      c->candidates = c->affected = c->full = c->fallback = 0;
-      c->cand_n = c->touched_n = c->a_n = 0;
-    }
+    auto work = [&](int dir) {
+      const uint32_t o = dir ? 0u : off;
+      return ArcWork{&q, &s, dir ? &p.g.in : &p.g.out, dir, s.fu[dir] + o, s.fv[dir] + o, s.ff[dir] + o, s.fpos[dir] + o,
+                     dir ? *s.cnt[1] : F, 0ll, 0u};
+    };
     stamp(q, 0);
-    // A: classification against the pre-batch graph; tombstone the deleted base arcs
-    {
-      // arcs dealt round-robin over the blocks (arc i to block i mod gridDim),
-      // so a small batch's searches spread over every SM
-      const vxb::DevAdj& a = p.g.out;
-      long long tombs = 0;
-      uint32_t dirtied = 0, removals = 0;
-      for (uint32_t i = threadIdx.x * gridDim.x + blockIdx.x; i < F; i += nthreads()) {
-        uint8_t f = s.ff[off + i];
-        if (!s.classified) {
-          f = gdev::classify_arc(a, s.fu[off + i], s.fv[off + i], f, s.fpos[off + i]);
-          s.ff[off + i] = f;
-        }
-        removals += !(f & kFAdd) && (f & kFChanged);
-        tombs += gdev::tomb_arc(a, s.fu[off + i], f, s.fpos[off + i], 0, dirtied);
-      }
-      tombs = vxb::warp_sum(tombs);
-      dirtied = vxb::warp_sum(dirtied);
-      removals = vxb::warp_sum(removals);
-      if (lane == 0 && tombs) atomicAdd(&s.gc->tombs[0], (unsigned long long)tombs);
-      if (lane == 0 && dirtied) atomicAdd(&s.gc->dirty_rows[0], (unsigned long long)dirtied);
-      if (lane == 0 && removals) atomicAdd(&c->rmb[bi & 1], removals);
-      if (s.digest && bi > 0) digest_pass(p.dist, lpre, &s.digest[bi - 1]);
+    // A: classification against the pre-batch graph, removals, deletion candidates
+    for (int dir = 0; dir < ndir; ++dir) {
+      ArcWork w = work(dir);
+      removal_pass(w, sm);
     }
-    if (!sync_grid(p)) return;
+    if (s.digest && bi > 0) digest_pass(p.dist, lpre, &s.digest[bi - 1]);
+    if (!sync_words(p, sm.w)) return;
     phase(0);
-    // B: delta removals; deletion candidates registered.  A batch without a
-    // removal arc has neither, and skips the phase and its barrier.  The other
-    // parity's counter was last read before the previous batch's later
-    // barriers: it is cleared here for the next batch.
-    const uint32_t nrm = ld_cg(&c->rmb[bi & 1]);
-    if (gtid() == 0) c->rmb[(bi + 1) & 1] = 0u;
-    if (nrm) {
-      commit_runs<false>(q, s, off, F, sm);
-      register_candidates(q);
-      if (!sync_grid(p)) return;
+    if (sm.w.multi_rm) {
+      for (int dir = 0; dir < ndir; ++dir) {
+        ArcWork w = work(dir);
+        removal_runs(w, sm);
+      }
+      if (!sync_words(p, sm.w)) return;
     }
     phase(1);
     stamp(q, 1);
-    // C: the cascade over the graph without the batch's deletions
-    const uint32_t ncand = ld_cg(&c->cand_n);
+    // B: the cascade over the graph without the batch's deletions
+    const uint32_t ncand = sm.w.touched;
     if (gtid() == 0) {
+      // last_* counters (bfs.hpp:30-33); the last reader of the previous
+      // batch's was this thread, at its end
       c->candidates = ncand;
+      c->affected = c->full = 0;
       acct_add(p, 1, ncand + F);  // candidate checks, heads of the canonical arcs
       acct_add(p, 3, F);
       acct_add(p, 4, 1);
@@ -2353,30 +2675,27 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     }
     phase(2);
     stamp(q, 2);
-    // D: revive re-added base arcs, delta insertions; new vertices start unreachable
-    {
-      const vxb::DevAdj& a = p.g.out;
-      long long tombs = 0;
-      uint32_t dirtied = 0;
-      for (uint32_t i = threadIdx.x * gridDim.x + blockIdx.x; i < F; i += nthreads())
-        tombs += gdev::tomb_arc(a, s.fu[off + i], s.ff[off + i], s.fpos[off + i], 1, dirtied);
-      tombs = vxb::warp_sum(tombs);
-      dirtied = vxb::warp_sum(dirtied);
-      if (lane == 0 && tombs) atomicAdd(&s.gc->tombs[0], (unsigned long long)tombs);
-      if (lane == 0 && dirtied) atomicAdd(&s.gc->dirty_rows[0], (unsigned long long)dirtied);
-      for (uint32_t v = lpre + gtid(); v < Vpost; v += nthreads()) p.dist[v] = kUnreachable;
+    // C: insertions; new vertices start unreachable and, unless a BFS gives
+    // the distances, the affected ones are invalidated
+    for (int dir = 0; dir < ndir; ++dir) {
+      ArcWork w = work(dir);
+      insertion_pass(w, sm);
     }
-    commit_runs<true>(q, s, off, F, sm);
-    if (!sync_grid(p)) return;
+    for (uint32_t v = lpre + gtid(); v < Vpost; v += nthreads()) p.dist[v] = kUnreachable;
+    if (!sm.w.cbig && !sm.w.fallback) invalidate(q, sm.w.affected);
+    if (!sync_words(p, sm.w)) return;
     phase(3);
-    // E: the post-batch repair (or the fallback full BFS) on the new graph
+    // D: the post-batch repair (or the fallback full BFS) on the new graph
     q.V = Vpost;
     q.dist_len = Vpost;
-    repair_post(q, sm, lb, bq);
-    if (ld_cg(&c->err)) return;
+    repair_post<true>(q, sm, lb, bq);
     phase(4);
-    // every block's counter updates are in before they are recorded, and
-    // recorded before the next batch resets them (same thread)
+    // the repair lists start empty in the next batch (and launch); every block
+    // has their lengths in sm.w
+    if (gtid() == 0) c->touched_n = c->a_n = c->fallback = c->multi_rm = 0;
+    if (bi + 1 == s.nb && !s.digest && !s.bstats) break;
+    // every block's counter updates are in before they are recorded and the
+    // next batch begins
     if (!sync_grid(p)) return;
     phase(5);
     if (gtid() == 0 && s.bstats) {
@@ -2387,8 +2706,6 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     }
   }
   if (s.digest && s.nb) digest_pass(p.dist, s.vpost[s.nb - 1], &s.digest[s.nb - 1]);
-  // every read of the removal counters came before the last end-of-batch barrier
-  if (gtid() == 0) c->rmb[0] = c->rmb[1] = 0u;
 }
 
 // The full BFS has a kernel of its own (the repair kernels run it too, for the
@@ -2419,7 +2736,7 @@ __global__ void __launch_bounds__(kThreads, 2) bfs_kernel(Params p, int mode) {
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
   if (mode == kModePre) repair_pre(p, sm, lb, bq);
-  else repair_post(p, sm, lb, bq);
+  else repair_post<false>(p, sm, lb, bq);
 }
 
 // Registers for two blocks per SM: the launches of two graphs (on their own
@@ -2898,6 +3215,11 @@ static int launch_stream(Bfs* b, Params& p, StreamArgs& sa) {
   const uint32_t want = b->tune.update_blocks ? b->tune.update_blocks : (uint32_t)sm_count();
   p.nblocks = want < (uint32_t)b->stream_grid ? want : (uint32_t)b->stream_grid;
   p.deltas = 1;  // the launch inserts delta rows itself
+  if (b->lists_left) {  // the update launch starts from empty repair lists and leaves them empty
+    VX_CUDA_TRY(cudaMemsetAsync(&b->ctr->cand_n, 0, 3 * sizeof(uint32_t), b->g->stream));
+    VX_CUDA_TRY(cudaMemsetAsync(&b->ctr->fallback, 0, sizeof(uint32_t), b->g->stream));
+    b->lists_left = false;
+  }
   void* args[] = {&p, &sa};
   count_launch();
   VX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bfs_stream_kernel, dim3(p.nblocks), dim3(kThreads), args,
@@ -2913,14 +3235,14 @@ static int repair_fused(Bfs* b) {
   const size_t n = b->staged_ops, m = 2 * n;
   StreamArgs sa;
   memset(&sa, 0, sizeof(sa));
-  sa.fu = g->batch.fu;
-  sa.fv = g->batch.fv;
-  sa.ff = g->batch.ff;
-  sa.fpos = g->batch.fpos;
-  sa.bcnt = &g->ctr->final_arcs;
-  sa.scratch = g->batch.lu;
+  sa.fu[0] = g->batch.fu;
+  sa.fv[0] = g->batch.fv;
+  sa.ff[0] = g->batch.ff;
+  sa.fpos[0] = g->batch.fpos;
+  sa.cnt[0] = &g->ctr->final_arcs;
+  sa.scratch[0] = g->batch.lu;
   sa.gc = g->ctr;
-  sa.arena_cap = g->adj[0].arena_cap;
+  sa.arena_cap[0] = g->adj[0].arena_cap;
   sa.frac = b->frac;
   sa.nb = 1;
   sa.V0 = (uint32_t)b->staged_V_pre;
@@ -2947,6 +3269,7 @@ int bfs_repair_staged(Bfs* b) {
   VX_CUDA_TRY(cudaMemsetAsync(b->ctr->handovers, 0, sizeof(b->ctr->handovers), s));
   const size_t V_pre = b->staged_V_pre, len_pre = b->staged_len_pre;
   const size_t V_post = g->V;
+  b->lists_left = true;
   // fallback limit: max(1, size_t(double(V) * fraction))  (bfs.hpp:225-226)
   unsigned long long lim = (unsigned long long)((double)V_pre * b->frac);
   if (lim < 1) lim = 1;
@@ -3197,18 +3520,18 @@ int bfs_apply_stream(Bfs* b, const uint32_t* hs, const uint32_t* hd, const uint8
   if (digests) VX_CUDA_TRY(cudaMemsetAsync(S.digest, 0, nb * 8, st));
   StreamArgs sa;
   memset(&sa, 0, sizeof(sa));
-  sa.fu = S.fu;
-  sa.fv = S.fv;
-  sa.ff = S.ff;
-  sa.fpos = S.fpos;
+  sa.fu[0] = S.fu;
+  sa.fv[0] = S.fv;
+  sa.ff[0] = S.ff;
+  sa.fpos[0] = S.fpos;
   sa.boff = S.boff;
-  sa.bcnt = S.bcnt;
+  sa.cnt[0] = S.bcnt;
   sa.vpost = S.vpost;
-  sa.scratch = S.scratch;
+  sa.scratch[0] = S.scratch;
   sa.digest = digests ? S.digest : nullptr;
   sa.bstats = stats ? S.bstats : nullptr;
   sa.gc = g->ctr;
-  sa.arena_cap = a.arena_cap;
+  sa.arena_cap[0] = a.arena_cap;
   sa.frac = b->frac;
   sa.nb = (uint32_t)nb;
   sa.V0 = (uint32_t)Vbefore;

@@ -39,10 +39,10 @@ struct BfsCounters {
   // (classify + tombstones, removals + candidates, cascade, insertions,
   // post-batch repair, end-of-batch barrier), summed over its batches, ns
   unsigned long long stream_ns[6];
-  // removal arcs of the update launch's current batch (two slots, by batch
-  // parity; zero between launches): a batch without any skips the removal
-  // phase and its barrier
-  uint32_t rmb[2];
+  // a delta removal of the update launch's current batch lies in a run of
+  // several arcs (zero between batches)
+  uint32_t multi_rm;
+  uint32_t unused;  // (the size of this struct is what stats() reports as read back)
   // the post-batch relaxation passed its time budget and the batch's
   // distances come from a full BFS (zero between batches)
   uint32_t rbig;
@@ -51,7 +51,7 @@ struct BfsCounters {
   // the number of vertices whose distance that BFS raised
   uint32_t cbig;
   uint32_t a_bfs;
-  // ns the last full BFS took (or would have inside an update launch), and the time at which the running
+  // ns the last full BFS took, and the time at which the running
   // repair phase hands over to a BFS (~0: never)
   unsigned long long full_ns;
   unsigned long long deadline;
@@ -73,7 +73,7 @@ struct BfsTuning {
   // fraction of the vertices
   float window_pull_frac = 0.02f;
   // a repair phase (the cascade, the relaxation) that has run longer than this
-  // multiple of the last full BFS's time hands over to a BFS (0: at its first
+  // multiple of the last full BFS's time (+ 0.1 ms) hands over to a BFS (0: at its first
   // work-ring round; negative: never)
   float handover = 1.0f;
 };
@@ -129,6 +129,7 @@ struct Bfs {
   BfsTuning tune;
   int grid = 0;       // blocks of the repair kernel
   int stream_grid = 0;
+  bool lists_left = false;  // the per-phase path left its repair lists' lengths in ctr
   unsigned long long* acct = nullptr;  // algorithmic-byte accounting (5 counters), when on
   bool acct_on = false;
   StreamBufs sb;
