@@ -273,8 +273,8 @@ int vx_bfs_set_window_pull_fraction(vx_bfs* b, float frac);
  * negative value never.  Same distances and counters for every value.  No
  * reference counterpart. */
 int vx_bfs_set_handover(vx_bfs* b, float multiple);
-/* fused != 0 (default): an undirected batch's commit and repair run in one
- * persistent launch after staging; 0: the per-phase path (a launch per commit
+/* fused != 0 (default): a batch's commit and repair run in one persistent
+ * launch after staging; 0: the per-phase path (a launch per commit
  * step and for each half of the repair) -- the plain baseline the batched
  * stream path is measured against.  Same results either way.  No reference
  * counterpart. */

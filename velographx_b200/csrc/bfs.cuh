@@ -64,7 +64,7 @@ struct BfsTuning {
   float alpha = 14.0f;       // top-down -> bottom-up when m_f * alpha > m_u
   float beta = 24.0f;        // bottom-up -> top-down when n_f * beta < V (shrinking)
   uint32_t large_row = 1024; // rows this long are expanded by the whole grid
-  bool fused = true;         // undirected batches: one persistent launch after staging
+  bool fused = true;         // one persistent launch per batch after staging
   uint32_t update_blocks = 0;  // blocks of the update launch (0: every co-resident block)
   // batches per version-parallel window of a stream whose per-batch repair
   // counters are not asked for (0: every batch by the update launch)

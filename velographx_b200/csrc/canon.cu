@@ -104,7 +104,7 @@ template <int ITEMS>
 __global__ void __launch_bounds__(kThreads, 1)
     canon_cluster_kernel(const uint32_t* src, const uint32_t* dst, const uint8_t* add, uint32_t n, int directed,
                          int b, int sh, uint32_t bound, int passes, uint32_t* fu, uint32_t* fv, uint8_t* ff,
-                         GraphCounters* ctr) {
+                         uint32_t* count, GraphCounters* ctr) {
   constexpr int kItems = Tile<ITEMS>::kItems;
   constexpr int kTile = Tile<ITEMS>::kTile;
   cg::cluster_group cluster = cg::this_cluster();
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t base = 0;
     for (uint32_t rr = 0; rr < r; ++rr) base += cluster.map_shared_rank(misc, rr)[32];
     misc[33] = base;
-    if (r == C - 1) ctr->final_arcs = base + misc[32];
+    if (r == C - 1) *count = base + misc[32];
   }
   __syncthreads();
   uint32_t out = misc[33] + misc[warp] + incl - cnt;
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 size_t canon_cluster_capacity() { return (size_t)kMaxCluster * Tile<11>::kTile; }
 
 template <int ITEMS>
-static int launch_canon(Graph* g, size_t n, size_t m, int b, int sh, uint32_t bound, bool* launched) {
+static int launch_canon(Graph* g, size_t n, size_t m, int b, int sh, uint32_t bound, int dir, bool* launched) {
   using T = Tile<ITEMS>;
   *launched = false;
   static bool attr = false;
@@ -290,15 +290,17 @@ static int launch_canon(Graph* g, size_t n, size_t m, int b, int sh, uint32_t bo
   const int passes = (2 * b + 7) / 8;
   BatchBuffers& B = g->batch;
   count_launch();
-  VX_CUDA_TRY(cudaLaunchKernelEx(&cfg, canon_cluster_kernel<ITEMS>, B.in_src, B.in_dst, B.in_add, (uint32_t)n,
-                                 (int)g->directed, b, sh, bound, passes, B.fu, B.fv, B.ff, g->ctr));
+  const uint32_t *src = dir ? B.in_dst : B.in_src, *dst = dir ? B.in_src : B.in_dst;
+  VX_CUDA_TRY(cudaLaunchKernelEx(&cfg, canon_cluster_kernel<ITEMS>, src, dst, B.in_add, (uint32_t)n, (int)g->directed,
+                                 b, sh, bound, passes, dir ? B.ru : B.fu, dir ? B.rv : B.fv, dir ? B.rf : B.ff,
+                                 dir ? &g->ctr->rev_arcs : &g->ctr->final_arcs, g->ctr));
   *launched = true;
   return 0;
 }
 
 // Canonicalises the staged batch when it fits one cluster (*done = true);
 // returns a negative status on a launch error.
-int canon_cluster(Graph* g, size_t n, int b, uint32_t bound, bool* done) {
+int canon_cluster(Graph* g, size_t n, int b, uint32_t bound, int dir, bool* done) {
   *done = false;
   const size_t m = g->directed ? n : 2 * n;
   int sbits = 1;
@@ -307,12 +309,12 @@ int canon_cluster(Graph* g, size_t n, int b, uint32_t bound, bool* done) {
   if (m == 0 || m > canon_cluster_capacity() || 2 * b + sh > 64) return 0;
   bool launched = false;
   int rc = 0;
-  if (m <= (size_t)kMaxClusterNP * Tile<1>::kTile) rc = launch_canon<1>(g, n, m, b, sh, bound, &launched);
+  if (m <= (size_t)kMaxClusterNP * Tile<1>::kTile) rc = launch_canon<1>(g, n, m, b, sh, bound, dir, &launched);
   if (!rc && !launched && m <= (size_t)kMaxClusterNP * Tile<2>::kTile)
-    rc = launch_canon<2>(g, n, m, b, sh, bound, &launched);
+    rc = launch_canon<2>(g, n, m, b, sh, bound, dir, &launched);
   if (!rc && !launched && m <= (size_t)kMaxCluster * Tile<4>::kTile)
-    rc = launch_canon<4>(g, n, m, b, sh, bound, &launched);
-  if (!rc && !launched) rc = launch_canon<11>(g, n, m, b, sh, bound, &launched);
+    rc = launch_canon<4>(g, n, m, b, sh, bound, dir, &launched);
+  if (!rc && !launched) rc = launch_canon<11>(g, n, m, b, sh, bound, dir, &launched);
   *done = launched;
   return rc;
 }

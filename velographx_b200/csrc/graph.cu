@@ -846,6 +846,32 @@ int graph_prepare_batch(Graph* g, size_t n, size_t vertex_bound) {
   return graph_grow(g, std::max<size_t>(g->V, vertex_bound));
 }
 
+// The canonical arcs of the staged batch (dir 1: reversed).
+static int canon_list(Graph* g, size_t n, int b, int dir) {
+  cudaStream_t s = g->stream;
+  BatchBuffers& B = g->batch;
+  const size_t m = g->directed ? n : 2 * n;
+  bool done = false;
+  if (int rc = canon_cluster(g, n, b, (uint32_t)g->V, dir, &done)) return rc;
+  if (done) return 0;
+  vxh::count_launch();
+  expand_ops_kernel<<<grid_for(n), kBlock, 0, s>>>(dir ? B.in_dst : B.in_src, dir ? B.in_src : B.in_dst, B.in_add, n,
+                                                    g->directed, b, (uint32_t)g->V, B.keys, B.vals, g->ctr);
+  VX_CUDA_TRY(cudaGetLastError());
+  bool in_alt = false;
+  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, s)) return rc;
+  uint64_t* keys = in_alt ? B.keys_alt : B.keys;
+  uint32_t* vals = in_alt ? B.vals_alt : B.vals;
+  vxh::count_launch();
+  last_of_run_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, B.flag);
+  if (int rc = scan_count(g, B.flag, B.pos, m, dir ? &g->ctr->rev_arcs : &g->ctr->final_arcs)) return rc;
+  vxh::count_launch();
+  compact_final_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, vals, B.flag, B.pos, m, b, dir ? B.ru : B.fu,
+                                                       dir ? B.rv : B.fv, dir ? B.rf : B.ff);
+  VX_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 int graph_stage_batch(Graph* g, size_t n, size_t vertex_bound, bool classify) {
   cudaStream_t s = g->stream;
   BatchBuffers& B = g->batch;
@@ -856,31 +882,8 @@ int graph_stage_batch(Graph* g, size_t n, size_t vertex_bound, bool classify) {
     VX_CUDA_TRY(cudaMemsetAsync(&g->ctr->final_arcs, 0, 5 * sizeof(uint32_t), s));
     return 0;
   }
-  bool done = false;
-  if (int rc = canon_cluster(g, n, b, (uint32_t)g->V, &done)) return rc;
-  if (done) {
-    if (!classify) return 0;
-    vxh::count_launch();
-    classify_kernel<<<grid_for(m), kBlock, 0, s>>>(devadj(g->adj[0]), B.fu, B.fv, B.ff, B.fpos,
-                                                    &g->ctr->final_arcs);
-    VX_CUDA_TRY(cudaGetLastError());
-    return 0;
-  }
-  vxh::count_launch();
-  expand_ops_kernel<<<grid_for(n), kBlock, 0, s>>>(B.in_src, B.in_dst, B.in_add, n, g->directed, b, (uint32_t)g->V,
-                                                    B.keys, B.vals, g->ctr);
-  VX_CUDA_TRY(cudaGetLastError());
-  bool in_alt = false;
-  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, s)) return rc;
-  uint64_t* keys = in_alt ? B.keys_alt : B.keys;
-  uint32_t* vals = in_alt ? B.vals_alt : B.vals;
-  vxh::count_launch();
-  last_of_run_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, B.flag);
-  if (int rc = scan_count(g, B.flag, B.pos, m, &g->ctr->final_arcs)) return rc;
-  vxh::count_launch();
-  compact_final_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, vals, B.flag, B.pos, m, b, B.fu, B.fv, B.ff);
-  VX_CUDA_TRY(cudaGetLastError());
-  if (!classify) return 0;
+  if (int rc = canon_list(g, n, b, 0)) return rc;
+  if (!classify) return g->directed ? canon_list(g, n, b, 1) : 0;
   vxh::count_launch();
   classify_kernel<<<grid_for(m), kBlock, 0, s>>>(devadj(g->adj[0]), B.fu, B.fv, B.ff, B.fpos,
                                                   &g->ctr->final_arcs);

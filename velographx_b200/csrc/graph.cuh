@@ -73,7 +73,8 @@ struct BatchBuffers {
   uint32_t* lu = nullptr;
   uint32_t* lv = nullptr;
   uint32_t* runs = nullptr;
-  // reversed canonical arcs (in direction, directed graphs)
+  // reversed canonical arcs (in direction, directed graphs; the per-phase
+  // commit keeps only those that change)
   uint32_t* ru = nullptr;
   uint32_t* rv = nullptr;
   uint8_t* rf = nullptr;
@@ -106,7 +107,8 @@ int graph_grow(Graph* g, size_t vertices);
 int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n_edges);
 // Stage a batch already in g->batch.{src,dst,add}: canonicalise + classify on
 // the pre-batch graph.  vertex_bound bounds every non-self-loop id + 1.
-// classify = false leaves the arcs unclassified (a fused repair classifies them itself).
+// classify = false leaves the arcs unclassified, and a directed graph's reversed
+// arcs canonicalised as well (a fused repair classifies both itself).
 int graph_stage_batch(Graph* g, size_t n, size_t vertex_bound, bool classify = true);
 // The part of staging that precedes canonicalisation: arena room for a batch
 // of n ops (consolidating first when the arena would pass its limit) and the
@@ -121,9 +123,10 @@ int graph_commit_insertions(Graph* g);
 int graph_consolidate(Graph* g);
 int graph_reserve_stream(Graph* g, uint64_t entries, int* fits);
 // One-launch canonicalisation of the staged batch in a thread-block cluster
-// (sort, last-op-wins dedupe, compaction, classification); *done = false when
-// the batch exceeds one cluster's capacity.
-int canon_cluster(Graph* g, size_t n, int b, uint32_t bound, bool* done);
+// (sort, last-op-wins dedupe, compaction); *done = false when the batch exceeds
+// one cluster's capacity.  dir 1 (directed graphs): the reversed arcs (v, u),
+// into batch.{ru,rv,rf} and ctr->rev_arcs.
+int canon_cluster(Graph* g, size_t n, int b, uint32_t bound, int dir, bool* done);
 size_t canon_cluster_capacity();
 // maybe_compact(threshold) (dynamic_graph.hpp:620-631, 764-789): consolidates when
 // any dirty row's overlay density reaches the threshold; *compacted = 1 then.
