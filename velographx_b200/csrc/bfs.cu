@@ -470,10 +470,11 @@ constexpr uint32_t kSoloArcs = 4096;
 constexpr uint32_t kSoloLevels = 4096;
 
 // Words of the barrier array past the barrier word (zero between searches):
-// what a stretch hands back (two sets of 8), and the length of a queue made
-// from a bitmap.
-constexpr uint32_t kSoloWord = 8, kQueueWord = 28;
-static_assert(kQueueWord < vxb::kBarrierWords, "the barrier array holds these words");
+// what a stretch hands back (two sets of 8), the length of a queue made from a
+// bitmap, and the lengths of the arc lists of a batch that the update launch
+// canonicalises itself.
+constexpr uint32_t kSoloWord = 8, kQueueWord = 28, kRawWord = 30;
+static_assert(kRawWord + 2 <= vxb::kBarrierWords, "the barrier array holds these words");
 
 struct SoloState {
   uint32_t level, n_f, reached;
@@ -1170,7 +1171,7 @@ __device__ void block_rows(const DevAdj& a, const T* items, uint32_t n, LbStage&
 // The words a repair phase decides by, as of the last grid barrier.
 struct RepairWords {
   unsigned long long deadline;
-  uint32_t failed, touched, affected, fallback, cbig, rbig, tail, big_b, multi_rm;
+  uint32_t failed, touched, affected, fallback, cbig, rbig, tail, big_b, later, raw_f[2];
 };
 
 // Grid barrier of the repair phases: thread 0 of each block loads the words
@@ -1189,7 +1190,9 @@ __device__ __forceinline__ bool sync_words(const Params& p, RepairWords& w) {
     r.rbig = ld_cg(&c->rbig);
     r.tail = ld_cg(p.rq_tail);
     r.big_b = ld_cg(&c->big_b);
-    r.multi_rm = ld_cg(&c->multi_rm);
+    r.later = ld_cg(&c->later);
+    r.raw_f[0] = ld_cg(p.bar + kRawWord);
+    r.raw_f[1] = ld_cg(p.bar + kRawWord + 1);
     r.deadline = __ldcg(&c->deadline);
     w = r;
   });
@@ -1318,6 +1321,43 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
       atomicMax(&p.rq_stat[5], dt);
     }
   }
+}
+
+// A phase's first items are taken in rounds with a grid barrier between them, a
+// warp per item, before the ring is drained asynchronously: most batches leave a
+// few dozen items of one or two hops, and a drain's tickets, polls and
+// termination test take longer than a barrier (1,000 directed ops at 300,000
+// vertices, 2 items: cascade 20 us drained, 16 in rounds; 10,000 ops at R-MAT 22, 58
+// items: 33 and 27).  A phase that is not done after kSyncRounds rounds,
+// or has more items than blocks, is deep or wide enough to drain.  w.one
+// handles an item (whole warp) that it has taken out of the ring.  sm.w is of
+// the last barrier; true when the ring is empty, false to drain (or on an
+// error, sm.w.failed).
+constexpr uint32_t kSyncRounds = 2;
+
+template <class W>
+__device__ bool sync_rounds(const Params& p, RepairSmem& sm, W& w) {
+  if (p.handover == 0.0f) return false;  // hands over at its first drain round
+  uint32_t lo = 0;
+  for (uint32_t r = 0; r < kSyncRounds; ++r) {
+    const uint32_t hi = sm.w.tail;
+    if (lo == hi) return true;
+    if (hi - lo > gridDim.x || sm.w.fallback) return false;
+    if (gtid() == 0) *p.rq_head = *p.rq_done = hi;  // a drain starts behind them
+    const uint32_t i = lo + dealt_warp();
+    if (i < hi) {
+      const unsigned long long it = __ldcg(&p.ring[i & p.ring_mask]);
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) {
+        __stcg(&p.ring[i & p.ring_mask], kSent);
+        acct_add(p, 1, 1);
+      }
+      w.one(it);
+    }
+    lo = hi;
+    if (!sync_words(p, sm.w)) return false;
+  }
+  return sm.w.tail == lo;
 }
 
 // --------------------------------------------------- pre-batch fixpoint --
@@ -1579,9 +1619,45 @@ __device__ void chunk_check(const Params& p, uint32_t x, uint32_t c) {
   ring_push(p, aff, (unsigned long long)(x | kKindBit));
 }
 
+// An expand item (y, chunk) by one warp: the item's arcs of y's out-row, all of
+// a short row's; the other chunks of a longer one are queued by its first.
+__device__ void expand_one(const Params& p, unsigned long long it) {
+  const DevAdj& a = p.g.out;
+  const uint32_t lane = threadIdx.x & 31, y = item_vertex(it), c = item_chunk(it);
+  const uint32_t dy = p.dist[y];
+  uint64_t b, e;
+  vxb::base_range(a, y, b, e);
+  const uint2 dr = a.drow[y];
+  const uint32_t nb = (uint32_t)(e - b), total = nb + dr.y;
+  const uint32_t hi = min(total, (c + 1) * kChunk);
+  if (c == 0)
+    for (uint32_t k = 1 + lane; (k - lane) * kChunk < total; k += 32)
+      ring_push(p, k * kChunk < total, (unsigned long long)(y | kKindBit) | ((unsigned long long)k << 32));
+  if (lane == 0) acct_add(p, 0, hi - c * kChunk);
+  ExpandChildren ec{&p, y, dy};
+  for (uint32_t k0 = c * kChunk; k0 < hi; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    const uint32_t x = k >= hi ? kTomb : k < nb ? a.col[b + k] : a.darena[dr.x + (k - nb)];
+    ec(!(x & kTomb), x & kIdMask, 0u);
+  }
+}
+
 struct Cascade {
   const Params* p;
   LbStage* lb;
+  // One item by one warp.  Past the fallback limit it is dropped like process
+  // drops its items.
+  __device__ void one(unsigned long long it) {
+    if (ld_cg(&p->c->fallback)) {
+      if (!(it & kChunkCheckBit) && !((uint32_t)it & kKindBit) && (threadIdx.x & 31) == 0)
+        atomicAnd(&p->inq[1][(uint32_t)it >> 5], ~(1u << ((uint32_t)it & 31)));
+      return;
+    }
+    __threadfence();  // expand items were pushed after their affected bits
+    if (it & kChunkCheckBit) chunk_check(*p, item_vertex(it), item_chunk(it));
+    else if ((uint32_t)it & kKindBit) expand_one(*p, it);
+    else check_vertex<false>(*p, (uint32_t)it);
+  }
   __device__ void process(RepairSmem& sm, uint32_t n) {
     const Params& P = *p;
     BfsCounters* c = P.c;
@@ -1748,8 +1824,11 @@ __device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue
   if (!sync_words(p, sm.w)) return false;
   if (sm.w.tail) {
     Cascade w{&p, &lb};
-    drain(p, sm, w, p.cascade_bfs ? sm.w.deadline : kNever);
-    if (!sync_words(p, sm.w)) return false;
+    if (!sync_rounds(p, sm, w)) {
+      if (sm.w.failed) return false;
+      drain(p, sm, w, p.cascade_bfs ? sm.w.deadline : kNever);
+      if (!sync_words(p, sm.w)) return false;
+    }
   }
   if (gtid() == 0) {  // the drain statistics of the phase trace
     p.c->rtrace[7] = sm.w.tail;
@@ -1816,17 +1895,46 @@ __device__ __forceinline__ void push_one(const Params& p, uint32_t x) {
 
 constexpr uint32_t kInlineRelax = 8;  // rows this short are relaxed where they are lowered
 
+// Arcs [lo, hi) of u's row relaxed from label du, whole warp, four arcs per
+// lane in flight; the vertices lowered are queued.
+__device__ __forceinline__ void relax_arcs(const Params& p, uint64_t b, uint32_t nb, uint32_t dx, uint32_t lo, uint32_t hi,
+                                           uint32_t du, long long& reach) {
+  const DevAdj& a = p.g.out;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t k0 = lo; k0 < hi; k0 += 128) {
+    uint32_t x[4], d[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint32_t k = k0 + 32 * j + lane;
+      x[j] = k >= hi ? kTomb : k < nb ? a.col[b + k] : a.darena[dx + (k - nb)];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) d[j] = !(x[j] & kTomb) && x[j] < p.dist_len ? ld_cg(&p.dist[x[j]]) : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+      if (d[j] > du + 1 && lower(p, x[j], du + 1, reach)) push_one(p, x[j]);
+  }
+}
+
+constexpr uint32_t kInlineRows = 4;    // longer rows of one warp's seeds relaxed in place
+constexpr uint32_t kInlineArcs = 512;  // their length
+
 // A seed v just lowered: a short row is relaxed here by its lane (the
-// vertices it lowers are queued), a longer one is queued.  Any later lowering
+// vertices it lowers are queued), a few longer ones by the warp, others are
+// queued (a batch whose seeds queue nothing ends without draining the ring).  Any later lowering
 // of v queues v again, so relaxing from the current label loses nothing.
 __device__ void seed_relax(const Params& p, bool lowered, uint32_t v, long long& reach) {
+  const DevAdj& a = p.g.out;
   bool queue = false;
+  uint64_t b = 0;
+  uint32_t nb = 0, deg = 0;
+  uint2 dr = make_uint2(0u, 0u);
   if (lowered) {
-    const DevAdj& a = p.g.out;
-    uint64_t b, e;
+    uint64_t e;
     vxb::base_range(a, v, b, e);
-    const uint2 dr = a.drow[v];
-    const uint32_t deg = (uint32_t)(e - b) + dr.y;
+    dr = a.drow[v];
+    nb = (uint32_t)(e - b);
+    deg = nb + dr.y;
     if (deg > kInlineRelax) {
       queue = true;
     } else {
@@ -1836,13 +1944,25 @@ __device__ void seed_relax(const Params& p, bool lowered, uint32_t v, long long&
       uint32_t x[kInlineRelax], dx[kInlineRelax];
 #pragma unroll
       for (uint32_t k = 0; k < kInlineRelax; ++k)
-        x[k] = k < e - b ? a.col[b + k] : k < deg ? a.darena[dr.x + (k - (uint32_t)(e - b))] : kTomb;
+        x[k] = k < nb ? a.col[b + k] : k < deg ? a.darena[dr.x + (k - nb)] : kTomb;
 #pragma unroll
       for (uint32_t k = 0; k < kInlineRelax; ++k)
         dx[k] = !(x[k] & kTomb) && x[k] < p.dist_len ? ld_cg(&p.dist[x[k]]) : 0u;
 #pragma unroll
       for (uint32_t k = 0; k < kInlineRelax; ++k)
         if (dx[k] > dv + 1 && lower(p, x[k], dv + 1, reach)) push_one(p, x[k]);
+    }
+  }
+  uint32_t rows = __ballot_sync(FULL, queue && deg <= kInlineArcs);
+  if (rows && __popc(rows) <= kInlineRows) {
+    if ((rows >> (threadIdx.x & 31)) & 1u) queue = false;
+    while (rows) {
+      const int l = __ffs(rows) - 1;
+      rows &= rows - 1;
+      const uint32_t n = __shfl_sync(FULL, deg, l);
+      if ((threadIdx.x & 31) == 0) acct_add(p, 0, n);
+      relax_arcs(p, __shfl_sync(FULL, b, l), __shfl_sync(FULL, nb, l), __shfl_sync(FULL, dr.x, l), 0u, n,
+                 ld_cg(&p.dist[__shfl_sync(FULL, v, l)]), reach);
     }
   }
   lower_and_push(p, queue, v);
@@ -1856,6 +1976,29 @@ struct Relax {
   const Params* p;
   LbStage* lb;
   long long* reach;
+  // One item by one warp (the other chunks of a long row are queued by its first).
+  __device__ void one(unsigned long long it) {
+    const Params& P = *p;
+    const DevAdj& a = P.g.out;
+    const uint32_t lane = threadIdx.x & 31, u = item_vertex(it), c = item_chunk(it);
+    if (c == 0) {
+      if (lane == 0) atomicAnd(&P.inq[0][u >> 5], ~(1u << (u & 31)));
+      __syncwarp();
+      __threadfence();  // the queued bit is clear before the label is read
+    }
+    const uint32_t du = ld_cg(&P.dist[u]);
+    uint64_t b, e;
+    vxb::base_range(a, u, b, e);
+    const uint2 dr = a.drow[u];
+    const uint32_t nb = (uint32_t)(e - b), total = nb + dr.y;
+    const uint32_t hi = min(total, (c + 1) * kChunk);
+    if (c == 0)
+      for (uint32_t k = 1 + lane; (k - lane) * kChunk < total; k += 32)
+        ring_push(P, k * kChunk < total, (unsigned long long)u | ((unsigned long long)k << 32));
+    if (du == kUnreachable) return;
+    if (lane == 0) acct_add(P, 0, hi - c * kChunk);
+    relax_arcs(P, b, nb, dr.x, c * kChunk, hi, du, *reach);
+  }
   __device__ void process(RepairSmem& sm, uint32_t n) {
     const Params& P = *p;
     const uint32_t t = threadIdx.x;
@@ -2082,8 +2225,11 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
   stamp(p, 5);
   if (sm.w.tail) {  // the relaxation runs only when a seed left work queued
     Relax w{&p, &lb, &reach};
-    drain(p, sm, w, sm.w.deadline);
-    if (!sync_words(p, sm.w)) return false;
+    if (!sync_rounds(p, sm, w)) {
+      if (sm.w.failed) return false;
+      drain(p, sm, w, sm.w.deadline);
+      if (!sync_words(p, sm.w)) return false;
+    }
     if (sm.w.rbig) {
       // the relaxation passed its budget: a full BFS of the post-batch graph
       // gives the distances and the reachable count (the repair's counters
@@ -2159,7 +2305,207 @@ struct StreamArgs {
   uint32_t nb, V0, len0;
   uint32_t v_single;    // vertex count after the batch when vpost is null (one staged batch)
   uint32_t classified;  // the arcs carry their classification already (a staged batch)
+  // raw_n > 0: one batch whose op arrays the launch canonicalises itself (the
+  // arc lists above are written by it); ids take b bits, below bound, and
+  // raw_sh bits hold an op's index and its add flag
+  const uint32_t* raw_src;
+  const uint32_t* raw_dst;
+  const uint8_t* raw_add;
+  uint32_t raw_n, raw_b, raw_sh, raw_bound;
 };
+
+// A batch of at most kRawOps ops is canonicalised inside the launch: every block
+// reads all ops and keeps the arcs whose row hashes to it (a dozen of 2,000), sorts
+// them, keeps the last of each arc and appends them to the batch's list, so
+// the arcs of a row are consecutive there and the block that has them in
+// shared memory can process them at once.  A launch of its own with a cluster's
+// barriers between the radix passes took 12 to 21 us; every block sorting
+// all arcs 2 us for 128 arcs but 7 for 1,024 and 13 for 2,048, bound by the
+// instructions of the one block an SM runs; now 2 to 3.
+constexpr uint32_t kRawOps = 1024;
+constexpr unsigned long long kRawDir = 1ull << 63;  // a directed graph's reversed arcs sort last
+// A block with more arcs than this (hub rows) leaves them to the whole grid,
+// behind a barrier: its 16 warps take one arc each at a time.
+constexpr uint32_t kRawMine = 64;
+constexpr uint8_t kFPending = 0x80;  // flag of an arc left to the grid
+struct RawArcs {
+  unsigned long long key[2 * kRawOps];  // [dir] | u | v | op index | add
+  uint32_t wsum[kThreads / 32];
+  uint32_t n[2];                        // arcs, and those of direction 0 among them
+  uint32_t base[2];                     // their places in the batch's lists
+};
+static_assert(sizeof(RawArcs) <= sizeof(LbStage), "the arcs are kept in the row stage's memory");
+
+// Bitonic sort of a warp's 32 * E keys, key e * 32 + lane in x[e].  The loops
+// over the steps stay rolled: the code runs once per launch, and unrolled it
+// is bound by fetching its instructions.
+template <int E>
+__device__ __forceinline__ void warp_sort(unsigned long long (&x)[E]) {
+  const uint32_t lane = threadIdx.x & 31;
+  auto exchange = [&](uint32_t e, uint32_t o, uint32_t k) {
+    if ((x[e] > x[o]) == (((e * 32 + lane) & k) == 0)) {
+      const unsigned long long t = x[e];
+      x[e] = x[o];
+      x[o] = t;
+    }
+  };
+#pragma unroll 1
+  for (uint32_t k = 2; k <= 32 * E; k <<= 1) {
+    if (E == 4 && k == 128) {
+      exchange(0, 2 % E, k);
+      exchange(1 % E, 3 % E, k);
+    }
+    if (E >= 2 && k >= 64) {
+      exchange(0, 1 % E, k);
+      if (E == 4) exchange(2 % E, 3 % E, k);
+    }
+#pragma unroll 1
+    for (uint32_t j = min(k >> 1, 16u); j > 0; j >>= 1) {
+      const bool low = (lane & j) == 0;
+#pragma unroll
+      for (uint32_t e = 0; e < E; ++e) {
+        const bool up = ((e * 32 + lane) & k) == 0;
+        const unsigned long long y = __shfl_xor_sync(FULL, x[e], j);
+        x[e] = (x[e] < y) == (low == up) ? x[e] : y;
+      }
+    }
+  }
+}
+
+// Sorts the block's n arc keys, padded to N (a power of two, 32 * E per warp in
+// use), and keeps the last of each arc.  Every warp sorts its keys in
+// registers; the runs are then merged pairwise, each key finding its place by a
+// binary search of the other run.
+template <int E>
+__device__ void canon_sort(const StreamArgs& s, bool directed, RawArcs& r, uint32_t n, uint32_t N) {
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const bool on = warp * 32 * E < N;
+  unsigned long long x[E];
+  uint32_t g[E];  // the keys' places
+#pragma unroll
+  for (uint32_t e = 0; e < E; ++e) {
+    g[e] = warp * 32 * E + e * 32 + lane;
+    x[e] = g[e] < n ? r.key[g[e]] : ~0ull;
+  }
+  __syncthreads();  // every key is read
+  if (on) {
+    warp_sort<E>(x);
+#pragma unroll
+    for (uint32_t e = 0; e < E; ++e) r.key[g[e]] = x[e];
+  }
+  if (t < 2) r.n[t] = 0;
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t L = 32 * E; L < N; L <<= 1) {
+    uint32_t to[E];
+    if (on) {
+      uint32_t lo[E];
+      const unsigned long long* other[E];
+      bool right[E];
+#pragma unroll
+      for (uint32_t e = 0; e < E; ++e) {
+        lo[e] = 0;
+        right[e] = (g[e] & L) != 0;
+        other[e] = r.key + ((g[e] & ~(L - 1)) ^ L);
+      }
+      // padding keys are equal: those of the left run stay first
+#pragma unroll 1
+      for (uint32_t step = L >> 1; step > 0; step >>= 1) {
+#pragma unroll
+        for (uint32_t e = 0; e < E; ++e) {
+          const unsigned long long y = other[e][lo[e] + step - 1];
+          if (y < x[e] || (right[e] && y == x[e])) lo[e] += step;
+        }
+      }
+#pragma unroll
+      for (uint32_t e = 0; e < E; ++e) {
+        const unsigned long long y = other[e][lo[e]];
+        if (y < x[e] || (right[e] && y == x[e])) ++lo[e];
+        to[e] = (g[e] & ~(2 * L - 1)) + (g[e] & (L - 1)) + lo[e];
+      }
+    }
+    __syncthreads();
+    if (on) {
+#pragma unroll
+      for (uint32_t e = 0; e < E; ++e) {
+        g[e] = to[e];
+        r.key[g[e]] = x[e];
+      }
+    }
+    __syncthreads();
+  }
+  // the last key of every arc, compacted in place
+  unsigned long long keep[E];
+  uint32_t cnt = 0, cnt0 = 0;
+#pragma unroll
+  for (uint32_t h = 0; h < E; ++h) {
+    const uint32_t j = t * E + h;
+    keep[h] = ~0ull;
+    if (j < N) {
+      const unsigned long long k = r.key[j], y = j + 1 < N ? r.key[j + 1] : ~0ull;
+      if (k != ~0ull && (k >> s.raw_sh) != (y >> s.raw_sh)) {
+        keep[h] = k;
+        ++cnt;
+        cnt0 += !(directed && (k & kRawDir));
+      }
+    }
+  }
+  uint32_t incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, incl, o);
+    if ((int)lane >= o) incl += y;
+  }
+  cnt0 = __reduce_add_sync(FULL, cnt0);
+  if (lane == 31) r.wsum[warp] = incl;
+  if (lane == 0 && cnt0) atomicAdd(&r.n[1], cnt0);
+  __syncthreads();  // every key is read, too
+  uint32_t pos = incl - cnt;
+  for (uint32_t k = 0; k < warp; ++k) pos += r.wsum[k];
+#pragma unroll
+  for (uint32_t h = 0; h < E; ++h)
+    if (keep[h] != ~0ull) r.key[pos++] = keep[h];
+  if (t == kThreads - 1) r.n[0] = pos;
+  __syncthreads();
+}
+
+// The block's arcs of the batch in r, and their places in the batch's lists
+// (whose lengths are f[0] and f[1], zero before).  Block-uniform.
+__device__ void canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32_t* f) {
+  if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < s.raw_n; i += kThreads) {
+    const uint32_t a = s.raw_src[i], b = s.raw_dst[i];
+    const unsigned long long low = ((unsigned long long)i << 1) | (s.raw_add[i] ? 1ull : 0ull);
+    bool ok = a != b;
+    if (ok && (a >= s.raw_bound || b >= s.raw_bound)) {
+      if (blockIdx.x == 0) atomicOr(&s.gc->err, vxb::kErrBadVertex);
+      ok = false;
+    }
+    if (!ok) continue;
+#pragma unroll
+    for (int rev = 0; rev < 2; ++rev) {
+      const unsigned long long u = rev ? b : a, v = rev ? a : b;
+      if (__umulhi((uint32_t)u * 0x9E3779B1u, gridDim.x) != blockIdx.x) continue;
+      r.key[atomicAdd(&r.n[0], 1u)] =
+          (directed && rev ? kRawDir : 0ull) | (u << (s.raw_b + s.raw_sh)) | (v << s.raw_sh) | low;
+    }
+  }
+  __syncthreads();
+  const uint32_t n = r.n[0];
+  __syncthreads();
+  uint32_t N = 32;
+  while (N < n) N <<= 1;
+  static_assert(2 * kRawOps == 4 * kThreads, "four keys per thread at most");
+  if (N <= kThreads) canon_sort<1>(s, directed, r, n, N);
+  else if (N <= 2 * kThreads) canon_sort<2>(s, directed, r, n, N);
+  else canon_sort<4>(s, directed, r, n, N);
+  if (threadIdx.x < 2) {
+    const uint32_t k = threadIdx.x ? r.n[0] - r.n[1] : r.n[1];
+    r.base[threadIdx.x] = k ? atomicAdd(&f[threadIdx.x], k) : 0u;
+  }
+  __syncthreads();
+}
 
 // Order-independent 64-bit digest of dist[0, n): sum of splitmix64(v << 32 | dist[v]).
 using vxb::mix64;
@@ -2314,6 +2660,11 @@ struct ArcWork {
   uint8_t* ff;
   uint64_t* fpos;
   uint32_t F;
+  // the arcs this block canonicalised, F of them, whose list place is base on
+  // (null: the whole batch's, in fu, fv, ff)
+  const unsigned long long* raw;
+  uint32_t base;
+  bool pending;        // only the arcs marked kFPending
   long long tombs;     // this lane's change of the tombstone count, and rows it dirtied
   uint32_t dirtied;
 
@@ -2329,14 +2680,32 @@ struct ArcWork {
     if (first) p->lst_t[slot] = v;
   }
 
+  __device__ __forceinline__ uint32_t tail_of(uint32_t i) const {
+    return raw ? (uint32_t)((raw[i] & ~kRawDir) >> (s->raw_b + s->raw_sh)) : fu[i];
+  }
+  // Arc i; a block's own are also written to the list the later passes read.
+  __device__ __forceinline__ void arc(uint32_t i, uint32_t& u, uint32_t& v, uint8_t& f) const {
+    if (raw) {
+      const unsigned long long k = raw[i];
+      u = tail_of(i);
+      v = (uint32_t)(k >> s->raw_sh) & ((1u << s->raw_b) - 1u);
+      f = (uint8_t)(k & 1ull);
+      const_cast<uint32_t*>(fu)[base + i] = u;
+      const_cast<uint32_t*>(fv)[base + i] = v;
+    } else {
+      u = fu[i];
+      v = fv[i];
+      f = ff[i];
+    }
+  }
   // Whether arc i's row has other arcs in the batch.
   __device__ __forceinline__ bool in_run(uint32_t i, uint32_t u) const {
-    return (i > 0 && fu[i - 1] == u) || (i + 1 < F && fu[i + 1] == u);
+    return (i > 0 && tail_of(i - 1) == u) || (i + 1 < F && tail_of(i + 1) == u);
   }
 
-  // The delta removals of run [st, ...), classified before; whole warp.
-  __device__ void remove_run(uint32_t st) {
-    run_remove(*a, dir, fv, ff, st, run_end(fu, st, F), fu[st], s->gc, p->acct ? p->acct + 2 : nullptr);
+  // The delta removals of run [st, en), classified before; whole warp.
+  __device__ void remove_run(uint32_t st, uint32_t en) {
+    run_remove(*a, dir, fv, ff, st, en, fu[st], s->gc, p->acct ? p->acct + 2 : nullptr);
   }
 
   // The sums of the pass into the graph's counters.
@@ -2373,20 +2742,37 @@ struct SmallRow {
   }
 };
 
+// What the first removal pass left for later (bits of BfsCounters::later).
+constexpr uint32_t kLaterRuns = 1u;  // delta removals of runs of several arcs
+constexpr uint32_t kLaterArcs = 2u;  // arcs marked kFPending
+
 // The removal pass.  A batch of few arcs takes a warp per arc: its row searches
 // read 32 pivots per round trip instead of 7, and the chain of such a batch is
 // its longest row's.  With the classification, the removals and the candidates
 // in three passes and two barriers 950 arcs at R-MAT 20 took 20 us, now 7 to 8;
 // 20,000 arcs at R-MAT 22 22 us, now 15.  Block-uniform.
 __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
+  if (w.raw && w.F > kRawMine) {  // hub rows: listed, and left to the grid
+    for (uint32_t i = threadIdx.x; i < w.F; i += kThreads) {
+      uint32_t u, v;
+      uint8_t f;
+      w.arc(i, u, v, f);
+      w.ff[w.base + i] = f | kFPending;
+    }
+    if (threadIdx.x == 0) atomicOr(&w.p->c->later, kLaterArcs);
+    return;
+  }
   const Params& p = *w.p;
   const vxb::DevAdj& a = *w.a;
   const uint32_t lane = threadIdx.x & 31;
   bool multi = false;  // a delta removal left to removal_runs
-  if (w.F <= 2 * nwarps()) {
-    for (uint32_t i = dealt_warp(); i < w.F; i += nwarps()) {
-      const uint32_t u = w.fu[i], v = w.fv[i];
-      uint8_t f = w.ff[i];
+  const uint32_t base = w.base;
+  if (w.raw || w.F <= 2 * nwarps()) {
+    for (uint32_t i = w.raw ? threadIdx.x >> 5 : dealt_warp(); i < w.F; i += w.raw ? kThreads / 32 : nwarps()) {
+      uint32_t u, v;
+      uint8_t f;
+      w.arc(i, u, v, f);
+      if (w.pending && !(f & kFPending)) continue;
       uint64_t b, e;
       vxb::base_range(a, u, b, e);
       const uint2 row = a.drow[u];
@@ -2408,11 +2794,11 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
         if (cur) f |= kFCur;
         if (cur != ((f & kFAdd) != 0)) f |= kFChanged;
         if (lane == 0) {
-          w.ff[i] = f;
-          w.fpos[i] = q;
+          w.ff[base + i] = f;
+          w.fpos[base + i] = q;
         }
       } else {
-        q = w.fpos[i];
+        q = w.fpos[base + i];
       }
       // lane 0 does what is not a search
       if (lane == 0) w.tombs += gdev::tomb_arc(a, u, f, q, 0, w.dirtied);
@@ -2431,7 +2817,7 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
         }
       } else {
         __syncwarp();
-        w.remove_run(i);
+        w.remove_run(base + i, base + i + 1);
       }
     }
   } else {
@@ -2439,15 +2825,13 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
       if (threadIdx.x == 0) sm.nsv = 0;
       __syncthreads();
       const uint32_t i = r0 + dealt_thread();
-      const bool act = i < w.F;
+      bool act = i < w.F && !(w.pending && !(w.ff[i] & kFPending));
       bool queue = false;
       uint32_t u = 0, v = 0;
       uint8_t f = 0;
       long long dlive = 0;
       if (act) {
-        u = w.fu[i];
-        v = w.fv[i];
-        f = w.ff[i];
+        w.arc(i, u, v, f);
         uint64_t b, e;
         vxb::base_range(a, u, b, e);
         const uint2 row = a.drow[u];
@@ -2498,11 +2882,11 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
       if (queue) sm.sv[atomicAdd(&sm.nsv, 1u)] = i;
       __syncthreads();
       const uint32_t nq = sm.nsv;
-      for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k]);
+      for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k], sm.sv[k] + 1);
       __syncthreads();  // the list is rebuilt by the next round
     }
   }
-  if (__any_sync(FULL, multi) && lane == 0) p.c->multi_rm = 1u;
+  if (__any_sync(FULL, multi) && lane == 0) atomicOr(&p.c->later, kLaterRuns);
   w.flush();
 }
 
@@ -2519,7 +2903,8 @@ __device__ void removal_runs(ArcWork& w, RepairSmem& sm) {
     }
     __syncthreads();
     const uint32_t nq = sm.nsv;
-    for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k]);
+    for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32)
+      w.remove_run(sm.sv[k], run_end(w.fu, sm.sv[k], w.F));
     __syncthreads();  // the list is rebuilt by the next round
   }
 }
@@ -2622,14 +3007,22 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
   }
   const int ndir = p.g.directed ? 2 : 1;
   for (uint32_t bi = 0; bi < s.nb; ++bi) {
-    const uint32_t off = s.boff ? s.boff[bi] : 0u, F = s.cnt[0][bi];
+    RawArcs& raw = reinterpret_cast<RawArcs&>(lb);
+    uint32_t off = 0, F = 0, Frev = 0;
+    if (s.raw_n) {
+      canon_raw(s, p.g.directed, raw, p.bar + kRawWord);
+    } else {
+      if (s.boff) off = s.boff[bi];
+      F = s.cnt[0][bi];
+      if (s.cnt[1]) Frev = *s.cnt[1];
+    }
     const uint32_t Vpre = bi ? s.vpost[bi - 1] : s.V0, lpre = bi ? s.vpost[bi - 1] : s.len0;
     const uint32_t Vpost = s.vpost ? s.vpost[bi] : s.v_single;
     Params q = p;
     q.fu = s.fu[0] + off;
     q.fv = s.fv[0] + off;
     q.ff = s.ff[0] + off;
-    q.F = &s.cnt[0][bi];
+    q.F = s.raw_n ? p.bar + kRawWord : &s.cnt[0][bi];
     q.V = Vpre;
     q.dist_len = lpre;
     const unsigned long long lim = (unsigned long long)((double)Vpre * s.frac);
@@ -2637,18 +3030,35 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     auto work = [&](int dir) {
       const uint32_t o = dir ? 0u : off;
       return ArcWork{&q, &s, dir ? &p.g.in : &p.g.out, dir, s.fu[dir] + o, s.fv[dir] + o, s.ff[dir] + o, s.fpos[dir] + o,
-                     dir ? *s.cnt[1] : F, 0ll, 0u};
+                     dir ? Frev : F, nullptr, 0u, false, 0ll, 0u};
     };
     stamp(q, 0);
     // A: classification against the pre-batch graph, removals, deletion candidates
     for (int dir = 0; dir < ndir; ++dir) {
       ArcWork w = work(dir);
+      if (s.raw_n) {
+        w.raw = raw.key + (dir ? raw.n[1] : 0u);
+        w.base = raw.base[dir];
+        w.F = dir ? raw.n[0] - raw.n[1] : raw.n[1];
+      }
       removal_pass(w, sm);
     }
     if (s.digest && bi > 0) digest_pass(p.dist, lpre, &s.digest[bi - 1]);
     if (!sync_words(p, sm.w)) return;
     phase(0);
-    if (sm.w.multi_rm) {
+    if (s.raw_n) {
+      F = sm.w.raw_f[0];
+      Frev = sm.w.raw_f[1];
+    }
+    if (sm.w.later & kLaterArcs) {
+      for (int dir = 0; dir < ndir; ++dir) {
+        ArcWork w = work(dir);
+        w.pending = true;
+        removal_pass(w, sm);
+      }
+      if (!sync_words(p, sm.w)) return;
+    }
+    if (sm.w.later & kLaterRuns) {
       for (int dir = 0; dir < ndir; ++dir) {
         ArcWork w = work(dir);
         removal_runs(w, sm);
@@ -2692,7 +3102,10 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     phase(4);
     // the repair lists start empty in the next batch (and launch); every block
     // has their lengths in sm.w
-    if (gtid() == 0) c->touched_n = c->a_n = c->fallback = c->multi_rm = 0;
+    if (gtid() == 0) {
+      c->touched_n = c->a_n = c->fallback = c->later = 0;
+      p.bar[kRawWord] = p.bar[kRawWord + 1] = 0u;
+    }
     if (bi + 1 == s.nb && !s.digest && !s.bstats) break;
     // every block's counter updates are in before they are recorded and the
     // next batch begins
@@ -3180,6 +3593,15 @@ int bfs_accounting(Bfs* b, unsigned long long* out5) {
   return 0;
 }
 
+constexpr uint32_t kRawShift = 11;  // an op index below kRawOps and the add flag
+static_assert((1u << (kRawShift - 1)) >= kRawOps, "an op's index fits its bits");
+
+static int raw_bits(size_t V) {  // bits of a vertex id below max(V, 2)
+  int b = 1;
+  while (((size_t)1 << b) < V) ++b;
+  return b;
+}
+
 int bfs_stage(Bfs* b, size_t n, size_t vertex_bound, bool classify) {
   Graph* g = b->g;
   cudaStream_t s = g->stream;
@@ -3194,7 +3616,13 @@ int bfs_stage(Bfs* b, size_t n, size_t vertex_bound, bool classify) {
   // consumes it: the fused launch in its first phase, the per-phase and full
   // paths on the host before their kernels
   b->staged_classified = classify;
-  if (int rc = graph_stage_batch(g, n, vertex_bound, classify)) return rc;
+  b->staged_raw = false;
+  if (!classify && n <= kRawOps) {  // keys of 2 * bits + kRawShift bits and the direction
+    if (int rc = graph_prepare_batch(g, n, vertex_bound)) return rc;
+    b->staged_raw = 2 * raw_bits(g->V) + (int)kRawShift <= 62;
+  }
+  if (!b->staged_raw)
+    if (int rc = graph_stage_batch(g, n, vertex_bound, classify)) return rc;
   if (int rc = ensure_capacity(b, std::max<size_t>(g->V, 1))) return rc;
   return ensure_ring(b);
 }
@@ -3260,6 +3688,16 @@ static int repair_fused(Bfs* b) {
   sa.len0 = (uint32_t)b->staged_len_pre;
   sa.v_single = (uint32_t)g->V;
   sa.classified = b->staged_classified ? 1u : 0u;
+  if (b->staged_raw) {
+    sa.raw_src = g->batch.in_src;
+    sa.raw_dst = g->batch.in_dst;
+    sa.raw_add = g->batch.in_add;
+    sa.raw_n = (uint32_t)n;
+    sa.raw_b = (uint32_t)raw_bits(g->V);
+    sa.raw_sh = kRawShift;
+    sa.raw_bound = (uint32_t)g->V;
+    b->staged_raw = false;
+  }
   Params p = make_params(b, (uint32_t)g->V, (uint32_t)g->V);
   if (int rc = launch_stream(b, p, sa)) return rc;
   for (int d = 0; d < (g->directed ? 2 : 1); ++d) g->adj[d].arena_bound += 8ull * m + 8;  // what the staging reserved

@@ -39,9 +39,9 @@ struct BfsCounters {
   // (classify + tombstones, removals + candidates, cascade, insertions,
   // post-batch repair, end-of-batch barrier), summed over its batches, ns
   unsigned long long stream_ns[6];
-  // a delta removal of the update launch's current batch lies in a run of
-  // several arcs (zero between batches)
-  uint32_t multi_rm;
+  // what the first removal pass of the update launch's current batch left to
+  // later passes (zero between batches)
+  uint32_t later;
   uint32_t unused;  // (the size of this struct is what stats() reports as read back)
   // the post-batch relaxation passed its time budget and the batch's
   // distances come from a full BFS (zero between batches)
@@ -126,6 +126,7 @@ struct Bfs {
   float* features = nullptr;            // selector features of the staged batch
   size_t staged_ops = 0, staged_V_pre = 0, staged_len_pre = 0;  // batch staged by bfs_stage
   bool staged_classified = true;
+  bool staged_raw = false;  // the update launch canonicalises the staged batch itself
   BfsTuning tune;
   int grid = 0;       // blocks of the repair kernel
   int stream_grid = 0;
