@@ -66,8 +66,11 @@ struct Params {
   unsigned long long* sw;  // support words of the pre-batch cascade (zero between batches)
   unsigned long long* ring;  // work ring of the repair phases (kSent between phases)
   uint32_t ring_mask;
+  uint32_t rq_base;        // slot of the current epoch's first item (sync_rounds)
+  uint32_t touched_base;   // length of the touched list before touched_n counts
   uint32_t* rq_head;       // ring counters, each on its own 128-byte line: the
-  uint32_t* rq_tail;       // idle blocks poll them while the working ones push
+  uint32_t* rq_tail0;      // idle blocks poll them while the working ones push
+  uint32_t* rq_tail;       // the current epoch's (rq_tail0 + epoch)
   uint32_t* rq_done;
   uint32_t* rq_fin;        // set by the first block that sees the phase finished
   unsigned long long* rq_stat;  // drain statistics of the last phase (own line)
@@ -1065,7 +1068,7 @@ constexpr uint32_t kDrainIdleLimit = 1u << 20;  // idle rounds of a block (up to
 
 __device__ __forceinline__ void ring_push(const Params& p, bool pred, unsigned long long item) {
   const uint32_t s = vxb::warp_append(pred, p.rq_tail);  // warp-uniform
-  if (pred) __stcg(&p.ring[s & p.ring_mask], item);
+  if (pred) __stcg(&p.ring[(p.rq_base + s) & p.ring_mask], item);
 }
 
 __device__ __forceinline__ uint32_t item_vertex(unsigned long long it) { return (uint32_t)it & ~kKindBit; }
@@ -1099,7 +1102,7 @@ __device__ void block_rows(const DevAdj& a, const T* items, uint32_t n, LbStage&
       const uint32_t lo = c * kChunk, hi = min(total, lo + kChunk);
       if (c == 0 && total > kChunk) {  // hand the other chunks to other blocks
         const uint32_t more = (total - 1) / kChunk;
-        const uint32_t s0 = atomicAdd(p->rq_tail, more);
+        const uint32_t s0 = p->rq_base + atomicAdd(p->rq_tail, more);
         for (uint32_t k = 0; k < more; ++k)
           __stcg(&p->ring[(s0 + k) & p->ring_mask], ((unsigned long long)it & 0xFFFFFFFFull) |
                                                         ((unsigned long long)(k + 1) << 32));
@@ -1171,19 +1174,23 @@ __device__ void block_rows(const DevAdj& a, const T* items, uint32_t n, LbStage&
 // The words a repair phase decides by, as of the last grid barrier.
 struct RepairWords {
   unsigned long long deadline;
-  uint32_t failed, touched, affected, fallback, cbig, rbig, tail, big_b, later, raw_f[2];
+  uint32_t failed, candidates, touched, affected, fallback, cbig, rbig, tail, big_b, later, raw_f[2];
 };
 
 // Grid barrier of the repair phases: thread 0 of each block loads the words
 // above once, all in flight together (each phase loading what it needs in
 // every thread cost a dependent round trip per word and thousands of requests
-// for one line).  False once any block recorded a device error.
+// for one line).  A block may load them while another is already in the next
+// phase, so a word may be used only where the next phase does not change it, or
+// only in a direction that does not change what is decided by it.  False once
+// any block recorded a device error.
 __device__ __forceinline__ bool sync_words(const Params& p, RepairWords& w) {
   BfsCounters* c = p.c;
   vxb::grid_barrier_then(p.bar, p.nblocks, &c->err, [&] {
     RepairWords r;
     r.failed = __ldcg(&c->err);
-    r.touched = ld_cg(&c->touched_n);
+    r.candidates = ld_cg(&c->cand_n);
+    r.touched = p.touched_base + ld_cg(&c->touched_n);
     r.affected = ld_cg(&c->a_n);
     r.fallback = ld_cg(&c->fallback);
     r.cbig = ld_cg(&c->cbig);
@@ -1265,12 +1272,12 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
         }
         const uint32_t k = cur + lane;
         unsigned long long v = kSent;
-        if (k < end) v = __ldcg(&p.ring[k & p.ring_mask]);
+        if (k < end) v = __ldcg(&p.ring[(p.rq_base + k) & p.ring_mask]);
         const uint32_t have = __ballot_sync(FULL, v != kSent);
         n = have == FULL ? 32u : (uint32_t)(__ffs(~have) - 1);  // leading filled slots
         if ((uint32_t)lane < n) {
           sm.items[lane] = v;
-          __stcg(&p.ring[k & p.ring_mask], kSent);
+          __stcg(&p.ring[(p.rq_base + k) & p.ring_mask], kSent);
         }
         cur += n;
         if (n == 0) {
@@ -1333,31 +1340,40 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
 // handles an item (whole warp) that it has taken out of the ring.  sm.w is of
 // the last barrier; true when the ring is empty, false to drain (or on an
 // error, sm.w.failed).
+//
+// What a round pushes is an epoch of its own, with its own length word and the
+// slots behind the epoch before: a block that is late to read a round's length
+// must not see pushes of the next round in it.  (A first epoch that is drained
+// only grows, past the limit that sends it to the drain.)
 constexpr uint32_t kSyncRounds = 2;
 
+__device__ __forceinline__ void ring_epoch(Params& p, uint32_t epoch, uint32_t base) {
+  p.rq_tail = p.rq_tail0 + epoch;
+  p.rq_base = base;
+}
+
 template <class W>
-__device__ bool sync_rounds(const Params& p, RepairSmem& sm, W& w) {
+__device__ bool sync_rounds(Params& p, RepairSmem& sm, W& w) {
   if (p.handover == 0.0f) return false;  // hands over at its first drain round
-  uint32_t lo = 0;
   for (uint32_t r = 0; r < kSyncRounds; ++r) {
-    const uint32_t hi = sm.w.tail;
-    if (lo == hi) return true;
-    if (hi - lo > gridDim.x || sm.w.fallback) return false;
-    if (gtid() == 0) *p.rq_head = *p.rq_done = hi;  // a drain starts behind them
-    const uint32_t i = lo + dealt_warp();
-    if (i < hi) {
-      const unsigned long long it = __ldcg(&p.ring[i & p.ring_mask]);
+    const uint32_t lo = p.rq_base, n = sm.w.tail;
+    if (n == 0) return true;
+    if (n > gridDim.x) return false;
+    ring_epoch(p, r + 1, lo + n);
+    const uint32_t i = dealt_warp();
+    if (i < n) {
+      unsigned long long* slot = &p.ring[(lo + i) & p.ring_mask];
+      const unsigned long long it = __ldcg(slot);
       __syncwarp();
       if ((threadIdx.x & 31) == 0) {
-        __stcg(&p.ring[i & p.ring_mask], kSent);
+        __stcg(slot, kSent);
         acct_add(p, 1, 1);
       }
       w.one(it);
     }
-    lo = hi;
     if (!sync_words(p, sm.w)) return false;
   }
-  return sm.w.tail == lo;
+  return sm.w.tail == 0;
 }
 
 // --------------------------------------------------- pre-batch fixpoint --
@@ -1419,8 +1435,8 @@ __device__ __forceinline__ void request_check(const Params& p, bool pred, uint32
   bf = __shfl_sync(FULL, bf, lf);
   bp = __shfl_sync(FULL, bp, lp);
   const uint32_t lt = vxb::lanemask_lt();
-  if (first) p.lst_t[bf + __popc(mf & lt)] = x;
-  if (push) __stcg(&p.ring[(bp + __popc(mp & lt)) & p.ring_mask], (unsigned long long)x);
+  if (first) p.lst_t[p.touched_base + bf + __popc(mf & lt)] = x;
+  if (push) __stcg(&p.ring[(p.rq_base + bp + __popc(mp & lt)) & p.ring_mask], (unsigned long long)x);
 }
 
 // expand(y) for a newly affected y at distance dy, applied to one arc (y, x)
@@ -1722,10 +1738,11 @@ struct Cascade {
   }
 };
 
-__device__ void reset_ring(const Params& p) {
+__device__ void reset_ring(Params& p) {
+  ring_epoch(p, 0, 0);
   if (gtid() == 0) {
     *p.rq_head = 0;
-    *p.rq_tail = 0;
+    for (uint32_t k = 0; k <= kSyncRounds; ++k) p.rq_tail0[k] = 0;
     *p.rq_done = 0;
     *p.rq_fin = 0;
     for (int k = 0; k < 6; ++k) p.rq_stat[k] = 0;
@@ -1774,7 +1791,7 @@ __device__ void clear_workspace(const Params& p, uint32_t touched, uint32_t affe
 // affected list stays empty, so the post-batch repair only relaxes the
 // insertions.  The BFS distances go to tent (zero between phases), which the
 // comparison pass zeroes again.
-__device__ __noinline__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
+__device__ __noinline__ bool cascade_by_bfs(Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
   BfsCounters* c = p.c;
   clear_workspace(p, sm.w.touched, sm.w.affected);
   reset_ring(p);
@@ -1818,7 +1835,7 @@ __device__ __noinline__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, Blo
 // is drained only when a check left work in it (an affected vertex to expand,
 // chunks of a long in-row), which most small batches never do.  Records the
 // batch's affected count.
-__device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t ncand) {
+__device__ bool cascade(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t ncand) {
   if (gtid() == 0) set_deadline(p);
   for (uint32_t i = dealt_warp(); i < ncand; i += nwarps()) check_vertex<true>(p, p.lst_t[i]);
   if (!sync_words(p, sm.w)) return false;
@@ -1831,7 +1848,7 @@ __device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue
     }
   }
   if (gtid() == 0) {  // the drain statistics of the phase trace
-    p.c->rtrace[7] = sm.w.tail;
+    p.c->rtrace[7] = p.rq_base + sm.w.tail;
     for (int k = 0; k < 6; ++k) p.c->rtrace[9 + k] = __ldcg(&p.rq_stat[k]);
   }
   if (sm.w.cbig) return cascade_by_bfs(p, sm, bq, lb);
@@ -1839,7 +1856,7 @@ __device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue
   return true;
 }
 
-__device__ void repair_pre(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
+__device__ void repair_pre(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
   stamp(p, 0);
   reset_ring(p);
@@ -1889,7 +1906,7 @@ __device__ __forceinline__ void lower_and_push(const Params& p, bool lowered, ui
 __device__ __forceinline__ void push_one(const Params& p, uint32_t x) {
   const uint32_t bit = 1u << (x & 31);
   if (atomicOr(&p.inq[0][x >> 5], bit) & bit) return;
-  const uint32_t s = atomicAdd(p.rq_tail, 1u);
+  const uint32_t s = p.rq_base + atomicAdd(p.rq_tail, 1u);
   __stcg(&p.ring[s & p.ring_mask], (unsigned long long)x);
 }
 
@@ -2166,7 +2183,7 @@ __device__ __forceinline__ void invalidate(const Params& p, uint32_t na) {
 }
 
 template <bool kInvalidated>
-__device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
+__device__ bool repair_relax(Params& p, RepairSmem& sm, LbStage& lb) {
   BfsCounters* c = p.c;
   const int lane = threadIdx.x & 31;
   // the ring counters are zero here: the pre-batch kernel (or the previous
@@ -2174,7 +2191,10 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
   // kernel or a kernel boundary
   stamp(p, 3);
   if (gtid() == 0) set_deadline(p);
+  // the lists' lengths as of the barrier before: gtid 0 resets them once the
+  // repair is done, when another block may just be reading the last barrier's words
   const uint32_t na = kInvalidated ? sm.w.affected : ld_cg(&c->a_n);
+  const uint32_t nt = kInvalidated ? sm.w.touched : ld_cg(&c->touched_n);
   if (gtid() == 0) acct_add(p, 1, na);  // invalidated and re-seeded
   long long reach = 0;
   if (na > 0) {
@@ -2234,19 +2254,19 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
       // the relaxation passed its budget: a full BFS of the post-batch graph
       // gives the distances and the reachable count (the repair's counters
       // -- candidates, affected, no full recompute -- stand)
-      clear_workspace(p, sm.w.touched, sm.w.affected);
+      clear_workspace(p, nt, na);
       reset_ring(p);
       return true;
     }
   }
   stamp(p, 6);
   if (gtid() == 0) {
-    c->rtrace[8] = sm.w.tail;
+    c->rtrace[8] = p.rq_base + sm.w.tail;
     for (int k = 0; k < 6; ++k) c->rtrace[15 + k] = __ldcg(&p.rq_stat[k]);
   }
   reach = vxb::warp_sum(reach);
   if (lane == 0) reach_add(p, reach);
-  clear_workspace(p, sm.w.touched, sm.w.affected);
+  clear_workspace(p, nt, na);
   reset_ring(p);
   return false;
 }
@@ -2254,7 +2274,7 @@ __device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
 // Post-batch repair (bfs.hpp:72-97): the fallback's full BFS or the repair,
 // which may itself hand over to a full BFS; one call site serves both.
 template <bool kInvalidated>
-__device__ void repair_post(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
+__device__ void repair_post(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
   const bool fallback = kInvalidated ? sm.w.fallback != 0u : ld_cg(&c->fallback) != 0u;
   if (fallback) {
@@ -2669,14 +2689,14 @@ struct ArcWork {
   uint32_t dirtied;
 
   // A deletion candidate (bfs.hpp:52-63) is the head of a deleted
-  // shortest-parent arc; its first touch records it in the touched list, whose
-  // length after the pass is their number.  Warp-uniform.
+  // shortest-parent arc; its first touch records it at the front of the touched
+  // list.  Warp-uniform.
   __device__ __forceinline__ void candidate(bool arc, uint32_t u, uint32_t v, uint8_t f) {
     if (dir) return;
     bool first = false;
     if (arc && !(f & kFAdd) && (f & kFCur) && is_sp(*p, u, v))
       first = !(atomicOr(&p->sw[v], kSwTouched) & kSwTouched);
-    const uint32_t slot = vxb::warp_append(first, &p->c->touched_n);
+    const uint32_t slot = vxb::warp_append(first, &p->c->cand_n);
     if (first) p->lst_t[slot] = v;
   }
 
@@ -3044,7 +3064,7 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
       removal_pass(w, sm);
     }
     if (s.digest && bi > 0) digest_pass(p.dist, lpre, &s.digest[bi - 1]);
-    if (!sync_words(p, sm.w)) return;
+    if (!sync_words(q, sm.w)) return;
     phase(0);
     if (s.raw_n) {
       F = sm.w.raw_f[0];
@@ -3056,19 +3076,20 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
         w.pending = true;
         removal_pass(w, sm);
       }
-      if (!sync_words(p, sm.w)) return;
+      if (!sync_words(q, sm.w)) return;
     }
     if (sm.w.later & kLaterRuns) {
       for (int dir = 0; dir < ndir; ++dir) {
         ArcWork w = work(dir);
         removal_runs(w, sm);
       }
-      if (!sync_words(p, sm.w)) return;
+      if (!sync_words(q, sm.w)) return;
     }
     phase(1);
     stamp(q, 1);
     // B: the cascade over the graph without the batch's deletions
-    const uint32_t ncand = sm.w.touched;
+    const uint32_t ncand = sm.w.candidates;
+    q.touched_base = ncand;
     if (gtid() == 0) {
       // last_* counters (bfs.hpp:30-33); the last reader of the previous
       // batch's was this thread, at its end
@@ -3093,7 +3114,7 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     }
     for (uint32_t v = lpre + gtid(); v < Vpost; v += nthreads()) p.dist[v] = kUnreachable;
     if (!sm.w.cbig && !sm.w.fallback) invalidate(q, sm.w.affected);
-    if (!sync_words(p, sm.w)) return;
+    if (!sync_words(q, sm.w)) return;
     phase(3);
     // D: the post-batch repair (or the fallback full BFS) on the new graph
     q.V = Vpost;
@@ -3103,7 +3124,7 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     // the repair lists start empty in the next batch (and launch); every block
     // has their lengths in sm.w
     if (gtid() == 0) {
-      c->touched_n = c->a_n = c->fallback = c->later = 0;
+      c->cand_n = c->touched_n = c->a_n = c->fallback = c->later = 0;
       p.bar[kRawWord] = p.bar[kRawWord + 1] = 0u;
     }
     if (bi + 1 == s.nb && !s.digest && !s.bstats) break;
@@ -3365,7 +3386,7 @@ static Params make_params(Bfs* b, uint32_t V, uint32_t dist_len) {
   p.ring = b->ring;
   p.ring_mask = b->ring_slots ? (uint32_t)(b->ring_slots - 1) : 0u;
   p.rq_head = b->rq;
-  p.rq_tail = b->rq + 32;
+  p.rq_tail = p.rq_tail0 = b->rq + 32;
   p.rq_done = b->rq + 64;
   p.rq_fin = b->rq + 128;
   p.rq_stat = reinterpret_cast<unsigned long long*>(b->rq + 96);
