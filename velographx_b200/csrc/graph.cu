@@ -10,6 +10,7 @@
 //     delta entry removed again;
 //   * compact (:633-639): the overlay is merged into a fresh base CSR.
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 
 #include "graph.cuh"
@@ -646,13 +647,15 @@ int graph_create(Graph** out, size_t vertices, bool directed) {
   if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&g->ctr, sizeof(GraphCounters)) != cudaSuccess ||
       cudaMallocHost(&g->hctr, sizeof(GraphCounters)) != cudaSuccess ||
-      cudaMallocHost(&g->pinned_scalar, 4096) != cudaSuccess) {
+      cudaMallocHost(&g->pinned_scalar, 4096) != cudaSuccess ||
+      cudaEventCreateWithFlags(&g->arena_ev, cudaEventDisableTiming) != cudaSuccess) {
     set_error("CUDA initialisation failed: %s", cudaGetErrorString(cudaGetLastError()));
     graph_destroy(g);
     return -3;
   }
   cudaMemsetAsync(g->ctr, 0, sizeof(GraphCounters), g->stream);
   memset(g->hctr, 0, sizeof(GraphCounters));
+  g->arena_tops = g->pinned_scalar + 256;  // the other readbacks stay below it
   g->arena_limit_entries = (size_t)1 << 28;
   const int ndir = directed ? 2 : 1;
   for (int d = 0; d < ndir; ++d) {
@@ -682,14 +685,20 @@ void graph_destroy(Graph* g) {
   cudaFree(g->ctr);
   cudaFreeHost(g->hctr);
   cudaFreeHost(g->pinned_scalar);
+  if (g->arena_ev) cudaEventDestroy(g->arena_ev);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }
 
+// A bound of arena_top for which room has been made when nothing else is
+// inserted (see reserve_arena): the rows' next blocks.
+static uint64_t arena_bound_from(uint64_t top, uint64_t live) { return top + 4 * live; }
+
 int graph_sync_counters(Graph* g) {
   VX_CUDA_TRY(cudaMemcpyAsync(g->hctr, g->ctr, sizeof(GraphCounters), cudaMemcpyDeviceToHost, g->stream));
   VX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  for (int d = 0; d < 2; ++d) g->adj[d].arena_bound = std::max<uint64_t>(g->hctr->arena_top[d], 0);
+  for (int d = 0; d < 2; ++d) g->adj[d].arena_bound = arena_bound_from(g->hctr->arena_top[d], g->hctr->delta_live[d]);
+  g->arena_pending = false;  // an older readback says less
   if (g->hctr->err) {
     const uint32_t e = g->hctr->err;
     set_error("device error word 0x%x (%s%s%s%s)", e, (e & vxb::kErrBadVertex) ? "vertex id out of bound " : "",
@@ -729,6 +738,7 @@ static int build_adjacency(Graph* g, Adjacency& a, uint64_t* keys, size_t m, int
   VX_CUDA_TRY(cudaGetLastError());
   a.Vb = (uint32_t)g->V;
   a.A = A;
+  g->arena_pending = false;
   VX_CUDA_TRY(cudaMemsetAsync(a.drow, 0, g->Vcap * sizeof(uint2), s));
   VX_CUDA_TRY(cudaMemsetAsync(a.dcap, 0, g->Vcap * sizeof(uint32_t), s));
   VX_CUDA_TRY(cudaMemsetAsync(a.tcnt, 0, g->Vcap * sizeof(uint32_t), s));
@@ -793,16 +803,80 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
   return 0;
 }
 
-// Reserve arena room for `arcs` insertions in adjacency a (host-side bound:
-// a row's blocks sum to < 8 entries per insertion ever made into it).
-static int reserve_arena(Graph* g, Adjacency& a, size_t arcs, int* need_consolidate) {
-  const uint64_t need = a.arena_bound + 8ull * arcs + 8;
-  if (need <= a.arena_cap) return 0;
-  if (need > g->arena_limit_entries || need >= 0xFFFFFFF0ull) {
-    *need_consolidate = 1;
+// ---- arena room ----
+// The host bounds arena_top by 8 entries per arc ever inserted: a row without a
+// block takes 8, and the blocks of a row that outgrows them double, so they sum
+// to less than 4 times its entries.  Almost all arcs find room in the block
+// their row has, and the bound alone would grow the arena fourfold every few dozen batches
+// and consolidate the graph in the end (100,000-op batches at R-MAT 20: to 1 GB
+// and a consolidation every 160 batches, calls of 4 to 95 ms, now and then
+// hundreds on a busy host).  So the top and the live entries are read back when
+// half of the room is used up by it: a 32-byte copy on the stream, looked at
+// when it has arrived.  From then on the rows that hold those entries can take
+// at most 4 times them in new blocks, before the 8 per further arc.
+
+static_assert(offsetof(GraphCounters, delta_live) == 16 && offsetof(GraphCounters, arena_top) == 0,
+              "one copy reads the tops and the live entries");
+
+// Enqueues the readback (not while the stream is being captured).
+static int arena_ask(Graph* g) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (g->arena_pending || cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     return 0;
+  VX_CUDA_TRY(cudaMemcpyAsync(g->arena_tops, g->ctr->arena_top, 32, cudaMemcpyDeviceToHost, g->stream));
+  VX_CUDA_TRY(cudaEventRecord(g->arena_ev, g->stream));
+  for (int d = 0; d < 2; ++d) g->arena_seen[d] = g->adj[d].arena_bound;
+  g->arena_pending = true;
+  return 0;
+}
+
+// Takes a readback into the bounds, if one is in flight and has arrived (or,
+// with wait, when it has).
+static int arena_take(Graph* g, bool wait) {
+  if (!g->arena_pending) return 0;
+  if (wait) {
+    VX_CUDA_TRY(cudaEventSynchronize(g->arena_ev));
+  } else {
+    const cudaError_t e = cudaEventQuery(g->arena_ev);
+    if (e == cudaErrorNotReady) return 0;
+    VX_CUDA_TRY(e);
   }
-  return grow_arena(a, need, g->stream);
+  for (int d = 0; d < 2; ++d)
+    g->adj[d].arena_bound = arena_bound_from(g->arena_tops[d], g->arena_tops[2 + d]) +
+                            (g->adj[d].arena_bound - g->arena_seen[d]);
+  g->arena_pending = false;
+  return 0;
+}
+
+// Room for `arcs` insertions in every adjacency: *need_consolidate when the
+// arena would pass its limit.
+static int reserve_arena(Graph* g, size_t arcs, int* need_consolidate) {
+  const int ndir = g->directed ? 2 : 1;
+  const uint64_t add = 8ull * arcs + 8;
+  if (int rc = arena_take(g, false)) return rc;
+  bool over = false, half = false;
+  for (int d = 0; d < ndir; ++d) {
+    over = over || g->adj[d].arena_bound + add > g->adj[d].arena_cap;
+    half = half || g->adj[d].arena_bound + add > g->adj[d].arena_cap / 2;
+  }
+  if (over) {
+    if (int rc = arena_ask(g)) return rc;
+    if (int rc = arena_take(g, true)) return rc;
+  } else if (half) {
+    if (int rc = arena_ask(g)) return rc;
+  }
+  for (int d = 0; d < ndir; ++d) {
+    Adjacency& a = g->adj[d];
+    const uint64_t need = a.arena_bound + add;
+    // a top that takes up half of the room is asked for with every batch: grow
+    if (need <= a.arena_cap && !(over && need > a.arena_cap / 2)) continue;
+    if (need > g->arena_limit_entries || need >= 0xFFFFFFF0ull) {
+      if (need > a.arena_cap) *need_consolidate = 1;
+      continue;
+    }
+    if (int rc = grow_arena(a, need, g->stream)) return rc;
+  }
+  return 0;
 }
 
 // Arena room for a whole update stream whose batches insert at most
@@ -812,6 +886,10 @@ static int reserve_arena(Graph* g, Adjacency& a, size_t arcs, int* need_consolid
 int graph_reserve_stream(Graph* g, uint64_t entries, int* fits) {
   *fits = 1;
   Adjacency& a = g->adj[0];
+  if (a.arena_bound + entries + 8 > a.arena_cap) {
+    if (int rc = arena_ask(g)) return rc;
+    if (int rc = arena_take(g, true)) return rc;
+  }
   if (a.arena_bound + entries + 8 > g->arena_limit_entries || a.arena_bound + entries + 8 >= 0xFFFFFFF0ull) {
     if (int rc = graph_consolidate(g)) return rc;
     if (a.arena_bound + entries + 8 > g->arena_limit_entries || a.arena_bound + entries + 8 >= 0xFFFFFFF0ull) {
@@ -836,12 +914,10 @@ int graph_prepare_batch(Graph* g, size_t n, size_t vertex_bound) {
   const size_t m = g->directed ? n : 2 * n;
   // arena room (consolidate first if the bound passed the limit)
   int consolidate = 0;
-  for (int d = 0; d < (g->directed ? 2 : 1); ++d)
-    if (int rc = reserve_arena(g, g->adj[d], m, &consolidate)) return rc;
+  if (int rc = reserve_arena(g, m, &consolidate)) return rc;
   if (consolidate) {
     if (int rc = graph_consolidate(g)) return rc;
-    for (int d = 0; d < (g->directed ? 2 : 1); ++d)
-      if (int rc = reserve_arena(g, g->adj[d], m, &consolidate)) return rc;
+    if (int rc = reserve_arena(g, m, &consolidate)) return rc;
   }
   return graph_grow(g, std::max<size_t>(g->V, vertex_bound));
 }
@@ -1015,6 +1091,7 @@ int graph_consolidate(Graph* g) {
     a.col_cap = A;
     a.Vb = V;
     a.A = A;
+    g->arena_pending = false;
     VX_CUDA_TRY(cudaMemsetAsync(a.drow, 0, g->Vcap * sizeof(uint2), s));
     VX_CUDA_TRY(cudaMemsetAsync(a.dcap, 0, g->Vcap * sizeof(uint32_t), s));
     VX_CUDA_TRY(cudaMemsetAsync(a.tcnt, 0, g->Vcap * sizeof(uint32_t), s));

@@ -14,7 +14,7 @@ namespace vxh {
 // Device counters of one graph; lives in device memory, mirrored to pinned
 // host memory on demand.
 struct GraphCounters {
-  unsigned long long arena_top[2];   // per direction (0 = out, 1 = in)
+  unsigned long long arena_top[2];   // per direction (0 = out, 1 = in); read back with the next two
   unsigned long long delta_live[2];  // delta entries (overlay "present")
   unsigned long long tombs[2];       // tombstoned base arcs (overlay "absent")
   unsigned long long dirty_rows[2];  // rows touched since last compaction
@@ -96,6 +96,12 @@ struct Graph {
   uint64_t* pinned_scalar = nullptr;  // small pinned buffer for readbacks
   size_t batch_ops = 0;               // ops of the batch currently staged
   size_t arena_limit_entries = 0;     // consolidate instead of growing past this
+  // a readback of arena_top and delta_live in flight (arena_tops, pinned), and
+  // the bounds when it was enqueued
+  cudaEvent_t arena_ev = nullptr;
+  uint64_t* arena_tops = nullptr;
+  uint64_t arena_seen[2] = {0, 0};
+  bool arena_pending = false;
 
   Adjacency& in() { return directed ? adj[1] : adj[0]; }
   vxb::DevGraph view();
