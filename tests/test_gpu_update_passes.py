@@ -1,8 +1,8 @@
 """GPU: the update launch's passes against the per-phase path, directed and
 undirected, at the batch sizes where they change: one op, the most ops the
-launch canonicalises itself and one more, up to and past two arcs per warp
-(2 x 2,368 on 148 SMs), past one cluster's canonicalisation; with hub rows (runs of
-several arcs, delta rows of more than 8 and 32 arcs), repeated ops on one
+launch canonicalises itself (16,384) and one more, past one cluster's
+canonicalisation; with hub rows (runs of several arcs, blocks with more arcs
+than they process or sort at once, one arc repeated more often than that, delta rows of more than 8 and 32 arcs), repeated ops on one
 arc, self-loops, growth, and batches that undo the one before.  After every
 batch: distances, counters, edge and delta counts, dirty rows, and the rows
 of touched vertices in both directions; at the end the mirrored edge set."""
@@ -13,6 +13,22 @@ import workloads as w
 
 pytestmark = pytest.mark.gpu
 vx = pytest.importorskip("velographx_b200")
+
+
+def star_batches(rng, V, e, ops):
+    """Most ops on one row; then half of a batch on one arc."""
+    out = []
+    for t in range(2):
+        s = np.full(ops, 3, np.uint32)
+        d = rng.integers(0, V, ops, dtype=np.uint32)
+        s[: ops // 8] = rng.integers(0, V, ops // 8, dtype=np.uint32)
+        a = (rng.random(ops) < 0.8).astype(np.uint8)
+        p = rng.permutation(ops)
+        out += [(s[p], d[p], a[p]), (s[p], d[p], (1 - a[p]).astype(np.uint8))]
+        d = d.copy()
+        d[ops // 8: ops // 8 + ops // 2] = 17
+        out += [(s, d, a), (s[::-1].copy(), d[::-1].copy(), a[::-1].copy())]
+    return out
 
 
 def batches(rng, V, e, ops):
@@ -39,8 +55,9 @@ def batches(rng, V, e, ops):
 
 
 @pytest.mark.parametrize("directed", [False, True])
-@pytest.mark.parametrize("ops", [1, 33, 511, 512, 513, 1024, 1025, 2368, 4800, 46000])
-def test_passes_match_the_per_phase_path(ops, directed):
+@pytest.mark.parametrize("star,ops", [(False, n) for n in (1, 33, 512, 1024, 2368, 4800, 16384, 16385, 46000)] +
+                         [(True, n) for n in (600, 2100, 2500, 9000, 16384)])
+def test_passes_match_the_per_phase_path(star, ops, directed):
     rng = np.random.default_rng(ops + directed)
     V = 20_011
     e = w.rmat_edges(14, 8, seed=3)
@@ -54,7 +71,7 @@ def test_passes_match_the_per_phase_path(ops, directed):
         b = vx.IncrementalBFS(g, int(e[0, 0]))
         b.set_fused(fused)
         pair.append((g, b))
-    for t, (s, d, a) in enumerate(batches(rng, V, e, ops)):
+    for t, (s, d, a) in enumerate((star_batches if star else batches)(rng, V, e, ops)):
         for u, v, x in zip(s.tolist(), d.tolist(), a.tolist()):
             if u == v:
                 continue

@@ -2339,20 +2339,24 @@ struct StreamArgs {
 // them, keeps the last of each arc and appends them to the batch's list, so
 // the arcs of a row are consecutive there and the block that has them in
 // shared memory can process them at once.  A launch of its own with a cluster's
-// barriers between the radix passes took 12 to 21 us; every block sorting
+// barriers between the radix passes took 12 to 44 us; every block sorting
 // all arcs 2 us for 128 arcs but 7 for 1,024 and 13 for 2,048, bound by the
-// instructions of the one block an SM runs; now 2 to 3.
-constexpr uint32_t kRawOps = 1024;
+// instructions of the one block an SM runs; now 2 to 8 (10,000 ops).  The limit keeps a
+// block's reading (9 bytes an op from L2) at a few microseconds.
+constexpr uint32_t kRawOps = 16384;
+constexpr uint32_t kRawKeys = 2048;  // arcs a block sorts at once (canon_long beyond)
 constexpr unsigned long long kRawDir = 1ull << 63;  // a directed graph's reversed arcs sort last
 // A block with more arcs than this (hub rows) leaves them to the whole grid,
-// behind a barrier: its 16 warps take one arc each at a time.
-constexpr uint32_t kRawMine = 64;
+// behind a barrier; with more than kRawWarps it gives each a lane, not a warp.
+constexpr uint32_t kRawMine = 1024;
+constexpr uint32_t kRawWarps = 32;
 constexpr uint8_t kFPending = 0x80;  // flag of an arc left to the grid
+constexpr uint8_t kFDead = 0x40;     // flag of a list slot without an arc of its own
 struct RawArcs {
-  unsigned long long key[2 * kRawOps];  // [dir] | u | v | op index | add
+  unsigned long long key[kRawKeys];  // [dir] | u | v | op index | add
   uint32_t wsum[kThreads / 32];
-  uint32_t n[2];                        // arcs, and those of direction 0 among them
-  uint32_t base[2];                     // their places in the batch's lists
+  uint32_t n[2];                     // arcs, and those of direction 0 among them
+  uint32_t base[2];                  // their places in the batch's lists
 };
 static_assert(sizeof(RawArcs) <= sizeof(LbStage), "the arcs are kept in the row stage's memory");
 
@@ -2489,17 +2493,16 @@ __device__ void canon_sort(const StreamArgs& s, bool directed, RawArcs& r, uint3
   __syncthreads();
 }
 
-// The block's arcs of the batch in r, and their places in the batch's lists
-// (whose lengths are f[0] and f[1], zero before).  Block-uniform.
-__device__ void canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32_t* f) {
-  if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
-  __syncthreads();
+// The keys of the batch's arcs that are this block's, f(key) each (a lane at a
+// time).  first: reports ids out of bound.
+template <class F>
+__device__ __forceinline__ void raw_scan(const StreamArgs& s, bool directed, bool first, F&& f) {
   for (uint32_t i = threadIdx.x; i < s.raw_n; i += kThreads) {
     const uint32_t a = s.raw_src[i], b = s.raw_dst[i];
     const unsigned long long low = ((unsigned long long)i << 1) | (s.raw_add[i] ? 1ull : 0ull);
     bool ok = a != b;
     if (ok && (a >= s.raw_bound || b >= s.raw_bound)) {
-      if (blockIdx.x == 0) atomicOr(&s.gc->err, vxb::kErrBadVertex);
+      if (first && blockIdx.x == 0) atomicOr(&s.gc->err, vxb::kErrBadVertex);
       ok = false;
     }
     if (!ok) continue;
@@ -2507,24 +2510,125 @@ __device__ void canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32
     for (int rev = 0; rev < 2; ++rev) {
       const unsigned long long u = rev ? b : a, v = rev ? a : b;
       if (__umulhi((uint32_t)u * 0x9E3779B1u, gridDim.x) != blockIdx.x) continue;
-      r.key[atomicAdd(&r.n[0], 1u)] =
-          (directed && rev ? kRawDir : 0ull) | (u << (s.raw_b + s.raw_sh)) | (v << s.raw_sh) | low;
+      f((directed && rev ? kRawDir : 0ull) | (u << (s.raw_b + s.raw_sh)) | (v << s.raw_sh) | low);
     }
   }
-  __syncthreads();
-  const uint32_t n = r.n[0];
-  __syncthreads();
+}
+
+__device__ void canon_keys(const StreamArgs& s, bool directed, RawArcs& r, uint32_t n) {
   uint32_t N = 32;
   while (N < n) N <<= 1;
-  static_assert(2 * kRawOps == 4 * kThreads, "four keys per thread at most");
+  static_assert(kRawKeys == 4 * kThreads, "four keys per thread at most");
   if (N <= kThreads) canon_sort<1>(s, directed, r, n, N);
   else if (N <= 2 * kThreads) canon_sort<2>(s, directed, r, n, N);
   else canon_sort<4>(s, directed, r, n, N);
+}
+
+// A block's n arcs that do not fit its shared memory (a batch most of whose ops
+// share a row): listed in ascending ranges of their (dir, u, v) value that do,
+// halved and doubled as they come, each found by another scan of the ops.  Slow
+// (some 20 us for 1,000 arcs) but for any batch.  The arcs are left to the
+// grid; slots that repeated ops on an arc leave over hold a copy without effect.
+__device__ __noinline__ void canon_long(const StreamArgs& s, bool directed, RawArcs& r) {
+  const uint32_t bits = 2 * s.raw_b;
+  auto value = [&](unsigned long long key) {
+    return ((key & ~kRawDir) >> s.raw_sh) | (key & kRawDir ? 1ull << bits : 0ull);
+  };
+  const unsigned long long top = (directed ? 2ull : 1ull) << bits;
+  uint32_t place[2] = {r.base[0], r.base[1]}, end[2];
+  end[0] = place[0] + r.n[1];
+  end[1] = place[1] + (r.n[0] - r.n[1]);
+  unsigned long long lo = 0, width = top;
+  __syncthreads();  // r.n and r.base are read
+  while (lo < top) {
+    const unsigned long long hi = top - lo < width ? top : lo + width;
+    if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+    __syncthreads();
+    raw_scan(s, directed, false, [&](unsigned long long key) {
+      const unsigned long long x = value(key);
+      if (x < lo || x >= hi) return;
+      const uint32_t k = atomicAdd(&r.n[0], 1u);
+      if (k < kRawKeys) r.key[k] = key;
+    });
+    __syncthreads();
+    uint32_t n = r.n[0];
+    __syncthreads();
+    if (n > kRawKeys && hi - lo > 1) {
+      width = (hi - lo + 1) / 2;
+      continue;
+    }
+    if (n > kRawKeys) {  // one arc, more ops than fit: its last op
+      if (threadIdx.x == 0) r.key[0] = 0;
+      __syncthreads();
+      raw_scan(s, directed, false, [&](unsigned long long key) {
+        if (value(key) == lo) atomicMax(&r.key[0], key);
+      });
+      __syncthreads();
+      n = 1;
+    }
+    if (n) {
+      if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+      __syncthreads();
+      canon_keys(s, directed, r, n);
+      const uint32_t kept = r.n[0], kept0 = r.n[1];
+      for (uint32_t i = threadIdx.x; i < kept; i += kThreads) {
+        const int dir = i >= kept0;
+        const uint32_t at = place[dir] + i - (dir ? kept0 : 0u);
+        const unsigned long long k = r.key[i];
+        const_cast<uint32_t*>(s.fu[dir])[at] = (uint32_t)((k & ~kRawDir) >> (s.raw_b + s.raw_sh));
+        const_cast<uint32_t*>(s.fv[dir])[at] = (uint32_t)(k >> s.raw_sh) & ((1u << s.raw_b) - 1u);
+        s.ff[dir][at] = (uint8_t)(k & 1ull) | kFPending;
+      }
+      place[0] += kept0;
+      place[1] += kept - kept0;
+      __syncthreads();
+    }
+    if (n < kRawKeys / 2 && width <= top / 2) width *= 2;
+    lo = hi;
+  }
+  for (int dir = 0; dir < (directed ? 2 : 1); ++dir)
+    for (uint32_t at = place[dir] + threadIdx.x; at < end[dir]; at += kThreads) {
+      const_cast<uint32_t*>(s.fu[dir])[at] = s.fu[dir][place[dir] - 1];
+      const_cast<uint32_t*>(s.fv[dir])[at] = s.fv[dir][place[dir] - 1];
+      s.ff[dir][at] = kFDead;
+    }
+}
+
+// The block's arcs of the batch in r, and their places in the batch's lists
+// (whose lengths are f[0] and f[1], zero before); true when the block has too
+// many and listed them itself, all pending.  Block-uniform.
+__device__ bool canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32_t* f) {
+  if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+  __syncthreads();
+  raw_scan(s, directed, true, [&](unsigned long long key) {
+    const uint32_t k = atomicAdd(&r.n[0], 1u);
+    if (k < kRawKeys) r.key[k] = key;
+  });
+  __syncthreads();
+  const uint32_t n = r.n[0];
+  __syncthreads();
+  const bool fits = n <= kRawKeys;
+  if (fits) {
+    if (threadIdx.x == 0) r.n[0] = 0;
+    __syncthreads();
+    canon_keys(s, directed, r, n);
+  } else {
+    raw_scan(s, directed, false, [&](unsigned long long key) {
+      if (!(directed && (key & kRawDir))) atomicAdd(&r.n[1], 1u);
+    });
+    __syncthreads();
+  }
   if (threadIdx.x < 2) {
     const uint32_t k = threadIdx.x ? r.n[0] - r.n[1] : r.n[1];
     r.base[threadIdx.x] = k ? atomicAdd(&f[threadIdx.x], k) : 0u;
   }
   __syncthreads();
+  if (fits) return false;
+  canon_long(s, directed, r);
+  __syncthreads();
+  if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+  __syncthreads();
+  return true;
 }
 
 // Order-independent 64-bit digest of dist[0, n): sum of splitmix64(v << 32 | dist[v]).
@@ -2787,7 +2891,7 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
   const uint32_t lane = threadIdx.x & 31;
   bool multi = false;  // a delta removal left to removal_runs
   const uint32_t base = w.base;
-  if (w.raw || w.F <= 2 * nwarps()) {
+  if (w.raw ? w.F <= kRawWarps : w.F <= 2 * nwarps()) {
     for (uint32_t i = w.raw ? threadIdx.x >> 5 : dealt_warp(); i < w.F; i += w.raw ? kThreads / 32 : nwarps()) {
       uint32_t u, v;
       uint8_t f;
@@ -2841,10 +2945,10 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
       }
     }
   } else {
-    for (uint32_t r0 = 0; r0 < w.F; r0 += nthreads()) {
+    for (uint32_t r0 = 0; r0 < w.F; r0 += w.raw ? kThreads : nthreads()) {
       if (threadIdx.x == 0) sm.nsv = 0;
       __syncthreads();
-      const uint32_t i = r0 + dealt_thread();
+      const uint32_t i = r0 + (w.raw ? threadIdx.x : dealt_thread());
       bool act = i < w.F && !(w.pending && !(w.ff[i] & kFPending));
       bool queue = false;
       uint32_t u = 0, v = 0;
@@ -2872,10 +2976,10 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
           }
           if (cur) f |= kFCur;
           if (cur != ((f & kFAdd) != 0)) f |= kFChanged;
-          w.ff[i] = f;
-          w.fpos[i] = q;
+          w.ff[base + i] = f;
+          w.fpos[base + i] = q;
         } else {
-          q = w.fpos[i];
+          q = w.fpos[base + i];
         }
         w.tombs += gdev::tomb_arc(a, u, f, q, 0, w.dirtied);
         if (delta_op(f, false)) {
@@ -2899,7 +3003,7 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
       w.candidate(act, u, v, f);
       dlive = vxb::warp_sum(dlive);
       if (lane == 0 && dlive) atomicAdd(&w.s->gc->delta_live[w.dir], (unsigned long long)dlive);
-      if (queue) sm.sv[atomicAdd(&sm.nsv, 1u)] = i;
+      if (queue) sm.sv[atomicAdd(&sm.nsv, 1u)] = base + i;
       __syncthreads();
       const uint32_t nq = sm.nsv;
       for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k], sm.sv[k] + 1);
@@ -3030,7 +3134,7 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     RawArcs& raw = reinterpret_cast<RawArcs&>(lb);
     uint32_t off = 0, F = 0, Frev = 0;
     if (s.raw_n) {
-      canon_raw(s, p.g.directed, raw, p.bar + kRawWord);
+      if (canon_raw(s, p.g.directed, raw, p.bar + kRawWord) && threadIdx.x == 0) atomicOr(&c->later, kLaterArcs);
     } else {
       if (s.boff) off = s.boff[bi];
       F = s.cnt[0][bi];
@@ -3614,8 +3718,11 @@ int bfs_accounting(Bfs* b, unsigned long long* out5) {
   return 0;
 }
 
-constexpr uint32_t kRawShift = 11;  // an op index below kRawOps and the add flag
-static_assert((1u << (kRawShift - 1)) >= kRawOps, "an op's index fits its bits");
+static int raw_shift(size_t n) {  // bits of an op's index and its add flag
+  int sh = 2;
+  while (((size_t)1 << (sh - 1)) < n) ++sh;
+  return sh;
+}
 
 static int raw_bits(size_t V) {  // bits of a vertex id below max(V, 2)
   int b = 1;
@@ -3638,9 +3745,9 @@ int bfs_stage(Bfs* b, size_t n, size_t vertex_bound, bool classify) {
   // paths on the host before their kernels
   b->staged_classified = classify;
   b->staged_raw = false;
-  if (!classify && n <= kRawOps) {  // keys of 2 * bits + kRawShift bits and the direction
+  if (!classify && n <= kRawOps) {  // keys of two ids, an op's index, its add flag and the direction
     if (int rc = graph_prepare_batch(g, n, vertex_bound)) return rc;
-    b->staged_raw = 2 * raw_bits(g->V) + (int)kRawShift <= 62;
+    b->staged_raw = 2 * raw_bits(g->V) + raw_shift(n) <= 62;
   }
   if (!b->staged_raw)
     if (int rc = graph_stage_batch(g, n, vertex_bound, classify)) return rc;
@@ -3715,7 +3822,7 @@ static int repair_fused(Bfs* b) {
     sa.raw_add = g->batch.in_add;
     sa.raw_n = (uint32_t)n;
     sa.raw_b = (uint32_t)raw_bits(g->V);
-    sa.raw_sh = kRawShift;
+    sa.raw_sh = (uint32_t)raw_shift(n);
     sa.raw_bound = (uint32_t)g->V;
     b->staged_raw = false;
   }
