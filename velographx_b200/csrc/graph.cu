@@ -785,7 +785,7 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
       }
     }
     bool in_alt = false;
-    rc = radix_sort_u64(keys, alt, nullptr, nullptr, m, 2 * b, &in_alt, g->scratch, s);
+    rc = radix_sort_u64(keys, alt, nullptr, nullptr, m, 2 * b, &in_alt, g->scratch, &g->ctr->err, s);
     if (!rc) rc = build_adjacency(g, g->adj[d], in_alt ? alt : keys, m, b, flag, pos);
   }
   cudaStreamSynchronize(s);
@@ -935,7 +935,7 @@ static int canon_list(Graph* g, size_t n, int b, int dir) {
                                                     g->directed, b, (uint32_t)g->V, B.keys, B.vals, g->ctr);
   VX_CUDA_TRY(cudaGetLastError());
   bool in_alt = false;
-  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, s)) return rc;
+  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, &g->ctr->err, s)) return rc;
   uint64_t* keys = in_alt ? B.keys_alt : B.keys;
   uint32_t* vals = in_alt ? B.vals_alt : B.vals;
   vxh::count_launch();
@@ -1019,7 +1019,7 @@ static int prepare_reverse(Graph* g, size_t m) {
   vxh::count_launch();
   reverse_keys_kernel<<<grid_for(m), kBlock, 0, s>>>(B.fu, B.fv, B.ff, &g->ctr->final_arcs, m, b, B.keys, B.vals);
   bool in_alt = false;
-  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, s)) return rc;
+  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, &g->ctr->err, s)) return rc;
   uint64_t* keys = in_alt ? B.keys_alt : B.keys;
   uint32_t* vals = in_alt ? B.vals_alt : B.vals;
   vxh::count_launch();

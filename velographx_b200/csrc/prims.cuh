@@ -21,9 +21,10 @@ struct Scratch {
 // Sort (keys, vals) ascending by the low `key_bits` bits of the keys; stable.
 // keys/vals are double-buffered with keys_alt/vals_alt (same sizes).  On
 // return *in_alt says whether the sorted data ended in the *_alt buffers.
-// vals may be null (keys-only sort).
+// vals may be null (keys-only sort).  *err (device) gets kErrBarrierTimeout if a
+// bounded wait of the sort expires.
 int radix_sort_u64(uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, size_t n,
-                   int key_bits, bool* in_alt, Scratch& scratch, cudaStream_t s);
+                   int key_bits, bool* in_alt, Scratch& scratch, uint32_t* err, cudaStream_t s);
 
 // Scratch bytes radix_sort_u64 needs for n items.
 size_t radix_sort_scratch_bytes(size_t n);
