@@ -11,6 +11,7 @@
 //   * compact (:633-639): the overlay is merged into a fresh base CSR.
 #include <algorithm>
 #include <cstddef>
+#include <cstdlib>
 #include <cstring>
 
 #include "graph.cuh"
@@ -548,9 +549,13 @@ int BatchBuffers::ensure(size_t ops) {
   size_t c = std::max<size_t>(ops, 1024);
   const size_t arcs = 2 * c;
   int rc = 0;
-  rc |= alloc_array(&src, c);
-  rc |= alloc_array(&dst, c);
-  rc |= alloc_array(&add, c);
+  uint8_t* ops9 = nullptr;
+  rc |= alloc_array(&ops9, 9 * c);
+  if (!rc) {
+    src = reinterpret_cast<uint32_t*>(ops9);
+    dst = src + c;
+    add = ops9 + 8 * c;
+  }
   rc |= alloc_array(&keys, arcs);
   rc |= alloc_array(&keys_alt, arcs);
   rc |= alloc_array(&vals, arcs);
@@ -577,9 +582,10 @@ int BatchBuffers::ensure(size_t ops) {
 }
 
 void BatchBuffers::free_all() {
-  void* ptrs[] = {src, dst, add, keys, keys_alt, vals, vals_alt, flag, pos, fu,
+  void* ptrs[] = {src, keys, keys_alt, vals, vals_alt, flag, pos, fu,
                   fv, ff, fpos, lu, lv, runs, ru, rv, rf, rpos};
   for (void* p : ptrs) cudaFree(p);
+  free(host);
   *this = BatchBuffers();
 }
 

@@ -50,7 +50,8 @@ enum : uint8_t { kFAdd = 1, kFInBase = 2, kFCur = 4, kFChanged = 8 };
 
 struct BatchBuffers {
   size_t cap = 0;       // op capacity
-  uint32_t* src = nullptr;
+  uint8_t* host = nullptr;    // a small host batch packed for one copy
+  uint32_t* src = nullptr;    // one allocation of 9 bytes an op holds src, dst and add
   uint32_t* dst = nullptr;
   uint8_t* add = nullptr;
   // the op arrays the next staging reads: src/dst/add after a host upload, or
