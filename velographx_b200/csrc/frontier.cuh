@@ -53,18 +53,30 @@ __device__ __forceinline__ void load_words(const uint32_t* base, uint32_t* out) 
 }
 
 // The listed rows (lengths len[0, n)) of which this warp holds a slice, when
-// row r is cut into slices of `slice` arcs and its slices are dealt to the
-// warps starting at warp r (mod the warp count): f(r, len_r, first slice)
-// for each, warp-uniformly.  The lengths are read 32 at a time, so a warp
-// passes the rows it has no slice of without a round trip per row.
+// every row is cut into slices of `slice` arcs and the slices of all rows, in
+// list order, are dealt to the warps in turn: f(r, len_r, first slice) for
+// each, warp-uniformly; the warp's further slices of the row follow nwarps()
+// apart.  The lengths are read 32 at a time, so a warp passes the rows it has
+// no slice of without a round trip per row.  (With the slices of row r dealt
+// from warp r on, the few hub rows of a small frontier all lay on the same
+// warps: 55 rows with 478,438 arcs 286 us, so 21 us.)
 template <class F>
 __device__ __forceinline__ void for_my_rows(const uint32_t* len, uint32_t n, uint32_t slice, F&& f) {
   const uint32_t lane = threadIdx.x & 31, nw = nwarps(), gw = gwarp();
+  uint32_t first = 0;  // slices of the rows before r0, mod the warp count
   for (uint32_t r0 = 0; r0 < n; r0 += 32) {
     const uint32_t r = r0 + lane;
     const uint32_t l = r < n ? __ldcg(&len[r]) : 0u;
-    const uint32_t s0 = (gw + nw - r % nw) % nw;
-    uint32_t mine = __ballot_sync(0xFFFFFFFFu, r < n && s0 < (l + slice - 1) / slice);
+    const uint32_t sl = (l + slice - 1) / slice;
+    uint32_t incl = sl;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= d) incl += t;
+    }
+    const uint32_t s0 = (gw + nw - (first + incl - sl) % nw) % nw;
+    first = (first + __shfl_sync(0xFFFFFFFFu, incl, 31)) % nw;
+    uint32_t mine = __ballot_sync(0xFFFFFFFFu, s0 < sl);
     while (mine) {
       const uint32_t k = __ffs(mine) - 1;
       mine &= mine - 1;

@@ -552,11 +552,9 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
   if (!vs_sync(p)) return false;
   const uint32_t nb = __ldcg(nbig);
   if (nb == 0) return true;
-  // long rows: every warp takes 32 * kSlots-arc slices, the slices of row r
-  // starting at warp r (mod the warp count); a warp skips, from the listed
-  // length alone, the rows it has no slice of
-  const uint32_t nw_ = nwarps(), gw = gwarp();
-  for_my_rows(p.biglen, nb, 32 * kSlots, [&](uint32_t r, uint32_t, uint32_t) {
+  // long rows: the grid's warps take 32 * kSlots-arc slices
+  const uint32_t nw_ = nwarps();
+  for_my_rows(p.biglen, nb, 32 * kSlots, [&](uint32_t r, uint32_t, uint32_t sl) {
     const uint32_t v = p.big[r];
     uint32_t vis[W];
 #pragma unroll
@@ -564,7 +562,7 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
     const VsRow rw = vs_row(p, v);
     const uint32_t total = rw.nb + rw.dy + rw.tn;
     const uint32_t nslices = (total + 32 * kSlots - 1) / (32 * kSlots);
-    for (uint32_t sl = (gw + nw_ - r % nw_) % nw_; sl < nslices; sl += nw_) {
+    for (; sl < nslices; sl += nw_) {
       bool full = true;
 #pragma unroll
       for (uint32_t w = 0; w < W; ++w) full = full && (vis[w] | __ldcg(&p.nxt[(size_t)v * W + w])) == vmask(p.K, w);
@@ -671,8 +669,7 @@ __device__ bool vs_push(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
   bq_flush(vs_bq, tn, p.tl);
   if (!vs_sync(p)) return false;
   const uint32_t nb = __ldcg(nbig);
-  // hub rows: kVsPushSlice-arc slices, the slices of row j starting at warp j
-  // (mod the warp count); a warp skips the rows it has no slice of
+  // hub rows: the grid's warps take kVsPushSlice-arc slices
   const uint32_t nw = nwarps();
   for_my_rows(p.biglen, nb, kVsPushSlice, [&](uint32_t j, uint32_t total, uint32_t sl) {
     const uint32_t nsl = (total + kVsPushSlice - 1) / kVsPushSlice;
