@@ -71,9 +71,14 @@ constexpr uint32_t kVsWarps = kVsThreads / 32;
 // 32-vertex groups a warp claims per atomic of a pull level (one counter
 // per level: a claim per group serialised on it)
 constexpr uint32_t kClaimGroups = 4;
+constexpr uint32_t kClaimsPerWarp = 4;  // claims of one group where a warp would get fewer than these
 constexpr uint32_t kVsHead = 8;        // in-arcs a lane reads itself before the flattened rounds
 constexpr uint32_t kVsHeadStep = 4;    // of which it loads this many at a time
 constexpr uint32_t kVsBigPull = 2048;  // pull rows this long are read by the whole grid
+// Pull rows this long are read by a warp each: in the groups, a power-law
+// graph's heavy vertices made the level's tail.  512 versions of 1M vertices
+// 5.32 -> 5.0-5.2 ms, of 100k vertices 5.5 -> 4.3 ms.
+constexpr uint32_t kVsMidPull = 256;
 constexpr uint32_t kVsBigPush = 1024;  // push rows this long are expanded by the whole grid
 constexpr uint32_t kVsPushSlice = 128; // arcs of a hub row a warp takes at a time
 constexpr int kVsTBits = 8;            // version field of the sort keys
@@ -385,25 +390,61 @@ struct VsStage {
   uint32_t acc[32 * 8];
 };
 
+// The frontier words of 32 * kSlots arcs of a row from arc k0 on, the lane's
+// arcs OR-ed into add (masked by the versions that a touched arc is in).
+template <uint32_t W>
+__device__ __forceinline__ void vs_or_arcs(const VsParams& p, const VsRow& rw, const uint32_t* fc, uint32_t k0,
+                                           uint32_t total, uint32_t* add) {
+  constexpr uint32_t kSlots = VsSlots<W>::value;
+  uint32_t x[kSlots], e[kSlots];
+#pragma unroll
+  for (uint32_t u = 0; u < kSlots; ++u) {
+    const uint32_t k = k0 + u * 32 + (threadIdx.x & 31);
+    x[u] = kTomb;
+    e[u] = kNoEntry;
+    if (k < total) x[u] = vs_arc(p, rw.b, rw.nb, rw.dx, rw.dy, rw.tb, rw.tn, rw.pre, k, e[u]);
+  }
+#pragma unroll
+  for (uint32_t w = 0; w < W; ++w) add[w] = 0u;
+#pragma unroll
+  for (uint32_t u = 0; u < kSlots; ++u) {
+    if (x[u] & kTomb) continue;
+    uint32_t f[W];
+    load_words<W>(fc + (size_t)x[u] * W, f);
+    if (e[u] != kNoEntry) {
+      uint32_t mk[W];
+      load_words<W>(p.tmask + (size_t)e[u] * W, mk);
+#pragma unroll
+      for (uint32_t w = 0; w < W; ++w) f[w] &= mk[w];
+    }
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) add[w] |= f[w];
+  }
+}
+
 // Pull level: groups of 32 consecutive vertices from a counter; the rows of
 // the group's vertices that some version has not reached are read as one
 // flattened arc list, kSlots arcs per lane per round, each arc's frontier
 // words (masked by its presence for touched arcs) OR-ed into its owner's
-// accumulator; owners reached in every version stop.  Long rows are read by
-// the whole grid after a barrier, through nxt.  Ends with a grid barrier.
+// accumulator; owners reached in every version stop.  Longer rows that their
+// first arcs leave open are read after a barrier: from kVsMidPull arcs on by a
+// warp each (nmid, mid), from kVsBigPull on by the whole grid, through nxt.
+// Ends with a grid barrier.
 template <uint32_t W>
 __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uint32_t level, uint32_t* gnext,
-                        uint32_t* nbig, uint32_t* qn, uint32_t* qout, unsigned long long* mf, VsStage& ws,
+                        uint32_t* nbig, uint32_t* nmid, uint32_t* mid, uint32_t* qn, uint32_t* qout,
+                        unsigned long long* mf, VsStage& ws,
                         VsSums& s, unsigned long long* sdig) {
   constexpr uint32_t kSlots = VsSlots<W>::value;
   const uint32_t lane = threadIdx.x & 31;
+  const uint32_t claim = p.V / 32 >= kClaimsPerWarp * kClaimGroups * nwarps() ? kClaimGroups : 1u;
   uint32_t cur = 0, end = 0;  // the warp's claimed groups [cur, end), warp-uniform
   for (;;) {
     if (cur == end) {
       uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(gnext, kClaimGroups);
+      if (lane == 0) c0 = atomicAdd(gnext, claim);
       cur = __shfl_sync(FULL, c0, 0);
-      end = cur + kClaimGroups;
+      end = cur + claim;
     }
     const uint32_t base = cur++ * 32;
     if (base >= p.V) break;
@@ -421,12 +462,6 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
       const VsRow r = vs_row(p, v);
       len = r.nb + r.dy + r.tn;
       rowlen = len;
-      if (len >= kVsBigPull) {  // the whole grid reads it after the barrier
-        const uint32_t slot = atomicAdd(nbig, 1u);
-        p.big[slot] = v;
-        p.biglen[slot] = len;
-        len = 0;
-      }
       ws.rb[lane] = r.b;
       ws.nb[lane] = r.nb;
       ws.dx[lane] = r.dx;
@@ -441,6 +476,7 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
       uint32_t hacc[W];
 #pragma unroll
       for (uint32_t w = 0; w < W; ++w) hacc[w] = 0u;
+      bool fin = false;
       for (uint32_t h0 = 0; h0 < hn; h0 += kVsHeadStep) {
         uint32_t hx[kVsHeadStep], he[kVsHeadStep];
 #pragma unroll
@@ -462,15 +498,24 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
 #pragma unroll
           for (uint32_t w = 0; w < W; ++w) hacc[w] |= f[w];
         }
-        bool fin = true;
+        fin = true;
 #pragma unroll
         for (uint32_t w = 0; w < W; ++w) fin = fin && (vis[w] | hacc[w]) == vmask(p.K, w);
-        if (fin) {
-          len = hn;  // nothing left for the rounds
-          break;
-        }
+        if (fin) break;
       }
-      len -= hn;
+      len = fin ? 0u : len - hn;
+      if (!fin && rowlen >= kVsMidPull) {  // all of it is read after the barrier
+        if (rowlen >= kVsBigPull) {
+          const uint32_t slot = atomicAdd(nbig, 1u);
+          p.big[slot] = v;
+          p.biglen[slot] = rowlen;
+        } else {
+          mid[atomicAdd(nmid, 1u)] = v;
+        }
+        len = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < W; ++w) hacc[w] = 0u;
+      }
 #pragma unroll
       for (uint32_t w = 0; w < W; ++w) ws.acc[lane * W + w] = hacc[w];
     }
@@ -550,8 +595,44 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
   bq_flush(vs_bq, qn, qout);
   mf_flush(mf);
   if (!vs_sync(p)) return false;
-  const uint32_t nb = __ldcg(nbig);
-  if (nb == 0) return true;
+  const uint32_t nb = __ldcg(nbig), nm = __ldcg(nmid);
+  if ((nb | nm) == 0) return true;
+  // rows of a warp each: no other warp adds to them, so they are finished here
+  for (uint32_t i = gwarp(); i < nm; i += nwarps()) {
+    const uint32_t v = mid[i];
+    const VsRow rw = vs_row(p, v);
+    const uint32_t total = rw.nb + rw.dy + rw.tn;
+    uint32_t vis[W], nw[W];
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) {
+      vis[w] = __ldcg(&p.vis[(size_t)v * W + w]);
+      nw[w] = 0u;
+    }
+    for (uint32_t k0 = 0; k0 < total; k0 += 32 * kSlots) {
+      uint32_t add[W];
+      vs_or_arcs<W>(p, rw, fc, k0, total, add);
+      bool full = true;
+#pragma unroll
+      for (uint32_t w = 0; w < W; ++w) {
+        nw[w] |= __reduce_or_sync(FULL, add[w]);
+        full = full && (vis[w] | nw[w]) == vmask(p.K, w);
+      }
+      if (full) break;
+    }
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) nw[w] &= ~vis[w];
+    bool any = false;
+    if (lane == 0) {
+      any = vs_discover<W>(p, v, vis, nw, fn, level + 1, s);
+      if (p.dig) vs_digest<W>(p, v, nw, level + 1, s, sdig);
+      if (any) atomicAdd(&vs_mf, (unsigned long long)total);
+    }
+    __syncwarp();
+    bq_push(vs_bq, any, v, qn, qout);
+  }
+  bq_flush(vs_bq, qn, qout);
+  mf_flush(mf);
+  if (nb == 0) return vs_sync(p);
   // long rows: the grid's warps take 32 * kSlots-arc slices
   const uint32_t nw_ = nwarps();
   for_my_rows(p.biglen, nb, 32 * kSlots, [&](uint32_t r, uint32_t, uint32_t sl) {
@@ -567,31 +648,8 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
 #pragma unroll
       for (uint32_t w = 0; w < W; ++w) full = full && (vis[w] | __ldcg(&p.nxt[(size_t)v * W + w])) == vmask(p.K, w);
       if (full) break;
-      uint32_t x[kSlots], e[kSlots];
-#pragma unroll
-      for (uint32_t u = 0; u < kSlots; ++u) {
-        const uint32_t k = sl * 32 * kSlots + u * 32 + lane;
-        x[u] = kTomb;
-        e[u] = kNoEntry;
-        if (k < total) x[u] = vs_arc(p, rw.b, rw.nb, rw.dx, rw.dy, rw.tb, rw.tn, rw.pre, k, e[u]);
-      }
       uint32_t add[W];
-#pragma unroll
-      for (uint32_t w = 0; w < W; ++w) add[w] = 0u;
-#pragma unroll
-      for (uint32_t u = 0; u < kSlots; ++u) {
-        if (x[u] & kTomb) continue;
-        uint32_t f[W];
-        load_words<W>(fc + (size_t)x[u] * W, f);
-        if (e[u] != kNoEntry) {
-          uint32_t mk[W];
-          load_words<W>(p.tmask + (size_t)e[u] * W, mk);
-#pragma unroll
-          for (uint32_t w = 0; w < W; ++w) f[w] &= mk[w];
-        }
-#pragma unroll
-        for (uint32_t w = 0; w < W; ++w) add[w] |= f[w];
-      }
+      vs_or_arcs<W>(p, rw, fc, sl * 32 * kSlots, total, add);
 #pragma unroll
       for (uint32_t w = 0; w < W; ++w) {
         const uint32_t red = __reduce_or_sync(FULL, add[w]) & ~vis[w];
@@ -774,8 +832,8 @@ __global__ void __launch_bounds__(kVsThreads, 2) vs_bfs_kernel(VsParams p) {
     }
     bool ok;
     if (pull)
-      ok = vs_pull<W>(p, fc, fn, level, &c->gnext[cur], &c->nbig[cur], &c->qn[nx], p.q[nx], &c->mf[nx],
-                      stage[threadIdx.x >> 5], s, sdig);
+      ok = vs_pull<W>(p, fc, fn, level, &c->gnext[cur], &c->nbig[cur], &c->tn[cur], p.tl, &c->qn[nx], p.q[nx],
+                      &c->mf[nx], stage[threadIdx.x >> 5], s, sdig);
     else
       ok = vs_push<W>(p, fc, fn, level, n_f, p.q[cur], &c->tn[cur], &c->nbig[cur], &c->qn[nx], p.q[nx], &c->mf[nx],
                       s, sdig);
