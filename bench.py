@@ -434,7 +434,7 @@ def run_b200(args, rank, world, local):
                                   / (float(np.median(bfs_ms)) * 1e-3) / 1e9 / hbm) if traffic else None,
         },
         "roofline_step": {
-            "kernel": "one update step: canon_cluster_kernel + bfs_stream_kernel (fused commit and repair)",
+            "kernel": "one update step: bfs_stream_kernel (canonicalisation, commit and repair)",
             "bound": "hbm",
             "achieved": step_achieved,
             "peak": hbm,

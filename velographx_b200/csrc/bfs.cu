@@ -7,11 +7,12 @@
 //   kModeFull  recompute (bfs.hpp:100-120) as a direction-optimising BFS:
 //              top-down levels expand a frontier queue with warp-cooperative
 //              gathers (rows < 32 arcs flattened across the warp, medium rows
-//              expanded by the whole warp, rows >= tune.large_row expanded by
-//              the whole grid), bottom-up levels scan candidate lists a warp
-//              per 32 vertices and stop each scan at the first parent in the
-//              frontier bitmap.  Claims are atomicOr on the visited bitmap,
-//              frontier queues are appended with warp-aggregated atomics.
+//              expanded by the whole warp, rows >= tune.large_row by the whole
+//              grid; the smallest levels by one block alone), bottom-up levels
+//              look through every block's own vertices and stop each scan at
+//              the first parent in the frontier bitmap.  Top-down claims are
+//              atomicOr on the visited bitmap; queues are appended through the
+//              blocks' shared memory.
 //   kModePre   the pre-batch part of apply (bfs.hpp:38-70, 222-259): deletion
 //              candidates and the support-count fixpoint, run as one
 //              asynchronous cascade over a work ring (no barrier per level).
