@@ -4084,7 +4084,7 @@ int bfs_apply_stream(Bfs* b, const uint32_t* hs, const uint32_t* hd, const uint8
   stream_keys_kernel<<<grid_n, 256, 0, st>>>(S.src, S.dst, S.add, S.off, (uint32_t)nb, n, bbits, S.keys, S.vals);
   VX_CUDA_TRY(cudaGetLastError());
   bool in_alt = false;
-  if (int rc = radix_sort_u64(S.keys, S.keys_alt, S.vals, S.vals_alt, m, 2 * bbits + tbits, &in_alt, g->scratch, &g->ctr->err, st))
+  if (int rc = radix_sort_u64(S.keys, S.keys_alt, S.vals, S.vals_alt, m, 2 * bbits + tbits, &in_alt, g->scratch, g->sort_wait(), st))
     return rc;
   uint64_t* keys = in_alt ? S.keys_alt : S.keys;
   uint32_t* vals = in_alt ? S.vals_alt : S.vals;

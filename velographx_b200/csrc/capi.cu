@@ -324,6 +324,12 @@ int vx_graph_stream(vx_graph* g, void** stream) {
   return VX_OK;
 }
 
+int vx_graph_set_sort_wait(vx_graph* g, uint32_t looks) {
+  if (!g) return fail(VX_ERR_INVALID, "null argument");
+  g->g->sort_looks = looks;
+  return VX_OK;
+}
+
 int vx_graph_synchronize(vx_graph* g) {
   if (!g) return fail(VX_ERR_INVALID, "null argument");
   return vxh::graph_sync_counters(g->g);

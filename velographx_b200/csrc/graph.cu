@@ -721,7 +721,9 @@ uint64_t graph_edge_count_directed(const Graph* g) {
 }
 
 // Builds adjacency a from sorted keys holding (u << b | v) arcs (duplicates
-// and ~0 padding allowed).  flag/pos are scratch arrays of m entries.
+// and ~0 padding allowed).  flag/pos are scratch arrays of m entries.  The word
+// of the sort that made the keys (ctr->scratch32) is read with the arc count,
+// before any offset is written at a place that the keys name.
 static int build_adjacency(Graph* g, Adjacency& a, uint64_t* keys, size_t m, int b, uint32_t* flag,
                            uint32_t* pos) {
   cudaStream_t s = g->stream;
@@ -732,8 +734,13 @@ static int build_adjacency(Graph* g, Adjacency& a, uint64_t* keys, size_t m, int
   unique_flag_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, flag);
   if (int rc = scan_exclusive_u32(flag, pos, m, total, g->scratch, s)) return rc;
   VX_CUDA_TRY(cudaMemcpyAsync(g->pinned_scalar, total, 4, cudaMemcpyDeviceToHost, s));
+  VX_CUDA_TRY(cudaMemcpyAsync(g->pinned_scalar + 1, &g->ctr->scratch32, 4, cudaMemcpyDeviceToHost, s));
   VX_CUDA_TRY(cudaStreamSynchronize(s));
   const uint32_t A = *reinterpret_cast<uint32_t*>(g->pinned_scalar);
+  if (*reinterpret_cast<uint32_t*>(g->pinned_scalar + 1)) {
+    set_error("bulk load: a wait of the radix sort ran out");
+    return -5;
+  }
   if (alloc_array(&a.col, A) || alloc_array(&a.off, g->V + 1)) return -4;
   a.col_cap = A;
   a.off_cap = g->V + 1;
@@ -758,6 +765,7 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
   // vertex growth: max id + 1 over non-self-loop edges
   uint32_t* mx = reinterpret_cast<uint32_t*>(&g->ctr->max_vertex_plus1);
   VX_CUDA_TRY(cudaMemsetAsync(mx, 0, 4, s));
+  VX_CUDA_TRY(cudaMemsetAsync(&g->ctr->scratch32, 0, 4, s));
   if (n) {
     vxh::count_launch();
     max_id_kernel<<<grid_for(n), kBlock, 0, s>>>(d_uv, n, mx);
@@ -791,7 +799,9 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
       }
     }
     bool in_alt = false;
-    rc = radix_sort_u64(keys, alt, nullptr, nullptr, m, 2 * b, &in_alt, g->scratch, &g->ctr->err, s);
+    // a word of its own: the load's last step clears the counters and ctr->err with them
+    const SortWait wait{&g->ctr->scratch32, g->sort_looks};
+    rc = radix_sort_u64(keys, alt, nullptr, nullptr, m, 2 * b, &in_alt, g->scratch, wait, s);
     if (!rc) rc = build_adjacency(g, g->adj[d], in_alt ? alt : keys, m, b, flag, pos);
   }
   cudaStreamSynchronize(s);
@@ -941,7 +951,7 @@ static int canon_list(Graph* g, size_t n, int b, int dir) {
                                                     g->directed, b, (uint32_t)g->V, B.keys, B.vals, g->ctr);
   VX_CUDA_TRY(cudaGetLastError());
   bool in_alt = false;
-  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, &g->ctr->err, s)) return rc;
+  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, g->sort_wait(), s)) return rc;
   uint64_t* keys = in_alt ? B.keys_alt : B.keys;
   uint32_t* vals = in_alt ? B.vals_alt : B.vals;
   vxh::count_launch();
@@ -1025,7 +1035,7 @@ static int prepare_reverse(Graph* g, size_t m) {
   vxh::count_launch();
   reverse_keys_kernel<<<grid_for(m), kBlock, 0, s>>>(B.fu, B.fv, B.ff, &g->ctr->final_arcs, m, b, B.keys, B.vals);
   bool in_alt = false;
-  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, &g->ctr->err, s)) return rc;
+  if (int rc = radix_sort_u64(B.keys, B.keys_alt, B.vals, B.vals_alt, m, 2 * b, &in_alt, g->scratch, g->sort_wait(), s)) return rc;
   uint64_t* keys = in_alt ? B.keys_alt : B.keys;
   uint32_t* vals = in_alt ? B.vals_alt : B.vals;
   vxh::count_launch();

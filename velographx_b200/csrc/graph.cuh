@@ -24,7 +24,7 @@ struct GraphCounters {
   uint32_t err;                      // vxb::kErr* bits
   uint32_t max_vertex_plus1;         // max(src,dst)+1 over non-self-loop ops
   uint32_t rev_arcs;                 // reversed changed arcs (directed graphs)
-  uint32_t scratch32;                // single-value readbacks (has_edge, maybe_compact)
+  uint32_t scratch32;                // single-value readbacks (has_edge, maybe_compact, a load's sort)
 };
 
 struct Adjacency {
@@ -97,6 +97,7 @@ struct Graph {
   uint64_t* pinned_scalar = nullptr;  // small pinned buffer for readbacks
   size_t batch_ops = 0;               // ops of the batch currently staged
   size_t arena_limit_entries = 0;     // consolidate instead of growing past this
+  uint32_t sort_looks = kSortLooks;   // bound of the sorts' waits (SortWait)
   // a readback of arena_top and delta_live in flight (arena_tops, pinned), and
   // the bounds when it was enqueued
   cudaEvent_t arena_ev = nullptr;
@@ -104,6 +105,7 @@ struct Graph {
   uint64_t arena_seen[2] = {0, 0};
   bool arena_pending = false;
 
+  SortWait sort_wait() { return SortWait{&ctr->err, sort_looks}; }
   Adjacency& in() { return directed ? adj[1] : adj[0]; }
   vxb::DevGraph view();
 };

@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(kDigits) radix_bases_kernel(unsigned long long
 // A tile's word for one digit: its count, or the count of it and all tiles
 // before it, once published.
 constexpr unsigned long long kTileSum = 1ull << 62, kTilePrefix = 2ull << 62, kTileMask = (1ull << 62) - 1;
-constexpr uint32_t kLookBack = 8;          // words of earlier tiles in flight per step
-constexpr uint32_t kLookLimit = 1u << 22;  // steps without progress before a tile gives up
+constexpr uint32_t kLookBack = 8;  // words of earlier tiles in flight per look
 
 // One pass.  Tiles take their numbers from a ticket, so every tile before a
 // running one is running or done, and the look-back ends.  33.5M keys: 358 us a
@@ -327,7 +326,7 @@ __global__ void __launch_bounds__(kBigBlock, 3) radix_pass_kernel(const uint64_t
                                                                uint64_t* keys_out, uint32_t* vals_out, size_t n,
                                                                int shift, const unsigned long long* bases,
                                                                unsigned long long* state, uint32_t* ticket,
-                                                               uint32_t* err) {
+                                                               SortWait wait) {
   __shared__ __align__(16) uint64_t stage[kBigTile];
   __shared__ uint32_t warp_hist[(kBigBlock / 32) * kDigits];
   __shared__ uint32_t total[kDigits];
@@ -364,8 +363,12 @@ __global__ void __launch_bounds__(kBigBlock, 3) radix_pass_kernel(const uint64_t
   }
   unsigned long long before = 0;
   if (tile > 0) {
-    uint32_t idle = 0;
+    uint32_t idle = 0;  // looks since the last word that was there
     for (int64_t j = (int64_t)tile - 1; j >= 0;) {
+      if (idle++ == wait.looks) {
+        atomicOr(wait.err, vxb::kErrBarrierTimeout);
+        break;
+      }
       unsigned long long w[kLookBack];
 #pragma unroll
       for (uint32_t q = 0; q < kLookBack; ++q)
@@ -379,12 +382,9 @@ __global__ void __launch_bounds__(kBigBlock, 3) radix_pass_kernel(const uint64_t
         before += w[q] & kTileMask;
         done = (w[q] & kTilePrefix) != 0ull;
         --j;
+        idle = 0;
       }
       if (done) break;
-      if (stuck && ++idle > kLookLimit) {
-        atomicOr(err, vxb::kErrBarrierTimeout);
-        break;
-      }
     }
     __stcg(word, kTilePrefix | (before + mine));
   }
@@ -471,7 +471,7 @@ size_t radix_sort_scratch_bytes(size_t n) {
 }
 
 int radix_sort_u64(uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, size_t n,
-                   int key_bits, bool* in_alt, Scratch& scratch, uint32_t* err, cudaStream_t s) {
+                   int key_bits, bool* in_alt, Scratch& scratch, const SortWait& wait, cudaStream_t s) {
   *in_alt = false;
   if (n <= 1) return 0;
   if (key_bits < 1) key_bits = 1;
@@ -507,7 +507,7 @@ int radix_sort_u64(uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t*
     VX_CUDA_TRY(cudaMemsetAsync(state, 0, (size_t)tiles * kDigits * 8, s));
     vxh::count_launch();
     radix_pass_kernel<<<tiles, kBigBlock, 0, s>>>(ki, vi, ko, vo, n, shift, counts + p * kDigits, state, tickets + p,
-                                                  err);
+                                                  wait);
     VX_CUDA_TRY(cudaGetLastError());
     uint64_t* tk = ki;
     ki = ko;

@@ -18,13 +18,22 @@ struct Scratch {
   ~Scratch() { release(); }
 };
 
+// How long a tile of a sort waits for the tiles before it, in looks at their
+// words without progress (0: it gives up without looking); then *err (device)
+// gets kErrBarrierTimeout.
+constexpr uint32_t kSortLooks = 1u << 22;
+struct SortWait {
+  uint32_t* err;
+  uint32_t looks;
+};
+
 // Sort (keys, vals) ascending by the low `key_bits` bits of the keys; stable.
 // keys/vals are double-buffered with keys_alt/vals_alt (same sizes).  On
 // return *in_alt says whether the sorted data ended in the *_alt buffers.
-// vals may be null (keys-only sort).  *err (device) gets kErrBarrierTimeout if a
-// bounded wait of the sort expires.
+// vals may be null (keys-only sort).  A sort whose wait ran out leaves slots of
+// its output unwritten: nothing may be indexed by them before wait.err is tested.
 int radix_sort_u64(uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, size_t n,
-                   int key_bits, bool* in_alt, Scratch& scratch, uint32_t* err, cudaStream_t s);
+                   int key_bits, bool* in_alt, Scratch& scratch, const SortWait& wait, cudaStream_t s);
 
 // Scratch bytes radix_sort_u64 needs for n items.
 size_t radix_sort_scratch_bytes(size_t n);

@@ -1050,7 +1050,7 @@ int stream_versions(Bfs* b, const uint32_t* d_src, const uint32_t* d_dst, const 
     VX_CUDA_TRY(cudaGetLastError());
     bool in_alt = false;
     if (int rc = radix_sort_u64(S.keys, S.keys_alt, S.vals, S.vals_alt, m, 2 * bbits + kVsTBits, &in_alt,
-                                g->scratch, &g->ctr->err, st))
+                                g->scratch, g->sort_wait(), st))
       return rc;
     keys = in_alt ? S.keys_alt : S.keys;
     vals = in_alt ? S.vals_alt : S.vals;
