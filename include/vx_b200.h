@@ -149,8 +149,9 @@ int vx_graph_scan_rows(vx_graph* g, uint64_t* arcs, double* ns);
 /* Bound of the radix sort behind loads and large batches: the looks without
  * progress (default 2^22, some seconds) after which a part of the sort gives up
  * waiting for the parts before it; 0 gives up without looking.  A load then
- * fails with VX_ERR_DEVICE and must be repeated before the graph is used.  No
- * reference counterpart (failure detection). */
+ * fails with VX_ERR_DEVICE and must be repeated before the graph is used; a
+ * batch holds no arcs and every synchronising call after it fails (VX_ERR_DEVICE)
+ * until the graph is loaded anew.  No reference counterpart (failure detection). */
 int vx_graph_set_sort_wait(vx_graph* g, uint32_t looks);
 /* The graph's CUDA stream (cudaStream_t) and a host-side wait for it. */
 int vx_graph_stream(vx_graph* g, void** stream);

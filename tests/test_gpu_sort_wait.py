@@ -48,3 +48,64 @@ def test_a_load_reports_it_and_can_be_repeated(n, directed):
     for u in (0, 17, 29_999):
         lo, hi = np.searchsorted(want, [u << 32, u + 1 << 32])
         assert g.neighbors(u) == (want[lo:hi] & np.uint64(0xFFFFFFFF)).tolist()
+
+
+def big_batch(ops=60_000, V=30_000, seed=2):
+    rng = np.random.default_rng(seed)
+    return (rng.integers(0, V, ops, dtype=np.uint32), rng.integers(0, V, ops, dtype=np.uint32),
+            (rng.random(ops) < 0.7).astype(np.uint8))
+
+
+def small_graph(directed, V=30_000):
+    g = vx.Graph(V, directed)
+    g.bulk_load_edges(np.random.default_rng(1).integers(0, V, (2 * V, 2), dtype=np.uint32))
+    return g
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("fused", [True, False])
+def test_a_batch_reports_it_and_holds_no_arcs(fused, directed):
+    g = small_graph(directed)
+    b = vx.IncrementalBFS(g, 5)
+    b.set_fused(fused)
+    before = [g.neighbors(u) for u in range(40)]
+    set_sort_wait(g, 0)
+    b.apply_arrays(*big_batch(100_000))
+    for call in (b.stats, b.distances_array, g.edge_count_directed):
+        with pytest.raises(RuntimeError):
+            call()
+    assert [g.neighbors(u) for u in range(40)] == before
+    set_sort_wait(g, DEFAULT_LOOKS)  # the error stays
+    b.apply_arrays(*big_batch(10))
+    with pytest.raises(RuntimeError):
+        b.stats()
+
+
+@pytest.mark.parametrize("directed", [False, True])
+def test_a_graph_batch_reports_it(directed):
+    g = small_graph(directed)
+    set_sort_wait(g, 0)
+    g.apply_arrays(*big_batch(100_000))
+    with pytest.raises(RuntimeError):
+        g.edge_count_directed()
+
+
+@pytest.mark.parametrize("stats", [False, True])
+def test_a_stream_reports_it(stats):
+    g = small_graph(False)
+    b = vx.IncrementalBFS(g, 5)
+    set_sort_wait(g, 0)
+    s, d, a = big_batch()
+    with pytest.raises(RuntimeError):
+        b.apply_stream(s, d, a, np.arange(0, 60_001, 6000, dtype=np.uint64), digests=True, stats=stats)
+
+
+def test_components_report_it():
+    g = small_graph(False)
+    c = vx.IncrementalComponents(g)
+    set_sort_wait(g, 0)
+    c.apply_arrays(*big_batch())
+    with pytest.raises(RuntimeError):
+        c.labels_array()
+    with pytest.raises(RuntimeError):
+        c.last_repaired_vertices

@@ -90,6 +90,7 @@ struct Params {
   uint32_t large_row;
   uint32_t nblocks;
   uint32_t deltas;  // the graph may hold delta rows (zero: their table need not be read)
+  const uint32_t* graph_err;  // the graph's error word (null: none)
   unsigned long long* trace;  // optional per-level {time, n_f | bottom-up << 63}
   // optional accounting of the update launch's algorithmic bytes (null: off):
   // [0] row arcs scanned by the repair, [1] vertices it visited, [2] delta-row
@@ -127,11 +128,21 @@ __device__ __forceinline__ void acct_add(const Params& p, int k, unsigned long l
   if (p.acct && v) atomicAdd(&p.acct[k], v);
 }
 
+// The errors a block's thread 0 looks at behind a barrier: the object's own, and
+// a wait of the graph's sort that ran out (its batch holds no arcs then), which
+// becomes the object's, so that the next synchronising call on it fails.
+__device__ __forceinline__ uint32_t barrier_errors(const Params& p) {
+  const uint32_t own = __ldcg(&p.c->err);
+  const uint32_t sort = p.graph_err ? __ldcg(p.graph_err) & vxb::kErrBarrierTimeout : 0u;
+  if (sort) atomicOr(&p.c->err, sort);
+  return own | sort;
+}
+
 // Grid barrier; returns false once any block recorded a device error (a
 // barrier that gave up waiting, a loop bound), so every persistent loop ends.
 __device__ __forceinline__ bool sync_grid(const Params& p) {
   __shared__ uint32_t failed;
-  vxb::grid_barrier_then(p.bar, p.nblocks, &p.c->err, [&] { failed = __ldcg(&p.c->err); });
+  vxb::grid_barrier_then(p.bar, p.nblocks, &p.c->err, [&] { failed = barrier_errors(p); });
   return failed == 0u;
 }
 
@@ -1189,7 +1200,7 @@ __device__ __forceinline__ bool sync_words(const Params& p, RepairWords& w) {
   BfsCounters* c = p.c;
   vxb::grid_barrier_then(p.bar, p.nblocks, &c->err, [&] {
     RepairWords r;
-    r.failed = __ldcg(&c->err);
+    r.failed = barrier_errors(p);
     r.candidates = ld_cg(&c->cand_n);
     r.touched = p.touched_base + ld_cg(&c->touched_n);
     r.affected = ld_cg(&c->a_n);
@@ -3313,10 +3324,11 @@ __global__ void stream_keys_kernel(const uint32_t* src, const uint32_t* dst, con
   }
 }
 
-__global__ void stream_last_kernel(const uint64_t* keys, size_t m, uint32_t* flag) {
+__global__ void stream_last_kernel(const uint64_t* keys, size_t m, const uint32_t* err, uint32_t* flag) {
+  const bool sorted = !(*err & vxb::kErrBarrierTimeout);  // no arcs after a sort whose wait ran out
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
-    flag[i] = (k != ~0ull) && (i + 1 == m || keys[i + 1] != k);
+    flag[i] = sorted && (k != ~0ull) && (i + 1 == m || keys[i + 1] != k);
   }
 }
 
@@ -3503,6 +3515,7 @@ static Params make_params(Bfs* b, uint32_t V, uint32_t dist_len) {
   p.ff = g->batch.ff;
   p.F = &g->ctr->final_arcs;
   p.c = b->ctr;
+  p.graph_err = &g->ctr->err;
   p.total_arcs = g->adj[0].A;  // estimate for the direction switch
   p.alpha = b->tune.alpha;
   p.beta = b->tune.beta;
@@ -4089,7 +4102,7 @@ int bfs_apply_stream(Bfs* b, const uint32_t* hs, const uint32_t* hd, const uint8
   uint64_t* keys = in_alt ? S.keys_alt : S.keys;
   uint32_t* vals = in_alt ? S.vals_alt : S.vals;
   count_launch();
-  stream_last_kernel<<<grid_m, 256, 0, st>>>(keys, m, S.flag);
+  stream_last_kernel<<<grid_m, 256, 0, st>>>(keys, m, &g->ctr->err, S.flag);
   if (int rc = scan_exclusive_u32(S.flag, S.pos, m, S.total, g->scratch, st)) return rc;
   count_launch();
   stream_compact_kernel<<<grid_m, 256, 0, st>>>(keys, vals, S.flag, S.pos, m, bbits, S.fu, S.fv, S.ff, S.bid);
@@ -4122,9 +4135,8 @@ int bfs_apply_stream(Bfs* b, const uint32_t* hs, const uint32_t* hd, const uint8
   b->staged_ops = 0;
   if (digests) VX_CUDA_TRY(cudaMemcpyAsync(digests, S.digest, nb * 8, cudaMemcpyDeviceToHost, st));
   if (stats) VX_CUDA_TRY(cudaMemcpyAsync(stats, S.bstats, nb * 16, cudaMemcpyDeviceToHost, st));
-  if (digests || stats) VX_CUDA_TRY(cudaStreamSynchronize(st));
   *applied = nb;
-  return 0;
+  return digests || stats ? bfs_sync(b) : 0;
 }
 
 int bfs_digest(Bfs* b, uint64_t* out) {

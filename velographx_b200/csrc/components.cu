@@ -419,10 +419,23 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
   return 0;
 }
 
+// Waits for the stream; fails when a wait of the graph's sort ran out (the batch
+// held no arcs then).
+static int cc_sync(Components* c) {
+  Graph* g = c->g;
+  VX_CUDA_TRY(cudaMemcpyAsync(g->pinned_scalar + 1, &g->ctr->err, 4, cudaMemcpyDeviceToHost, g->stream));
+  VX_CUDA_TRY(cudaStreamSynchronize(g->stream));
+  if (*reinterpret_cast<uint32_t*>(g->pinned_scalar + 1) & vxb::kErrBarrierTimeout) {
+    set_error("components: a wait of the radix sort ran out");
+    return -5;
+  }
+  return 0;
+}
+
 int cc_last_repaired(Components* c, uint64_t* out) {
   if (c->repaired_pending) {
     VX_CUDA_TRY(cudaMemcpyAsync(c->g->pinned_scalar, c->ctr + 2, 8, cudaMemcpyDeviceToHost, c->g->stream));
-    VX_CUDA_TRY(cudaStreamSynchronize(c->g->stream));
+    if (int rc = cc_sync(c)) return rc;
     c->last_repaired = (size_t)c->g->pinned_scalar[0];
     c->repaired_pending = false;
   }
@@ -434,8 +447,7 @@ int cc_labels(Components* c, uint32_t* host_out, size_t cap, size_t* n) {
   *n = c->n;
   const size_t k = std::min(cap, c->n);
   if (host_out && k) VX_CUDA_TRY(cudaMemcpyAsync(host_out, c->label, k * 4, cudaMemcpyDeviceToHost, c->g->stream));
-  VX_CUDA_TRY(cudaStreamSynchronize(c->g->stream));
-  return 0;
+  return cc_sync(c);
 }
 
 }  // namespace vxh

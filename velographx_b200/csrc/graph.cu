@@ -138,11 +138,13 @@ __global__ void expand_ops_kernel(const uint32_t* src, const uint32_t* dst, cons
 }
 
 // Last element of every run of equal keys (stable sort keeps op order, so it
-// carries the batch's final op for that arc).
-__global__ void last_of_run_kernel(const uint64_t* keys, size_t m, uint32_t* flag) {
+// carries the batch's final op for that arc).  None after a sort whose wait ran
+// out: its keys may be anything, and the arcs made of them are indices.
+__global__ void last_of_run_kernel(const uint64_t* keys, size_t m, const uint32_t* err, uint32_t* flag) {
+  const bool sorted = !(*err & vxb::kErrBarrierTimeout);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
-    flag[i] = (k != ~0ull) && (i + 1 == m || keys[i + 1] != k);
+    flag[i] = sorted && (k != ~0ull) && (i + 1 == m || keys[i + 1] != k);
   }
 }
 
@@ -182,9 +184,10 @@ __global__ void reverse_keys_kernel(const uint32_t* fu, const uint32_t* fv, cons
   }
 }
 
-__global__ void count_valid_kernel(const uint64_t* keys, size_t m, uint32_t* flag) {
+__global__ void count_valid_kernel(const uint64_t* keys, size_t m, const uint32_t* err, uint32_t* flag) {
+  const bool sorted = !(*err & vxb::kErrBarrierTimeout);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x)
-    flag[i] = keys[i] != ~0ull;
+    flag[i] = sorted && keys[i] != ~0ull;
 }
 
 // --------------------------------------------------------- batch commit --
@@ -955,7 +958,7 @@ static int canon_list(Graph* g, size_t n, int b, int dir) {
   uint64_t* keys = in_alt ? B.keys_alt : B.keys;
   uint32_t* vals = in_alt ? B.vals_alt : B.vals;
   vxh::count_launch();
-  last_of_run_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, B.flag);
+  last_of_run_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, &g->ctr->err, B.flag);
   if (int rc = scan_count(g, B.flag, B.pos, m, dir ? &g->ctr->rev_arcs : &g->ctr->final_arcs)) return rc;
   vxh::count_launch();
   compact_final_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, vals, B.flag, B.pos, m, b, dir ? B.ru : B.fu,
@@ -1039,7 +1042,7 @@ static int prepare_reverse(Graph* g, size_t m) {
   uint64_t* keys = in_alt ? B.keys_alt : B.keys;
   uint32_t* vals = in_alt ? B.vals_alt : B.vals;
   vxh::count_launch();
-  count_valid_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, B.flag);
+  count_valid_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, m, &g->ctr->err, B.flag);
   if (int rc = scan_count(g, B.flag, B.pos, m, &g->ctr->rev_arcs)) return rc;
   vxh::count_launch();
   compact_final_kernel<<<grid_for(m), kBlock, 0, s>>>(keys, vals, B.flag, B.pos, m, b, B.ru, B.rv, B.rf);

@@ -151,10 +151,13 @@ __global__ void vs_keys_kernel(const uint32_t* src, const uint32_t* dst, size_t 
 }
 
 // flag[j] = key j starts the run of a distinct arc
-__global__ void vs_runs_kernel(const uint64_t* keys, size_t m, uint32_t* flag) {
+__global__ void vs_runs_kernel(const uint64_t* keys, size_t m, const uint32_t* err, uint32_t* flag,
+                               uint32_t* window_err) {
+  const uint32_t bad = *err & vxb::kErrBarrierTimeout;  // no arcs after a sort whose wait ran out
+  if (bad && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(window_err, bad);
   for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < m; j += (size_t)gridDim.x * blockDim.x) {
     const uint64_t x = keys[j];
-    flag[j] = x != ~0ull && (j == 0 || (keys[j - 1] >> kVsTBits) != (x >> kVsTBits)) ? 1u : 0u;
+    flag[j] = !bad && x != ~0ull && (j == 0 || (keys[j - 1] >> kVsTBits) != (x >> kVsTBits)) ? 1u : 0u;
   }
 }
 
@@ -1055,7 +1058,7 @@ int stream_versions(Bfs* b, const uint32_t* d_src, const uint32_t* d_dst, const 
     keys = in_alt ? S.keys_alt : S.keys;
     vals = in_alt ? S.vals_alt : S.vals;
     count_launch();
-    vs_runs_kernel<<<gm, 256, 0, st>>>(keys, m, S.flag);
+    vs_runs_kernel<<<gm, 256, 0, st>>>(keys, m, &g->ctr->err, S.flag, &S.ctr->err);
     if (int rc = scan_exclusive_u32(S.flag, S.pos, m, &S.ctr->runs, g->scratch, st)) return rc;
     VX_CUDA_TRY(cudaMemcpyAsync(&g->ctr->final_arcs, &S.ctr->runs, 4, cudaMemcpyDeviceToDevice, st));
     switch (words) {
