@@ -109,3 +109,21 @@ def test_components_report_it():
         c.labels_array()
     with pytest.raises(RuntimeError):
         c.last_repaired_vertices
+
+
+@pytest.mark.parametrize("directed", [False, True])
+def test_batches_after_an_error_stay_within_the_lists(directed):
+    # each of them would append its arcs behind the lengths the one before left
+    g = small_graph(directed)
+    b = vx.IncrementalBFS(g, 5)
+    set_sort_wait(g, 0)
+    b.apply_arrays(*big_batch(100_000))
+    for t in range(60):
+        b.apply_arrays(*big_batch(16_384, seed=t))
+    with pytest.raises(RuntimeError):
+        b.stats()
+    set_sort_wait(g, DEFAULT_LOOKS)  # the memory around the lists is sound
+    h = small_graph(directed)
+    c = vx.IncrementalBFS(h, 5)
+    c.apply_arrays(*big_batch(16_384))
+    assert np.array_equal(c.distances_array(), vx.IncrementalBFS(h, 5).distances_array())

@@ -2364,6 +2364,7 @@ constexpr uint32_t kRawMine = 1024;
 constexpr uint32_t kRawWarps = 32;
 constexpr uint8_t kFPending = 0x80;  // flag of an arc left to the grid
 constexpr uint8_t kFDead = 0x40;     // flag of a list slot without an arc of its own
+constexpr uint32_t kNoRoom = 0xFFFFFFFFu;
 struct RawArcs {
   unsigned long long key[kRawKeys];  // [dir] | u | v | op index | add
   uint32_t wsum[kThreads / 32];
@@ -2631,11 +2632,20 @@ __device__ bool canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32
     __syncthreads();
   }
   if (threadIdx.x < 2) {
-    const uint32_t k = threadIdx.x ? r.n[0] - r.n[1] : r.n[1];
-    r.base[threadIdx.x] = k ? atomicAdd(&f[threadIdx.x], k) : 0u;
+    const uint32_t k = threadIdx.x ? r.n[0] - r.n[1] : r.n[1], room = directed ? s.raw_n : 2 * s.raw_n;
+    const uint32_t at = k ? atomicAdd(&f[threadIdx.x], k) : 0u;
+    r.base[threadIdx.x] = at <= room && k <= room - at ? at : kNoRoom;
   }
   __syncthreads();
-  if (fits) return false;
+  // A launch that ended on a device error left its lengths behind: the batches
+  // after it, whose launches end at their first barrier, must not run past the lists.
+  const bool room = r.base[0] != kNoRoom && r.base[1] != kNoRoom;
+  if (!room) {
+    __syncthreads();
+    if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+    __syncthreads();
+  }
+  if (fits || !room) return false;
   canon_long(s, directed, r);
   __syncthreads();
   if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
