@@ -706,7 +706,9 @@ static uint64_t arena_bound_from(uint64_t top, uint64_t live) { return top + 4 *
 int graph_sync_counters(Graph* g) {
   VX_CUDA_TRY(cudaMemcpyAsync(g->hctr, g->ctr, sizeof(GraphCounters), cudaMemcpyDeviceToHost, g->stream));
   VX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  for (int d = 0; d < 2; ++d) g->adj[d].arena_bound = arena_bound_from(g->hctr->arena_top[d], g->hctr->delta_live[d]);
+  for (int d = 0; d < 2; ++d)
+    g->adj[d].arena_bound =
+        std::min(g->adj[d].arena_bound, arena_bound_from(g->hctr->arena_top[d], g->hctr->delta_live[d]));
   g->arena_pending = false;  // an older readback says less
   if (g->hctr->err) {
     const uint32_t e = g->hctr->err;
@@ -832,7 +834,10 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
 // hundreds on a busy host).  So the top and the live entries are read back when
 // half of the room is used up by it: a 32-byte copy on the stream, looked at
 // when it has arrived.  From then on the rows that hold those entries can take
-// at most 4 times them in new blocks, before the 8 per further arc.
+// at most 4 times them in new blocks, before the 8 per further arc.  That bound is
+// above the host's own where the rows are new (12 entries for each arc in a row of
+// its own): both hold, so the smaller one counts, and room reserved for a stream
+// by the 8 lasts for it.
 
 static_assert(offsetof(GraphCounters, delta_live) == 16 && offsetof(GraphCounters, arena_top) == 0,
               "one copy reads the tops and the live entries");
@@ -860,9 +865,11 @@ static int arena_take(Graph* g, bool wait) {
     if (e == cudaErrorNotReady) return 0;
     VX_CUDA_TRY(e);
   }
-  for (int d = 0; d < 2; ++d)
-    g->adj[d].arena_bound = arena_bound_from(g->arena_tops[d], g->arena_tops[2 + d]) +
-                            (g->adj[d].arena_bound - g->arena_seen[d]);
+  for (int d = 0; d < 2; ++d) {
+    Adjacency& a = g->adj[d];
+    a.arena_bound = std::min(a.arena_bound, arena_bound_from(g->arena_tops[d], g->arena_tops[2 + d]) +
+                                                (a.arena_bound - g->arena_seen[d]));
+  }
   g->arena_pending = false;
   return 0;
 }
