@@ -842,11 +842,16 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
 static_assert(offsetof(GraphCounters, delta_live) == 16 && offsetof(GraphCounters, arena_top) == 0,
               "one copy reads the tops and the live entries");
 
-// Enqueues the readback (not while the stream is being captured).
-static int arena_ask(Graph* g) {
+// A stream capture holds the batch's own launches alone: no readback is enqueued
+// in it, and an event may be neither queried nor waited for.
+static bool capturing(Graph* g) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (g->arena_pending || cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-    return 0;
+  return cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
+// Enqueues the readback.
+static int arena_ask(Graph* g) {
+  if (g->arena_pending || capturing(g)) return 0;
   VX_CUDA_TRY(cudaMemcpyAsync(g->arena_tops, g->ctr->arena_top, 32, cudaMemcpyDeviceToHost, g->stream));
   VX_CUDA_TRY(cudaEventRecord(g->arena_ev, g->stream));
   for (int d = 0; d < 2; ++d) g->arena_seen[d] = g->adj[d].arena_bound;
@@ -857,7 +862,7 @@ static int arena_ask(Graph* g) {
 // Takes a readback into the bounds, if one is in flight and has arrived (or,
 // with wait, when it has).
 static int arena_take(Graph* g, bool wait) {
-  if (!g->arena_pending) return 0;
+  if (!g->arena_pending || capturing(g)) return 0;
   if (wait) {
     VX_CUDA_TRY(cudaEventSynchronize(g->arena_ev));
   } else {
