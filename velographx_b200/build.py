@@ -42,7 +42,7 @@ def _run(cmd):
 
 def build_library(verbose_ptxas: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + [os.path.join(INCLUDE, "vx_b200.h")]
+    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + [os.path.join(INCLUDE, "vx_b200.h")]
     objs = []
     for src in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
         obj = os.path.join(BUILD, os.path.basename(src)[:-3] + ".o")

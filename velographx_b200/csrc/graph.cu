@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "arena_room.h"
 #include "graph.cuh"
 #include "graph_dev.cuh"
 
@@ -699,16 +700,14 @@ void graph_destroy(Graph* g) {
   delete g;
 }
 
-// A bound of arena_top for which room has been made when nothing else is
-// inserted (see reserve_arena): the rows' next blocks.
-static uint64_t arena_bound_from(uint64_t top, uint64_t live) { return top + 4 * live; }
-
 int graph_sync_counters(Graph* g) {
   VX_CUDA_TRY(cudaMemcpyAsync(g->hctr, g->ctr, sizeof(GraphCounters), cudaMemcpyDeviceToHost, g->stream));
   VX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  for (int d = 0; d < 2; ++d)
-    g->adj[d].arena_bound =
-        std::min(g->adj[d].arena_bound, arena_bound_from(g->hctr->arena_top[d], g->hctr->delta_live[d]));
+  for (int d = 0; d < 2; ++d) {
+    Adjacency& a = g->adj[d];
+    a.arena_read = arena_bound_from(g->hctr->arena_top[d], g->hctr->delta_live[d]);
+    a.arena_bound = std::min(a.arena_bound, a.arena_read);
+  }
   g->arena_pending = false;  // an older readback says less
   if (g->hctr->err) {
     const uint32_t e = g->hctr->err;
@@ -761,7 +760,7 @@ static int build_adjacency(Graph* g, Adjacency& a, uint64_t* keys, size_t m, int
   VX_CUDA_TRY(cudaMemsetAsync(a.dcap, 0, g->Vcap * sizeof(uint32_t), s));
   VX_CUDA_TRY(cudaMemsetAsync(a.tcnt, 0, g->Vcap * sizeof(uint32_t), s));
   VX_CUDA_TRY(cudaMemsetAsync(a.dirty, 0, ((g->Vcap + 31) / 32) * sizeof(uint32_t), s));
-  a.arena_bound = 0;
+  a.arena_bound = a.arena_read = 0;
   return 0;
 }
 
@@ -832,8 +831,8 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
 // and consolidate the graph in the end (100,000-op batches at R-MAT 20: to 1 GB
 // and a consolidation every 160 batches, calls of 4 to 95 ms, now and then
 // hundreds on a busy host).  So the top and the live entries are read back when
-// half of the room is used up by it: a 32-byte copy on the stream, looked at
-// when it has arrived.  From then on the rows that hold those entries can take
+// the bound has used up most of the room left (arena_ask_due): a 32-byte copy on
+// the stream, looked at when it has arrived.  From then on the rows that hold those entries can take
 // at most 4 times them in new blocks, before the 8 per further arc.  That bound is
 // above the host's own where the rows are new (12 entries for each arc in a row of
 // its own): both hold, so the smaller one counts, and room reserved for a stream
@@ -872,8 +871,8 @@ static int arena_take(Graph* g, bool wait) {
   }
   for (int d = 0; d < 2; ++d) {
     Adjacency& a = g->adj[d];
-    a.arena_bound = std::min(a.arena_bound, arena_bound_from(g->arena_tops[d], g->arena_tops[2 + d]) +
-                                                (a.arena_bound - g->arena_seen[d]));
+    a.arena_read = arena_bound_from(g->arena_tops[d], g->arena_tops[2 + d]);
+    a.arena_bound = std::min(a.arena_bound, a.arena_read + (a.arena_bound - g->arena_seen[d]));
   }
   g->arena_pending = false;
   return 0;
@@ -885,15 +884,16 @@ static int reserve_arena(Graph* g, size_t arcs, int* need_consolidate) {
   const int ndir = g->directed ? 2 : 1;
   const uint64_t add = 8ull * arcs + 8;
   if (int rc = arena_take(g, false)) return rc;
-  bool over = false, half = false;
+  bool over = false, due = false;
   for (int d = 0; d < ndir; ++d) {
-    over = over || g->adj[d].arena_bound + add > g->adj[d].arena_cap;
-    half = half || g->adj[d].arena_bound + add > g->adj[d].arena_cap / 2;
+    const Adjacency& a = g->adj[d];
+    over = over || a.arena_bound + add > a.arena_cap;
+    due = due || arena_ask_due(a.arena_bound + add, a.arena_read, a.arena_cap);
   }
   if (over) {
     if (int rc = arena_ask(g)) return rc;
     if (int rc = arena_take(g, true)) return rc;
-  } else if (half) {
+  } else if (due) {
     if (int rc = arena_ask(g)) return rc;
   }
   for (int d = 0; d < ndir; ++d) {
@@ -1131,7 +1131,7 @@ int graph_consolidate(Graph* g) {
     VX_CUDA_TRY(cudaMemsetAsync(&g->ctr->delta_live[d], 0, 8, s));
     VX_CUDA_TRY(cudaMemsetAsync(&g->ctr->tombs[d], 0, 8, s));
     VX_CUDA_TRY(cudaMemsetAsync(&g->ctr->dirty_rows[d], 0, 8, s));
-    a.arena_bound = 0;
+    a.arena_bound = a.arena_read = 0;
   }
   return 0;
 }

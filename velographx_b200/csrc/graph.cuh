@@ -40,6 +40,7 @@ struct Adjacency {
   uint32_t* darena = nullptr;
   size_t arena_cap = 0;
   uint64_t arena_bound = 0;    // host-side upper bound of arena_top
+  uint64_t arena_read = 0;     // that bound by the last readback alone
   void free_all();
 };
 
