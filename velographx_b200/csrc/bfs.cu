@@ -128,21 +128,19 @@ __device__ __forceinline__ void acct_add(const Params& p, int k, unsigned long l
   if (p.acct && v) atomicAdd(&p.acct[k], v);
 }
 
-// The errors a block's thread 0 looks at behind a barrier: the object's own, and
-// a wait of the graph's sort that ran out (its batch holds no arcs then), which
-// becomes the object's, so that the next synchronising call on it fails.
-__device__ __forceinline__ uint32_t barrier_errors(const Params& p) {
-  const uint32_t own = __ldcg(&p.c->err);
-  const uint32_t sort = p.graph_err ? __ldcg(p.graph_err) & vxb::kErrBarrierTimeout : 0u;
-  if (sort) atomicOr(&p.c->err, sort);
-  return own | sort;
+// A wait of the graph's sort that ran out (its batch holds no arcs then) becomes
+// the object's error, so that the next synchronising call on it fails: one thread
+// loads the word at the start of a launch and looks at it before the first barrier
+// (with the words of every barrier it cost 1 us a batch).
+__device__ __forceinline__ uint32_t sort_error(const Params& p) {
+  return gtid() == 0 && p.graph_err ? __ldcg(p.graph_err) & vxb::kErrBarrierTimeout : 0u;
 }
 
 // Grid barrier; returns false once any block recorded a device error (a
 // barrier that gave up waiting, a loop bound), so every persistent loop ends.
 __device__ __forceinline__ bool sync_grid(const Params& p) {
   __shared__ uint32_t failed;
-  vxb::grid_barrier_then(p.bar, p.nblocks, &p.c->err, [&] { failed = barrier_errors(p); });
+  vxb::grid_barrier_then(p.bar, p.nblocks, &p.c->err, [&] { failed = __ldcg(&p.c->err); });
   return failed == 0u;
 }
 
@@ -802,6 +800,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
                          uint32_t wbits_n, uint32_t* dist, unsigned long long* trace) {
   BfsCounters* c = p.c;
   const unsigned long long t_start = gtid() == 0 ? globaltimer() : 0ull;  // the repair phases' time budget
+  const uint32_t sort_err = kInRepair ? 0u : sort_error(p);
   __shared__ uint32_t seg_n[2];  // entries of this block's segment of each candidate list
   __shared__ unsigned long long red[kT / 32];
   __shared__ LevelWords lw;
@@ -834,6 +833,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     p.fb[0][i] = p.fb[1][i] = p.fb[2][i] = 0u;
   }
   if (gtid() == 0) {
+    if (sort_err) atomicOr(&c->err, sort_err);
     for (int k = 0; k < 3; ++k) {
       c->lvl_n[k] = 0;
       c->lvl_big[k] = 0;
@@ -1200,7 +1200,7 @@ __device__ __forceinline__ bool sync_words(const Params& p, RepairWords& w) {
   BfsCounters* c = p.c;
   vxb::grid_barrier_then(p.bar, p.nblocks, &c->err, [&] {
     RepairWords r;
-    r.failed = barrier_errors(p);
+    r.failed = __ldcg(&c->err);
     r.candidates = ld_cg(&c->cand_n);
     r.touched = p.touched_base + ld_cg(&c->touched_n);
     r.affected = ld_cg(&c->a_n);
@@ -3138,6 +3138,7 @@ __device__ void insertion_pass(ArcWork& w, RepairSmem& sm) {
 
 __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
+  const uint32_t sort_err = sort_error(p);
   unsigned long long tmark = globaltimer();
   auto phase = [&](int k) {  // gtid 0 accumulates the time since the previous mark
     if (gtid() == 0) {
@@ -3190,6 +3191,7 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
       removal_pass(w, sm);
     }
     if (s.digest && bi > 0) digest_pass(p.dist, lpre, &s.digest[bi - 1]);
+    if (sort_err) atomicOr(&c->err, sort_err);
     if (!sync_words(q, sm.w)) return;
     phase(0);
     if (s.raw_n) {
@@ -3295,6 +3297,7 @@ __global__ void __launch_bounds__(kThreads, 2) bfs_kernel(Params p, int mode) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
+  if (const uint32_t e = sort_error(p)) atomicOr(&p.c->err, e);
   if (mode == kModePre) repair_pre(p, sm, lb, bq);
   else repair_post<false>(p, sm, lb, bq);
 }
