@@ -2343,6 +2343,7 @@ struct StreamArgs {
   const uint32_t* raw_src;
   const uint32_t* raw_dst;
   const uint8_t* raw_add;
+  uint32_t* over;  // canon_grid: per block, rows left to the grid, then two counts
   uint32_t raw_n, raw_b, raw_sh, raw_bound;
 };
 
@@ -2350,26 +2351,29 @@ struct StreamArgs {
 // reads all ops and keeps the arcs whose row hashes to it (a dozen of 2,000), sorts
 // them, keeps the last of each arc and appends them to the batch's list, so
 // the arcs of a row are consecutive there and the block that has them in
-// shared memory can process them at once.  A launch of its own with a cluster's
+// shared memory can process them at once.  Rows of more arcs than a block sorts are
+// listed by the whole grid (canon_grid).  A launch of its own with a cluster's
 // barriers between the radix passes took 12 to 44 us; every block sorting
 // all arcs 2 us for 128 arcs but 7 for 1,024 and 13 for 2,048, bound by the
 // instructions of the one block an SM runs; now 2 to 8 (10,000 ops).  The limit keeps a
 // block's reading (9 bytes an op from L2) at a few microseconds.
 constexpr uint32_t kRawOps = 16384;
-constexpr uint32_t kRawKeys = 2048;  // arcs a block sorts at once (canon_long beyond)
+constexpr uint32_t kRawKeys = 2048;  // arcs a block sorts at once (canon_grid beyond)
+constexpr uint32_t kRawBlocks = 512;  // blocks of a launch at most
 constexpr unsigned long long kRawDir = 1ull << 63;  // a directed graph's reversed arcs sort last
 // A block with more arcs than this (hub rows) leaves them to the whole grid,
 // behind a barrier; with more than kRawWarps it gives each a lane, not a warp.
 constexpr uint32_t kRawMine = 1024;
 constexpr uint32_t kRawWarps = 32;
 constexpr uint8_t kFPending = 0x80;  // flag of an arc left to the grid
-constexpr uint8_t kFDead = 0x40;     // flag of a list slot without an arc of its own
 constexpr uint32_t kNoRoom = 0xFFFFFFFFu;
 struct RawArcs {
   unsigned long long key[kRawKeys];  // [dir] | u | v | op index | add
   uint32_t wsum[kThreads / 32];
   uint32_t n[2];                     // arcs, and those of direction 0 among them
   uint32_t base[2];                  // their places in the batch's lists
+  uint32_t over[kRawBlocks / 32];    // canon_grid: blocks whose rows are left to the grid
+  uint32_t sum[4];
 };
 static_assert(sizeof(RawArcs) <= sizeof(LbStage), "the arcs are kept in the row stage's memory");
 
@@ -2410,11 +2414,11 @@ __device__ __forceinline__ void warp_sort(unsigned long long (&x)[E]) {
 }
 
 // Sorts the block's n arc keys, padded to N (a power of two, 32 * E per warp in
-// use), and keeps the last of each arc.  Every warp sorts its keys in
-// registers; the runs are then merged pairwise, each key finding its place by a
-// binary search of the other run.
+// use), and, unless all are wanted, keeps the last of each arc.  Every warp sorts
+// its keys in registers; the runs are then merged pairwise, each key finding its
+// place by a binary search of the other run.
 template <int E>
-__device__ void canon_sort(const StreamArgs& s, bool directed, RawArcs& r, uint32_t n, uint32_t N) {
+__device__ void canon_sort(const StreamArgs& s, bool directed, RawArcs& r, uint32_t n, uint32_t N, bool all) {
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const bool on = warp * 32 * E < N;
   unsigned long long x[E];
@@ -2471,6 +2475,7 @@ __device__ void canon_sort(const StreamArgs& s, bool directed, RawArcs& r, uint3
     }
     __syncthreads();
   }
+  if (all) return;
   // the last key of every arc, compacted in place
   unsigned long long keep[E];
   uint32_t cnt = 0, cnt0 = 0;
@@ -2506,131 +2511,57 @@ __device__ void canon_sort(const StreamArgs& s, bool directed, RawArcs& r, uint3
   __syncthreads();
 }
 
-// The keys of the batch's arcs that are this block's, f(key) each (a lane at a
-// time).  first: reports ids out of bound.
-template <class F>
-__device__ __forceinline__ void raw_scan(const StreamArgs& s, bool directed, bool first, F&& f) {
-  for (uint32_t i = threadIdx.x; i < s.raw_n; i += kThreads) {
-    const uint32_t a = s.raw_src[i], b = s.raw_dst[i];
-    const unsigned long long low = ((unsigned long long)i << 1) | (s.raw_add[i] ? 1ull : 0ull);
-    bool ok = a != b;
-    if (ok && (a >= s.raw_bound || b >= s.raw_bound)) {
-      if (first && blockIdx.x == 0) atomicOr(&s.gc->err, vxb::kErrBadVertex);
-      ok = false;
-    }
-    if (!ok) continue;
+// The keys of op i's arcs whose row hashes to a block that mine(block) takes,
+// f(key) each.  first: reports ids out of bound.
+template <class Mine, class F>
+__device__ __forceinline__ void raw_op(const StreamArgs& s, bool directed, uint32_t i, bool first, Mine&& mine, F&& f) {
+  const uint32_t a = s.raw_src[i], b = s.raw_dst[i];
+  const unsigned long long low = ((unsigned long long)i << 1) | (s.raw_add[i] ? 1ull : 0ull);
+  bool ok = a != b;
+  if (ok && (a >= s.raw_bound || b >= s.raw_bound)) {
+    if (first && blockIdx.x == 0) atomicOr(&s.gc->err, vxb::kErrBadVertex);
+    ok = false;
+  }
+  if (!ok) return;
 #pragma unroll
-    for (int rev = 0; rev < 2; ++rev) {
-      const unsigned long long u = rev ? b : a, v = rev ? a : b;
-      if (__umulhi((uint32_t)u * 0x9E3779B1u, gridDim.x) != blockIdx.x) continue;
-      f((directed && rev ? kRawDir : 0ull) | (u << (s.raw_b + s.raw_sh)) | (v << s.raw_sh) | low);
-    }
+  for (int rev = 0; rev < 2; ++rev) {
+    const unsigned long long u = rev ? b : a, v = rev ? a : b;
+    if (!mine(__umulhi((uint32_t)u * 0x9E3779B1u, gridDim.x))) continue;
+    f((directed && rev ? kRawDir : 0ull) | (u << (s.raw_b + s.raw_sh)) | (v << s.raw_sh) | low);
   }
 }
 
-__device__ void canon_keys(const StreamArgs& s, bool directed, RawArcs& r, uint32_t n) {
+__device__ void canon_keys(const StreamArgs& s, bool directed, RawArcs& r, uint32_t n, bool all = false) {
   uint32_t N = 32;
   while (N < n) N <<= 1;
   static_assert(kRawKeys == 4 * kThreads, "four keys per thread at most");
-  if (N <= kThreads) canon_sort<1>(s, directed, r, n, N);
-  else if (N <= 2 * kThreads) canon_sort<2>(s, directed, r, n, N);
-  else canon_sort<4>(s, directed, r, n, N);
-}
-
-// A block's n arcs that do not fit its shared memory (a batch most of whose ops
-// share a row): listed in ascending ranges of their (dir, u, v) value that do,
-// halved and doubled as they come, each found by another scan of the ops.  Slow
-// (some 20 us for 1,000 arcs) but for any batch.  The arcs are left to the
-// grid; slots that repeated ops on an arc leave over hold a copy without effect.
-__device__ __noinline__ void canon_long(const StreamArgs& s, bool directed, RawArcs& r) {
-  const uint32_t bits = 2 * s.raw_b;
-  auto value = [&](unsigned long long key) {
-    return ((key & ~kRawDir) >> s.raw_sh) | (key & kRawDir ? 1ull << bits : 0ull);
-  };
-  const unsigned long long top = (directed ? 2ull : 1ull) << bits;
-  uint32_t place[2] = {r.base[0], r.base[1]}, end[2];
-  end[0] = place[0] + r.n[1];
-  end[1] = place[1] + (r.n[0] - r.n[1]);
-  unsigned long long lo = 0, width = top;
-  __syncthreads();  // r.n and r.base are read
-  while (lo < top) {
-    const unsigned long long hi = top - lo < width ? top : lo + width;
-    if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
-    __syncthreads();
-    raw_scan(s, directed, false, [&](unsigned long long key) {
-      const unsigned long long x = value(key);
-      if (x < lo || x >= hi) return;
-      const uint32_t k = atomicAdd(&r.n[0], 1u);
-      if (k < kRawKeys) r.key[k] = key;
-    });
-    __syncthreads();
-    uint32_t n = r.n[0];
-    __syncthreads();
-    if (n > kRawKeys && hi - lo > 1) {
-      width = (hi - lo + 1) / 2;
-      continue;
-    }
-    if (n > kRawKeys) {  // one arc, more ops than fit: its last op
-      if (threadIdx.x == 0) r.key[0] = 0;
-      __syncthreads();
-      raw_scan(s, directed, false, [&](unsigned long long key) {
-        if (value(key) == lo) atomicMax(&r.key[0], key);
-      });
-      __syncthreads();
-      n = 1;
-    }
-    if (n) {
-      if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
-      __syncthreads();
-      canon_keys(s, directed, r, n);
-      const uint32_t kept = r.n[0], kept0 = r.n[1];
-      for (uint32_t i = threadIdx.x; i < kept; i += kThreads) {
-        const int dir = i >= kept0;
-        const uint32_t at = place[dir] + i - (dir ? kept0 : 0u);
-        const unsigned long long k = r.key[i];
-        const_cast<uint32_t*>(s.fu[dir])[at] = (uint32_t)((k & ~kRawDir) >> (s.raw_b + s.raw_sh));
-        const_cast<uint32_t*>(s.fv[dir])[at] = (uint32_t)(k >> s.raw_sh) & ((1u << s.raw_b) - 1u);
-        s.ff[dir][at] = (uint8_t)(k & 1ull) | kFPending;
-      }
-      place[0] += kept0;
-      place[1] += kept - kept0;
-      __syncthreads();
-    }
-    if (n < kRawKeys / 2 && width <= top / 2) width *= 2;
-    lo = hi;
-  }
-  for (int dir = 0; dir < (directed ? 2 : 1); ++dir)
-    for (uint32_t at = place[dir] + threadIdx.x; at < end[dir]; at += kThreads) {
-      const_cast<uint32_t*>(s.fu[dir])[at] = s.fu[dir][place[dir] - 1];
-      const_cast<uint32_t*>(s.fv[dir])[at] = s.fv[dir][place[dir] - 1];
-      s.ff[dir][at] = kFDead;
-    }
+  if (N <= kThreads) canon_sort<1>(s, directed, r, n, N, all);
+  else if (N <= 2 * kThreads) canon_sort<2>(s, directed, r, n, N, all);
+  else canon_sort<4>(s, directed, r, n, N, all);
 }
 
 // The block's arcs of the batch in r, and their places in the batch's lists
-// (whose lengths are f[0] and f[1], zero before); true when the block has too
-// many and listed them itself, all pending.  Block-uniform.
+// (whose lengths are f[0] and f[1], zero before); true, and no arcs, when the block
+// has too many: canon_grid lists them.  Block-uniform.
 __device__ bool canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32_t* f) {
   if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
   __syncthreads();
-  raw_scan(s, directed, true, [&](unsigned long long key) {
-    const uint32_t k = atomicAdd(&r.n[0], 1u);
-    if (k < kRawKeys) r.key[k] = key;
-  });
+  for (uint32_t i = threadIdx.x; i < s.raw_n; i += kThreads)
+    raw_op(s, directed, i, true, [&](uint32_t b) { return b == blockIdx.x; }, [&](unsigned long long key) {
+      if (*(volatile uint32_t*)&r.n[0] > kRawKeys) return;
+      const uint32_t k = atomicAdd(&r.n[0], 1u);
+      if (k < kRawKeys) r.key[k] = key;
+    });
   __syncthreads();
   const uint32_t n = r.n[0];
   __syncthreads();
   const bool fits = n <= kRawKeys;
-  if (fits) {
-    if (threadIdx.x == 0) r.n[0] = 0;
-    __syncthreads();
-    canon_keys(s, directed, r, n);
-  } else {
-    raw_scan(s, directed, false, [&](unsigned long long key) {
-      if (!(directed && (key & kRawDir))) atomicAdd(&r.n[1], 1u);
-    });
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    r.n[0] = 0;
+    s.over[blockIdx.x] = fits ? 0u : 1u;
   }
+  __syncthreads();
+  if (fits) canon_keys(s, directed, r, n);
   if (threadIdx.x < 2) {
     const uint32_t k = threadIdx.x ? r.n[0] - r.n[1] : r.n[1], room = directed ? s.raw_n : 2 * s.raw_n;
     const uint32_t at = k ? atomicAdd(&f[threadIdx.x], k) : 0u;
@@ -2639,17 +2570,157 @@ __device__ bool canon_raw(const StreamArgs& s, bool directed, RawArcs& r, uint32
   __syncthreads();
   // A launch that ended on a device error left its lengths behind: the batches
   // after it, whose launches end at their first barrier, must not run past the lists.
-  const bool room = r.base[0] != kNoRoom && r.base[1] != kNoRoom;
-  if (!room) {
+  if (r.base[0] == kNoRoom || r.base[1] == kNoRoom) {
     __syncthreads();
     if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
     __syncthreads();
   }
-  if (fits || !room) return false;
-  canon_long(s, directed, r);
+  return !fits;
+}
+
+// Ascending ranges of [lo, hi) of the arcs' (dir, u, v) value whose arcs fit r,
+// halved and doubled as they come: emit() for each, its arcs in r (the last op of
+// each, r.n as canon_keys leaves it).  One range, the whole of it, where
+// canon_grid's samples do not deceive.  Returns their number.  Block-uniform.
+template <class Mine, class Emit>
+__device__ uint32_t raw_ranges(const StreamArgs& s, bool directed, RawArcs& r, unsigned long long lo,
+                               unsigned long long end, Mine&& mine, Emit&& emit) {
+  const uint32_t bits = 2 * s.raw_b;
+  auto value = [&](unsigned long long key) {
+    return ((key & ~kRawDir) >> s.raw_sh) | (key & kRawDir ? 1ull << bits : 0ull);
+  };
+  unsigned long long width = end - lo;
+  uint32_t ranges = 0;
+  while (lo < end) {
+    const unsigned long long hi = end - lo < width ? end : lo + width;
+    __syncthreads();  // the range before is done with
+    if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+    if (threadIdx.x == 0) r.key[0] = 0;
+    __syncthreads();
+    uint32_t n;
+    if (hi - lo == 1) {  // one arc, of any number of ops: its last
+      unsigned long long last = 0;
+      for (uint32_t i = threadIdx.x; i < s.raw_n; i += kThreads)
+        raw_op(s, directed, i, false, mine, [&](unsigned long long key) {
+          if (value(key) == lo && key > last) last = key;
+        });
+      if (last) atomicMax(&r.key[0], last);  // ids of an arc differ, so no key is 0
+      __syncthreads();
+      n = r.key[0] ? 1u : 0u;
+    } else {
+      for (uint32_t i = threadIdx.x; i < s.raw_n; i += kThreads)
+        raw_op(s, directed, i, false, mine, [&](unsigned long long key) {
+          const unsigned long long x = value(key);
+          if (x < lo || x >= hi || *(volatile uint32_t*)&r.n[0] > kRawKeys) return;
+          const uint32_t k = atomicAdd(&r.n[0], 1u);
+          if (k < kRawKeys) r.key[k] = key;
+        });
+      __syncthreads();
+      n = r.n[0];
+    }
+    __syncthreads();
+    if (n > kRawKeys) {
+      width = (hi - lo + 1) / 2;
+      continue;
+    }
+    if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+    __syncthreads();
+    canon_keys(s, directed, r, n);
+    emit();
+    ++ranges;
+    if (n < kRawKeys / 2 && width <= (end - lo) / 2) width *= 2;
+    lo = hi;
+  }
+  return ranges;
+}
+
+// The arcs of rows whose block has too many of them, listed by the whole grid in
+// the order of their (dir, u, v) value: all blocks sort the same sample of the
+// ops, take the range between two of its entries each, sort their range's arcs,
+// and write them behind those of the blocks before (marked kFPending: a row's arcs
+// lie with several blocks).  An arc that fills a block's share of the sample or
+// more is a range by itself.  The hub's block alone, range after range of 2,048
+// arcs, took the launch 1.5 ms longer than a cluster's sort of the batch does
+// (16,384 ops on one row at R-MAT 20: 2.88 ms a call against 1.38).  words: as of
+// the last barrier; false on a device error.  Grid-uniform.
+constexpr uint32_t kRawSamples = 512;  // ops
+__device__ __noinline__ bool canon_grid(const Params& p, const StreamArgs& s, RawArcs& r,
+                                        const RepairWords& words) {
+  const bool directed = p.g.directed;
+  const uint32_t t = threadIdx.x, G = gridDim.x, b = blockIdx.x;
+  if (t < 2) r.n[t] = 0;
+  if (t < 4) r.sum[t] = 0;
+  for (uint32_t i = t; i < kRawBlocks / 32; i += kThreads) r.over[i] = 0;
   __syncthreads();
-  if (threadIdx.x < 2) r.n[threadIdx.x] = 0;
+  for (uint32_t i = t; i < G; i += kThreads)
+    if (ld_cg(&s.over[i])) atomicOr(&r.over[i >> 5], 1u << (i & 31));
   __syncthreads();
+  auto left = [&](uint32_t block) { return (r.over[block >> 5] >> (block & 31)) & 1u; };
+  const uint32_t S = min(s.raw_n, kRawSamples);
+  for (uint32_t i = t; i < S; i += kThreads) {
+    const uint32_t lo = (uint32_t)((uint64_t)i * s.raw_n / S), hi = (uint32_t)((uint64_t)(i + 1) * s.raw_n / S);
+    raw_op(s, directed, lo + (uint32_t)(vxb::mix64(i) % (hi - lo)), false, left,
+           [&](unsigned long long key) { r.key[atomicAdd(&r.n[0], 1u)] = key; });
+  }
+  __syncthreads();
+  const uint32_t ns = r.n[0];
+  __syncthreads();
+  static_assert(2 * kRawSamples <= kRawKeys, "the samples' arcs are sorted at once");
+  canon_keys(s, directed, r, ns, true);
+  const uint32_t bits = 2 * s.raw_b;
+  auto split = [&](uint32_t k) {  // first value of block k's range
+    if (k == 0 || ns == 0) return k < G ? 0ull : (directed ? 2ull : 1ull) << bits;
+    if (k >= G) return (directed ? 2ull : 1ull) << bits;
+    const unsigned long long key = r.key[(uint64_t)k * ns / G];
+    return ((key & ~kRawDir) >> s.raw_sh) | (key & kRawDir ? 1ull << bits : 0ull);
+  };
+  unsigned long long lo = split(b), hi = split(b + 1);
+  const bool again = b > 0 && split(b - 1) == lo;  // the block before begins at the same arc
+  if (lo == hi) hi = again ? lo : lo + 1;          // the first of them takes that arc,
+  else if (again) ++lo;                            // the last what lies behind it
+  uint32_t kept[2] = {0, 0};
+  const uint32_t ranges = raw_ranges(s, directed, r, lo, hi, left, [&] {
+    kept[0] += r.n[1];
+    kept[1] += r.n[0] - r.n[1];
+  });
+  if (t == 0) {
+    s.over[G + b] = kept[0];
+    s.over[2 * G + b] = kept[1];
+  }
+  if (!sync_grid(p)) return false;
+  for (uint32_t i0 = t & ~31u; i0 < G; i0 += kThreads) {
+    const uint32_t i = i0 + (t & 31);
+    for (uint32_t d = 0; d < 2; ++d) {
+      const uint32_t c = i < G ? ld_cg(&s.over[(d + 1) * G + i]) : 0u;
+      const uint32_t before = __reduce_add_sync(FULL, i < b ? c : 0u), sum = __reduce_add_sync(FULL, c);
+      if ((t & 31) == 0) {
+        atomicAdd(&r.sum[d], before);
+        atomicAdd(&r.sum[2 + d], sum);
+      }
+    }
+  }
+  __syncthreads();
+  uint32_t place[2] = {words.raw_f[0] + r.sum[0], words.raw_f[1] + r.sum[1]};
+  if (gtid() == 0) {  // the lists' new lengths, read behind the next barrier
+    p.bar[kRawWord] = words.raw_f[0] + r.sum[2];
+    p.bar[kRawWord + 1] = words.raw_f[1] + r.sum[3];
+  }
+  auto write = [&] {
+    const uint32_t n = r.n[0], n0 = r.n[1];
+    for (uint32_t i = t; i < n; i += kThreads) {
+      const int dir = i >= n0;
+      const uint32_t at = place[dir] + i - (dir ? n0 : 0u);
+      const unsigned long long k = r.key[i];
+      const_cast<uint32_t*>(s.fu[dir])[at] = (uint32_t)((k & ~kRawDir) >> (s.raw_b + s.raw_sh));
+      const_cast<uint32_t*>(s.fv[dir])[at] = (uint32_t)(k >> s.raw_sh) & ((1u << s.raw_b) - 1u);
+      s.ff[dir][at] = (uint8_t)(k & 1ull) | kFPending;
+    }
+    place[0] += n0;
+    place[1] += n - n0;
+  };
+  if (ranges == 1) write();
+  else if (ranges) raw_ranges(s, directed, r, lo, hi, left, write);
+  __syncthreads();  // r is used by others
   return true;
 }
 
@@ -2663,14 +2734,19 @@ __device__ void digest_pass(const uint32_t* dist, uint32_t n, unsigned long long
   if ((threadIdx.x & 31) == 0 && h) atomicAdd(out, h);
 }
 
-// End of the row run of canonical arcs starting at s (same u), whole warp.
+// End of the row run of canonical arcs starting at s (same u), whole warp: 32
+// probes a step, 1, 32, 1,024 ... arcs apart while all of them are the row's, then
+// closer again (a row's arcs are consecutive).
 __device__ __forceinline__ uint32_t run_end(const uint32_t* fu, uint32_t s, uint32_t F) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t u = fu[s];
-  for (uint32_t k = s + 1;; k += 32) {
-    const uint32_t i = k + lane;
+  const uint32_t lane = threadIdx.x & 31, u = fu[s];
+  uint64_t last = s, stride = 1;  // last: an arc of the row
+  for (;;) {
+    const uint64_t i = last + (lane + 1) * stride;
     const uint32_t m = __ballot_sync(FULL, i >= F || fu[i] != u);
-    if (m) return k + (uint32_t)(__ffs(m) - 1);
+    last += (m ? (uint32_t)(__ffs(m) - 1) : 32u) * stride;
+    if (!m) stride *= 32;
+    else if (stride == 1) return (uint32_t)last + 1;
+    else stride /= 32;
   }
 }
 
@@ -2680,9 +2756,13 @@ __device__ __forceinline__ bool delta_op(uint8_t f, bool insertion) {
 
 // Delta removals of one row run (whole warp): the row's sorted delta list
 // keeps every entry that is not a removal of the run (delta_remove_kernel of
-// the per-batch path, on the canonical arcs directly).
+// the per-batch path, on the canonical arcs directly).  128 entries a step, their
+// searches in the run side by side: a hub's run is one warp's chain.  9,000 ops on
+// one row at R-MAT 20, 6,300 removals: with run_end's probes the pass takes 232 us
+// instead of 337, and the insertions back 92 instead of 176.
 __device__ void run_remove(const vxb::DevAdj& a, int dir, const uint32_t* fv, const uint8_t* ff, uint32_t s, uint32_t e,
                            uint32_t u, GraphCounters* gc, unsigned long long* acct) {
+  constexpr int kStep = 4;
   const int lane = threadIdx.x & 31;
   bool any = false;
   for (uint32_t k = s + lane; k < e; k += 32) any |= delta_op(ff[k], false);
@@ -2690,20 +2770,31 @@ __device__ void run_remove(const vxb::DevAdj& a, int dir, const uint32_t* fv, co
   const uint2 row = a.drow[u];
   uint32_t* A = a.darena + row.x;
   uint32_t written = 0;
-  for (uint32_t base = 0; base < row.y; base += 32) {
-    const uint32_t j = base + lane;
-    const bool in = j < row.y;
-    const uint32_t x = in ? A[j] : 0u;
-    bool keep = in;
-    if (in) {
-      const uint32_t q = vxb::lower_bound_u32(fv, s, e, x);
-      if (q < e && fv[q] == x && delta_op(ff[q], false)) keep = false;
+  for (uint32_t base = 0; base < row.y; base += 32 * kStep) {
+    uint32_t x[kStep], lo[kStep];
+#pragma unroll
+    for (int r = 0; r < kStep; ++r) {
+      const uint32_t j = base + 32 * r + lane;
+      x[r] = j < row.y ? A[j] : 0u;
+      lo[r] = s;
     }
-    const uint32_t mask = __ballot_sync(FULL, keep);
-    const uint32_t p = written + __popc(mask & vxb::lanemask_lt());
-    __syncwarp();
-    if (keep) A[p] = x;
-    written += __popc(mask);
+    for (uint32_t len = e - s; len > 1;) {  // x's place in the run is lo or, at the end, lo + 1
+      const uint32_t half = len >> 1;
+#pragma unroll
+      for (int r = 0; r < kStep; ++r)
+        if (fv[lo[r] + half - 1] < x[r]) lo[r] += half;
+      len -= half;
+    }
+    __syncwarp();  // every entry of the step is read
+#pragma unroll
+    for (int r = 0; r < kStep; ++r) {
+      if (base + 32 * r >= row.y) break;
+      const uint32_t q = lo[r] + (fv[lo[r]] < x[r] ? 1u : 0u);
+      const bool keep = base + 32 * r + lane < row.y && !(q < e && fv[q] == x[r] && delta_op(ff[q], false));
+      const uint32_t mask = __ballot_sync(FULL, keep);
+      if (keep) A[written + __popc(mask & vxb::lanemask_lt())] = x[r];
+      written += __popc(mask);
+    }
     __syncwarp();
   }
   if (lane == 0) {
@@ -2723,12 +2814,21 @@ __device__ void run_insert(const vxb::DevAdj& a, int dir, const uint32_t* fv, co
                            unsigned long long* acct) {
   const int lane = threadIdx.x & 31;
   uint32_t nB = 0;
-  for (uint32_t base = s; base < e; base += 32) {
-    const uint32_t k = base + lane;
-    const bool ins = k < e && delta_op(ff[k], true);
-    const uint32_t m = __ballot_sync(FULL, ins);
-    if (ins) scratch[s + nB + __popc(m & vxb::lanemask_lt())] = fv[k];
-    nB += __popc(m);
+  for (uint32_t base = s; base < e; base += 128) {  // 128 arcs in flight
+    uint32_t v[4];
+    bool ins[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t k = base + 32 * r + lane;
+      ins[r] = k < e && delta_op(ff[k], true);
+      v[r] = k < e ? fv[k] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t m = __ballot_sync(FULL, ins[r]);
+      if (ins[r]) scratch[s + nB + __popc(m & vxb::lanemask_lt())] = v[r];
+      nB += __popc(m);
+    }
   }
   if (nB == 0) return;
   __syncwarp();
@@ -2849,9 +2949,25 @@ struct ArcWork {
     return (i > 0 && tail_of(i - 1) == u) || (i + 1 < F && tail_of(i + 1) == u);
   }
 
-  // The delta removals of run [st, en), classified before; whole warp.
-  __device__ void remove_run(uint32_t st, uint32_t en) {
-    run_remove(*a, dir, fv, ff, st, en, fu[st], s->gc, p->acct ? p->acct + 2 : nullptr);
+  // Arc (u, v) leaves u's delta row; whole warp.
+  __device__ void remove_one(uint32_t u, uint32_t v) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint2 row = a->drow[u];
+    uint32_t* A = a->darena + row.x;
+    uint32_t written = 0;
+    for (uint32_t base = 0; base < row.y; base += 32) {
+      const uint32_t x = base + lane < row.y ? A[base + lane] : v;
+      const uint32_t mask = __ballot_sync(FULL, x != v);
+      if (x != v) A[written + __popc(mask & vxb::lanemask_lt())] = x;
+      written += __popc(mask);
+      __syncwarp();
+    }
+    if (lane == 0) {
+      a->drow[u].y = written;
+      acct_add(*p, 2, (unsigned long long)row.y + written);
+      atomicAdd(&s->gc->delta_live[dir], (unsigned long long)(-(long long)(row.y - written)));
+      gdev::mark_dirty(a->dirty, u, &s->gc->dirty_rows[dir]);
+    }
   }
 
   // The sums of the pass into the graph's counters.
@@ -2891,6 +3007,7 @@ struct SmallRow {
 // What the first removal pass left for later (bits of BfsCounters::later).
 constexpr uint32_t kLaterRuns = 1u;  // delta removals of runs of several arcs
 constexpr uint32_t kLaterArcs = 2u;  // arcs marked kFPending
+constexpr uint32_t kLaterRows = 4u;  // rows of blocks with too many arcs (canon_grid)
 
 // The removal pass.  A batch of few arcs takes a warp per arc: its row searches
 // read 32 pivots per round trip instead of 7, and the chain of such a batch is
@@ -2963,7 +3080,7 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
         }
       } else {
         __syncwarp();
-        w.remove_run(base + i, base + i + 1);
+        w.remove_one(u, v);
       }
     }
   } else {
@@ -3028,7 +3145,7 @@ __device__ void removal_pass(ArcWork& w, RepairSmem& sm) {
       if (queue) sm.sv[atomicAdd(&sm.nsv, 1u)] = base + i;
       __syncthreads();
       const uint32_t nq = sm.nsv;
-      for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_run(sm.sv[k], sm.sv[k] + 1);
+      for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32) w.remove_one(w.fu[sm.sv[k]], w.fv[sm.sv[k]]);
       __syncthreads();  // the list is rebuilt by the next round
     }
   }
@@ -3050,7 +3167,8 @@ __device__ void removal_runs(ArcWork& w, RepairSmem& sm) {
     __syncthreads();
     const uint32_t nq = sm.nsv;
     for (uint32_t k = threadIdx.x >> 5; k < nq; k += kThreads / 32)
-      w.remove_run(sm.sv[k], run_end(w.fu, sm.sv[k], w.F));
+      run_remove(*w.a, w.dir, w.fv, w.ff, sm.sv[k], run_end(w.fu, sm.sv[k], w.F), w.fu[sm.sv[k]], w.s->gc,
+                 w.p->acct ? w.p->acct + 2 : nullptr);
     __syncthreads();  // the list is rebuilt by the next round
   }
 }
@@ -3136,7 +3254,7 @@ __device__ void insertion_pass(ArcWork& w, RepairSmem& sm) {
   w.flush();
 }
 
-__device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
+__device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
   const uint32_t sort_err = sort_error(p);
   unsigned long long tmark = globaltimer();
@@ -3157,7 +3275,7 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     RawArcs& raw = reinterpret_cast<RawArcs&>(lb);
     uint32_t off = 0, F = 0, Frev = 0;
     if (s.raw_n) {
-      if (canon_raw(s, p.g.directed, raw, p.bar + kRawWord) && threadIdx.x == 0) atomicOr(&c->later, kLaterArcs);
+      if (canon_raw(s, p.g.directed, raw, p.bar + kRawWord) && threadIdx.x == 0) atomicOr(&c->later, kLaterRows);
     } else {
       if (s.boff) off = s.boff[bi];
       F = s.cnt[0][bi];
@@ -3194,11 +3312,12 @@ __device__ void stream_kernel_body(Params p, const StreamArgs& s, RepairSmem& sm
     if (sort_err) atomicOr(&c->err, sort_err);
     if (!sync_words(q, sm.w)) return;
     phase(0);
+    if ((sm.w.later & kLaterRows) && !(canon_grid(p, s, raw, sm.w) && sync_words(q, sm.w))) return;
     if (s.raw_n) {
       F = sm.w.raw_f[0];
       Frev = sm.w.raw_f[1];
     }
-    if (sm.w.later & kLaterArcs) {
+    if (sm.w.later & (kLaterArcs | kLaterRows)) {
       for (int dir = 0; dir < ndir; ++dir) {
         ArcWork w = work(dir);
         w.pending = true;
@@ -3306,7 +3425,11 @@ __global__ void __launch_bounds__(kThreads, 2) bfs_kernel(Params p, int mode) {
 // streams) then run side by side, which a block with 128 registers a thread
 // (no spills, 2% faster alone) does not allow: 10,000-op batches on three R-MAT
 // 22 graphs in turn 86 us a batch, 111 us with 128 registers.
-__global__ void __launch_bounds__(kThreads, 2) bfs_stream_kernel(Params p, StreamArgs s) {
+// The arguments stay in the kernel's parameter space: as copies for the functions
+// that take them by reference they made a stack frame of 1,184 bytes a thread, now
+// 928 (10,000 ops at R-MAT 22, three graphs in turn: 67.8 us a batch, now 62.1).
+__global__ void __launch_bounds__(kThreads, 2) bfs_stream_kernel(const __grid_constant__ Params p,
+                                                                 const __grid_constant__ StreamArgs s) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
@@ -3796,7 +3919,7 @@ static int launch_stream(Bfs* b, Params& p, StreamArgs& sa) {
   // block) the grid barriers and the work ring's polling are cheaper, and the
   // update step measured 13% faster at R-MAT 22 and R-MAT 20
   const uint32_t want = b->tune.update_blocks ? b->tune.update_blocks : (uint32_t)sm_count();
-  p.nblocks = want < (uint32_t)b->stream_grid ? want : (uint32_t)b->stream_grid;
+  p.nblocks = std::min(std::min(want, (uint32_t)b->stream_grid), kRawBlocks);
   p.deltas = 1;  // the launch inserts delta rows itself
   if (b->lists_left) {  // the update launch starts from empty repair lists and leaves them empty
     VX_CUDA_TRY(cudaMemsetAsync(&b->ctr->cand_n, 0, 3 * sizeof(uint32_t), b->g->stream));
@@ -3844,6 +3967,7 @@ static int repair_fused(Bfs* b) {
   sa.v_single = (uint32_t)g->V;
   sa.classified = b->staged_classified ? 1u : 0u;
   if (b->staged_raw) {
+    sa.over = g->batch.flag;  // the staging's, unused here
     sa.raw_src = g->batch.in_src;
     sa.raw_dst = g->batch.in_dst;
     sa.raw_add = g->batch.in_add;
