@@ -3,7 +3,6 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <string>
 
@@ -73,12 +72,12 @@ int upload_batch(vxh::Graph* g, const uint32_t* src, const uint32_t* dst, const 
   if (vmax > vxb::kMaxVertices) return fail(VX_ERR_RANGE, "vertex id beyond the supported maximum (2^31 - 1)");
   if (int rc = g->batch.ensure(n)) return rc;
   cudaStream_t s = g->stream;
-  if (n <= kPackOps && !g->batch.host) g->batch.host = static_cast<uint8_t*>(malloc(9 * kPackOps));
-  if (n <= kPackOps && g->batch.host) {
+  uint8_t* h = nullptr;
+  if (n <= kPackOps)
+    if (int rc = vxh::graph_pack_room(g, 9 * n, &h)) return rc;
+  if (h) {
     // a small batch is one copy of its packed arrays, not three (some 3 us
-    // each to enqueue); the host buffer is pageable, so the call has taken the
-    // bytes when it returns
-    uint8_t* h = g->batch.host;
+    // each to enqueue)
     memcpy(h, src, 4 * n);
     memcpy(h + 4 * n, dst, 4 * n);
     memcpy(h + 8 * n, add, n);

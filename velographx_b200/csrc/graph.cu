@@ -589,7 +589,6 @@ void BatchBuffers::free_all() {
   void* ptrs[] = {src, keys, keys_alt, vals, vals_alt, flag, pos, fu,
                   fv, ff, fpos, lu, lv, runs, ru, rv, rf, rpos};
   for (void* p : ptrs) cudaFree(p);
-  free(host);
   *this = BatchBuffers();
 }
 
@@ -658,7 +657,9 @@ int graph_create(Graph** out, size_t vertices, bool directed) {
       cudaMalloc(&g->ctr, sizeof(GraphCounters)) != cudaSuccess ||
       cudaMallocHost(&g->hctr, sizeof(GraphCounters)) != cudaSuccess ||
       cudaMallocHost(&g->pinned_scalar, 4096) != cudaSuccess ||
-      cudaEventCreateWithFlags(&g->arena_ev, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&g->arena_ev, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&g->pack.done[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&g->pack.done[1], cudaEventDisableTiming) != cudaSuccess) {
     set_error("CUDA initialisation failed: %s", cudaGetErrorString(cudaGetLastError()));
     graph_destroy(g);
     return -3;
@@ -696,6 +697,9 @@ void graph_destroy(Graph* g) {
   cudaFreeHost(g->hctr);
   cudaFreeHost(g->pinned_scalar);
   if (g->arena_ev) cudaEventDestroy(g->arena_ev);
+  for (cudaEvent_t e : g->pack.done)
+    if (e) cudaEventDestroy(e);
+  free(g->pack.mem);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }
@@ -823,6 +827,28 @@ int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n) {
   return 0;
 }
 
+static bool capturing(Graph* g) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
+int graph_pack_room(Graph* g, size_t bytes, uint8_t** out) {
+  PackRing& r = g->pack;
+  *out = nullptr;
+  if (capturing(g)) return 0;
+  if (!r.mem && !(r.mem = static_cast<uint8_t*>(malloc(2 * PackRing::kHalf)))) return 0;
+  if (r.used + bytes > PackRing::kHalf) {
+    VX_CUDA_TRY(cudaEventRecord(r.done[r.half], g->stream));
+    r.copied[r.half] = true;
+    r.half ^= 1;
+    if (r.copied[r.half]) VX_CUDA_TRY(cudaEventSynchronize(r.done[r.half]));
+    r.used = 0;
+  }
+  *out = r.mem + r.half * PackRing::kHalf + r.used;
+  r.used += bytes;
+  return 0;
+}
+
 // ---- arena room ----
 // The host bounds arena_top by 8 entries per arc ever inserted: a row without a
 // block takes 8, and the blocks of a row that outgrows them double, so they sum
@@ -843,10 +869,6 @@ static_assert(offsetof(GraphCounters, delta_live) == 16 && offsetof(GraphCounter
 
 // A stream capture holds the batch's own launches alone: no readback is enqueued
 // in it, and an event may be neither queried nor waited for.
-static bool capturing(Graph* g) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
-}
 
 // Enqueues the readback.
 static int arena_ask(Graph* g) {

@@ -51,7 +51,6 @@ enum : uint8_t { kFAdd = 1, kFInBase = 2, kFCur = 4, kFChanged = 8 };
 
 struct BatchBuffers {
   size_t cap = 0;       // op capacity
-  uint8_t* host = nullptr;    // a small host batch packed for one copy
   uint32_t* src = nullptr;    // one allocation of 9 bytes an op holds src, dst and add
   uint32_t* dst = nullptr;
   uint8_t* add = nullptr;
@@ -85,6 +84,19 @@ struct BatchBuffers {
   void free_all();
 };
 
+// Packed host batches on their way to the device: two halves filled in turn, each
+// with an event behind its last copy, which is waited for before the half is
+// filled again (whether such a copy has taken its bytes when the call returns is
+// up to the driver).  One event per 256 KB: some 450 batches of 64 ops, 3 of 8,192.
+struct PackRing {
+  static constexpr size_t kHalf = 256 * 1024;
+  uint8_t* mem = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  bool copied[2] = {false, false};
+  int half = 0;
+  size_t used = 0;
+};
+
 struct Graph {
   bool directed = false;
   size_t V = 0, Vcap = 0;
@@ -105,6 +117,7 @@ struct Graph {
   uint64_t* arena_tops = nullptr;
   uint64_t arena_seen[2] = {0, 0};
   bool arena_pending = false;
+  PackRing pack;
 
   SortWait sort_wait() { return SortWait{&ctr->err, sort_looks}; }
   Adjacency& in() { return directed ? adj[1] : adj[0]; }
@@ -115,6 +128,10 @@ int graph_create(Graph** out, size_t vertices, bool directed);
 void graph_destroy(Graph* g);
 int graph_grow(Graph* g, size_t vertices);
 int graph_bulk_load(Graph* g, const uint32_t* d_uv, size_t n_edges);
+// Host room for `bytes` (at most PackRing::kHalf) that a copy on the graph's stream
+// reads next; null where there is none (no memory; a stream capture, whose copies
+// are run later).
+int graph_pack_room(Graph* g, size_t bytes, uint8_t** out);
 // Stage a batch already in g->batch.{src,dst,add}: canonicalise + classify on
 // the pre-batch graph.  vertex_bound bounds every non-self-loop id + 1.
 // classify = false leaves the arcs unclassified, and a directed graph's reversed
