@@ -1359,6 +1359,7 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
 // only grows, past the limit that sends it to the drain.)
 constexpr uint32_t kSyncRounds = 2;
 
+// One thread of a block (its Params are in shared memory).
 __device__ __forceinline__ void ring_epoch(Params& p, uint32_t epoch, uint32_t base) {
   p.rq_tail = p.rq_tail0 + epoch;
   p.rq_base = base;
@@ -1371,7 +1372,9 @@ __device__ bool sync_rounds(Params& p, RepairSmem& sm, W& w) {
     const uint32_t lo = p.rq_base, n = sm.w.tail;
     if (n == 0) return true;
     if (n > gridDim.x) return false;
-    ring_epoch(p, r + 1, lo + n);
+    __syncthreads();  // every warp has read the epoch before
+    if (threadIdx.x == 0) ring_epoch(p, r + 1, lo + n);
+    __syncthreads();
     const uint32_t i = dealt_warp();
     if (i < n) {
       unsigned long long* slot = &p.ring[(lo + i) & p.ring_mask];
@@ -1750,8 +1753,9 @@ struct Cascade {
   }
 };
 
+// Between a barrier after the ring's last use and one before its next.
 __device__ void reset_ring(Params& p) {
-  ring_epoch(p, 0, 0);
+  if (threadIdx.x == 0) ring_epoch(p, 0, 0);
   if (gtid() == 0) {
     *p.rq_head = 0;
     for (uint32_t k = 0; k <= kSyncRounds; ++k) p.rq_tail0[k] = 0;
@@ -3254,7 +3258,21 @@ __device__ void insertion_pass(ArcWork& w, RepairSmem& sm) {
   w.flush();
 }
 
-__device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
+// A block's own copy of the launch's parameters, in shared memory: the repair
+// phases change some of them (the vertex count, the ring's epoch) and hand them by
+// reference to functions that are not inlined.  A copy per thread was a stack frame
+// of 928 bytes (784 in bfs_kernel; now 448 and 288), written by every thread of a
+// launch: 10,000 ops at R-MAT 22, three graphs in turn, 62 us a batch, now 44; 64
+// ops at R-MAT 14 57, now 52.
+__device__ __forceinline__ void copy_params(Params& to, const Params& from) {
+  static_assert(sizeof(Params) % 4 == 0, "copied by words");
+  for (uint32_t i = threadIdx.x; i < sizeof(Params) / 4; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&to)[i] = reinterpret_cast<const uint32_t*>(&from)[i];
+  __syncthreads();
+}
+
+__device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params& q, RepairSmem& sm, LbStage& lb,
+                                   BlockQueue& bq) {
   BfsCounters* c = p.c;
   const uint32_t sort_err = sort_error(p);
   unsigned long long tmark = globaltimer();
@@ -3271,27 +3289,31 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairS
     c->handovers[0] = c->handovers[1] = 0;
   }
   const int ndir = p.g.directed ? 2 : 1;
+  copy_params(q, p);
   for (uint32_t bi = 0; bi < s.nb; ++bi) {
     RawArcs& raw = reinterpret_cast<RawArcs&>(lb);
     uint32_t off = 0, F = 0, Frev = 0;
+    if (s.boff) off = s.boff[bi];
+    const uint32_t Vpre = bi ? s.vpost[bi - 1] : s.V0, lpre = bi ? s.vpost[bi - 1] : s.len0;
+    if (threadIdx.x == 0) {  // the ring's epoch is the first again (reset_ring)
+      q.fu = s.fu[0] + off;
+      q.fv = s.fv[0] + off;
+      q.ff = s.ff[0] + off;
+      q.F = s.raw_n ? p.bar + kRawWord : &s.cnt[0][bi];
+      q.V = Vpre;
+      q.dist_len = lpre;
+      q.touched_base = 0;
+      const unsigned long long lim = (unsigned long long)((double)Vpre * s.frac);
+      q.fallback_limit = lim < 1 ? 1 : lim;
+    }
+    __syncthreads();
     if (s.raw_n) {
       if (canon_raw(s, p.g.directed, raw, p.bar + kRawWord) && threadIdx.x == 0) atomicOr(&c->later, kLaterRows);
     } else {
-      if (s.boff) off = s.boff[bi];
       F = s.cnt[0][bi];
       if (s.cnt[1]) Frev = *s.cnt[1];
     }
-    const uint32_t Vpre = bi ? s.vpost[bi - 1] : s.V0, lpre = bi ? s.vpost[bi - 1] : s.len0;
     const uint32_t Vpost = s.vpost ? s.vpost[bi] : s.v_single;
-    Params q = p;
-    q.fu = s.fu[0] + off;
-    q.fv = s.fv[0] + off;
-    q.ff = s.ff[0] + off;
-    q.F = s.raw_n ? p.bar + kRawWord : &s.cnt[0][bi];
-    q.V = Vpre;
-    q.dist_len = lpre;
-    const unsigned long long lim = (unsigned long long)((double)Vpre * s.frac);
-    q.fallback_limit = lim < 1 ? 1 : lim;
     auto work = [&](int dir) {
       const uint32_t o = dir ? 0u : off;
       return ArcWork{&q, &s, dir ? &p.g.in : &p.g.out, dir, s.fu[dir] + o, s.fv[dir] + o, s.ff[dir] + o, s.fpos[dir] + o,
@@ -3336,7 +3358,11 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairS
     stamp(q, 1);
     // B: the cascade over the graph without the batch's deletions
     const uint32_t ncand = sm.w.candidates;
-    q.touched_base = ncand;
+    if (threadIdx.x == 0) {
+      q.touched_base = ncand;
+      q.cascade_bfs = lpre == Vpre;
+    }
+    __syncthreads();
     if (gtid() == 0) {
       // last_* counters (bfs.hpp:30-33); the last reader of the previous
       // batch's was this thread, at its end
@@ -3347,7 +3373,6 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairS
       acct_add(p, 4, 1);
     }
     if (ncand) {
-      q.cascade_bfs = lpre == Vpre;
       if (!cascade(q, sm, lb, bq, ncand)) return;
       reset_ring(q);
     }
@@ -3364,8 +3389,8 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairS
     if (!sync_words(q, sm.w)) return;
     phase(3);
     // D: the post-batch repair (or the fallback full BFS) on the new graph
-    q.V = Vpost;
-    q.dist_len = Vpost;
+    if (threadIdx.x == 0) q.V = q.dist_len = Vpost;
+    __syncthreads();
     repair_post<true>(q, sm, lb, bq);
     phase(4);
     // the repair lists start empty in the next batch (and launch); every block
@@ -3412,10 +3437,12 @@ __global__ void __launch_bounds__(kT, 1024 / kT) bfs_full_kernel(Params p) {
   full_bfs<false>(p, sm.bq, sm.lb, sm.bu, sm.bits, 8192u, p.dist, p.trace);
 }
 
-__global__ void __launch_bounds__(kThreads, 2) bfs_kernel(Params p, int mode) {
+__global__ void __launch_bounds__(kThreads, 2) bfs_kernel(const __grid_constant__ Params args, int mode) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
+  __shared__ Params p;
+  copy_params(p, args);
   if (const uint32_t e = sort_error(p)) atomicOr(&p.c->err, e);
   if (mode == kModePre) repair_pre(p, sm, lb, bq);
   else repair_post<false>(p, sm, lb, bq);
@@ -3426,14 +3453,16 @@ __global__ void __launch_bounds__(kThreads, 2) bfs_kernel(Params p, int mode) {
 // (no spills, 2% faster alone) does not allow: 10,000-op batches on three R-MAT
 // 22 graphs in turn 86 us a batch, 111 us with 128 registers.
 // The arguments stay in the kernel's parameter space: as copies for the functions
-// that take them by reference they made a stack frame of 1,184 bytes a thread, now
-// 928 (10,000 ops at R-MAT 22, three graphs in turn: 67.8 us a batch, now 62.1).
+// that take them by reference they made a stack frame of 1,184 bytes a thread
+// instead of 928 (10,000 ops at R-MAT 22, three graphs in turn: 70 us a batch
+// instead of 62).
 __global__ void __launch_bounds__(kThreads, 2) bfs_stream_kernel(const __grid_constant__ Params p,
                                                                  const __grid_constant__ StreamArgs s) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
-  stream_kernel_body(p, s, sm, lb, bq);
+  __shared__ Params q;
+  stream_kernel_body(p, s, q, sm, lb, bq);
 }
 
 // Stream canonicalisation: both arcs of every non-self-loop op keyed by
