@@ -229,7 +229,11 @@ int vx_graph_reserve(vx_graph* g, size_t max_batch_ops, size_t total_ops);
  * `batches` batches, the largest max_batch_ops ops.  No reference counterpart. */
 int vx_bfs_reserve_stream(vx_bfs* b, size_t ops, size_t batches, size_t max_batch_ops);
 /* Direction switch (alpha, beta) and grid-expanded row length of the full BFS.
- * No reference counterpart: the reference BFS is top-down only. */
+ * A level goes bottom-up when its frontier's arcs m_f hold more than 1 / alpha of
+ * the arcs of unvisited vertices (m_f * alpha > m_u), and either m_f * alpha > 12 V
+ * or the frontier is wide beside what is left (at least a quarter of the unvisited
+ * and a sixteenth of all vertices); back when it shrinks below V / beta.  No
+ * reference counterpart: the reference BFS is top-down only. */
 int vx_bfs_set_tuning(vx_bfs* b, float alpha, float beta, uint32_t large_row);
 /* Autotuner of the full BFS: times a grid of 36 (alpha, beta, large_row)
  * candidates (alpha 4/14/40/120, beta 8/24/96, large_row 512/1024/4096) on a

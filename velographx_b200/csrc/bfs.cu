@@ -936,14 +936,20 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     m_visited += m_f;
     if (!bottom_up && !left_bu && level > 0) {
       // bottom-up when the frontier's rows hold more than 1 / alpha of the
-      // arcs of unvisited vertices, and (at the default alpha) more arcs than
-      // there are vertices: the first bottom-up level sweeps every vertex, so
-      // a thin frontier of a low-degree graph is cheaper pushed (4096 x 4096
-      // lattice, 620,000 vertices of frontier: three bottom-up levels took 480 us,
-      // top-down ones take 170)
+      // arcs of unvisited vertices, and (at the default alpha) nearly as many
+      // arcs as there are vertices: the first bottom-up level sweeps every
+      // vertex, so a thin frontier of a low-degree graph is cheaper pushed (4096 x
+      // 4096 lattice, 620,000 vertices of frontier: three bottom-up levels took 480
+      // us, top-down ones take 170; the hub of a star of 2^20 leaves, seen from a
+      // leaf: 15 us swept, 45 pushed).  Or when few vertices are left beside a wide
+      // frontier, whatever its arcs: the last levels of trees (262,144 and then
+      // 782,000 leaves of 2^20 vertices: 30 + 3 us, pushed 202 + 21).  A frontier
+      // vertex costs some 90 ps pushed, an unvisited one 15 ps looked at, and every
+      // vertex 2 ps swept.
       const unsigned long long m_u = p.total_arcs > m_visited ? p.total_arcs - m_visited : 0ull;
       const double am = (double)m_f * p.alpha;
-      bottom_up = am > (double)m_u && am > 14.0 * (double)V;
+      const bool few_left = (unsigned long long)(V - reached) <= 4ull * n_f && V <= 16ull * n_f;
+      bottom_up = am > (double)m_u && (am > 12.0 * (double)V || few_left);
     }
     if (gtid() == 0 && trace && level < kTraceLevels) {
       trace[2 * level] = globaltimer();

@@ -61,7 +61,7 @@ struct BfsCounters {
 };
 
 struct BfsTuning {
-  float alpha = 14.0f;       // top-down -> bottom-up when m_f * alpha > m_u
+  float alpha = 14.0f;       // top-down -> bottom-up when m_f * alpha > m_u and > 12 V, or little is left
   float beta = 24.0f;        // bottom-up -> top-down when n_f * beta < V (shrinking)
   uint32_t large_row = 1024; // rows this long are expanded by the whole grid
   bool fused = true;         // one persistent launch per batch after staging
