@@ -73,3 +73,15 @@ def test_a_lattice_is_pushed():
     r, c = np.divmod(np.arange(10**6, dtype=np.uint32), 1000)
     assert np.array_equal(b.distances_array(), r + c)
     assert not any(up for _, _, up in b.level_trace())
+
+
+def test_a_hub_of_a_million_leaves_is_pushed_at_the_rate_of_the_memory():
+    vertices = 1 << 20
+    hub = np.stack((np.full(vertices - 1, vertices - 1), np.arange(vertices - 1)), 1).astype(np.uint32)
+    g, b = search(vertices, hub, vertices - 1)
+    us = []
+    for _ in range(20):
+        b.recompute()
+        us.append(b.level_trace()[0][0])
+    # 2^20 claims: some 45 us are their atomics; with too few arcs in flight 118
+    assert min(us) < 80, us
