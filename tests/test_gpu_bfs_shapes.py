@@ -85,3 +85,21 @@ def test_a_hub_of_a_million_leaves_is_pushed_at_the_rate_of_the_memory():
         us.append(b.level_trace()[0][0])
     # 2^20 claims: some 45 us are their atomics; with too few arcs in flight 118
     assert min(us) < 80, us
+
+
+def test_a_level_of_a_thousand_vertices_takes_no_longer_than_one_of_two_thousand():
+    # a root with an arc to every vertex of a lattice's first row: each level is a row
+    rows, level = 200, []
+    for width in (1024, 2048):
+        e = np.concatenate((lattice(width, rows) + np.uint32(1),
+                            np.stack((np.zeros(width), np.arange(1, width + 1)), 1).astype(np.uint32)))
+        g, b = search(1 + width * rows, e, 0)
+        want = np.r_[0, np.repeat(np.arange(1, rows + 1), width)].astype(np.uint32)
+        assert np.array_equal(b.distances_array(), want)
+        best = np.full(rows + 1, np.inf)
+        for _ in range(6):
+            b.recompute()
+            best = np.minimum(best, [us for us, _, _ in b.level_trace()])
+        level.append(np.median(best[20:-20]))
+    # half of the arcs: by one block alone such a level took twice as long as the wider one
+    assert level[0] < 1.05 * level[1], level

@@ -477,10 +477,12 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v, un
 // as the grid takes to meet at a barrier: block 0 runs such levels by itself,
 // frontier in shared memory and block barriers only, until the frontier
 // outgrows it, while the others wait at the grid barrier that ends the
-// stretch.  A level takes 3 us instead of 8 to 10.  The limits are where a
-// level of one block (four arcs per thread and step) costs what a level of
-// the grid does.  A stretch is bounded so that the waiting blocks' barrier is.
-constexpr uint32_t kSoloArcs = 4096;
+// stretch.  A level takes 3 us instead of 8 to 10.  The limit is where a level of
+// one block (one step of four arcs per thread) costs what a level of the grid
+// does, 7 to 8 us: lattices 512 wide 8.3 us a level by one block, 600 wide 10.7 by
+// one block in two steps and 8.1 by the grid, 1,024 wide 18.6 and 9.4.  A stretch is
+// bounded so that the waiting blocks' barrier is.
+constexpr uint32_t kSoloArcs = 2048;
 constexpr uint32_t kSoloLevels = 4096;
 
 // Words of the barrier array past the barrier word (zero between searches):
