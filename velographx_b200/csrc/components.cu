@@ -38,29 +38,29 @@ unsigned cc_grid(uint64_t n) {
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + kCcThreads - 1) / kCcThreads, 148ull * 64));
 }
 
-__device__ __forceinline__ uint32_t cc_find(uint32_t* label, uint32_t x) {
-  // path halving; parents only ever move to smaller ids of the same set
-  uint32_t p = __ldcg(&label[x]);
-  while (p != x) {
-    const uint32_t gp = __ldcg(&label[p]);
-    if (gp != p) __stcg(&label[x], gp);
-    x = p;
-    p = gp;
-  }
-  return x;
-}
-
+// Unites the sets of a and b (Rem's algorithm with splicing; concurrent as in
+// Dhulipala, Hong and Shun, "ConnectIt", VLDB 2020).  The end with the larger parent
+// goes under the other's parent; if it was no root, its old parent's set is still to
+// be united, so the walk goes on from there.  Parents only ever move to smaller ids,
+// and the walk ends where the parents are equal: without looking at the root, whose
+// word all threads would load once the sets have grown together.  cc_link_kernel on
+// a uniform graph of 2^20 vertices and 8M edges 763 to 1,123 us with a find of both
+// roots, 125 so.
 __device__ __forceinline__ void cc_union(uint32_t* label, uint32_t a, uint32_t b) {
-  for (int guard = 0; guard < (1 << 20); ++guard) {
-    a = cc_find(label, a);
-    b = cc_find(label, b);
-    if (a == b) return;
-    if (a > b) {
-      const uint32_t t = a;
+  uint32_t pa = __ldcg(&label[a]), pb = __ldcg(&label[b]);
+  while (pa != pb) {
+    if (pa < pb) {
+      const uint32_t t = a, tp = pa;
       a = b;
+      pa = pb;
       b = t;
+      pb = tp;
     }
-    if (atomicCAS(&label[b], b, a) == b) return;  // hook the larger root under the smaller
+    const uint32_t old = atomicMin(&label[a], pb);
+    if (old == a) return;  // a root, now under pb
+    a = old;
+    pa = __ldcg(&label[a]);
+    pb = __ldcg(&label[b]);
   }
 }
 
@@ -87,11 +87,13 @@ __global__ void cc_identity_kernel(uint32_t* label, uint32_t lo, uint32_t hi) {
 // directions are stored, so the partition is the same whichever root is taken
 // (none when no sample hit the set).  Each pass is a coalesced sweep of the
 // vertices with a few dependent loads each, bound by their latency; at R-MAT
-// 2^20 they take 84 us together (hook 13, compress 29, link 24, sample 6, rows 12).
+// 2^20 they take some 90 us together (hook 13, compress 40, link 20, sample 6,
+// rows 12).
 
 constexpr uint32_t kNoRoot = 0xFFFFFFFFu;
 constexpr uint32_t kProbe = 4;     // arcs of each row part looked at for a live neighbour in the set
 constexpr uint32_t kSamples = 256;
+constexpr uint32_t kLaneRow = 8;   // rows this short are walked by one lane
 
 __device__ __forceinline__ bool in_set(const uint32_t* aff, uint32_t v) {
   return !aff || ((aff[v >> 5] >> (v & 31)) & 1u);
@@ -180,8 +182,12 @@ __global__ void __launch_bounds__(kSamples) cc_sample_kernel(const uint32_t* lab
   if (t == 0) *giant = (uint32_t)best;
 }
 
-// The rows of the set's vertices outside the giant: a lane each finds them, the
-// warp walks them.
+// The rows of the set's vertices outside the giant: a lane each finds them and
+// walks the short ones, the warp the others.  Rows of at most two arcs have been
+// hooked and linked whole; a short row's arcs are united without a look for its
+// root, which costs about as much.  A tree of 2^20 randomly numbered vertices with
+// three children each: 759 us with a warp per row (and a find of both roots), now
+// 70 to 95.
 __global__ void cc_rows_kernel(vxb::DevAdj a, uint32_t V, uint32_t n, uint32_t* label, const uint32_t* aff,
                                const uint32_t* any, const uint32_t* giant) {
   if (any && !*any) return;
@@ -189,8 +195,20 @@ __global__ void cc_rows_kernel(vxb::DevAdj a, uint32_t V, uint32_t n, uint32_t* 
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t v0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; v0 < n; v0 += nw * 32) {
     const uint32_t v = v0 + lane;
-    const bool mine = v < n && in_set(aff, v) && frontier::degree_of(a, v) != 0u && cc_root(label, v) != big;
-    uint32_t rows = __ballot_sync(0xFFFFFFFFu, mine);
+    uint32_t deg = 0;
+    if (v < n && in_set(aff, v) && __ldcg(&label[v]) != big) deg = frontier::degree_of(a, v);
+    if (deg > kLaneRow && cc_root(label, v) == big) deg = 0;
+    if (deg > 2u && deg <= kLaneRow) {
+      uint64_t b, e;
+      vxb::base_range(a, v, b, e);
+      const uint2 dr = a.drow[v];
+      const uint32_t nb = (uint32_t)(e - b);
+      for (uint32_t k = 0; k < nb + dr.y; ++k) {
+        const uint32_t x = k < nb ? a.col[b + k] : a.darena[dr.x + (k - nb)];
+        if (!(x & vxb::kTomb) && x < V && in_set(aff, x)) cc_union(label, v, x);
+      }
+    }
+    uint32_t rows = __ballot_sync(0xFFFFFFFFu, deg > kLaneRow);
     while (rows) {
       const uint32_t u = v0 + (uint32_t)__ffs(rows) - 1;
       rows &= rows - 1;
