@@ -89,6 +89,33 @@ __device__ __forceinline__ void for_my_rows(const uint32_t* len, uint32_t n, uin
 
 constexpr uint32_t FULL = 0xFFFFFFFFu;
 
+// The 32-vertex groups that a warp takes of a pull level: the first by its number,
+// further ones from one counter (zero before the level), one at a time where its last
+// group was a heavy one (arcs to read past the rows' heads, or much to write), else
+// kClaimGroups.  Claims serialise on the counter, which shows where a level does little
+// beside them: one root in a star of 2^20 vertices, two pull levels, 136 us a run with
+// single claims, 112 so, 104 with claims of four.  Those leave the grid waiting for a
+// warp with several heavy groups: 64 roots in a graph of 2^20 vertices and 2^21 edges
+// 574, 593 and 702 us.
+constexpr uint32_t kClaimGroups = 2;
+struct GroupClaims {
+  // warp-uniform; numbered across the blocks first, as a skewed graph's heavy groups
+  // may lie side by side
+  uint32_t cur = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, end = cur + 1;
+  bool heavy = false;  // the last group was (set by the caller)
+  // The next group, or one at or past the level's last when there are no more; whole warp.
+  __device__ __forceinline__ uint32_t next(uint32_t* counter) {
+    if (cur == end) {
+      const uint32_t n = heavy ? 1u : kClaimGroups;
+      uint32_t c = 0;
+      if ((threadIdx.x & 31) == 0) c = nwarps() + atomicAdd(counter, n);
+      cur = __shfl_sync(FULL, c, 0);
+      end = cur + n;
+    }
+    return cur++;
+  }
+};
+
 // The whole warp walks one row (all lanes pass the same u); f as above.
 template <class F>
 __device__ __forceinline__ void warp_row(const DevAdj& a, uint32_t u, F& f) {

@@ -135,11 +135,7 @@ constexpr uint32_t kMrBigPull = 2048;    // pull rows this long are read by the 
 // 128.
 constexpr uint32_t kMrMidPull = 256;
 constexpr uint32_t kMrWarps = kThreads / 32;
-// 32-vertex groups a warp claims per atomic of a pull level (one counter
-// per level: a claim per group serialised on it; one where that leaves a warp
-// fewer than kClaimsPerWarp claims)
-constexpr uint32_t kClaimGroups = 4;
-constexpr uint32_t kClaimsPerWarp = 4;
+constexpr uint32_t kHeavyRoots = 8;  // a pull group that more roots reach is a heavy one (GroupClaims)
 
 // Per-warp staging of one pull group: the rows of its 32 vertices and their
 // OR accumulators ([lane][word]).
@@ -152,18 +148,21 @@ struct MrWarpStage {
 
 // Newly reached roots of the warp's 32 consecutive vertices (v = base + lane)
 // at distance lvl, one root at a time, so every store of a root's row covers
-// the warp's vertices together.
+// the warp's vertices together.  Returns the number of roots.
 template <uint32_t W>
-__device__ __forceinline__ void write_dists_warp(const MrParams& p, uint32_t v, const uint32_t* acc, uint32_t lvl) {
+__device__ __forceinline__ uint32_t write_dists_warp(const MrParams& p, uint32_t v, const uint32_t* acc, uint32_t lvl) {
+  uint32_t n = 0;
 #pragma unroll
   for (uint32_t w = 0; w < W; ++w) {
     uint32_t roots = __reduce_or_sync(FULL, acc[w]);
+    n += __popc(roots);
     while (roots) {
       const uint32_t b = __ffs(roots) - 1;
       roots &= roots - 1;
       if ((acc[w] >> b) & 1u) p.dist[(size_t)(32 * w + b) * p.V + v] = lvl;
     }
   }
+  return n;
 }
 
 // A row that the whole warp holds: the roots of acc that are not in vis reach
@@ -207,17 +206,12 @@ __device__ bool pull_level(const MrParams& p, const uint32_t* fc, uint32_t* fn, 
   constexpr uint32_t kMrU = MrSlots<W>::value;
   const DevAdj& a = p.g.in;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t claim = p.V / 32 >= kClaimsPerWarp * kClaimGroups * nwarps() ? kClaimGroups : 1u;
-  uint32_t cur = 0, end = 0;  // the warp's claimed groups [cur, end), warp-uniform
+  const uint32_t groups = (p.V + 31) / 32;
+  GroupClaims claims;
   for (;;) {
-    if (cur == end) {
-      uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(gnext, claim);
-      cur = __shfl_sync(FULL, c0, 0);
-      end = cur + claim;
-    }
-    const uint32_t base = cur++ * 32;
-    if (base >= p.V) break;
+    const uint32_t group = claims.next(gnext);
+    if (group >= groups) break;
+    const uint32_t base = group * 32;
     const uint32_t v = base + lane;
     uint32_t vis[W];
     bool done = true;
@@ -353,7 +347,7 @@ __device__ bool pull_level(const MrParams& p, const uint32_t* fc, uint32_t* fn, 
         fn[(size_t)v * W + w] = acc[w];
       }
     }
-    write_dists_warp<W>(p, v, acc, level + 1);
+    claims.heavy = write_dists_warp<W>(p, v, acc, level + 1) > kHeavyRoots || T != 0u;
     bq_push(mr_bq, any, v, qn, qout);
     const unsigned long long dsum = vxb::warp_sum(any ? (unsigned long long)rowlen : 0ull);
     if (lane == 0 && dsum) atomicAdd(&mr_mf, dsum);
@@ -504,6 +498,7 @@ __global__ void __launch_bounds__(kThreads, 2) mrbfs_kernel(MrParams p) {
     }
     const int cur = level % 3, nx = (level + 1) % 3, clr = (level + 2) % 3;
     const uint32_t n_f = __ldcg(&c->qn[cur]);
+    const unsigned long long m_f = __ldcg(&c->mf[cur]);
     if (n_f == 0) break;
     if (gtid() == 0) {  // counters of level+2: no block uses them before the next barrier
       c->qn[clr] = 0;
@@ -523,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 2) mrbfs_kernel(MrParams p) {
     uint32_t* fn = p.frn[nx];
     // pull for a large frontier, or for one whose rows would cost more to
     // push than reading up to every arc costs to pull
-    const bool pull = (float)n_f > p.pull_frac * (float)p.V || __ldcg(&c->mf[cur]) * kPushArcCost > p.arcs;
+    const bool pull = (float)n_f > p.pull_frac * (float)p.V || m_f * kPushArcCost > p.arcs;
     if (gtid() == 0) {
       const uint32_t t = min(level, kMrTraceLevels - 1);
       c->trace[2 * t] = globaltimer();
@@ -546,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, 2) mrbfs_kernel(MrParams p) {
       // (the roots' level of a 100k vertex, 20 root run 84 -> 44 us)
       const bool few = n_f <= nwarps();
       const uint32_t big_row = few ? kMrFewRow : kMrBigRow;
-      const uint32_t slice = few && __ldcg(&c->mf[cur]) <= (unsigned long long)nwarps() * 64u ? 32u : kMrPushSlice;
+      const uint32_t slice = few && m_f <= (unsigned long long)nwarps() * 64u ? 32u : kMrPushSlice;
       for (uint32_t i = gwarp(); i < n_f; i += nwarps()) {
         const uint32_t u = p.q[cur][i];
         const uint32_t deg = degree_of(a, u);

@@ -68,10 +68,6 @@ __device__ __forceinline__ void mf_flush(unsigned long long* dst) {
   __syncthreads();
 }
 constexpr uint32_t kVsWarps = kVsThreads / 32;
-// 32-vertex groups a warp claims per atomic of a pull level (one counter
-// per level: a claim per group serialised on it)
-constexpr uint32_t kClaimGroups = 4;
-constexpr uint32_t kClaimsPerWarp = 4;  // claims of one group where a warp would get fewer than these
 constexpr uint32_t kVsHead = 8;        // in-arcs a lane reads itself before the flattened rounds
 constexpr uint32_t kVsHeadStep = 4;    // of which it loads this many at a time
 constexpr uint32_t kVsBigPull = 2048;  // pull rows this long are read by the whole grid
@@ -440,17 +436,12 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
                         VsSums& s, unsigned long long* sdig) {
   constexpr uint32_t kSlots = VsSlots<W>::value;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t claim = p.V / 32 >= kClaimsPerWarp * kClaimGroups * nwarps() ? kClaimGroups : 1u;
-  uint32_t cur = 0, end = 0;  // the warp's claimed groups [cur, end), warp-uniform
+  const uint32_t groups = (p.V + 31) / 32;
+  GroupClaims claims;
   for (;;) {
-    if (cur == end) {
-      uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(gnext, claim);
-      cur = __shfl_sync(FULL, c0, 0);
-      end = cur + claim;
-    }
-    const uint32_t base = cur++ * 32;
-    if (base >= p.V) break;
+    const uint32_t group = claims.next(gnext);
+    if (group >= groups) break;
+    const uint32_t base = group * 32;
     const uint32_t v = base + lane;
     uint32_t vis[W];
     bool done = true;
@@ -590,6 +581,7 @@ __device__ bool vs_pull(const VsParams& p, const uint32_t* fc, uint32_t* fn, uin
     for (uint32_t w = 0; w < W; ++w) nw[w] = ws.acc[lane * W + w] & ~vis[w];
     const bool any = v < p.V && vs_discover<W>(p, v, vis, nw, fn, level + 1, s);
     if (p.dig && v < p.V) vs_digest<W>(p, v, nw, level + 1, s, sdig);
+    claims.heavy = T != 0u || __any_sync(FULL, any);
     bq_push(vs_bq, any, v, qn, qout);
     const unsigned long long dsum = vxb::warp_sum(any ? (unsigned long long)rowlen : 0ull);
     if (lane == 0 && dsum) atomicAdd(&vs_mf, dsum);
