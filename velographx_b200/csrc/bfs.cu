@@ -67,11 +67,8 @@ struct Params {
   unsigned long long* sw;  // support words of the pre-batch cascade (zero between batches)
   unsigned long long* ring;  // work ring of the repair phases (kSent between phases)
   uint32_t ring_mask;
-  uint32_t rq_base;        // slot of the current epoch's first item (sync_rounds)
-  uint32_t touched_base;   // length of the touched list before touched_n counts
   uint32_t* rq_head;       // ring counters, each on its own 128-byte line: the
-  uint32_t* rq_tail0;      // idle blocks poll them while the working ones push
-  uint32_t* rq_tail;       // the current epoch's (rq_tail0 + epoch)
+  uint32_t* rq_tail;       // idle blocks poll them while the working ones push
   uint32_t* rq_done;
   uint32_t* rq_fin;        // set by the first block that sees the phase finished
   unsigned long long* rq_stat;  // drain statistics of the last phase (own line)
@@ -98,6 +95,26 @@ struct Params {
   unsigned long long* acct;
   uint32_t* bar;              // grid barrier words
 };
+
+// What a repair launch's phases change of its parameters, a copy per block (thread 0
+// writes it between block barriers; start_phases).  The other parameters are read
+// where the launch put them: with all of them in shared memory every use was a load
+// that no store could be moved past (a pair of 64-op batches at 2^20 vertices 67 us,
+// now 63; a vertex of a cascade along a path 5.8 us, now 5.6).
+struct PhaseParams {
+  uint32_t V;             // vertices of the graph in this phase
+  uint32_t dist_len;      // logical length of the distance vector in this phase
+  uint32_t rq_base;       // slot of the ring's current epoch's first item (sync_rounds)
+  uint32_t* rq_tail;      // the current epoch's length (Params::rq_tail + epoch)
+  uint32_t touched_base;  // length of the touched list before touched_n counts
+  uint32_t cascade_bfs;   // the cascade may hand over (the distance vector spans the graph)
+  const uint32_t* fu;     // the batch's canonical arcs
+  const uint32_t* fv;
+  const uint8_t* ff;
+  const uint32_t* F;
+  unsigned long long fallback_limit;
+};
+__shared__ PhaseParams ph;
 
 constexpr uint32_t kTraceLevels = 256;
 
@@ -727,7 +744,7 @@ __device__ __forceinline__ BuEntry bu_entry(uint32_t v, uint64_t b, uint32_t nb,
 // pass instead cost a chain of loads per 512 vertices of a block there, also in
 // searches that never go bottom-up.)
 template <int kT, int kR, class Queue>
-__device__ void bu_first_level(const Params& p, BuOut<Queue>& o, BuStage<kT, kR>& st) {
+__device__ void bu_first_level(const Params& p, uint32_t V, BuOut<Queue>& o, BuStage<kT, kR>& st) {
   const DevAdj& a = p.g.in;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t nw = o.tiles.words();
@@ -738,7 +755,7 @@ __device__ void bu_first_level(const Params& p, BuOut<Queue>& o, BuStage<kT, kR>
     vis0 = FULL;
     if (w >= nw) return;
     const uint64_t x = (uint64_t)o.tiles.word_of(w) * 32 + lane;
-    if (x >= p.V) return;
+    if (x >= V) return;
     v = (uint32_t)x;
     vis0 = p.vis[v >> 5];
     row_of(p, a, v, b0, n0, d0);
@@ -812,7 +829,8 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     lw.m = 0;
     lw.n = 0;
   }
-  const uint32_t V = p.V;
+  uint32_t V = p.V;
+  if constexpr (kInRepair) V = ph.V;
   const uint32_t words = (V + 31) >> 5;
   // one pass sets every vertex unreached and the source at level 0 (bits
   // past V count as visited, so bottom-up never scans them)
@@ -986,7 +1004,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
       uint32_t* lists = p.bul + (size_t)blockIdx.x * seg;
       BuOut<Queue> o{dist,  level, p.fb[cur], p.fb[nxt], local ? wbits : nullptr, tiles, lists + (size_t)lout * p.bul_half,
                      &seg_n[lout], push ? &bq : nullptr, p.q[nxt], &c->lvl_n[nxt], 0u};
-      if (!bu_listed) bu_first_level(p, o, bu);
+      if (!bu_listed) bu_first_level(p, V, o, bu);
       else bu_list_level(p, o, bu, lists + (size_t)lin * p.bul_half, seg_n[lin]);
       if (local) {
         __syncthreads();
@@ -1050,7 +1068,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
 // ------------------------------------------------------------- helpers --
 
 __device__ __forceinline__ bool is_sp(const Params& p, uint32_t u, uint32_t v) {
-  if (u >= p.dist_len || v >= p.dist_len) return false;
+  if (u >= ph.dist_len || v >= ph.dist_len) return false;
   const uint32_t du = p.dist[u], dv = p.dist[v];
   return du != kUnreachable && dv != kUnreachable && du + 1 == dv;
 }
@@ -1088,8 +1106,8 @@ constexpr unsigned long long kChunkCheckBit = 1ull << 63;  // cascade items: one
 constexpr uint32_t kDrainIdleLimit = 1u << 20;  // idle rounds of a block (up to 2 us each)
 
 __device__ __forceinline__ void ring_push(const Params& p, bool pred, unsigned long long item) {
-  const uint32_t s = vxb::warp_append(pred, p.rq_tail);  // warp-uniform
-  if (pred) __stcg(&p.ring[(p.rq_base + s) & p.ring_mask], item);
+  const uint32_t s = vxb::warp_append(pred, ph.rq_tail);  // warp-uniform
+  if (pred) __stcg(&p.ring[(ph.rq_base + s) & p.ring_mask], item);
 }
 
 __device__ __forceinline__ uint32_t item_vertex(unsigned long long it) { return (uint32_t)it & ~kKindBit; }
@@ -1123,7 +1141,7 @@ __device__ void block_rows(const DevAdj& a, const T* items, uint32_t n, LbStage&
       const uint32_t lo = c * kChunk, hi = min(total, lo + kChunk);
       if (c == 0 && total > kChunk) {  // hand the other chunks to other blocks
         const uint32_t more = (total - 1) / kChunk;
-        const uint32_t s0 = p->rq_base + atomicAdd(p->rq_tail, more);
+        const uint32_t s0 = ph.rq_base + atomicAdd(ph.rq_tail, more);
         for (uint32_t k = 0; k < more; ++k)
           __stcg(&p->ring[(s0 + k) & p->ring_mask], ((unsigned long long)it & 0xFFFFFFFFull) |
                                                         ((unsigned long long)(k + 1) << 32));
@@ -1211,12 +1229,12 @@ __device__ __forceinline__ bool sync_words(const Params& p, RepairWords& w) {
     RepairWords r;
     r.failed = __ldcg(&c->err);
     r.candidates = ld_cg(&c->cand_n);
-    r.touched = p.touched_base + ld_cg(&c->touched_n);
+    r.touched = ph.touched_base + ld_cg(&c->touched_n);
     r.affected = ld_cg(&c->a_n);
     r.fallback = ld_cg(&c->fallback);
     r.cbig = ld_cg(&c->cbig);
     r.rbig = ld_cg(&c->rbig);
-    r.tail = ld_cg(p.rq_tail);
+    r.tail = ld_cg(ph.rq_tail);
     r.big_b = ld_cg(&c->big_b);
     r.later = ld_cg(&c->later);
     r.raw_f[0] = ld_cg(p.bar + kRawWord);
@@ -1246,12 +1264,19 @@ struct RepairSmem {
 };
 
 // The full BFS inside a repair kernel, in the shared memory its phases do not
-// hold at that point.
+// hold at that point.  It is a function of its own (called, not inlined), which reads
+// the parameters faster from a copy in shared memory than by reference from the
+// kernel's (fallback batches on a 512 x 512 lattice 1,127 us each, so 1,080).
 __device__ __noinline__ void bfs_in_repair(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t* dist,
                               unsigned long long* trace) {
   using Stage = BuStage<kThreads, 1>;
   static_assert(sizeof(Stage) <= sizeof(LbStage) && alignof(LbStage) >= alignof(Stage), "the two share memory");
-  full_bfs<true, kVisit>(p, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm),
+  static_assert(sizeof(Params) % 4 == 0, "copied by words");
+  __shared__ Params own;
+  for (uint32_t i = threadIdx.x; i < sizeof(Params) / 4; i += kThreads)
+    reinterpret_cast<uint32_t*>(&own)[i] = reinterpret_cast<const uint32_t*>(&p)[i];
+  __syncthreads();
+  full_bfs<true, kVisit>(own, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm),
                  (uint32_t)(offsetof(RepairSmem, w) / 4), dist, trace);
 }
 
@@ -1293,12 +1318,12 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
         }
         const uint32_t k = cur + lane;
         unsigned long long v = kSent;
-        if (k < end) v = __ldcg(&p.ring[(p.rq_base + k) & p.ring_mask]);
+        if (k < end) v = __ldcg(&p.ring[(ph.rq_base + k) & p.ring_mask]);
         const uint32_t have = __ballot_sync(FULL, v != kSent);
         n = have == FULL ? 32u : (uint32_t)(__ffs(~have) - 1);  // leading filled slots
         if ((uint32_t)lane < n) {
           sm.items[lane] = v;
-          __stcg(&p.ring[(p.rq_base + k) & p.ring_mask], kSent);
+          __stcg(&p.ring[(ph.rq_base + k) & p.ring_mask], kSent);
         }
         cur += n;
         if (n == 0) {
@@ -1308,7 +1333,7 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
             if (!st && (idle & 3) == 3) {
               const uint32_t dn = ld_cg(p.rq_done);
               __threadfence();
-              st = dn == ld_cg(p.rq_tail);
+              st = dn == ld_cg(ph.rq_tail);
               if (st) atomicExch(p.rq_fin, 1u);  // releases the other blocks at their next idle round
               atomicAdd(&p.rq_stat[3], 1ull);
             }
@@ -1368,17 +1393,17 @@ __device__ void drain(const Params& p, RepairSmem& sm, W& w, unsigned long long 
 // only grows, past the limit that sends it to the drain.)
 constexpr uint32_t kSyncRounds = 2;
 
-// One thread of a block (its Params are in shared memory).
-__device__ __forceinline__ void ring_epoch(Params& p, uint32_t epoch, uint32_t base) {
-  p.rq_tail = p.rq_tail0 + epoch;
-  p.rq_base = base;
+// One thread of a block.
+__device__ __forceinline__ void ring_epoch(const Params& p, uint32_t epoch, uint32_t base) {
+  ph.rq_tail = p.rq_tail + epoch;
+  ph.rq_base = base;
 }
 
 template <class W>
-__device__ bool sync_rounds(Params& p, RepairSmem& sm, W& w) {
+__device__ bool sync_rounds(const Params& p, RepairSmem& sm, W& w) {
   if (p.handover == 0.0f) return false;  // hands over at its first drain round
   for (uint32_t r = 0; r < kSyncRounds; ++r) {
-    const uint32_t lo = p.rq_base, n = sm.w.tail;
+    const uint32_t lo = ph.rq_base, n = sm.w.tail;
     if (n == 0) return true;
     if (n > gridDim.x) return false;
     __syncthreads();  // every warp has read the epoch before
@@ -1433,7 +1458,7 @@ __device__ __forceinline__ bool mark_affected(const Params& p, uint32_t v) {
   if (atomicOr(&p.aff[v >> 5], bit) & bit) return false;
   const uint32_t slot = atomicAdd(&p.c->a_n, 1u);
   p.lst_a[slot] = v;
-  if (slot + 1 > p.fallback_limit) p.c->fallback = 1;
+  if (slot + 1 > ph.fallback_limit) p.c->fallback = 1;
   __threadfence();  // the affected bit is visible before the expand item is
   return true;
 }
@@ -1455,12 +1480,12 @@ __device__ __forceinline__ void request_check(const Params& p, bool pred, uint32
   const int lf = mf ? __ffs(mf) - 1 : 0, lp = mp ? __ffs(mp) - 1 : 0;
   uint32_t bf = 0, bp = 0;
   if (mf && lane == lf) bf = atomicAdd(&p.c->touched_n, (uint32_t)__popc(mf));
-  if (mp && lane == lp) bp = atomicAdd(p.rq_tail, (uint32_t)__popc(mp));
+  if (mp && lane == lp) bp = atomicAdd(ph.rq_tail, (uint32_t)__popc(mp));
   bf = __shfl_sync(FULL, bf, lf);
   bp = __shfl_sync(FULL, bp, lp);
   const uint32_t lt = vxb::lanemask_lt();
-  if (first) p.lst_t[p.touched_base + bf + __popc(mf & lt)] = x;
-  if (push) __stcg(&p.ring[(p.rq_base + bp + __popc(mp & lt)) & p.ring_mask], (unsigned long long)x);
+  if (first) p.lst_t[ph.touched_base + bf + __popc(mf & lt)] = x;
+  if (push) __stcg(&p.ring[(ph.rq_base + bp + __popc(mp & lt)) & p.ring_mask], (unsigned long long)x);
 }
 
 // expand(y) for a newly affected y at distance dy, applied to one arc (y, x)
@@ -1472,7 +1497,7 @@ struct ExpandChildren {
   uint32_t y, dy;
   __device__ __forceinline__ void operator()(bool valid, uint32_t x, uint32_t) {
     bool need = false;
-    if (valid && x < p->dist_len) {
+    if (valid && x < ph.dist_len) {
       const uint32_t dx = p->dist[x];
       const unsigned long long w = __ldcg(&p->sw[x]);
       const uint32_t wit = (uint32_t)(w >> 32) & 0x7FFFFFFFu;
@@ -1503,7 +1528,7 @@ __device__ __forceinline__ bool find_parent(const Params& p, const DevAdj& a, ui
     uint32_t dy[4], aw[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const bool live = !(y[j] & kTomb) && y[j] < p.dist_len;
+      const bool live = !(y[j] & kTomb) && y[j] < ph.dist_len;
       dy[j] = live ? p.dist[y[j]] : kUnreachable;
       aw[j] = live ? __ldcg(&p.aff[y[j] >> 5]) : 0u;
     }
@@ -1749,7 +1774,7 @@ struct Cascade {
       __syncthreads();
       auto expand = [&](bool valid, uint32_t x, uint32_t j) {
         bool need = false;
-        if (valid && x < P.dist_len) {  // both loads in flight together
+        if (valid && x < ph.dist_len) {  // both loads in flight together
           const uint32_t dx = P.dist[x];
           const unsigned long long w = __ldcg(&P.sw[x]);
           const uint32_t wit = (uint32_t)(w >> 32) & 0x7FFFFFFFu;
@@ -1763,11 +1788,11 @@ struct Cascade {
 };
 
 // Between a barrier after the ring's last use and one before its next.
-__device__ void reset_ring(Params& p) {
+__device__ void reset_ring(const Params& p) {
   if (threadIdx.x == 0) ring_epoch(p, 0, 0);
   if (gtid() == 0) {
     *p.rq_head = 0;
-    for (uint32_t k = 0; k <= kSyncRounds; ++k) p.rq_tail0[k] = 0;
+    for (uint32_t k = 0; k <= kSyncRounds; ++k) p.rq_tail[k] = 0;
     *p.rq_done = 0;
     *p.rq_fin = 0;
     for (int k = 0; k < 6; ++k) p.rq_stat[k] = 0;
@@ -1784,15 +1809,15 @@ __device__ __forceinline__ void stamp(const Params& p, int k) {
 __device__ void register_candidates(const Params& p) {
   BfsCounters* c = p.c;
   const int lane = threadIdx.x & 31;
-  const uint32_t F = *p.F;
+  const uint32_t F = *ph.F;
   for (uint32_t base = gwarp() * 32; base < F; base += nwarps() * 32) {
     const uint32_t i = base + lane;
     bool first = false;
     uint32_t v = 0;
     if (i < F) {
-      const uint8_t f = p.ff[i];
-      const uint32_t u = p.fu[i];
-      v = p.fv[i];
+      const uint8_t f = ph.ff[i];
+      const uint32_t u = ph.fu[i];
+      v = ph.fv[i];
       if (!(f & kFAdd) && (f & kFCur) && is_sp(p, u, v)) first = !(atomicOr(&p.sw[v], kSwTouched) & kSwTouched);
     }
     const uint32_t slot = vxb::warp_append(first, &c->touched_n);
@@ -1816,7 +1841,7 @@ __device__ void clear_workspace(const Params& p, uint32_t touched, uint32_t affe
 // affected list stays empty, so the post-batch repair only relaxes the
 // insertions.  The BFS distances go to tent (zero between phases), which the
 // comparison pass zeroes again.
-__device__ __noinline__ bool cascade_by_bfs(Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
+__device__ __noinline__ bool cascade_by_bfs(const Params& p, RepairSmem& sm, BlockQueue& bq, LbStage& lb) {
   BfsCounters* c = p.c;
   clear_workspace(p, sm.w.touched, sm.w.affected);
   reset_ring(p);
@@ -1833,7 +1858,7 @@ __device__ __noinline__ bool cascade_by_bfs(Params& p, RepairSmem& sm, BlockQueu
   bfs_in_repair(p, sm, lb, bq, p.tent, nullptr);  // also sets the reachable count of the graph without the deletions
   if (!sync_grid(p)) return false;
   uint32_t raised = 0;
-  for (uint32_t v = gtid(); v < p.dist_len; v += nthreads()) {
+  for (uint32_t v = gtid(); v < ph.dist_len; v += nthreads()) {
     const uint32_t d0 = p.dist[v], d1 = p.tent[v];
     p.tent[v] = 0u;
     raised += d0 != kUnreachable && d1 > d0;
@@ -1845,7 +1870,7 @@ __device__ __noinline__ bool cascade_by_bfs(Params& p, RepairSmem& sm, BlockQueu
   if (gtid() == 0) {
     const uint32_t na = c->a_bfs;
     c->affected = na;
-    if (na > p.fallback_limit) c->fallback = 1;  // bfs.hpp:249, 258: more than the limit falls back
+    if (na > ph.fallback_limit) c->fallback = 1;  // bfs.hpp:249, 258: more than the limit falls back
     c->arcs = arcs;
     c->levels = levels;
     c->cbig = 0u;
@@ -1860,7 +1885,7 @@ __device__ __noinline__ bool cascade_by_bfs(Params& p, RepairSmem& sm, BlockQueu
 // is drained only when a check left work in it (an affected vertex to expand,
 // chunks of a long in-row), which most small batches never do.  Records the
 // batch's affected count.
-__device__ bool cascade(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t ncand) {
+__device__ bool cascade(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, uint32_t ncand) {
   if (gtid() == 0) set_deadline(p);
   for (uint32_t i = dealt_warp(); i < ncand; i += nwarps()) check_vertex<true>(p, p.lst_t[i]);
   if (!sync_words(p, sm.w)) return false;
@@ -1868,12 +1893,12 @@ __device__ bool cascade(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, 
     Cascade w{&p, &lb};
     if (!sync_rounds(p, sm, w)) {
       if (sm.w.failed) return false;
-      drain(p, sm, w, p.cascade_bfs ? sm.w.deadline : kNever);
+      drain(p, sm, w, ph.cascade_bfs ? sm.w.deadline : kNever);
       if (!sync_words(p, sm.w)) return false;
     }
   }
   if (gtid() == 0) {  // the drain statistics of the phase trace
-    p.c->rtrace[7] = p.rq_base + sm.w.tail;
+    p.c->rtrace[7] = ph.rq_base + sm.w.tail;
     for (int k = 0; k < 6; ++k) p.c->rtrace[9 + k] = __ldcg(&p.rq_stat[k]);
   }
   if (sm.w.cbig) return cascade_by_bfs(p, sm, bq, lb);
@@ -1881,7 +1906,7 @@ __device__ bool cascade(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq, 
   return true;
 }
 
-__device__ void repair_pre(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
+__device__ void repair_pre(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
   stamp(p, 0);
   reset_ring(p);
@@ -1931,7 +1956,7 @@ __device__ __forceinline__ void lower_and_push(const Params& p, bool lowered, ui
 __device__ __forceinline__ void push_one(const Params& p, uint32_t x) {
   const uint32_t bit = 1u << (x & 31);
   if (atomicOr(&p.inq[0][x >> 5], bit) & bit) return;
-  const uint32_t s = p.rq_base + atomicAdd(p.rq_tail, 1u);
+  const uint32_t s = ph.rq_base + atomicAdd(ph.rq_tail, 1u);
   __stcg(&p.ring[s & p.ring_mask], (unsigned long long)x);
 }
 
@@ -1951,7 +1976,7 @@ __device__ __forceinline__ void relax_arcs(const Params& p, uint64_t b, uint32_t
       x[j] = k >= hi ? kTomb : k < nb ? a.col[b + k] : a.darena[dx + (k - nb)];
     }
 #pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) d[j] = !(x[j] & kTomb) && x[j] < p.dist_len ? ld_cg(&p.dist[x[j]]) : 0u;
+    for (uint32_t j = 0; j < 4; ++j) d[j] = !(x[j] & kTomb) && x[j] < ph.dist_len ? ld_cg(&p.dist[x[j]]) : 0u;
 #pragma unroll
     for (uint32_t j = 0; j < 4; ++j)
       if (d[j] > du + 1 && lower(p, x[j], du + 1, reach)) push_one(p, x[j]);
@@ -1989,7 +2014,7 @@ __device__ void seed_relax(const Params& p, bool lowered, uint32_t v, long long&
         x[k] = k < nb ? a.col[b + k] : k < deg ? a.darena[dr.x + (k - nb)] : kTomb;
 #pragma unroll
       for (uint32_t k = 0; k < kInlineRelax; ++k)
-        dx[k] = !(x[k] & kTomb) && x[k] < p.dist_len ? ld_cg(&p.dist[x[k]]) : 0u;
+        dx[k] = !(x[k] & kTomb) && x[k] < ph.dist_len ? ld_cg(&p.dist[x[k]]) : 0u;
 #pragma unroll
       for (uint32_t k = 0; k < kInlineRelax; ++k)
         if (dx[k] > dv + 1 && lower(p, x[k], dv + 1, reach)) push_one(p, x[k]);
@@ -2065,7 +2090,7 @@ struct Relax {
     __syncthreads();
     auto relax = [&](bool valid, uint32_t x, uint32_t j) {
       const uint32_t du = sm.d[j];
-      const bool lowered = valid && du != kUnreachable && x < P.dist_len && lower(P, x, du + 1, *reach);
+      const bool lowered = valid && du != kUnreachable && x < ph.dist_len && lower(P, x, du + 1, *reach);
       lower_and_push(P, lowered, x);
     };
     block_rows(P.g.out, sm.items, n, *lb, relax, &P, P.acct);
@@ -2094,7 +2119,7 @@ __device__ void boundary_seeds(const Params& p, RepairSmem& sm, LbStage& lb, uin
     }
     __syncthreads();
     auto bmin = [&](bool valid, uint32_t x, uint32_t j) {
-      if (!valid || x >= p.dist_len || test_bit(p.aff, x)) return;
+      if (!valid || x >= ph.dist_len || test_bit(p.aff, x)) return;
       const uint32_t dx = p.dist[x];
       if (dx != kUnreachable) atomicMin(&sm.cnt[j], dx + 1);
     };
@@ -2143,7 +2168,7 @@ __device__ void boundary_seeds_few(const Params& p, uint32_t na, long long& reac
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const bool live = !(x[j] & kTomb) && x[j] < p.dist_len;
+      const bool live = !(x[j] & kTomb) && x[j] < ph.dist_len;
       dx[j] = live ? p.dist[x[j]] : kUnreachable;
       aw[j] = live ? p.aff[x[j] >> 5] : FULL;
     }
@@ -2184,7 +2209,7 @@ __device__ void grid_boundary_min(const Params& p, uint32_t nb) {
       } else {
         x = a.darena[dr.x + (uint32_t)(k - nbase)];
       }
-      if (x >= p.dist_len || test_bit(p.aff, x)) continue;
+      if (x >= ph.dist_len || test_bit(p.aff, x)) continue;
       const uint32_t dx = p.dist[x];
       if (dx != kUnreachable && dx + 1 < best) best = dx + 1;
     }
@@ -2208,7 +2233,7 @@ __device__ __forceinline__ void invalidate(const Params& p, uint32_t na) {
 }
 
 template <bool kInvalidated>
-__device__ bool repair_relax(Params& p, RepairSmem& sm, LbStage& lb) {
+__device__ bool repair_relax(const Params& p, RepairSmem& sm, LbStage& lb) {
   BfsCounters* c = p.c;
   const int lane = threadIdx.x & 31;
   // the ring counters are zero here: the pre-batch kernel (or the previous
@@ -2232,15 +2257,15 @@ __device__ bool repair_relax(Params& p, RepairSmem& sm, LbStage& lb) {
     else boundary_seeds(p, sm, lb, na, reach);
   }
   // inserted arcs relax their heads (bfs.hpp:91-96)
-  const uint32_t F = *p.F;
+  const uint32_t F = *ph.F;
   for (uint32_t base = (dealt_thread() - lane * gridDim.x); base < F; base += nthreads()) {
     const uint32_t i = base + lane * gridDim.x;
     bool lowered = false;
     uint32_t v = 0;
-    if (i < F && (p.ff[i] & kFAdd)) {
-      const uint32_t u = p.fu[i];
-      v = p.fv[i];
-      if (u < p.dist_len && v < p.dist_len) {
+    if (i < F && (ph.ff[i] & kFAdd)) {
+      const uint32_t u = ph.fu[i];
+      v = ph.fv[i];
+      if (u < ph.dist_len && v < ph.dist_len) {
         const uint32_t du = ld_cg(&p.dist[u]);
         if (du != kUnreachable) lowered = lower(p, v, du + 1, reach);
       }
@@ -2286,7 +2311,7 @@ __device__ bool repair_relax(Params& p, RepairSmem& sm, LbStage& lb) {
   }
   stamp(p, 6);
   if (gtid() == 0) {
-    c->rtrace[8] = p.rq_base + sm.w.tail;
+    c->rtrace[8] = ph.rq_base + sm.w.tail;
     for (int k = 0; k < 6; ++k) c->rtrace[15 + k] = __ldcg(&p.rq_stat[k]);
   }
   reach = vxb::warp_sum(reach);
@@ -2299,7 +2324,7 @@ __device__ bool repair_relax(Params& p, RepairSmem& sm, LbStage& lb) {
 // Post-batch repair (bfs.hpp:72-97): the fallback's full BFS or the repair,
 // which may itself hand over to a full BFS; one call site serves both.
 template <bool kInvalidated>
-__device__ void repair_post(Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
+__device__ void repair_post(const Params& p, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
   const bool fallback = kInvalidated ? sm.w.fallback != 0u : ld_cg(&c->fallback) != 0u;
   if (fallback) {
@@ -3267,21 +3292,14 @@ __device__ void insertion_pass(ArcWork& w, RepairSmem& sm) {
   w.flush();
 }
 
-// A block's own copy of the launch's parameters, in shared memory: the repair
-// phases change some of them (the vertex count, the ring's epoch) and hand them by
-// reference to functions that are not inlined.  A copy per thread was a stack frame
-// of 928 bytes (784 in bfs_kernel; now 448 and 288), written by every thread of a
-// launch: 10,000 ops at R-MAT 22, three graphs in turn, 62 us a batch, now 44; 64
-// ops at R-MAT 14 57, now 52.
-__device__ __forceinline__ void copy_params(Params& to, const Params& from) {
-  static_assert(sizeof(Params) % 4 == 0, "copied by words");
-  for (uint32_t i = threadIdx.x; i < sizeof(Params) / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(&to)[i] = reinterpret_cast<const uint32_t*>(&from)[i];
+// The start of a repair launch: the block's own copy of what its phases change.
+__device__ __forceinline__ void start_phases(const Params& p) {
+  if (threadIdx.x == 0)
+    ph = PhaseParams{p.V, p.dist_len, 0u, p.rq_tail, 0u, p.cascade_bfs, p.fu, p.fv, p.ff, p.F, p.fallback_limit};
   __syncthreads();
 }
 
-__device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params& q, RepairSmem& sm, LbStage& lb,
-                                   BlockQueue& bq) {
+__device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairSmem& sm, LbStage& lb, BlockQueue& bq) {
   BfsCounters* c = p.c;
   const uint32_t sort_err = sort_error(p);
   unsigned long long tmark = globaltimer();
@@ -3298,22 +3316,22 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params&
     c->handovers[0] = c->handovers[1] = 0;
   }
   const int ndir = p.g.directed ? 2 : 1;
-  copy_params(q, p);
+  start_phases(p);
   for (uint32_t bi = 0; bi < s.nb; ++bi) {
     RawArcs& raw = reinterpret_cast<RawArcs&>(lb);
     uint32_t off = 0, F = 0, Frev = 0;
     if (s.boff) off = s.boff[bi];
     const uint32_t Vpre = bi ? s.vpost[bi - 1] : s.V0, lpre = bi ? s.vpost[bi - 1] : s.len0;
     if (threadIdx.x == 0) {  // the ring's epoch is the first again (reset_ring)
-      q.fu = s.fu[0] + off;
-      q.fv = s.fv[0] + off;
-      q.ff = s.ff[0] + off;
-      q.F = s.raw_n ? p.bar + kRawWord : &s.cnt[0][bi];
-      q.V = Vpre;
-      q.dist_len = lpre;
-      q.touched_base = 0;
+      ph.fu = s.fu[0] + off;
+      ph.fv = s.fv[0] + off;
+      ph.ff = s.ff[0] + off;
+      ph.F = s.raw_n ? p.bar + kRawWord : &s.cnt[0][bi];
+      ph.V = Vpre;
+      ph.dist_len = lpre;
+      ph.touched_base = 0;
       const unsigned long long lim = (unsigned long long)((double)Vpre * s.frac);
-      q.fallback_limit = lim < 1 ? 1 : lim;
+      ph.fallback_limit = lim < 1 ? 1 : lim;
     }
     __syncthreads();
     if (s.raw_n) {
@@ -3325,10 +3343,10 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params&
     const uint32_t Vpost = s.vpost ? s.vpost[bi] : s.v_single;
     auto work = [&](int dir) {
       const uint32_t o = dir ? 0u : off;
-      return ArcWork{&q, &s, dir ? &p.g.in : &p.g.out, dir, s.fu[dir] + o, s.fv[dir] + o, s.ff[dir] + o, s.fpos[dir] + o,
+      return ArcWork{&p, &s, dir ? &p.g.in : &p.g.out, dir, s.fu[dir] + o, s.fv[dir] + o, s.ff[dir] + o, s.fpos[dir] + o,
                      dir ? Frev : F, nullptr, 0u, false, 0ll, 0u};
     };
-    stamp(q, 0);
+    stamp(p, 0);
     // A: classification against the pre-batch graph, removals, deletion candidates
     for (int dir = 0; dir < ndir; ++dir) {
       ArcWork w = work(dir);
@@ -3341,9 +3359,9 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params&
     }
     if (s.digest && bi > 0) digest_pass(p.dist, lpre, &s.digest[bi - 1]);
     if (sort_err) atomicOr(&c->err, sort_err);
-    if (!sync_words(q, sm.w)) return;
+    if (!sync_words(p, sm.w)) return;
     phase(0);
-    if ((sm.w.later & kLaterRows) && !(canon_grid(p, s, raw, sm.w) && sync_words(q, sm.w))) return;
+    if ((sm.w.later & kLaterRows) && !(canon_grid(p, s, raw, sm.w) && sync_words(p, sm.w))) return;
     if (s.raw_n) {
       F = sm.w.raw_f[0];
       Frev = sm.w.raw_f[1];
@@ -3354,22 +3372,22 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params&
         w.pending = true;
         removal_pass(w, sm);
       }
-      if (!sync_words(q, sm.w)) return;
+      if (!sync_words(p, sm.w)) return;
     }
     if (sm.w.later & kLaterRuns) {
       for (int dir = 0; dir < ndir; ++dir) {
         ArcWork w = work(dir);
         removal_runs(w, sm);
       }
-      if (!sync_words(q, sm.w)) return;
+      if (!sync_words(p, sm.w)) return;
     }
     phase(1);
-    stamp(q, 1);
+    stamp(p, 1);
     // B: the cascade over the graph without the batch's deletions
     const uint32_t ncand = sm.w.candidates;
     if (threadIdx.x == 0) {
-      q.touched_base = ncand;
-      q.cascade_bfs = lpre == Vpre;
+      ph.touched_base = ncand;
+      ph.cascade_bfs = lpre == Vpre;
     }
     __syncthreads();
     if (gtid() == 0) {
@@ -3382,11 +3400,11 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params&
       acct_add(p, 4, 1);
     }
     if (ncand) {
-      if (!cascade(q, sm, lb, bq, ncand)) return;
-      reset_ring(q);
+      if (!cascade(p, sm, lb, bq, ncand)) return;
+      reset_ring(p);
     }
     phase(2);
-    stamp(q, 2);
+    stamp(p, 2);
     // C: insertions; new vertices start unreachable and, unless a BFS gives
     // the distances, the affected ones are invalidated
     for (int dir = 0; dir < ndir; ++dir) {
@@ -3394,13 +3412,13 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, Params&
       insertion_pass(w, sm);
     }
     for (uint32_t v = lpre + gtid(); v < Vpost; v += nthreads()) p.dist[v] = kUnreachable;
-    if (!sm.w.cbig && !sm.w.fallback) invalidate(q, sm.w.affected);
-    if (!sync_words(q, sm.w)) return;
+    if (!sm.w.cbig && !sm.w.fallback) invalidate(p, sm.w.affected);
+    if (!sync_words(p, sm.w)) return;
     phase(3);
     // D: the post-batch repair (or the fallback full BFS) on the new graph
-    if (threadIdx.x == 0) q.V = q.dist_len = Vpost;
+    if (threadIdx.x == 0) ph.V = ph.dist_len = Vpost;
     __syncthreads();
-    repair_post<true>(q, sm, lb, bq);
+    repair_post<true>(p, sm, lb, bq);
     phase(4);
     // the repair lists start empty in the next batch (and launch); every block
     // has their lengths in sm.w
@@ -3451,12 +3469,11 @@ __global__ void __launch_bounds__(kT, 1) bfs_full_kernel(Params p) {
   full_bfs<false, 4096 / kT>(p, sm.bq, sm.lb, sm.bu, sm.bits, 8192u, p.dist, p.trace);
 }
 
-__global__ void __launch_bounds__(kThreads, 2) bfs_kernel(const __grid_constant__ Params args, int mode) {
+__global__ void __launch_bounds__(kThreads, 2) bfs_kernel(const __grid_constant__ Params p, int mode) {
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
-  __shared__ Params p;
-  copy_params(p, args);
+  start_phases(p);
   if (const uint32_t e = sort_error(p)) atomicOr(&p.c->err, e);
   if (mode == kModePre) repair_pre(p, sm, lb, bq);
   else repair_post<false>(p, sm, lb, bq);
@@ -3475,8 +3492,7 @@ __global__ void __launch_bounds__(kThreads, 2) bfs_stream_kernel(const __grid_co
   __shared__ BlockQueue bq;
   __shared__ LbStage lb;
   __shared__ RepairSmem sm;
-  __shared__ Params q;
-  stream_kernel_body(p, s, q, sm, lb, bq);
+  stream_kernel_body(p, s, sm, lb, bq);
 }
 
 // Stream canonicalisation: both arcs of every non-self-loop op keyed by
@@ -3682,7 +3698,7 @@ static Params make_params(Bfs* b, uint32_t V, uint32_t dist_len) {
   p.ring = b->ring;
   p.ring_mask = b->ring_slots ? (uint32_t)(b->ring_slots - 1) : 0u;
   p.rq_head = b->rq;
-  p.rq_tail = p.rq_tail0 = b->rq + 32;
+  p.rq_tail = b->rq + 32;
   p.rq_done = b->rq + 64;
   p.rq_fin = b->rq + 128;
   p.rq_stat = reinterpret_cast<unsigned long long*>(b->rq + 96);
