@@ -195,9 +195,8 @@ __device__ __forceinline__ uint32_t row_len(const Params& p, const DevAdj& a, ui
 
 constexpr int kVisit = 4;  // arcs a lane has in flight per step
 
-template <class Queue, int kV = kVisit>
+template <class Queue>
 struct TdVisit {
-  static constexpr int kArcs = kV;  // arcs a lane has in flight per step
   const Params* p;
   uint32_t* dist;
   uint32_t level;
@@ -208,30 +207,57 @@ struct TdVisit {
   unsigned long long mloc;  // arcs of the vertices this lane claimed
   // Claims the heads of one step's arcs for the next level (warp-uniform);
   // bit 31 of an entry marks a dead arc or none.
-  __device__ __forceinline__ void visit(const uint32_t (&x)[kV]) {
-    uint32_t w[kV];
+  __device__ __forceinline__ void visit(const uint32_t (&x)[kVisit]) {
+    uint32_t w[kVisit];
 #pragma unroll
-    for (int j = 0; j < kV; ++j) w[j] = (x[j] & kTomb) ? FULL : p->vis[x[j] >> 5];
+    for (int j = 0; j < kVisit; ++j) w[j] = (x[j] & kTomb) ? FULL : p->vis[x[j] >> 5];
     // the row lengths are loaded before the claims, so both are in flight together
-    uint32_t deg[kV];
+    uint32_t deg[kVisit];
 #pragma unroll
-    for (int j = 0; j < kV; ++j) deg[j] = (w[j] >> (x[j] & 31)) & 1u ? 0u : row_len(*p, p->g.out, x[j]);
+    for (int j = 0; j < kVisit; ++j) deg[j] = (w[j] >> (x[j] & 31)) & 1u ? 0u : row_len(*p, p->g.out, x[j]);
+    // Heads side by side (a hub's leaves) share a word: where 16 lanes or more do, one
+    // of them claims for all, as atomics of a warp on one word are served one by one (a
+    // star of 2^20 leaves 154 us, with eight arcs per lane in flight 73, so 39).
+    uint32_t m[kVisit];  // lanes whose claim is made together
 #pragma unroll
-    for (int j = 0; j < kV; ++j) {
-      const uint32_t bit = 1u << (x[j] & 31);
-      if (!(w[j] & bit)) w[j] = atomicOr(&p->vis[x[j] >> 5], bit);
+    for (int j = 0; j < kVisit; ++j) {
+      const uint32_t bit = 1u << (x[j] & 31), word = x[j] >> 5;
+      const bool need = !(w[j] & bit);
+      const uint32_t middle = __shfl_sync(FULL, word, 16);  // every lane takes part
+      m[j] = __ballot_sync(FULL, need && word == middle);
+      uint32_t op = need ? bit : 0u;
+      if (__popc(m[j]) >= 16) {
+        const bool in = (m[j] >> (threadIdx.x & 31)) & 1u;
+        const uint32_t all = __reduce_or_sync(FULL, in ? bit : 0u);
+        if (__popc(all) != __popc(m[j])) m[j] = 0u;  // a head twice
+        else if (in) op = (m[j] & vxb::lanemask_lt()) == 0u ? all : 0u;
+      } else {
+        m[j] = 0u;
+      }
+      if (op) w[j] = atomicOr(&p->vis[word], op);
     }
-    uint32_t m[kV];
 #pragma unroll
-    for (int j = 0; j < kV; ++j) {
+    for (int j = 0; j < kVisit; ++j) {
       const uint32_t bit = 1u << (x[j] & 31);
+      if (m[j]) {  // warp-uniform
+        const uint32_t old = __shfl_sync(FULL, w[j], __ffs(m[j]) - 1);
+        if ((m[j] >> (threadIdx.x & 31)) & 1u) w[j] = old;
+      }
       const bool claim = !(w[j] & bit);
-      m[j] = __ballot_sync(FULL, claim);
       if (claim) {
         mloc += deg[j];
         dist[x[j]] = level + 1;
-        if (fbn) atomicOr(&fbn[x[j] >> 5], bit);
       }
+      if (fbn) {
+        uint32_t op = claim ? bit : 0u;
+        if (m[j]) {
+          const bool in = (m[j] >> (threadIdx.x & 31)) & 1u;
+          const uint32_t all = __reduce_or_sync(FULL, in ? op : 0u);
+          if (in) op = (m[j] & vxb::lanemask_lt()) == 0u ? all : 0u;
+        }
+        if (op) atomicOr(&fbn[x[j] >> 5], op);
+      }
+      m[j] = __ballot_sync(FULL, claim);
     }
     bq_push_n(*bq, m, x, cnt_n, qout);
   }
@@ -250,10 +276,10 @@ __device__ __forceinline__ void td_rows(Visit& t, const uint32_t* arr, uint64_t 
     med &= med - 1;
     const uint64_t s = __shfl_sync(FULL, start, l);
     const uint32_t n = __shfl_sync(FULL, len, l);
-    for (uint32_t k0 = 0; k0 < n; k0 += 32 * Visit::kArcs) {
-      uint32_t x[Visit::kArcs];
+    for (uint32_t k0 = 0; k0 < n; k0 += 32 * kVisit) {
+      uint32_t x[kVisit];
 #pragma unroll
-      for (int j = 0; j < Visit::kArcs; ++j) {
+      for (int j = 0; j < kVisit; ++j) {
         const uint32_t k = k0 + 32 * j + lane;
         x[j] = k < n ? arr[s + k] : kTomb;
       }
@@ -270,10 +296,10 @@ __device__ __forceinline__ void td_rows(Visit& t, const uint32_t* arr, uint64_t 
   const uint32_t excl = incl - len;
   const uint32_t total = __shfl_sync(FULL, incl, 31);
   start -= excl;  // arc k of the list is arr[start + k] in its owner's lane
-  for (uint32_t k0 = 0; k0 < total; k0 += 32 * Visit::kArcs) {
-    uint32_t x[Visit::kArcs];
+  for (uint32_t k0 = 0; k0 < total; k0 += 32 * kVisit) {
+    uint32_t x[kVisit];
 #pragma unroll
-    for (int j = 0; j < Visit::kArcs; ++j) {
+    for (int j = 0; j < kVisit; ++j) {
       const uint32_t k = k0 + 32 * j + lane;
       int owner = 0;
 #pragma unroll
@@ -388,10 +414,10 @@ template <class Visit>
 __device__ void lb_visit(const Params& p, Visit& t, uint32_t n_f, const LbStage& st, uint32_t warp, uint32_t warps) {
   const DevAdj& a = p.g.out;
   const uint32_t M = st.pref[n_f];
-  for (uint32_t e0 = warp * 32; e0 < M; e0 += warps * 32 * Visit::kArcs) {
-    uint32_t x[Visit::kArcs];
+  for (uint32_t e0 = warp * 32; e0 < M; e0 += warps * 32 * kVisit) {
+    uint32_t x[kVisit];
 #pragma unroll
-    for (int j = 0; j < Visit::kArcs; ++j) {
+    for (int j = 0; j < kVisit; ++j) {
       const uint32_t e = e0 + j * warps * 32 + (threadIdx.x & 31);
       x[j] = kTomb;
       if (e < M) {
@@ -415,16 +441,16 @@ template <class Visit>
 __device__ void grid_rows(const Params& p, Visit& t, uint32_t n) {
   const DevAdj& a = p.g.out;
   const uint32_t lane = threadIdx.x & 31;
-  constexpr uint32_t kSlice = 32 * Visit::kArcs;
+  constexpr uint32_t kSlice = 32 * kVisit;
   for_my_rows(p.bul, n, kSlice, [&](uint32_t r, uint32_t len, uint32_t s0) {
     uint64_t b;
     uint32_t nb;
     uint2 dr;
     row_of(p, a, p.big[r], b, nb, dr);
     for (uint64_t k0 = (uint64_t)s0 * kSlice; k0 < len; k0 += (uint64_t)nwarps() * kSlice) {
-      uint32_t x[Visit::kArcs];
+      uint32_t x[kVisit];
 #pragma unroll
-      for (int j = 0; j < Visit::kArcs; ++j) {
+      for (int j = 0; j < kVisit; ++j) {
         const uint64_t k = k0 + 32 * j + lane;
         x[j] = k >= len ? kTomb : (k < nb ? a.col[b + k] : a.darena[dr.x + (uint32_t)(k - nb)]);
       }
@@ -815,7 +841,7 @@ __device__ void bu_list_level(const Params& p, BuOut<Queue>& o, BuStage<kT, kR>&
 
 // kT threads per block; lbst and bu may share memory.  wbits[0, wbits_n): shared
 // words for the block's part of a bitmap.
-template <bool kInRepair, int kV, int kT, int kR, class Queue>
+template <bool kInRepair, int kT, int kR, class Queue>
 __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, kR>& bu, uint32_t* wbits,
                          uint32_t wbits_n, uint32_t* dist, unsigned long long* trace) {
   BfsCounters* c = p.c;
@@ -1026,7 +1052,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
       // a small frontier's level keeps the bitmap (few claims); after a
       // larger one a bottom-up level makes it from the queue
       const bool keep = n_f <= kLbMax && !left_bu;
-      TdVisit<Queue, kV> t{&p, dist, level, p.q[nxt], keep ? p.fb[nxt] : nullptr, &c->lvl_n[nxt], &bq, 0ull};
+      TdVisit<Queue> t{&p, dist, level, p.q[nxt], keep ? p.fb[nxt] : nullptr, &c->lvl_n[nxt], &bq, 0ull};
       if (n_f <= kLbMax) {
         lb_stage<kT>(p, p.q[cur], n_f, lbst);
         lb_visit(p, t, n_f, lbst, gwarp(), nwarps());
@@ -1041,7 +1067,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     if (!level_end(p, lw, bq, nloc, mloc, nxt, td ? &c->lvl_big[cur] : nullptr)) return;
     prev_n = n_f;
     if (lw.nbig) {  // hub rows remain
-      TdVisit<Queue, kV> t{&p, dist, level, p.q[nxt], nullptr, &c->lvl_n[nxt], &bq, 0ull};
+      TdVisit<Queue> t{&p, dist, level, p.q[nxt], nullptr, &c->lvl_n[nxt], &bq, 0ull};
       grid_rows(p, t, lw.nbig);
       if (!level_end(p, lw, bq, 0u, t.mloc, nxt, nullptr)) return;
     }
@@ -1276,7 +1302,7 @@ __device__ __noinline__ void bfs_in_repair(const Params& p, RepairSmem& sm, LbSt
   for (uint32_t i = threadIdx.x; i < sizeof(Params) / 4; i += kThreads)
     reinterpret_cast<uint32_t*>(&own)[i] = reinterpret_cast<const uint32_t*>(&p)[i];
   __syncthreads();
-  full_bfs<true, kVisit>(own, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm),
+  full_bfs<true>(own, bq, lb, reinterpret_cast<Stage&>(lb), reinterpret_cast<uint32_t*>(&sm),
                  (uint32_t)(offsetof(RepairSmem, w) / 4), dist, trace);
 }
 
@@ -3447,13 +3473,12 @@ __device__ void stream_kernel_body(const Params& p, const StreamArgs& s, RepairS
 // four arcs per lane in flight keep the memory as busy as 48 with one did.
 // R-MAT of 30,000 vertices: 75 us with 444 blocks of 512 threads, 56 with 296,
 // 45 with 148.  Graphs of fewer than kWideArcs arcs take 512 threads, whose
-// block barriers are cheaper (40 us), with eight arcs per lane in flight and 110
-// registers: with four, wide levels of graphs below the limit took up to twice as
-// long (star of 2^20 leaves 118 -> 54 us, uniform directed 4M vertices and 16M arcs
-// 493 -> 344 in all).  Both sides of the limit: uniform 2^20 vertices, 16M arcs 110
-// us with 512 threads and 111 with 1,024; 4M vertices, 16M arcs directed 344 and
-// 319; R-MAT 2^18, 8M arcs 60.6 and 60.7; 1000 x 1000 lattice 749 and 785; R-MAT
-// 2^20, 31M arcs 89 (with four arcs per lane) and 77; R-MAT 2^22 244 and 168.
+// block barriers are cheaper (40 us; R-MAT 2^20, 31M arcs: 89 us with 512, 77 with
+// 1,024; R-MAT 2^22: 244 and 168), and 64 registers, so that the searches of two
+// graphs run side by side: three graphs in turn, us a search, and one alone: R-MAT of
+// 24,821 vertices 21 and 41, 500,000 38 and 80, 700 x 700 lattice 350 and 635.  With
+// eight arcs per lane and 110 registers one launch had the SMs to itself: 37 and 40,
+// 63 and 74, 611 and 619.
 template <int kT>
 struct FullSmem {
   BlockQueueOf<8192> bq;
@@ -3463,10 +3488,10 @@ struct FullSmem {
 };
 
 template <int kT>
-__global__ void __launch_bounds__(kT, 1) bfs_full_kernel(Params p) {
+__global__ void __launch_bounds__(kT, 1024 / kT) bfs_full_kernel(Params p) {
   extern __shared__ __align__(16) unsigned char full_smem[];
   FullSmem<kT>& sm = *reinterpret_cast<FullSmem<kT>*>(full_smem);
-  full_bfs<false, 4096 / kT>(p, sm.bq, sm.lb, sm.bu, sm.bits, 8192u, p.dist, p.trace);
+  full_bfs<false>(p, sm.bq, sm.lb, sm.bu, sm.bits, 8192u, p.dist, p.trace);
 }
 
 __global__ void __launch_bounds__(kThreads, 2) bfs_kernel(const __grid_constant__ Params p, int mode) {
