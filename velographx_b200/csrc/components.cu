@@ -290,7 +290,9 @@ __global__ void cc_mark_vertices_kernel(const uint32_t* label, uint32_t n_old, c
 
 // Step 5: the final additions of the batch (their edges exist now).
 __global__ void cc_union_adds_kernel(const uint32_t* fu, const uint32_t* fv, const uint8_t* ff, const uint32_t* F,
-                                     uint32_t* label) {
+                                     uint32_t* label, const uint32_t* graph_err, uint32_t* err) {
+  // the graph's error word goes out with the affected count: a copy of its own was 7 us a read
+  if (blockIdx.x == 0 && threadIdx.x == 0) *err = *graph_err;
   const uint32_t nf = *F;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x)
     if ((ff[i] & kFAdd) && fu[i] < fv[i]) cc_union(label, fu[i], fv[i]);
@@ -358,7 +360,7 @@ int cc_rebuild(Components* c) {
   }
   c->n = V;
   c->last_repaired = V;
-  c->repaired_pending = false;
+  c->repaired_pending = c->err_pending = false;
   return 0;
 }
 
@@ -370,7 +372,7 @@ int cc_create(Components** out, Graph* g) {
   }
   Components* c = new Components();
   c->g = g;
-  if (cudaMalloc(&c->ctr, 16) != cudaSuccess) {
+  if (cudaMalloc(&c->ctr, 32) != cudaSuccess) {
     set_error("components: counter allocation failed");
     cc_destroy(c);
     return -4;
@@ -409,7 +411,7 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
   const uint32_t words_old = (n_old + 31) / 32;
   uint32_t* any = c->ctr;                                                   // effective deletion seen
   unsigned long long* count = reinterpret_cast<unsigned long long*>(c->ctr + 2);  // affected vertices
-  VX_CUDA_TRY(cudaMemsetAsync(c->ctr, 0, 16, s));
+  VX_CUDA_TRY(cudaMemsetAsync(c->ctr, 0, 20, s));
   const uint64_t m = 2 * n;  // canonical arcs of an undirected batch, at most
   if (n_old) {
     count_launch();
@@ -417,7 +419,7 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
     count_launch();
     cc_mark_vertices_kernel<<<std::min(cc_grid(n_old), 148u * 8u), kCcThreads, 0, s>>>(c->label, n_old, c->aroot, c->aff, any, count);
   }
-  c->repaired_pending = true;  // the count is read by cc_last_repaired
+  c->repaired_pending = c->err_pending = true;  // read by cc_sync
   if (int rc = graph_commit_batch(g)) return rc;
   if (V > n_old) {
     count_launch();
@@ -426,7 +428,7 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
   }
   if (n_old) unite_rows(c, (uint32_t)V, n_old, c->aff, any);
   count_launch();
-  cc_union_adds_kernel<<<cc_grid(m), kCcThreads, 0, s>>>(B.fu, B.fv, B.ff, F, c->label);
+  cc_union_adds_kernel<<<cc_grid(m), kCcThreads, 0, s>>>(B.fu, B.fv, B.ff, F, c->label, &g->ctr->err, c->ctr + 4);
   count_launch();
   cc_compress_kernel<<<cc_grid(V), kCcThreads, 0, s>>>(c->label, (uint32_t)V, nullptr);
   // the marks start clear for the next batch
@@ -437,25 +439,40 @@ int cc_apply_staged(Components* c, size_t n, size_t vertex_bound) {
   return 0;
 }
 
-// Waits for the stream; fails when a wait of the graph's sort ran out (the batch
-// held no arcs then).
+// Waits for the stream; reads the last batch's affected count and the error word
+// unless they have been read, and fails when a wait of the graph's sort ran out (the
+// batch held no arcs then).
 static int cc_sync(Components* c) {
   Graph* g = c->g;
-  VX_CUDA_TRY(cudaMemcpyAsync(g->pinned_scalar + 1, &g->ctr->err, 4, cudaMemcpyDeviceToHost, g->stream));
   VX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  if (*reinterpret_cast<uint32_t*>(g->pinned_scalar + 1) & vxb::kErrBarrierTimeout) {
-    set_error("components: a wait of the radix sort ran out");
-    return -5;
+  if (!c->err_pending) return 0;
+  volatile uint32_t* err = reinterpret_cast<uint32_t*>(g->pinned_scalar + 1);
+  if (*err & vxb::kErrBarrierTimeout) {
+    // (a load since then has cleared the graph's word)
+    VX_CUDA_TRY(cudaMemcpyAsync(g->pinned_scalar + 1, &g->ctr->err, 4, cudaMemcpyDeviceToHost, g->stream));
+    VX_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    if (*err & vxb::kErrBarrierTimeout) {
+      set_error("components: a wait of the radix sort ran out");
+      return -5;
+    }
   }
+  c->err_pending = false;
+  if (c->repaired_pending) c->last_repaired = (size_t)g->pinned_scalar[0];
+  c->repaired_pending = false;
+  return 0;
+}
+
+// Enqueues the read that cc_sync looks at.
+static int cc_ask(Components* c) {
+  if (c->err_pending)
+    VX_CUDA_TRY(cudaMemcpyAsync(c->g->pinned_scalar, c->ctr + 2, 12, cudaMemcpyDeviceToHost, c->g->stream));
   return 0;
 }
 
 int cc_last_repaired(Components* c, uint64_t* out) {
   if (c->repaired_pending) {
-    VX_CUDA_TRY(cudaMemcpyAsync(c->g->pinned_scalar, c->ctr + 2, 8, cudaMemcpyDeviceToHost, c->g->stream));
+    if (int rc = cc_ask(c)) return rc;
     if (int rc = cc_sync(c)) return rc;
-    c->last_repaired = (size_t)c->g->pinned_scalar[0];
-    c->repaired_pending = false;
   }
   *out = c->last_repaired;
   return 0;
@@ -464,6 +481,7 @@ int cc_last_repaired(Components* c, uint64_t* out) {
 int cc_labels(Components* c, uint32_t* host_out, size_t cap, size_t* n) {
   *n = c->n;
   const size_t k = std::min(cap, c->n);
+  if (int rc = cc_ask(c)) return rc;
   if (host_out && k) VX_CUDA_TRY(cudaMemcpyAsync(host_out, c->label, k * 4, cudaMemcpyDeviceToHost, c->g->stream));
   return cc_sync(c);
 }

@@ -17,9 +17,10 @@ struct Components {
   uint32_t* label = nullptr;  // label[v] = smallest id of v's component
   uint32_t* aroot = nullptr;  // bitmap of affected roots (clear between batches)
   uint32_t* aff = nullptr;    // bitmap of affected vertices (clear between batches)
-  uint32_t* ctr = nullptr;    // {effective deletion seen, giant root, affected count (u64)}
+  uint32_t* ctr = nullptr;    // {effective deletion seen, giant root, affected count (u64), the graph's error word}
   size_t last_repaired = 0;
   bool repaired_pending = false;  // last_repaired is still in ctr
+  bool err_pending = false;       // and so is the error word of the last batch
 };
 
 int cc_create(Components** out, Graph* g);
