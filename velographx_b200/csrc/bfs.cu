@@ -195,7 +195,7 @@ __device__ __forceinline__ uint32_t row_len(const Params& p, const DevAdj& a, ui
 
 constexpr int kVisit = 4;  // arcs a lane has in flight per step
 
-template <class Queue>
+template <class Queue, bool kTogether>
 struct TdVisit {
   const Params* p;
   uint32_t* dist;
@@ -217,16 +217,21 @@ struct TdVisit {
     for (int j = 0; j < kVisit; ++j) deg[j] = (w[j] >> (x[j] & 31)) & 1u ? 0u : row_len(*p, p->g.out, x[j]);
     // Heads side by side (a hub's leaves) share a word: where 16 lanes or more do, one
     // of them claims for all, as atomics of a warp on one word are served one by one (a
-    // star of 2^20 leaves 154 us, with eight arcs per lane in flight 73, so 39).
+    // star of 2^20 leaves 154 us, with eight arcs per lane in flight 73, so 39).  Not in
+    // levels of one block (a 59 x 59 lattice 78 us, so 87) and not with 1,024 threads,
+    // which have no registers left for it (R-MAT of 3.9M vertices 134 us, so 136).
     uint32_t m[kVisit];  // lanes whose claim is made together
 #pragma unroll
     for (int j = 0; j < kVisit; ++j) {
       const uint32_t bit = 1u << (x[j] & 31), word = x[j] >> 5;
       const bool need = !(w[j] & bit);
-      const uint32_t middle = __shfl_sync(FULL, word, 16);  // every lane takes part
-      m[j] = __ballot_sync(FULL, need && word == middle);
       uint32_t op = need ? bit : 0u;
-      if (__popc(m[j]) >= 16) {
+      m[j] = 0u;
+      if (kTogether) {
+        const uint32_t middle = __shfl_sync(FULL, word, 16);  // every lane takes part
+        m[j] = __ballot_sync(FULL, need && word == middle);
+      }
+      if (kTogether && __popc(m[j]) >= 16) {
         const bool in = (m[j] >> (threadIdx.x & 31)) & 1u;
         const uint32_t all = __reduce_or_sync(FULL, in ? bit : 0u);
         if (__popc(all) != __popc(m[j])) m[j] = 0u;  // a head twice
@@ -239,7 +244,7 @@ struct TdVisit {
 #pragma unroll
     for (int j = 0; j < kVisit; ++j) {
       const uint32_t bit = 1u << (x[j] & 31);
-      if (m[j]) {  // warp-uniform
+      if (kTogether && m[j]) {  // warp-uniform
         const uint32_t old = __shfl_sync(FULL, w[j], __ffs(m[j]) - 1);
         if ((m[j] >> (threadIdx.x & 31)) & 1u) w[j] = old;
       }
@@ -250,7 +255,7 @@ struct TdVisit {
       }
       if (fbn) {
         uint32_t op = claim ? bit : 0u;
-        if (m[j]) {
+        if (kTogether && m[j]) {
           const bool in = (m[j] >> (threadIdx.x & 31)) & 1u;
           const uint32_t all = __reduce_or_sync(FULL, in ? op : 0u);
           if (in) op = (m[j] & vxb::lanemask_lt()) == 0u ? all : 0u;
@@ -314,7 +319,7 @@ __device__ __forceinline__ void td_rows(Visit& t, const uint32_t* arr, uint64_t 
   }
 }
 
-// A frontier of more than kLbMax vertices: up to 32 of them per warp, fewer
+// A wide frontier: up to 32 of its vertices per warp, fewer
 // when that leaves warps without any.  Rows of at least large_row arcs are
 // listed (p.big, their lengths in p.bul, free outside the bottom-up levels)
 // for grid_rows.
@@ -348,6 +353,9 @@ __device__ void td_level(const Params& p, Visit& t, const uint32_t* qin, uint32_
 // finds their owners by binary search -- the same number of edges per warp
 // however skewed the rows are (a 30-vertex frontier of hubs included).
 constexpr uint32_t kLbMax = 1024;
+// Levels of the grid take the flat edge space up to here: staging 1,024 rows of four
+// arcs made a level 7.3 us, by td_level it takes 6.9.
+constexpr uint32_t kFlatMax = 1000;
 struct LbStage {
   uint32_t pref[kLbMax + 1];
   uint64_t base[kLbMax];
@@ -563,7 +571,7 @@ __device__ void solo_levels(const Params& p, uint32_t* dist, const uint32_t* qin
     if (threadIdx.x == 0) bq.cnt = 0;
     __syncthreads();
     // an overflow of bq's slots goes to qout: more than kLbMax entries, so it is the last level here
-    TdVisit<Queue> t{&p, dist, s.level, qout, nullptr, cnt_n, &bq, 0ull};
+    TdVisit<Queue, false> t{&p, dist, s.level, qout, nullptr, cnt_n, &bq, 0ull};
     lb_visit(p, t, s.n_f, st, threadIdx.x >> 5, kT / 32);
     s.m_f = block_sum<kT>(t.mloc, red);  // its barriers also cover the pushes
     s.n_f = bq.cnt;
@@ -1051,9 +1059,9 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     } else {
       // a small frontier's level keeps the bitmap (few claims); after a
       // larger one a bottom-up level makes it from the queue
-      const bool keep = n_f <= kLbMax && !left_bu;
-      TdVisit<Queue> t{&p, dist, level, p.q[nxt], keep ? p.fb[nxt] : nullptr, &c->lvl_n[nxt], &bq, 0ull};
-      if (n_f <= kLbMax) {
+      const bool keep = n_f <= kFlatMax && !left_bu;
+      TdVisit<Queue, kT <= 512> t{&p, dist, level, p.q[nxt], keep ? p.fb[nxt] : nullptr, &c->lvl_n[nxt], &bq, 0ull};
+      if (n_f <= kFlatMax) {
         lb_stage<kT>(p, p.q[cur], n_f, lbst);
         lb_visit(p, t, n_f, lbst, gwarp(), nwarps());
       } else {
@@ -1067,7 +1075,7 @@ __device__ void full_bfs(const Params& p, Queue& bq, LbStage& lbst, BuStage<kT, 
     if (!level_end(p, lw, bq, nloc, mloc, nxt, td ? &c->lvl_big[cur] : nullptr)) return;
     prev_n = n_f;
     if (lw.nbig) {  // hub rows remain
-      TdVisit<Queue> t{&p, dist, level, p.q[nxt], nullptr, &c->lvl_n[nxt], &bq, 0ull};
+      TdVisit<Queue, kT <= 512> t{&p, dist, level, p.q[nxt], nullptr, &c->lvl_n[nxt], &bq, 0ull};
       grid_rows(p, t, lw.nbig);
       if (!level_end(p, lw, bq, 0u, t.mloc, nxt, nullptr)) return;
     }
