@@ -605,8 +605,8 @@ __device__ __forceinline__ void seg_append(bool pred, uint32_t v, uint32_t* seg,
 // loads in flight), and scans the longer rows still looking four at a time,
 // eight lanes each (one after another by the whole warp, each paid its own
 // chain).  R-MAT 22, the level that reaches 1.8M of 2.4M vertices: 103 us with
-// one vertex per lane and step, 87 us with two (of about 40 us for its 250 MB
-// of mostly single 32-byte sectors); one is enough, and 10% faster in all, on
+// one vertex per lane and step, 87 us with two (the whole launch moves 193 MB
+// of DRAM traffic, mostly single 32-byte sectors: 30 us at the copy rate); one is enough, and 10% faster in all, on
 // graphs of a few thousand arcs per block, which kT = 512 serves.  Putting the
 // long rows back into the ring instead (24 or 56 arcs left): no gain on large
 // graphs, 41 -> 44 us in all at 30,000 vertices.
@@ -3708,9 +3708,6 @@ static Params make_params(Bfs* b, uint32_t V, uint32_t dist_len) {
   memset(&p, 0, sizeof(p));
   p.g = g->view();
   p.V = V;
-  // a full BFS reads every arc once; a relaxation that has processed this
-  // many items is past the point where one would have been cheaper on a
-  // deep graph
   p.handover = b->tune.handover;
   p.cascade_bfs = dist_len == V;
   p.dist_len = dist_len;
@@ -4029,7 +4026,7 @@ static int launch_stream(Bfs* b, Params& p, StreamArgs& sa) {
 // cascade, delta insertions and the post-batch repair in one persistent launch
 // (a directed graph's two adjacencies one after the other within each pass).  A
 // directed 1,000-op batch at 300,000 vertices took some 22 launches and 213 us;
-// now three and 122.
+// now one and 73.
 static int repair_fused(Bfs* b) {
   Graph* g = b->g;
   const size_t n = b->staged_ops, m = g->directed ? n : 2 * n;
